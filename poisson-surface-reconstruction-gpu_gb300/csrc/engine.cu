@@ -342,6 +342,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.cg_r, (size_t)nodes); A.add(ws.cg_p, (size_t)nodes); A.add(ws.cg_q, (size_t)nodes);
     A.add(ws.cg_ap, (size_t)nodes);
     A.add(ws.cg_blk, (size_t)nodes * 8 + 64);
+    A.add(ws.cg_desc, 14 * ((size_t)nodes / 8 + 8));
     A.add(ws.cg_loop, (size_t)kMaxDepth + 1);
     A.add(ws.cg_loop_part, (size_t)(kMaxDepth + 1) * kLoopMaxBlocks);
     A.add(ws.cg_loop_ctl, (size_t)kLoopControlWords);
@@ -477,7 +478,13 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
         std::vector<float> dff32(dff.begin(), dff.end());   // the kernels use float entries
         e = cudaMemcpy(ws.dff, dff32.data(), dff32.size() * sizeof(float), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(ws.stencil, st.data(), st.size() * sizeof(float), cudaMemcpyHostToDevice);
-        std::copy(st.begin(), st.end(), ws.stencil_host);   // the CG launch passes some as parameters
+        // the CG takes four values per depth: an entry depends only on the axes its offset moves on
+        for (int d = 0; d <= kMaxDepth && e == cudaSuccess; ++d)
+            for (int k = 0; k < 27; ++k) {
+                const int first[4] = {13, 14, 17, 26};
+                const int axes = (k / 9 != 1) + ((k / 3) % 3 != 1) + (k % 3 != 1);
+                if (st[27 * d + k] != st[27 * d + first[axes]]) e = cudaErrorInvalidValue;
+            }
     }
     // the other cloud slots start as copies of slot 0 (tables, zeroed scan counters)
     for (int k = 1; k < h->clouds && e == cudaSuccess; ++k)

@@ -33,8 +33,8 @@ namespace psr {
 // ---- per-depth CG ---------------------------------------------------------------------
 // Every depth is an independent system.  The two finest depths (most rows, most
 // iterations) get one thread-block cluster each (k_cg_cluster: cluster barriers, sums
-// through distributed shared memory); the coarser depths get one CTA each (k_cg_cta,
-// launched concurrently on a second stream).  Both run the same solver body: a cluster
+// through distributed shared memory); the coarser depths get one CTA each (a cluster
+// of one, launched concurrently on a second stream).  Both run the same solver body: a cluster
 // of one CTA is a CTA.
 //
 // Reductions: every product enters exactly (fma: TwoProduct) into a per-thread float pair,
@@ -71,27 +71,37 @@ namespace psr {
 //   x = fma(alpha, p, x)            r = fma(-alpha, Ap, r)    beta = rr_new / rr
 // Missing neighbours contribute fma(st_k, 0, y) = y, the same as skipping them.
 //
-// Resident path (depth >= 1 and at most kCgSmemRows rows per CTA): each CTA owns a
-// contiguous, sibling-group aligned chunk of rows and keeps (r_k, p_{k-1}) in shared
-// memory (two buffers alternating per iteration), plus A p and x.  The operator is
-// applied per sibling group: the 8 children of one parent have all their 27-neighbours
-// inside one 4x4x4 block of same-depth nodes, listed once per group in the block table
-// (k_cg_blocks).  Each lane of a warp (4 groups of 8 siblings) fetches 8 block entries
-// (local shared memory or a remote CTA's through distributed shared memory), the group's
-// 64 p values go to a per-warp shared block, and each lane applies its 27-point stencil
-// from there.  Otherwise (the root, or more rows than fit) the vectors live in global
-// memory and the neighbour table is read row by row.
+// Resident path (depth >= 1 and fewer than kCgGroups sibling groups per CTA): each CTA owns
+// a contiguous chunk of sibling groups and keeps (r_k, p_{k-1}), x and A p of their rows in
+// shared memory, 16 bytes a row, sibling-major: row `sib` of local group g sits at element
+// sib * GP + g, so the lanes of a warp (consecutive groups) read consecutive words.
+// The 27-neighbourhoods of a group's 8 rows are one 4x4x4 block of same-depth nodes, made of
+// parts of the 27 sibling groups around it (one per neighbour of its parent); which sibling
+// of which neighbour group a block position is, is known at compile time.  So one thread
+// applies the operator to a whole group: it visits the 64 positions in order, loads each
+// (r, p) once (own shared memory, or a peer's through distributed shared memory) and adds
+// it to every row it belongs to, which keeps each row's sum in neighbour order.  Nothing is
+// staged and nothing is reread: a group costs 64 loads and 216 FMAs, and the neighbour
+// groups (CTA rank, local group: 15 bits) are found once per solve and stay packed in 14
+// words a group, in shared memory where they fit (up to 1024 groups).
+// A chunk of at most kCgRowGroups groups (the coarser depths) gives every row a thread of
+// its own instead, 27 loads each, for a shorter chain.  The first version fetched a group's
+// block with 8 lanes through a staging block in shared memory (8 stores and 27 reads a row
+// besides the 8 loads) and was bound by the shared-memory queue.  Since p is rebuilt from
+// (r, p) after the first barrier, phase B overwrites the one copy of the pair that phase A
+// read.  Otherwise (the root, or more rows than fit) the vectors live in global memory and
+// the neighbour table is read row by row.
 constexpr int kCgcBlock = 1024;
 constexpr int kCgWarps = kCgcBlock / 32;
-constexpr int kCgSmemRows = 7168;
-constexpr size_t kCgRowBytes = 2 * sizeof(float2) + 2 * sizeof(float);   // r/p x2, A p, x
-// per-warp shared block of 4 sibling groups: group gi at gi * 80 + {0, 18, 8, 26}[gi]
-// floats, so the 4 groups start in banks 0, 2, 8, 10 and the 32 lanes' stencil reads (at
+constexpr int kCgGroups = 1792;                   // local groups of a CTA's arrays; the last one is the zero group
+                                                  //   (absent neighbours: (0, 0), x = 0)
+constexpr int kCgRowGroups = kCgcBlock / 8;       // at most this many groups: a thread per row
+constexpr int kCgDescWords = 14;                  // 27 neighbour groups, two per word
+constexpr size_t kCgSmemBytes = (size_t)kCgGroups * 8 * (sizeof(float2) + 2 * sizeof(float));   // (r, p), x, A p
+// per-warp shared block of 4 sibling groups (device loop): group gi at gi * 80 + {0, 18, 8,
+// 26}[gi] floats, so the 4 groups start in banks 0, 2, 8, 10 and the 32 lanes' stencil reads (at
 // sibling offsets {0,1,4,5,16,17,20,21} + a common neighbour offset) hit 32 distinct banks
 constexpr int kCgWarpBlockFloats = 352;
-constexpr size_t kCgBlockBytes = (size_t)kCgWarps * kCgWarpBlockFloats * sizeof(float);
-constexpr size_t kCgSmemBytes = (size_t)kCgSmemRows * kCgRowBytes + kCgBlockBytes;
-static_assert(kCgSmemRows % 32 == 0, "whole warp slots");
 
 constexpr int kCgMaxRefine = 4;
 
@@ -101,7 +111,10 @@ struct CgcVec {
     const Counters* c;
     Counters* cw;
     const int* neigh;
-    const int* blk;     // block table: 64 entries per sibling group of depth >= 1
+    const int* parent;
+    const int* first_child;
+    const int* blk;     // device loop: 64 entries per sibling group of depth >= 1
+    unsigned* desc;     // [kCgDescWords][dstride]: packed neighbour groups of CTAs with more than one group a thread
     const float* stencil;
     const float* b;
     float* x;
@@ -109,7 +122,7 @@ struct CgcVec {
     float* pa;
     float* pb;
     float* ap;
-    __device__ void rebase() { PSR_CLOUD(c, cw, neigh, blk, stencil, b, x, r, pa, pb, ap); }
+    __device__ void rebase() { PSR_CLOUD(c, cw, neigh, parent, first_child, blk, desc, stencil, b, x, r, pa, pb, ap); }
 };
 
 // a workspace pointer of cloud 0 moved to cloud k (null stays null)
@@ -123,39 +136,50 @@ struct CgcArgs {
     int depth;
     int first;          // depth of cluster / CTA 0; unit u solves depth first - u
     size_t stride;
+    size_t dstride;     // sibling groups of the workspace
     float tol2;
     int max_iter;
     int res_period;     // > 0: true residual every res_period iterations; 0: only at
                         // convergence; < 0: never (the recursive residual alone)
     unsigned loop_mask; // depths the device loop solves when they do not fit the cluster
-    float stp[3][27];   // stencils of units 0..2 of k_cg_cluster (depth first - u)
 };
 
-// The resident path holds a depth when its cluster's chunk of rows fits a CTA's shared
-// memory (the last row is the zero row); the root never does.
-__device__ __forceinline__ int cg_chunk(int m, int nblk) { return ((m + nblk - 1) / nblk + 7) & ~7; }
+// The resident path holds a depth when its cluster's chunk of groups fits a CTA's shared
+// memory (the last group is the zero group); the root never does.
+__device__ __forceinline__ int cg_chunk_groups(int m, int nblk) { return ((m >> 3) + nblk - 1) / nblk; }
 __device__ __forceinline__ bool cg_fits_resident(int d, int m, int nblk) {
-    return d >= 1 && cg_chunk(m, nblk) < kCgSmemRows;
+    return d >= 1 && cg_chunk_groups(m, nblk) < kCgGroups;
 }
 
+// A sum in fixed point: m * 2^(e - 183), |m| < 2^62.  The lanes of a warp are added as 57-bit
+// integers aligned to the largest of them, in three integer warp reductions (what falls off a
+// smaller term is below 2^-57 of the largest); warps and CTAs the same way.
+struct alignas(16) CgSum {
+    long long m;
+    long long e;      // >= 512: not a number
+};
+
 struct CgcShared {
-    FF warp[kCgWarps];
-    double slot[2];
-    double rr;          // r.r of the recursive residual (FP64)
-    double rr_prev;     // the same one iteration earlier
-    double pap;
+    int4 warp[kCgWarps];           // the warps' sums: three pieces and their exponent
+    CgSum slot[2][16];             // the cluster's CTA sums, written by the CTAs
+    unsigned long long bar[2];     // their arrivals
+    CgSum rr;           // r.r of the recursive residual
+    CgSum pap;
     double floor2;      // (2^-20 ||b||)^2: what the true residual of an FP32 solution can reach
     double rr_true;     // r.r of the last true residual (-1: none yet)
+    float rrf;          // r.r rounded to float
     float alpha, beta;
     int go;             // the iteration continues
     int check;          // the true residual is due
     int replace;        // the true residual replaces r (a refinement restart)
     int checks;         // true-residual evaluations
     int restarts;       // refinement restarts
+    int until_check;    // iterations until the next periodic true residual
     float st[27];
 };
 static_assert(kCgWarps == 32, "one FP64 lane per warp partial");
 static_assert(kCgSmemBytes + sizeof(CgcShared) <= 227 * 1024, "shared memory of one CTA");
+static_assert(kCgGroups <= 2048, "11 bits of a packed neighbour group");
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -163,28 +187,150 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// Sum of every thread's `v` over the cluster (FP64).  Thread 0 hands the sum to `post`,
-// which sets the shared scalars the next step reads; every thread sees them when this
-// returns.  Contains the cluster barrier; identical in every CTA.
-template <class Post>
-__device__ __forceinline__ void cgc_allreduce(cg::cluster_group& cl, CgcShared& sh, int& buf, FF v, Post post) {
+// the lanes' sum of m, each |m| <= 2^57, in every lane: three 21-bit pieces, whose sums fit 32 bits
+__device__ __forceinline__ long long cgs_add_lanes(long long m) {
+    const int p0 = (int)(m & 0x1fffff), p1 = (int)((m >> 21) & 0x1fffff), p2 = (int)(m >> 42);
+    const int s0 = __reduce_add_sync(0xffffffffu, p0), s1 = __reduce_add_sync(0xffffffffu, p1),
+              s2 = __reduce_add_sync(0xffffffffu, p2);
+    return ((long long)s2 << 42) + ((long long)s1 << 21) + (long long)s0;
+}
+
+// the sum of the lanes' fixed-point values, in every lane
+__device__ __forceinline__ CgSum cgs_warp_sum(CgSum v) {
+    const long long mag = v.m < 0 ? -v.m : v.m;
+    const int len = 64 - __clzll(mag);   // bits of |m|
+    const int top = __reduce_max_sync(0xffffffffu, v.m != 0 ? (int)v.e + len : 0);
+    // the largest value takes 57 bits
+    const int e = top - 57, d = e - (int)v.e;
+    long long m = 0;
+    if (d <= 0) m = d > -64 ? v.m << -d : 0;           // to the left: only values of fewer than 57 bits
+    else if (d < 63) m = ((v.m >> (d - 1)) + 1) >> 1;  // to the right, to nearest
+    return CgSum{cgs_add_lanes(v.m != 0 ? m : 0), e};
+}
+
+// 2^x for |x| <= 126
+__device__ __forceinline__ float pow2f_exact(int x) { return __int_as_float((127 + x) << 23); }
+
+// The sum of the lanes' float pairs in three pieces (x + y 2^-21 + z 2^-42) 2^(w - 147), in every
+// lane.  A piece of a float against 1.5 * 2^23 units of the piece: the addition rounds to the unit
+// and leaves the integer in the low bits; what is left over is exact.
+__device__ __forceinline__ int4 cgs_warp_sum(FF v) {
+    int top = __reduce_max_sync(0xffffffffu, max((__float_as_int(v.hi) >> 23) & 255, (__float_as_int(v.lo) >> 23) & 255));
+    if (top == 255) return make_int4(0, 0, 0, 1024);   // infinite or not a number
+    int e = top;
+    if (top > 200 || top < 64) {   // uniform: keep the units of the pieces normal numbers
+        const int sh = top > 200 ? -64 : 64;
+        v.hi *= pow2f_exact(sh);
+        v.lo *= pow2f_exact(sh);
+        top += sh;
+    }
+    const int c0 = ((top - 20 + 23) << 23) | 0x400000, c1 = c0 - (21 << 23), c2 = c1 - (21 << 23);
+    auto take = [](float& r, int c) -> int {
+        const float f = __int_as_float(c);
+        const float t = __fadd_rn(r, f);
+        r = __fsub_rn(r, __fsub_rn(t, f));
+        return __float_as_int(t) - c;
+    };
+    int i0 = take(v.hi, c0), i1 = take(v.hi, c1), i2 = take(v.hi, c2);
+    i1 += take(v.lo, c1);
+    i2 += take(v.lo, c2);
+    i0 = __reduce_add_sync(0xffffffffu, i0);
+    i1 = __reduce_add_sync(0xffffffffu, i1);
+    i2 = __reduce_add_sync(0xffffffffu, i2);
+    return make_int4(i0, i1, i2, e);
+}
+// the pieces as one number, |m| <= 2^62
+__device__ __forceinline__ CgSum cgs_join(int4 q) {
+    if (q.w >= 512) return CgSum{1ll << 56, 1024};
+    return CgSum{((long long)q.x << 35) + ((long long)q.y << 14) + ((q.z + 64) >> 7), (long long)q.w + 1};
+}
+
+__device__ __forceinline__ float cgs_float(const CgSum& s) {
+    if (s.e >= 512) return __int_as_float(0x7fc00000);
+    // in two steps: the exponent may leave the float's range half way
+    const int x = max((int)s.e - 183, -250), h = x / 2;
+    return (__ll2float_rn(s.m) * pow2f_exact(h)) * pow2f_exact(x - h);
+}
+__device__ __forceinline__ double cgs_double(const CgSum& s) {
+    if (s.e >= 512) return (double)__int_as_float(0x7fc00000);
+    return (double)s.m * __hiloint2double((1023 + max((int)s.e - 183, -1000)) << 20, 0);   // a power of two: exact
+}
+
+// a shared-memory address of this CTA in the window of cluster CTA `rank`
+__device__ __forceinline__ unsigned cg_map(unsigned sa, unsigned rank) {
+    unsigned ra;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(sa), "r"(rank));
+    return ra;
+}
+__device__ __forceinline__ void cgc_barriers_init(CgcShared& sh) {
+    if (threadIdx.x < 2) {
+        const unsigned b = (unsigned)__cvta_generic_to_shared(&sh.bar[threadIdx.x]);
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+}
+
+// Sum of every thread's `v` over the cluster.  Thread 0 hands the sum to `post`, which sets
+// the shared scalars the next step reads; every thread sees them when this returns.
+// Identical in every CTA.  It is also the cluster's barrier: when the CTA's threads have met, a
+// lane of warp 0 per peer sends the CTA's sum into the peer's slot (st.async, counted by the
+// peer's mbarrier), and nobody goes on before its own mbarrier has counted every CTA's.  That
+// orders the threads' earlier reads of their peers; with kPublish their earlier writes too (a
+// fence before the sends), so that peers may read them next.  Measured in a loop of reductions
+// over 16 CTAs of 1024 threads: 836 cycles, 1165 with the fence, against 1442 for
+// barrier.cluster and a remote read of the sums and 1574 for remote stores and
+// mbarrier arrivals with release.  `n` counts the reductions: they alternate between two
+// slots and barriers, and a CTA reuses a slot only after every peer has sent to the other one.
+// The wait is bounded; `error` is then flagged and the solve stops.
+template <bool kPublish, class Post>
+__device__ __forceinline__ void cgc_allreduce(unsigned nb, unsigned me, CgcShared& sh, unsigned& n, FF v,
+                                              unsigned* error, Post post) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v = ff_warp_sum(v);
-    if (lane == 0) sh.warp[warp] = v;
+    int4 ws = make_int4(0, 0, 0, 0);
+    if (__any_sync(0xffffffffu, v.hi != 0.0f)) ws = cgs_warp_sum(v);   // not a number differs from 0 too
+    if (lane == 0) sh.warp[warp] = ws;
     __syncthreads();
     if (warp == 0) {
-        const double w = dbl_warp_sum(ff_to_double(sh.warp[lane]));
-        if (lane == 0) sh.slot[buf] = w;
+        CgSum t = cgs_warp_sum(cgs_join(sh.warp[lane]));
+        bool late = false;
+        if (nb > 1) {
+            const int buf = (int)(n & 1u);
+            const unsigned parity = (n >> 1) & 1u;
+            const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[buf]);
+            if (kPublish) asm volatile("fence.acq_rel.cluster;" ::: "memory");
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(nb * 16u) : "memory");
+            __syncwarp();
+            if ((unsigned)lane < nb) {
+                const unsigned slot = cg_map((unsigned)__cvta_generic_to_shared(&sh.slot[buf][me]), (unsigned)lane);
+                asm volatile(
+                    "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(slot),
+                    "l"(t.m), "l"(t.e), "r"(cg_map(bar, (unsigned)lane))
+                    : "memory");
+            }
+            unsigned done = 0;
+            for (int spin = 0; spin < kSpinLimit && !done; ++spin)
+                asm volatile(
+                    "{\n.reg .pred p;\n"
+                    "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                    "selp.u32 %0, 1, 0, p;\n}"
+                    : "=r"(done)
+                    : "r"(bar), "r"(parity)
+                    : "memory");
+            late = !done;
+            t = CgSum{0, 0};
+            if ((unsigned)lane < nb) t = sh.slot[buf][lane];
+            t = cgs_warp_sum(t);
+        }
+        if (lane == 0) {
+            post(t);
+            if (late) {
+                atomicOr(error, kErrSpinTimeout);
+                sh.go = sh.check = sh.replace = 0;
+            }
+        }
     }
-    cl.sync();
-    if (warp == 0) {
-        const unsigned nb = cl.num_blocks();
-        double w = 0.0;
-        if ((unsigned)lane < nb) w = *cl.map_shared_rank(&sh.slot[buf], (unsigned)lane);
-        w = dbl_warp_sum(w);
-        if (lane == 0) post(w);
-    }
-    buf ^= 1;
+    ++n;
     __syncthreads();
 }
 
@@ -245,10 +391,68 @@ __device__ __forceinline__ void cg_start(St& sh, const Ar& a, double w) {
     sh.replace = 0;
 }
 
+// The same decisions from fixed-point sums (the cluster solver)
+__device__ __forceinline__ void cgc_alpha(CgcShared& sh, const CgSum& t) {
+    sh.pap = t;
+    sh.alpha = t.m != 0 ? __fdiv_rn(sh.rrf, cgs_float(t)) : 0.0f;
+}
+template <class Ar>
+__device__ __forceinline__ void cgc_after_rr(CgcShared& sh, const Ar& a, const CgSum& t, int it) {
+    const float w = cgs_float(t);
+    sh.beta = sh.rr.m != 0 ? __fdiv_rn(w, sh.rrf) : 0.0f;
+    sh.rr = t;
+    sh.rrf = w;
+    const bool conv = !(w > a.tol2);
+    const bool more = sh.pap.m != 0 && it + 1 <= a.max_iter;
+    sh.go = !conv && more;
+    const bool due = --sh.until_check == 0;   // every res_period iterations
+    if (due) sh.until_check = a.res_period;
+    sh.check = a.res_period >= 0 && sh.pap.m != 0 && (conv || (due && more));
+}
+template <class Ar>
+__device__ __forceinline__ void cgc_after_true(CgcShared& sh, const Ar& a, const CgSum& t, int it) {
+    ++sh.checks;
+    const double w = cgs_double(t), rr = cgs_double(sh.rr);
+    const double target = fmax((double)a.tol2, sh.floor2);
+    const bool drift = w > 4.0 * fmax(rr, sh.floor2);
+    const bool falling = sh.rr_true < 0.0 || w < 0.25 * sh.rr_true;
+    sh.replace = w > target && (!sh.go || drift) && sh.restarts < kCgMaxRefine && it <= a.max_iter && falling;
+    if (sh.replace) {
+        ++sh.restarts;
+        sh.beta = 0.0f;
+        sh.go = 1;
+        sh.rr = t;
+        sh.rrf = cgs_float(t);
+    }
+    sh.rr_true = w;
+}
+template <class Ar>
+__device__ __forceinline__ void cgc_start(CgcShared& sh, const Ar& a, const CgSum& t) {
+    sh.rr = t;
+    sh.rrf = cgs_float(t);
+    sh.beta = 0.0f;
+    sh.go = (sh.rrf > a.tol2) && a.max_iter >= 1;
+    sh.until_check = a.res_period > 0 ? a.res_period : 0;   // 0: never counts down to 0 again
+    sh.floor2 = cgs_double(t) * 0x1p-40;
+    sh.rr_true = -1.0;
+    sh.checks = 0;
+    sh.restarts = 0;
+    sh.replace = 0;
+}
+
 // Per-depth results of a finished solve (thread 0 of cluster CTA 0).
 template <class St>
 __device__ __forceinline__ void cg_report(const CgcVec& v, int d, const St& sh) {
     v.cw->cg_rr[d] = sh.rr;
+    v.cw->cg_rr_true[d] = sh.rr_true;
+    v.cw->cg_checks[d] = sh.checks;
+    v.cw->cg_restarts[d] = sh.restarts;
+}
+// The iteration count goes out here and not per iteration: a global store in flight would hold
+// up the release at every reduction.
+__device__ __forceinline__ void cgc_report(const CgcVec& v, int d, const CgcShared& sh, int iterations) {
+    v.cw->cg_iters[d] = iterations;
+    v.cw->cg_rr[d] = cgs_double(sh.rr);
     v.cw->cg_rr_true[d] = sh.rr_true;
     v.cw->cg_checks[d] = sh.checks;
     v.cw->cg_restarts[d] = sh.restarts;
@@ -283,202 +487,313 @@ struct CgUnit {
     int d, row0, row1;
 };
 
-// (r, p) pair at byte offset `off` of the `cur` buffer of cluster CTA `rank`: the shared
-// address of this CTA's buffer mapped into that CTA's window (mapa), then one
-// distributed-shared-memory load
-__device__ __forceinline__ float2 cg_ld_pair(unsigned cur_sa, unsigned desc) {
-    unsigned ra;
+__device__ __forceinline__ float2 cg_ld2(unsigned a) {
     float2 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(cur_sa + (desc & 0xffffffu)), "r"(desc >> 24));
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(ra));
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
     return v;
 }
-constexpr int kCgZeroRow = kCgSmemRows - 1;   // kept (0, 0) in both buffers: absent neighbours
-
-// x of the row whose (r, p) pair a descriptor addresses: the x array holds one float per
-// row, so the row's byte offset in the pair buffer halves
-__device__ __forceinline__ float cg_ld_x(unsigned x_sa, unsigned desc) {
-    unsigned ra;
+__device__ __forceinline__ float cg_ld1(unsigned a) {
     float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(x_sa + ((desc & 0xffffffu) >> 1)), "r"(desc >> 24));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
     return v;
 }
 
-// Resident path.  CTA k of the cluster owns rows [row0 + k*chunk, row0 + (k+1)*chunk).
-// U >= 0: the cluster unit whose stencil is a launch parameter (a.stp[U]), read as a
-// constant operand of the FMAs; U < 0: the stencil staged in shared memory.
-template <int U>
-__device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& sh, const CgcArgs& a,
-                                             const CgcVec& v, const CgUnit& u, int chunk, float2* rp0, float2* rp1, float* sap,
-                                             float* sx, float* sblk) {
-    const unsigned me = cl.block_rank();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int m = u.row1 - u.row0;
-    const int mlo = u.row0 + (int)me * chunk;
-    const int nloc = max(0, min(chunk, m - (int)me * chunk));
-    const int nslot = (nloc + 31) >> 5;
-    const int gi = lane >> 3, sib = lane & 7;
-    const int spos = cg_spos(sib);
-    float* myblk = sblk + warp * kCgWarpBlockFloats + gi * 80 + ((0x1a081200 >> (gi * 8)) & 0xff);
-    const int gbase = (mlo - 1) >> 3;   // block-table group of local row 0
-    // g / chunk = umulhi(g, ceil(2^32 / chunk)): exact while g * (magic * chunk - 2^32) < 2^32,
-    // true here (g < 2^17 rows, chunk <= kCgSmemRows)
-    const unsigned chunk_magic = chunk > 0 ? (unsigned)((0x100000000ull + (unsigned)chunk - 1) / (unsigned)chunk) : 0u;
-    // The block table of this CTA's groups becomes descriptors, once: (CTA rank << 24) |
-    // byte offset of the row inside that CTA's buffer (the zero row for an absent cell), so
-    // an iteration reads a neighbour with one mapped load instead of locating its owner.
-    // Only this CTA reads these groups' entries; the barrier below publishes them.
-    int* blkw = const_cast<int*>(v.blk);
-    for (int t = threadIdx.x; t < nloc * 8; t += kCgcBlock) {
-        const size_t at = (size_t)gbase * 64 + t;
-        const int nb = blkw[at];
-        const int gl = nb - mlo;
-        const int g = nb - u.row0;
-        unsigned desc = (me << 24) | (unsigned)(kCgZeroRow * 8);
-        if ((unsigned)gl < (unsigned)nloc) {
-            desc = (me << 24) | (unsigned)(gl * 8);
-        } else if (nb >= 0 && (unsigned)g < (unsigned)m) {
-            const int owner = (int)__umulhi((unsigned)g, chunk_magic);   // g / chunk
-            desc = ((unsigned)owner << 24) | (unsigned)((g - owner * chunk) * 8);
+// The stencil entry of offset slot k depends only on how many axes the offset is non-zero on
+// (0: centre, 1: face, 2: edge, 3: corner): four values per depth (checked at creation).
+__host__ __device__ constexpr int cg_class(int k) {
+    return (k / 9 != 1) + ((k / 3) % 3 != 1) + (k % 3 != 1);
+}
+// block position 16 bx + 4 by + bz: the neighbour of the parent it lies in, and its sibling there
+__host__ __device__ constexpr int cg_pos_axis(int b) { return b == 0 ? 0 : (b == 3 ? 2 : 1); }
+__host__ __device__ constexpr int cg_pos_group(int p) {
+    return 9 * cg_pos_axis(p >> 4) + 3 * cg_pos_axis((p >> 2) & 3) + cg_pos_axis(p & 3);
+}
+__host__ __device__ constexpr int cg_pos_sib(int p) {
+    return 4 * (((p >> 4) + 1) & 1) + 2 * ((((p >> 2) & 3) + 1) & 1) + (((p & 3) + 1) & 1);
+}
+
+// The sibling group on slot n of group G's parent (global group number), or -1.
+__device__ __forceinline__ int cg_neighbour_group(const CgcVec& v, size_t stride, int pa, int n) {
+    const int q = v.neigh[(size_t)n * stride + pa];
+    const int f = v.first_child[q >= 0 ? q : 0];
+    return (q >= 0 && f >= 1) ? (f - 1) >> 3 : -1;
+}
+
+// How a CTA's rows are dealt to its threads.
+enum CgMode {
+    kCgRows,     // a thread per row (thread t: sibling t / kCgRowGroups of group t % kCgRowGroups)
+    kCgOne,      // a thread per group, the packed neighbour groups in shared memory
+    kCgMany      // groups in turn, their neighbour groups packed in global memory
+};
+// groups of the sibling-major arrays of a mode (the last one is the zero group)
+__host__ __device__ constexpr int cg_pitch(int mode) {
+    return mode == kCgMany ? kCgGroups : mode == kCgOne ? kCgcBlock + 8 : kCgRowGroups + 8;
+}
+static_assert((size_t)cg_pitch(kCgOne) * 8 * 16 + (size_t)kCgDescWords * kCgcBlock * 4 <= kCgSmemBytes, "kCgOne");
+
+// The operator of one group: adds st * val(position) to every row the position neighbours, in
+// neighbour order per row.  `val(n, off)` gives the value of neighbour group n's element at
+// element offset `off` of the sibling-major arrays.
+template <int kPitch, class Val, class Add>
+__device__ __forceinline__ void cg_apply_group(Val val, Add add) {
+#pragma unroll
+    for (int p = 0; p < 64; ++p) {
+        const auto x = val(cg_pos_group(p), cg_pos_sib(p) * kPitch);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const int ox = (p >> 4) - (s >> 2), oy = ((p >> 2) & 3) - ((s >> 1) & 1), oz = (p & 3) - (s & 1);
+            if (ox >= 0 && ox < 3 && oy >= 0 && oy < 3 && oz >= 0 && oz < 3)
+                add(s, cg_class(9 * ox + 3 * oy + oz), x);
         }
-        blkw[at] = (int)desc;
     }
-    if (threadIdx.x == 0) {
-        rp0[kCgZeroRow] = make_float2(0.0f, 0.0f);
-        rp1[kCgZeroRow] = make_float2(0.0f, 0.0f);
-        sx[kCgZeroRow] = 0.0f;
+}
+
+// Resident path.  CTA k of the cluster owns the unit's groups [k * chunk, (k + 1) * chunk).
+template <int kMode>
+__device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& sh, const CgcArgs& a,
+                                             const CgcVec& v, const CgUnit& u, int chunk, float4* dyn) {
+    constexpr int GP = cg_pitch(kMode);
+    float2* rp = reinterpret_cast<float2*>(dyn);
+    float* sx = reinterpret_cast<float*>(rp + 8 * GP);
+    float* sap = sx + 8 * GP;
+    constexpr int kDescPitch = kMode == kCgOne ? kCgcBlock : kCgRowGroups;
+    unsigned* sdesc = reinterpret_cast<unsigned*>(sap + 8 * GP);   // [kCgDescWords][kDescPitch]
+    const unsigned me = cl.block_rank(), nb = cl.num_blocks();
+    unsigned* err = &v.cw->error;
+    const int tid = threadIdx.x;
+    const int ngroups = (u.row1 - u.row0) >> 3;
+    const int g0 = (int)me * chunk;                           // the CTA's first group, in the unit
+    const int ng = max(0, min(chunk, ngroups - g0));
+    const int gbase = ((u.row0 - 1) >> 3) + g0;               // global number of local group 0
+    const unsigned rp_sa = (unsigned)__cvta_generic_to_shared(rp);
+    const unsigned x_sa = (unsigned)__cvta_generic_to_shared(sx);
+    const float w[4] = {sh.st[13], sh.st[14], sh.st[17], sh.st[26]};   // centre, face, edge, corner
+    // q / chunk = umulhi(q, ceil(2^32 / chunk)): exact for q < 16 * chunk, chunk <= 2^11
+    const unsigned magic = (unsigned)((0x100000000ull + (unsigned)chunk - 1) / (unsigned)chunk);
+    // rank << 11 | local group of global group G (absent or outside the unit: the zero group)
+    auto locate = [&](int G) -> unsigned {
+        const unsigned q = (unsigned)(G - ((u.row0 - 1) >> 3));
+        if (G < 0 || q >= (unsigned)ngroups) return (me << 11) | (unsigned)(GP - 1);
+        const unsigned own = chunk > 1 ? __umulhi(q, magic) : q;   // q / chunk
+        return (own << 11) | (q - own * (unsigned)chunk);
+    };
+    auto base_of = [&](unsigned d, unsigned sa, unsigned elem) { return cg_map(sa + (d & 2047u) * elem, d >> 11); };
+
+    // kCgRows: this thread's row and the mapped addresses of its 27 neighbours' pairs
+    const int rs = tid / kCgRowGroups, rg = tid % kCgRowGroups;
+    const bool row_on = kMode == kCgRows && rg < ng;
+    // neighbour (kx, ky, kz) of sibling s: its neighbour group slot and sibling there
+    auto slot_of = [](int s, int kx, int ky, int kz, int& n, int& sib) {
+        const int bx = (s >> 2) + kx, by = ((s >> 1) & 1) + ky, bz = (s & 1) + kz;
+        n = 9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1) + ((bz + 1) >> 1);   // cg_pos_axis
+        sib = 4 * ((bx + 1) & 1) + 2 * ((by + 1) & 1) + ((bz + 1) & 1);
+    };
+    // The packed neighbour groups (parent, its neighbour row, first children), in loops of a few
+    // steps: long straight-line code that runs once comes from L2
+    auto find_word = [&](int g, int pa, int j) {
+        const unsigned lo = locate(cg_neighbour_group(v, a.stride, pa, 2 * j));
+        const unsigned hi = (2 * j + 1 < 27) ? locate(cg_neighbour_group(v, a.stride, pa, 2 * j + 1)) : 0u;
+        const unsigned q = lo | (hi << 16);
+        if (kMode == kCgMany) v.desc[(size_t)j * a.dstride + gbase + g] = q;
+        else sdesc[j * kDescPitch + g] = q;
+    };
+    if (kMode == kCgRows) {   // a word per thread and turn
+#pragma unroll 2
+        for (int i = tid; i < kCgDescWords * kCgRowGroups; i += kCgcBlock) {
+            const int j = i / kCgRowGroups, g = i % kCgRowGroups;
+            if (g < ng) find_word(g, v.parent[1 + 8 * (gbase + g)], j);
+        }
+    } else {
+        for (int g = tid; g < ng; g += kCgcBlock) {
+            const int pa = v.parent[1 + 8 * (gbase + g)];
+#pragma unroll 7
+            for (int j = 0; j < kCgDescWords; ++j) find_word(g, pa, j);
+        }
     }
-    // r0 = b, p_{-1} = 0, x0 = 0
+    // neighbour group slot n of group g (packed)
+    auto desc_of = [&](int g, int n) -> unsigned {
+        const unsigned q = kMode == kCgMany ? v.desc[(size_t)(n >> 1) * a.dstride + gbase + g]
+                                            : sdesc[(n >> 1) * kDescPitch + g];
+        return (n & 1) ? q >> 16 : q & 0xffffu;
+    };
+    // kCgRows: the mapped addresses of the row's 27 neighbours' pairs
+    unsigned adr[kMode == kCgRows ? 27 : 1];
+    if (kMode == kCgRows) {
+        __syncthreads();
+        if (row_on) {
+#pragma unroll
+            for (int k = 0; k < 27; ++k) {
+                int n, sib;
+                slot_of(rs, k / 9, (k / 3) % 3, k % 3, n, sib);
+                adr[kMode == kCgRows ? k : 0] = base_of(desc_of(rg, n), rp_sa, 8u) + (unsigned)(sib * GP * 8);
+            }
+        }
+    }
+    if (tid < 8) {
+        rp[tid * GP + GP - 1] = make_float2(0.0f, 0.0f);
+        sx[tid * GP + GP - 1] = 0.0f;
+    }
+    // every row of this thread: body(element, row of the unit's arrays)
+    auto for_rows = [&](auto body) {
+        if (kMode == kCgRows) {
+            if (row_on) body(rs * GP + rg);
+        } else {
+            for (int g = tid; g < ng; g += kCgcBlock)
+#pragma unroll
+                for (int s = 0; s < 8; ++s) body(s * GP + g);
+        }
+    };
+    // r0 = b, p_{-1} = 0, x0 = 0 (rows in order: coalesced; A p starts as scratch)
     FF acc = ff_zero();
-    for (int l = threadIdx.x; l < nloc; l += kCgcBlock) {
+    const int mlo = 1 + 8 * gbase;
+    for (int l = tid; l < 8 * ng; l += kCgcBlock) {
         const float bi = v.b[mlo + l];
-        rp0[l] = make_float2(bi, 0.0f);
-        sx[l] = 0.0f;
+        const int e = (l & 7) * GP + (l >> 3);
+        rp[e] = make_float2(bi, 0.0f);
+        sx[e] = 0.0f;
         acc = ff_add(acc, ff_prod(bi, bi));
     }
-    int buf = 0;
-    cgc_allreduce(cl, sh, buf, acc, [&](double w) { cg_start(sh, a, w); });
+    unsigned nred = 0;
+    cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_start(sh, a, t); });
     bool ran = false;
-    float2* cur = rp0;
-    float2* nxt = rp1;
     int it = 1;
     while (sh.go) {
         const float beta = sh.beta;
-        // (A) own p_k, A p_k from the neighbours' (r_k, p_{k-1}), p.Ap
+        // (A) A p_k from the neighbours' (r_k, p_{k-1}), p.Ap
         acc = ff_zero();
-        // the block-table entries of the warp's next slot are loaded while the current
-        // slot is processed (they do not change between iterations)
-        int4 q0 = make_int4(-1, -1, -1, -1), q1 = q0;
-        if (warp < nslot && warp * 32 + lane < nloc) {
-            const int4* bp = reinterpret_cast<const int4*>(v.blk + (size_t)(gbase + ((warp * 32 + lane) >> 3)) * 64 + sib * 8);
-            q0 = bp[0];
-            q1 = bp[1];
-        }
-        const unsigned cur_sa = (unsigned)__cvta_generic_to_shared(cur);
-        for (int sl = warp; sl < nslot; sl += kCgWarps) {
-            const int l = sl * 32 + lane;
-            const bool mine = l < nloc;   // whole groups: a group is all in or all out
-            const int ids[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-            const int ln = l + kCgWarps * 32;
-            if (ln < nloc) {
-                const int4* bp = reinterpret_cast<const int4*>(v.blk + (size_t)(gbase + (ln >> 3)) * 64 + sib * 8);
-                q0 = bp[0];
-                q1 = bp[1];
-            }
-            if (mine) {
-                // 8 independent mapped loads (own buffer, a peer's, or the zero row)
-                float2 vals[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) vals[e] = cg_ld_pair(cur_sa, (unsigned)ids[e]);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) myblk[e * 8 + sib] = fmaf(beta, vals[e].y, vals[e].x);
-            }
-            __syncwarp();
-            if (mine) {
+        if (kMode == kCgRows) {
+            if (row_on) {
+                const int e = rs * GP + rg;
                 float y = 0.0f;
 #pragma unroll
-                for (int k = 0; k < 27; ++k) y = fmaf(U >= 0 ? a.stp[U < 0 ? 0 : U][k] : sh.st[k], myblk[spos + cg_kpos(k)], y);
-                const float2 own = cur[l];
-                const float pi = fmaf(beta, own.y, own.x);
-                nxt[l].y = pi;
-                sap[l] = y;
-                acc = ff_add(acc, ff_prod(pi, y));
+                for (int k = 0; k < 27; ++k) {
+                    const float2 q = cg_ld2(adr[kMode == kCgRows ? k : 0]);
+                    y = fmaf(w[cg_class(k)], fmaf(beta, q.y, q.x), y);
+                }
+                const float2 own = rp[e];
+                sap[e] = y;
+                acc = ff_add(acc, ff_prod(fmaf(beta, own.y, own.x), y));
             }
-            __syncwarp();
+        } else {
+            for (int g = tid; g < ng; g += kCgcBlock) {
+                float y[8];
+#pragma unroll
+                for (int s = 0; s < 8; ++s) y[s] = 0.0f;
+                cg_apply_group<GP>(
+                    [&](int n, int off) {
+                        const float2 q = cg_ld2(base_of(desc_of(g, n), rp_sa, 8u) + (unsigned)(off * 8));
+                        return fmaf(beta, q.y, q.x);
+                    },
+                    [&](int s, int c, float p) { y[s] = fmaf(w[c], p, y[s]); });
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const float2 own = rp[s * GP + g];
+                    sap[s * GP + g] = y[s];
+                    acc = ff_add(acc, ff_prod(fmaf(beta, own.y, own.x), y[s]));
+                }
+            }
         }
-        cgc_allreduce(cl, sh, buf, acc, [&](double w) {
-            sh.pap = w;
-            sh.alpha = cg_quot(sh.rr, w);
-        });
+        cgc_allreduce<false>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_alpha(sh, t); });
         const float alpha = sh.alpha;
-        // (B) x and r, r.r
+        // (B) x and r, r.r; every CTA has read the pairs (the barrier of the last reduction)
         acc = ff_zero();
-        for (int sl = warp; sl < nslot; sl += kCgWarps) {
-            const int l = sl * 32 + lane;
-            if (l < nloc) {
-                const float pi = nxt[l].y;
-                sx[l] = fmaf(alpha, pi, sx[l]);
-                const float ri = fmaf(-alpha, sap[l], cur[l].x);
-                nxt[l].x = ri;
-                acc = ff_add(acc, ff_prod(ri, ri));
-            }
-        }
-        cgc_allreduce(cl, sh, buf, acc, [&](double w) { cg_after_rr(sh, a, w, it); });
+        for_rows([&](int e) {
+            const float2 own = rp[e];
+            const float pi = fmaf(beta, own.y, own.x);
+            sx[e] = fmaf(alpha, pi, sx[e]);
+            const float ri = fmaf(-alpha, sap[e], own.x);
+            rp[e] = make_float2(ri, pi);
+            acc = ff_add(acc, ff_prod(ri, ri));
+        });
+        cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_rr(sh, a, t, it); });
         ran = true;
-        if (me == 0 && threadIdx.x == 0) v.cw->cg_iters[u.d] = it;
-        float2* t = cur;
-        cur = nxt;
-        nxt = t;
         ++it;
         if (sh.check) {
             // (C) true residual b - A x of the current x from the neighbours' x (the barrier
             // of the last reduction published every CTA's x), with exact products and
-            // float-pair sums; staged in the A p buffer, which holds nothing live here
+            // float-pair sums; staged in the A p array, which holds nothing live here
             acc = ff_zero();
-            const unsigned x_sa = (unsigned)__cvta_generic_to_shared(sx);
-            for (int sl = warp; sl < nslot; sl += kCgWarps) {
-                const int l = sl * 32 + lane;
-                const bool mine = l < nloc;
-                if (mine) {
-                    const int4* bp = reinterpret_cast<const int4*>(v.blk + (size_t)(gbase + (l >> 3)) * 64 + sib * 8);
-                    const int4 d0 = bp[0], d1 = bp[1];
-                    const int ids[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-                    float vals[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) vals[e] = cg_ld_x(x_sa, (unsigned)ids[e]);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) myblk[e * 8 + sib] = vals[e];
-                }
-                __syncwarp();
-                if (mine) {
+            // the entry of an offset that moves on `axes` of x and y, and by kz - 1 on z
+            auto w_of = [&](int axes, int kz) {
+                return kz == 1 ? (axes == 0 ? w[0] : axes == 1 ? w[1] : w[2]) : (axes == 0 ? w[1] : axes == 1 ? w[2] : w[3]);
+            };
+            auto residual = [&](int g, int s, FF y) {
+                const float ri = ff_to_float(ff_add(FF{v.b[mlo + 8 * g + s], 0.0f}, FF{-y.hi, -y.lo}));
+                sap[s * GP + g] = ri;
+                acc = ff_add(acc, ff_prod(ri, ri));
+            };
+            // rolled over the z-lines of the block: straight-line code that runs twice per solve
+            // would come from L2
+            if (kMode == kCgRows) {
+                if (row_on) {
                     FF y = ff_zero();
+#pragma unroll 1
+                    for (int q = 0; q < 9; ++q) {
 #pragma unroll
-                    for (int k = 0; k < 27; ++k)
-                        y = ff_add(y, ff_prod(U >= 0 ? a.stp[U < 0 ? 0 : U][k] : sh.st[k], myblk[spos + cg_kpos(k)]));
-                    const float ri = ff_to_float(ff_add(FF{v.b[mlo + l], 0.0f}, FF{-y.hi, -y.lo}));
-                    sap[l] = ri;
-                    acc = ff_add(acc, ff_prod(ri, ri));
+                        for (int kz = 0; kz < 3; ++kz) {
+                            int n, sib;
+                            slot_of(rs, q / 3, q % 3, kz, n, sib);
+                            const float wk = w_of((q / 3 != 1) + (q % 3 != 1), kz);
+                            y = ff_add(y, ff_prod(wk, cg_ld1(base_of(desc_of(rg, n), x_sa, 4u) + (unsigned)(sib * GP * 4))));
+                        }
+                    }
+                    residual(rg, rs, y);
                 }
-                __syncwarp();
+            } else {
+                for (int g = tid; g < ng; g += kCgcBlock) {
+                    FF y[8];
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) y[s] = ff_zero();
+#pragma unroll 1
+                    for (int q = 0; q < 16; ++q) {
+                        const int bx = q >> 2, by = q & 3;
+                        const int nxy = 9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1);
+                        const int sxy = 4 * ((bx + 1) & 1) + 2 * ((by + 1) & 1);
+                        float xv[4];
+#pragma unroll
+                        for (int bz = 0; bz < 4; ++bz)
+                            xv[bz] = cg_ld1(base_of(desc_of(g, nxy + cg_pos_axis(bz)), x_sa, 4u) +
+                                            (unsigned)((sxy + ((bz + 1) & 1)) * GP * 4));
+#pragma unroll
+                        for (int sxy2 = 0; sxy2 < 4; ++sxy2) {   // the rows (sx, sy) this line neighbours
+                            const int ox = bx - (sxy2 >> 1), oy = by - (sxy2 & 1);
+                            if (ox < 0 || ox > 2 || oy < 0 || oy > 2) continue;
+                            const int axes = (ox != 1) + (oy != 1);
+#pragma unroll
+                            for (int sz = 0; sz < 2; ++sz)
+#pragma unroll
+                                for (int oz = 0; oz < 3; ++oz) {
+                                    FF& t = y[2 * sxy2 + sz];
+                                    t = ff_add(t, ff_prod(w_of(axes, oz), xv[sz + oz]));
+                                }
+                        }
+                    }
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) residual(g, s, y[s]);
+                }
             }
-            cgc_allreduce(cl, sh, buf, acc, [&](double w) { cg_after_true(sh, a, w, it); });
+            cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_true(sh, a, t, it); });
             if (sh.replace) {   // refinement restart: CG continues from the true residual
-                for (int l = threadIdx.x; l < nloc; l += kCgcBlock) cur[l].x = sap[l];
+                for_rows([&](int e) { rp[e].x = sap[e]; });
                 cl.sync();      // before any CTA reads a neighbour's new r
             }
         }
     }
-    for (int l = threadIdx.x; l < nloc; l += kCgcBlock) {
-        v.x[mlo + l] = sx[l];
-        v.r[mlo + l] = cur[l].x;
+    __syncthreads();
+    for (int l = tid; l < 8 * ng; l += kCgcBlock) {
+        const int e = (l & 7) * GP + (l >> 3);
+        v.x[mlo + l] = sx[e];
+        v.r[mlo + l] = rp[e].x;
     }
-    if (ran && me == 0 && threadIdx.x == 0) cg_report(v, u.d, sh);
+    if (ran && me == 0 && tid == 0) cgc_report(v, u.d, sh, it - 1);
 }
 
-// Global-memory path (any size, any depth).
+// Global-memory path (any size, any depth).  The peers' vectors are read through L1, so every
+// published step also passes the cluster barrier.
 __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh, const CgcArgs& a,
                                            const CgcVec& v, const CgUnit& u) {
+    const unsigned me = cl.block_rank(), nb = cl.num_blocks();
+    unsigned* err = &v.cw->error;
     const int tid = cl.block_rank() * blockDim.x + threadIdx.x;
     const int nthr = cl.num_blocks() * blockDim.x;
     FF acc = ff_zero();
@@ -489,8 +804,9 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
         v.x[i] = 0.0f;
         acc = ff_add(acc, ff_prod(bi, bi));
     }
-    int buf = 0;
-    cgc_allreduce(cl, sh, buf, acc, [&](double w) { cg_start(sh, a, w); });
+    unsigned nred = 0;
+    cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_start(sh, a, t); });
+    if (nb > 1) cl.sync();
     bool ran = false;
     const float* pprev = v.pa;
     float* pcur = v.pb;
@@ -510,10 +826,7 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
             v.ap[i] = y;
             acc = ff_add(acc, ff_prod(pi, y));
         }
-        cgc_allreduce(cl, sh, buf, acc, [&](double w) {
-            sh.pap = w;
-            sh.alpha = cg_quot(sh.rr, w);
-        });
+        cgc_allreduce<false>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_alpha(sh, t); });
         const float alpha = sh.alpha;
         acc = ff_zero();
         for (int i = u.row0 + tid; i < u.row1; i += nthr) {
@@ -522,9 +835,9 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
             v.r[i] = ri;
             acc = ff_add(acc, ff_prod(ri, ri));
         }
-        cgc_allreduce(cl, sh, buf, acc, [&](double w) { cg_after_rr(sh, a, w, it); });
+        cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_rr(sh, a, t, it); });
+        if (nb > 1) cl.sync();
         ran = true;
-        if (cl.block_rank() == 0 && threadIdx.x == 0) v.cw->cg_iters[u.d] = it;
         float* t = const_cast<float*>(pprev);
         pprev = pcur;
         pcur = t;
@@ -542,19 +855,18 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
                 v.ap[i] = ri;   // staged; A p holds nothing live here
                 acc = ff_add(acc, ff_prod(ri, ri));
             }
-            cgc_allreduce(cl, sh, buf, acc, [&](double w) { cg_after_true(sh, a, w, it); });
+            cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_true(sh, a, t, it); });
+            if (nb > 1) cl.sync();
             if (sh.replace) {   // refinement restart: CG continues from the true residual
                 for (int i = u.row0 + tid; i < u.row1; i += nthr) v.r[i] = v.ap[i];
                 cl.sync();
             }
         }
     }
-    if (ran && cl.block_rank() == 0 && threadIdx.x == 0) cg_report(v, u.d, sh);
+    if (ran && cl.block_rank() == 0 && threadIdx.x == 0) cgc_report(v, u.d, sh, it - 1);
 }
 
-// one depth per cluster (a CTA when the launch has no cluster dimension); kClusterUnits:
-// the unit's stencil is a launch parameter
-template <bool kClusterUnits>
+// one depth per cluster (a CTA when the launch has no cluster dimension)
 __device__ __forceinline__ void cg_unit_body(const CgcArgs& a, const CgcVec& v, int unit) {
     cg::cluster_group cl = cg::this_cluster();
     __shared__ CgcShared sh;
@@ -565,22 +877,17 @@ __device__ __forceinline__ void cg_unit_body(const CgcArgs& a, const CgcVec& v, 
     u.row0 = v.c->level_base[u.d];
     u.row1 = (u.d < a.depth) ? v.c->level_base[u.d + 1] : v.c->n_nodes;
     if (threadIdx.x < 27) sh.st[threadIdx.x] = v.stencil[u.d * 27 + threadIdx.x];
-    __syncthreads();
     const int nblk = (int)cl.num_blocks();
+    cgc_barriers_init(sh);
+    cl.sync();   // the barriers are up before a peer arrives at them
     const int m = u.row1 - u.row0;
-    const int chunk = cg_chunk(m, nblk);   // sibling-group aligned
+    const int chunk = cg_chunk_groups(m, nblk);
     const bool fits = cg_fits_resident(u.d, m, nblk);   // uniform over the cluster
     if (!fits && ((a.loop_mask >> u.d) & 1u)) return;    // the device loop solves this depth
     if (fits) {
-        float2* rp0 = reinterpret_cast<float2*>(cg_dyn);
-        float2* rp1 = rp0 + kCgSmemRows;
-        float* sap = reinterpret_cast<float*>(rp1 + kCgSmemRows);
-        float* sx = sap + kCgSmemRows;
-        float* sblk = sx + kCgSmemRows;
-        if (kClusterUnits && unit == 0) cgc_resident<0>(cl, sh, a, v, u, chunk, rp0, rp1, sap, sx, sblk);
-        else if (kClusterUnits && unit == 1) cgc_resident<1>(cl, sh, a, v, u, chunk, rp0, rp1, sap, sx, sblk);
-        else if (kClusterUnits && unit == 2) cgc_resident<2>(cl, sh, a, v, u, chunk, rp0, rp1, sap, sx, sblk);
-        else cgc_resident<-1>(cl, sh, a, v, u, chunk, rp0, rp1, sap, sx, sblk);
+        if (chunk <= kCgRowGroups) cgc_resident<kCgRows>(cl, sh, a, v, u, chunk, cg_dyn);
+        else if (chunk <= kCgcBlock) cgc_resident<kCgOne>(cl, sh, a, v, u, chunk, cg_dyn);
+        else cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);
     } else {
         cgc_global(cl, sh, a, v, u);
     }
@@ -592,13 +899,7 @@ __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
     cg::cluster_group cl = cg::this_cluster();
     CgcVec v = a.v;
     v.rebase();
-    cg_unit_body<true>(a, v, (int)(blockIdx.x / cl.num_blocks()));
-}
-
-__global__ void __launch_bounds__(kCgcBlock) k_cg_cta(CgcArgs a) {
-    CgcVec v = a.v;
-    v.rebase();
-    cg_unit_body<false>(a, v, (int)blockIdx.x);
+    cg_unit_body(a, v, (int)(blockIdx.x / cl.num_blocks()));
 }
 
 // ---- device-loop CG: the depths too large for a cluster's shared memory -----------------
@@ -1101,9 +1402,7 @@ void prepare_launch_configs(Workspace& ws) {
     if (g_cg_cluster == 0) {
         int size = 8;
         if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgSmemBytes) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_cg_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgSmemBytes) !=
-                cudaSuccess)
+            cudaSuccess)
             return;   // left unset: the CG launch reports the error
         if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cudaLaunchConfig_t cfg = {};
@@ -1206,7 +1505,11 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     a.v.cw = ws.cnt;
     a.depth = D;
     a.v.neigh = ws.neigh;
+    a.v.parent = ws.parent;
+    a.v.first_child = ws.first_child;
     a.v.blk = ws.cg_blk;
+    a.v.desc = ws.cg_desc;
+    a.dstride = (size_t)ws.cap.nodes / 8 + 8;
     a.stride = (size_t)ws.cap.nodes;
     a.v.stencil = ws.stencil;
     a.v.b = ws.divg;
@@ -1220,9 +1523,7 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     // test of the loop is kept (mesh/solver/CGAlgorithm.cu:36)
     a.max_iter = (cg_mode == 1 && cg_iters > 0) ? cg_iters : cg_max_iter;
     a.res_period = res_period;
-    k_cg_blocks<<<PSR_GRID(ws, grid_for(ws, 1 << 20)), kBlock, 0, s>>>(ws.cnt, ws.neigh, (size_t)ws.cap.nodes, ws.cg_blk);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     // The finest depths (D, D-1, and D-2 from depth 5 on; never the root) on clusters: depth
     // D on the widest cluster, D-1 and D-2 (fewer rows, done well before depth D) on clusters
     // of at most 8 CTAs, on a third stream, so that they hold fewer SMs; the rest one CTA
@@ -1248,6 +1549,8 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     if (e == cudaSuccess && ncl > 1) e = cudaStreamWaitEvent(ws.aux3, ws.ev_fork, 0);
     if (e == cudaSuccess && loop_units > 0) {
         e = cudaStreamWaitEvent(ws.aux4, ws.ev_fork, 0);
+        k_cg_blocks<<<PSR_GRID(ws, grid_for(ws, 1 << 20)), kBlock, 0, ws.aux4>>>(ws.cnt, ws.neigh, (size_t)ws.cap.nodes,
+                                                                                ws.cg_blk);
         CgLoopArgs L;
         L.v = a.v;
         L.st = ws.cg_loop;
@@ -1263,24 +1566,18 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
         L.res_period = a.res_period;
         if (e == cudaSuccess) e = launch_cg_loop(ws, L);
         if (e == cudaSuccess) e = cudaEventRecord(ws.ev_join4, ws.aux4);
-        // the coarse sample values and the depth-D terms wait for every depth's solution
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(ws.aux, ws.ev_join4, 0);
     }
     if (e == cudaSuccess && ncta > 0) {
         CgcArgs b = a;
         b.first = D - ncl;
-        e = launch_cg(k_cg_cta, b, ncta, 1, ws.batch, ws.aux);   // clusters of one CTA
+        e = launch_cg(k_cg_cluster, b, ncta, 1, ws.batch, ws.aux);   // clusters of one CTA
     }
+    // the coarse sample values and the depth-D terms wait for every depth's solution
+    if (e == cudaSuccess && loop_units > 0) e = cudaStreamWaitEvent(ws.aux, ws.ev_join4, 0);
     if (e != cudaSuccess) return e;
-    auto set_stencils = [&](CgcArgs& q) {
-        for (int u = 0; u < 3; ++u)
-            for (int k = 0; k < 27; ++k)
-                q.stp[u][k] = (q.first - u >= 0) ? ws.stencil_host[(q.first - u) * 27 + k] : 0.0f;
-    };
     if (ncl > 1) {
         CgcArgs b = a;
         b.first = D - 1;
-        set_stencils(b);
         e = launch_cg(k_cg_cluster, b, (ncl - 1) * cl2, cl2, ws.batch, ws.aux3);
         if (e == cudaSuccess) e = cudaEventRecord(ws.ev_join3, ws.aux3);
         if (e != cudaSuccess) return e;
@@ -1301,7 +1598,6 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     if (e != cudaSuccess) return e;
     if (ncl > 0) {
         a.first = D;
-        set_stencils(a);
         e = launch_cg(k_cg_cluster, a, cl1, cl1, ws.batch, s);
         if (e != cudaSuccess) return e;
     }

@@ -94,7 +94,6 @@ struct Workspace {
     int res;
     float* dff;             // d/dx F_i . F_j rounded to float (index i + res * j)
     float* stencil;         // [D+1][27] Laplacian coefficients (0 where dropped)
-    float stencil_host[(kMaxDepth + 1) * 27];   // the same on the host
 
     // field / solve
     float* vfield;          // 3 x dnodes (SoA: x block, y block, z block)
@@ -104,6 +103,7 @@ struct Workspace {
     unsigned ev_flags = 0;         // flags of the stage-timing event records (external in a capture)
     float *cg_r, *cg_p, *cg_q, *cg_ap;   // residual, two direction buffers, A p
     int* cg_blk;            // CG block table: 64 same-depth nodes per sibling group
+    unsigned* cg_desc;      // [14][cap.nodes / 8 + 8]: packed neighbour groups (solver.cu)
     CgLoopState* cg_loop;   // [D+1]: device-loop CG state per depth
     double* cg_loop_part;   // [D+1][kLoopMaxBlocks]: its per-block partial sums
     unsigned* cg_loop_ctl;  // loop control of a launch (passes, listed units; cloud 0's copy)
