@@ -239,7 +239,7 @@ psr_status psr_debug_array(psr_handle* h, const char* name, void* dst, size_t ds
  * Morton code at `depth` (1..9) and stably sorts by it.  `xyz` (3 * count floats),
  * `codes` and `order` (count uint32 each: sorted codes, original index of each sorted
  * point) are device pointers owned by the caller.  All scratch lives in a fixed
- * file-scope device array (about 9 MB, on every device that loads the library, until
+ * file-scope device array (about 11 MB, on every device that loads the library, until
  * exit), so at most 1,048,576 points per call (PSR_OUT_OF_CAPACITY above that).  Calls
  * share that array: calls whose GPU work overlaps race.  The first call on a device
  * looks up the array's address with that device current.  Every call synchronises

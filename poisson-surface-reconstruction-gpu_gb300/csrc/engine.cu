@@ -47,7 +47,7 @@ struct GraphEntry {
 struct psr_handle {
     psr_config cfg;
     Workspace ws;
-    int* h_params = nullptr;   // pinned: written by the host, copied to ws.d_params per call
+    InputRef* h_params = nullptr;   // pinned, one per slot: written by the host, copied to ws.d_params per call
     std::map<long long, GraphEntry> graphs;
     int use_graphs = 1;
     int last_kernels = 0;
@@ -303,7 +303,8 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.cnt, 1);
     A.add(ws.scan.words, (size_t)cap.scan_tiles + kScanHeader);
     A.add(ws.scan_aux.words, (size_t)cap.scan_tiles + kScanHeader);
-    A.add(ws.sort.hist, (size_t)kRadix * sort_tiles + 16);
+    A.add(ws.sort.bins, (size_t)kSortBinWords);
+    A.add(ws.sort.status, (size_t)kSortMaxPasses * kRadix * sort_tiles);
     A.add(ws.sort.keys_alt, (size_t)N);
     A.add(ws.sort.vals_alt, (size_t)N);
     A.add(ws.in_xyz, 3 * (size_t)N);
@@ -319,7 +320,6 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.ucode, (size_t)N);
     A.add(ws.ufirst, (size_t)N + 1);
     A.add(ws.uslot, (size_t)N);
-    A.add(ws.uaddr, (size_t)N);
     A.add(ws.tkey, (size_t)nodes); A.add(ws.tpidx, (size_t)nodes); A.add(ws.tpnum, (size_t)nodes);
     A.add(ws.tdidx, (size_t)nodes); A.add(ws.tdnum, (size_t)nodes); A.add(ws.tchild, (size_t)nodes);
     A.add(ws.tparent_slot, (size_t)nodes / 8 + 8);
@@ -415,7 +415,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.mb.parts, 4 * (size_t)nodes + 8);
     A.add(ws.mb.kept_prefix, (size_t)ws.part_cap_v);
     A.add(ws.mb.misc, 16);
-    A.add(ws.d_params, 16);
+    A.add(ws.d_params, 1);
 
     if (cfg.batch_clouds > kMaxBatchClouds || cfg.cg_cluster_ctas < 0 || cfg.cg_cluster_ctas > 16 ||
         cfg.cg_cluster_ctas_fine < 0 || cfg.cg_cluster_ctas_fine > 16) {
@@ -445,10 +445,9 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     // the device-loop CG's block tickets start at zero; each reduction leaves them at zero
     if (e == cudaSuccess) e = cudaMemset(ws.cg_loop, 0, sizeof(CgLoopState) * (kMaxDepth + 1));
     ws.sort.max_tiles = sort_tiles;
-    ws.sort.scan = ws.scan;   // sort shares the scan scratch (scans are sequential on one stream)
     e = cudaMallocHost(&h->cnt_host_all, sizeof(Counters) * (size_t)h->clouds);
     ws.cnt_host = h->cnt_host_all;
-    if (e == cudaSuccess) e = cudaMallocHost(&h->h_params, 16 * sizeof(int) * (size_t)h->clouds);
+    if (e == cudaSuccess) e = cudaMallocHost(&h->h_params, sizeof(InputRef) * (size_t)h->clouds);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking);
     for (int i = 0; i < 7 && e == cudaSuccess; ++i) e = cudaEventCreate(&h->ev[i]);
     h->ws.ev_cg = h->ev[6];
@@ -613,15 +612,13 @@ static cudaError_t issue_pipeline(psr_handle* h, cudaStream_t qs, int cg_iters, 
 // Launches the pipeline for `clouds` clouds (slots 0 .. clouds - 1) on `s`: captured once
 // per (clouds, depth, options) into a CUDA graph, replayed afterwards.
 static cudaError_t launch_pipeline(psr_handle* h, int depth, int cg_iters, int want_colour, int want_normals,
-                                   bool has_rgb, int clouds, cudaStream_t s) {
+                                   int clouds, cudaStream_t s) {
     Workspace& ws = h->ws;
     ws.depth = depth;
-    uint8_t* saved_rgb = ws.in_rgb;
-    if (!has_rgb) ws.in_rgb = nullptr;
     set_batch(ws, clouds);
     cudaError_t e = cudaSuccess;
     const long long gkey = ((long long)clouds << 44) | ((long long)depth << 40) | ((long long)cg_iters << 8) |
-                           (want_colour << 2) | (want_normals << 1) | (has_rgb ? 1 : 0);
+                           (want_colour << 2) | (want_normals << 1);
     h->last_graph = 0;
     if (h->use_graphs) {
         auto it = h->graphs.find(gkey);
@@ -665,24 +662,42 @@ static cudaError_t launch_pipeline(psr_handle* h, int depth, int cg_iters, int w
         h->last_kernels = -1;
     }
     set_batch(ws, 1);
-    ws.in_rgb = saved_rgb;
     ws.stream = s;
     return e;
 }
 
-// Copies the inputs of one cloud into slot k and enqueues its point count.
+// Whether the kernels may read the caller's array in place: memory of the handle's device (or
+// managed).  Anything else is staged by a copy, which reports what it cannot read.
+static bool readable_in_place(const psr_handle* h, const void* p) {
+    if (!p) return true;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == h->cfg.device;
+}
+
+// Enqueues the input reference of slot k: the caller's device arrays themselves (the sort reads
+// them once and gathers from them once, so a copy would only add traffic and three launches), or
+// copies of host arrays in the slot's staging buffers.
 static cudaError_t stage_inputs(psr_handle* h, const psr_points* pts, int k, cudaStream_t s) {
     Workspace& ws = h->ws;
     const int n = pts->count;
-    const cudaMemcpyKind kind = (pts->location == PSR_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    cudaError_t e = cudaMemcpyAsync(slot_ptr(ws.in_xyz, k), pts->xyz, 3 * sizeof(float) * (size_t)n, kind, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(slot_ptr(ws.in_nrm, k), pts->normals, 3 * sizeof(float) * (size_t)n, kind, s);
-    if (e == cudaSuccess && pts->rgb) e = cudaMemcpyAsync(slot_ptr(ws.in_rgb, k), pts->rgb, 3 * (size_t)n, kind, s);
-    if (e == cudaSuccess) {
-        int* hp = h->h_params + 16 * k;
-        hp[0] = n;
-        e = cudaMemcpyAsync(slot_ptr(ws.d_params, k), hp, sizeof(int), cudaMemcpyHostToDevice, s);
+    InputRef* hp = h->h_params + k;
+    cudaError_t e = cudaSuccess;
+    if (pts->location == PSR_DEVICE && readable_in_place(h, pts->xyz) && readable_in_place(h, pts->normals) &&
+        readable_in_place(h, pts->rgb)) {
+        *hp = InputRef{pts->xyz, pts->normals, pts->rgb, n};
+    } else {
+        const cudaMemcpyKind kind = (pts->location == PSR_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        *hp = InputRef{slot_ptr(ws.in_xyz, k), slot_ptr(ws.in_nrm, k), pts->rgb ? slot_ptr(ws.in_rgb, k) : nullptr, n};
+        e = cudaMemcpyAsync((void*)hp->xyz, pts->xyz, 3 * sizeof(float) * (size_t)n, kind, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync((void*)hp->nrm, pts->normals, 3 * sizeof(float) * (size_t)n, kind, s);
+        if (e == cudaSuccess && pts->rgb) e = cudaMemcpyAsync((void*)hp->rgb, pts->rgb, 3 * (size_t)n, kind, s);
     }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(slot_ptr(ws.d_params, k), hp, sizeof(InputRef), cudaMemcpyHostToDevice, s);
     return e;
 }
 
@@ -764,7 +779,7 @@ static psr_status submit_clouds(psr_handle* h, const psr_points* pts, int count,
     if (e != cudaSuccess) return cuda_fail(h, e, "cudaSetDevice");
     for (int k = 0; k < count && e == cudaSuccess; ++k) e = stage_inputs(h, pts + k, k, s);
     if (e != cudaSuccess) return cuda_fail(h, e, "input copy");
-    e = launch_pipeline(h, depth, cg_iters, want_colour, want_normals, has_rgb, count, s);
+    e = launch_pipeline(h, depth, cg_iters, want_colour, want_normals, count, s);
     h->pend_emitted.assign(count, 0);
     for (int k = 0; k < count && e == cudaSuccess; ++k) {
         bool em = false;

@@ -30,11 +30,11 @@ namespace psr {
 
 constexpr int kNoAllocMaxPoints = 1 << 20;
 constexpr int kNoAllocSortTiles = (kNoAllocMaxPoints + kSortTile - 1) / kSortTile + 1;
-constexpr int kNoAllocScanTiles = (kRadix * kNoAllocSortTiles + kScanTile - 1) / kScanTile + 2;
 
 struct NoAllocState {
     int n;
     unsigned error;
+    unsigned ticket;      // blocks of the encoder done
     int bmax[3], bmin[3];
     float center[3];
     float edge;
@@ -44,17 +44,18 @@ struct NoAllocState {
 constexpr size_t kNaState = 0;
 constexpr size_t kNaKeys = 256;
 constexpr size_t kNaVals = kNaKeys + 4ull * kNoAllocMaxPoints;
-constexpr size_t kNaHist = kNaVals + 4ull * kNoAllocMaxPoints;
-constexpr size_t kNaHistBytes = ((4ull * ((size_t)kRadix * kNoAllocSortTiles + 16)) + 255) & ~255ull;
-constexpr size_t kNaScan = kNaHist + kNaHistBytes;
-constexpr size_t kNaBytes = kNaScan + 8ull * (kNoAllocScanTiles + kScanHeader);
+constexpr size_t kNaBins = kNaVals + 4ull * kNoAllocMaxPoints;
+constexpr size_t kNaStatus = kNaBins + ((4ull * kSortBinWords + 255) & ~255ull);
+constexpr size_t kNaBytes = kNaStatus + 4ull * kSortMaxPasses * kRadix * kNoAllocSortTiles;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaBytes];
 
-__global__ void k_na_init(NoAllocState* st, int n) {
+__global__ void k_na_init(NoAllocState* st, int n, unsigned* sort_bins) {
+    for (int i = threadIdx.x; i < kSortBinWords; i += blockDim.x) sort_bins[i] = 0u;
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         st->n = n;
         st->error = 0;
+        st->ticket = 0u;
         for (int a = 0; a < 3; ++a) {
             // seeded like the pipeline's reduction (-FLT_MAX / FLT_MAX), so the two agree
             // for coordinates of any magnitude
@@ -105,8 +106,11 @@ __global__ void k_na_finalize(NoAllocState* st, float scale) {
     if (!(edge > 0.0f)) atomicOr(&st->error, kErrInvalid);
 }
 
-__global__ void __launch_bounds__(kBlock) k_na_encode(const float* xyz, const NoAllocState* st, int depth,
-                                                      unsigned* code, unsigned* order) {
+__global__ void __launch_bounds__(kBlock) k_na_encode(const float* xyz, NoAllocState* st, int depth, unsigned* code,
+                                                      SortScratch sc, int passes) {
+    __shared__ unsigned s_h[kSortMaxPasses][kRadix];
+    const SortCounter count{s_h, passes};
+    count.clear();
     const int n = st->n;
     const float e = st->edge;
     PSR_GRID_STRIDE(i, n) {
@@ -125,8 +129,9 @@ __global__ void __launch_bounds__(kBlock) k_na_encode(const float* xyz, const No
             w = __fdiv_rn(w, 2.0f);
         }
         code[i] = k;
-        order[i] = (unsigned)i;
+        count.count(k);
     }
+    count.finish(sc, n, &st->ticket, &st->error);
 }
 
 namespace {
@@ -161,19 +166,18 @@ extern "C" psr_status psr_morton_sort_noalloc(const float* xyz, int count, int d
     cudaStream_t s = (cudaStream_t)stream;
     NoAllocState* st = (NoAllocState*)(base + kNaState);
     SortScratch sc;
-    sc.hist = (unsigned*)(base + kNaHist);
+    sc.bins = (unsigned*)(base + kNaBins);
+    sc.status = (unsigned*)(base + kNaStatus);
     sc.keys_alt = (unsigned*)(base + kNaKeys);
     sc.vals_alt = (unsigned*)(base + kNaVals);
     sc.max_tiles = kNoAllocSortTiles;
-    sc.scan.words = (unsigned long long*)(base + kNaScan);
-    sc.scan.max_tiles = kNoAllocScanTiles;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = (sms > 0 ? sms : 148) * 4;
-    k_na_init<<<1, 1, 0, s>>>(st, count);
+    k_na_init<<<1, 256, 0, s>>>(st, count, sc.bins);
     k_na_bbox<<<grid, kBlock, 0, s>>>(xyz, st);
     k_na_finalize<<<1, 1, 0, s>>>(st, bbox_scale);
-    k_na_encode<<<grid, kBlock, 0, s>>>(xyz, st, depth, codes, order);
+    k_na_encode<<<grid, kBlock, 0, s>>>(xyz, st, depth, codes, sc, sort_passes(3 * depth));
     bool alt = false;
     cudaError_t e = radix_sort_pairs(codes, order, &st->n, 3 * depth, sc, &st->error, s, &alt);
     if (e == cudaSuccess && alt) {

@@ -86,8 +86,11 @@ __device__ __forceinline__ void nrm_visit(float qx, float qy, float qz, const fl
     nrm_insert<kNrmK>(bd, bi, d2, i);
 }
 
-__global__ void k_nrm_reset(Counters* c, int n) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void k_nrm_reset(Counters* c, InputRef* in, unsigned* sort_bins, const float* xyz, int n) {
+    for (int i = threadIdx.x; i < kSortBinWords; i += blockDim.x) sort_bins[i] = 0u;
+    if (threadIdx.x != 0) return;
+    *in = InputRef{xyz, xyz, nullptr, n};
+    c->ticket[0] = c->ticket[1] = 0u;
     c->n_points = n;
     c->error = 0u;
     c->n_colour_far = 0;
@@ -424,8 +427,7 @@ __global__ void __launch_bounds__(kBlock) k_nrm_pca(const Counters* c, const flo
     }
 }
 
-cudaError_t encode_sort_points(Workspace& ws, const float* xyz, int depth, const unsigned** scode,
-                               const unsigned** sidx);
+cudaError_t encode_sort_points(Workspace& ws, int depth, const unsigned** scode, const unsigned** sidx);
 
 // normals of the n points at xyz (device, 3 floats each) into out (device), on ws.stream;
 // uses the workspace's point, node-neighbour and colour scratch (no reconstruction runs
@@ -433,9 +435,9 @@ cudaError_t encode_sort_points(Workspace& ws, const float* xyz, int depth, const
 cudaError_t normals_build(Workspace& ws, const float* xyz, int n, float* out, float vpx, float vpy, float vpz) {
     cudaStream_t s = ws.stream;
     Counters* c = ws.cnt;
-    k_nrm_reset<<<1, 1, 0, s>>>(c, n);
+    k_nrm_reset<<<1, 256, 0, s>>>(c, ws.d_params, ws.sort.bins, xyz, n);
     const unsigned *scode = nullptr, *sidx = nullptr;
-    cudaError_t e = encode_sort_points(ws, xyz, kNrmGridLevel, &scode, &sidx);
+    cudaError_t e = encode_sort_points(ws, kNrmGridLevel, &scode, &sidx);
     if (e != cudaSuccess) return e;
     const int gp = grid_for(ws, n);
     k_nrm_gather<<<gp, kBlock, 0, s>>>(c, xyz, sidx, ws.px, ws.py, ws.pz);

@@ -13,14 +13,16 @@ namespace psr {
 // ------------------------------------------------------------------------------------
 // bounding box (mesh/BuildOctree.cu:51-133) and normalisation parameters (:619-631)
 // ------------------------------------------------------------------------------------
-__global__ void k_reset_counters(Counters* c, const int* params) {
-    PSR_CLOUD(c, params);
+// the counters of a call, and the sort's
+__global__ void k_reset_counters(Counters* c, const InputRef* in, unsigned* sort_bins) {
+    PSR_CLOUD(c, in, sort_bins);
     static_assert(sizeof(Counters) % 4 == 0, "Counters is cleared word by word");
     unsigned* w = (unsigned*)c;
     for (int i = threadIdx.x; i < (int)(sizeof(Counters) / 4); i += blockDim.x) w[i] = 0u;
+    for (int i = threadIdx.x; i < kSortBinWords; i += blockDim.x) sort_bins[i] = 0u;
     __syncthreads();
     if (threadIdx.x == 0) {
-        c->n_points = params[0];
+        c->n_points = in->n;
         for (int a = 0; a < 3; ++a) {
             // The reference seeds its reduction (padding threads, mesh/BuildOctree.cu:66-73)
             // and its host finish (mesh/BuildOctree.cpp:87-88) with -1e6 / 1e6, which gives a
@@ -33,8 +35,12 @@ __global__ void k_reset_counters(Counters* c, const int* params) {
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_bbox(const float* xyz, const float* nrm, Counters* c) {
-    PSR_CLOUD(xyz, nrm, c);
+// Bounding box; the last block to finish sets the normalisation parameters (a launch of one
+// thread of their own would cost as much as the box).
+__global__ void __launch_bounds__(kBlock) k_bbox(const InputRef* in, Counters* c, float scale) {
+    PSR_CLOUD(in, c);
+    const float* xyz = in->xyz;
+    const float* nrm = in->nrm;
     const int n = c->n_points;
     float mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
     bool bad = false;
@@ -56,6 +62,7 @@ __global__ void __launch_bounds__(kBlock) k_bbox(const float* xyz, const float* 
     if (__any_sync(0xffffffffu, bad) && lane_id() == 0) atomicOr(&c->error, kErrInvalid);
     // block reduction, then one set of atomics per block
     __shared__ float s_mx[3][kBlock / 32], s_mn[3][kBlock / 32];
+    __shared__ int s_last;
     const int w = threadIdx.x >> 5;
     if (lane_id() == 0)
         for (int a = 0; a < 3; ++a) { s_mx[a][w] = mx[a]; s_mn[a][w] = mn[a]; }
@@ -66,25 +73,26 @@ __global__ void __launch_bounds__(kBlock) k_bbox(const float* xyz, const float* 
         for (int q = 1; q < kBlock / 32; ++q) { bmx = fmaxf(bmx, s_mx[a][q]); bmn = fminf(bmn, s_mn[a][q]); }
         atomicMax(&((int*)c->bbox_max)[a], float_to_ordered(bmx));
         atomicMin(&((int*)c->bbox_min)[a], float_to_ordered(bmn));
+        __threadfence();
     }
-}
-
-__global__ void k_bbox_finalize(Counters* c, float scale) {
-    PSR_CLOUD(c);
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    float mx[3], mn[3];
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&c->ticket[0], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last || threadIdx.x != 0) return;
+    __threadfence();
+    float bx[3], bn[3];
     for (int a = 0; a < 3; ++a) {
-        mx[a] = ordered_to_float(((int*)c->bbox_max)[a]);
-        mn[a] = ordered_to_float(((int*)c->bbox_min)[a]);
-        c->bbox_max[a] = mx[a];
-        c->bbox_min[a] = mn[a];
+        bx[a] = ordered_to_float(__ldcg(&((int*)c->bbox_max)[a]));
+        bn[a] = ordered_to_float(__ldcg(&((int*)c->bbox_min)[a]));
+        c->bbox_max[a] = bx[a];
+        c->bbox_min[a] = bn[a];
     }
     float edge = 1.0f;
     float ctr[3];
     for (int a = 0; a < 3; ++a) {
-        float ext = __fsub_rn(mx[a], mn[a]);
+        float ext = __fsub_rn(bx[a], bn[a]);
         if (a == 0 || edge < ext) edge = ext;
-        ctr[a] = __fdiv_rn(__fadd_rn(mx[a], mn[a]), 2.0f);
+        ctr[a] = __fdiv_rn(__fadd_rn(bx[a], bn[a]), 2.0f);
     }
     edge = __fmul_rn(edge, __fmul_rn(scale, 1.0f));
     for (int a = 0; a < 3; ++a) ctr[a] = __fsub_rn(ctr[a], __fdiv_rn(edge, 2.0f));
@@ -99,10 +107,14 @@ __device__ __forceinline__ float normalise_coord(float v, float ctr, float edge)
 }
 
 // Morton code of a normalised point (mesh/BuildOctree.cu:167-208); bit 3l+2 = x of level
-// D-l, so the code equals the reference key's upper 32 bits.
-__global__ void __launch_bounds__(kBlock) k_encode(const float* xyz, const Counters* c, int depth,
-                                                   unsigned* code, unsigned* sidx) {
-    PSR_CLOUD(xyz, c, code, sidx);
+// D-l, so the code equals the reference key's upper 32 bits.  Counts the sort's digits.
+__global__ void __launch_bounds__(kBlock) k_encode(const InputRef* in, Counters* c, int depth, unsigned* code,
+                                                   SortScratch sc, int passes) {
+    PSR_CLOUD(in, c, code, sc);
+    __shared__ unsigned s_h[kSortMaxPasses][kRadix];
+    const SortCounter count{s_h, passes};
+    count.clear();
+    const float* xyz = in->xyz;
     const int n = c->n_points;
     const float c0 = c->center[0], c1 = c->center[1], c2 = c->center[2], e = c->max_edge;
     PSR_GRID_STRIDE(i, n) {
@@ -120,21 +132,27 @@ __global__ void __launch_bounds__(kBlock) k_encode(const float* xyz, const Count
             w = __fdiv_rn(w, 2.0f);
         }
         code[i] = k;
-        sidx[i] = (unsigned)i;
+        count.count(k);
     }
+    count.finish(sc, n, &c->ticket[1], &c->error);
 }
 
-// Gather the sorted points, scale the normals to 2^(D+1) (mesh/BuildOctree.cu:152-164)
-// and flag the first point of every unique leaf.
-__global__ void __launch_bounds__(kBlock) k_gather(const float* xyz, const float* nrm, const uint8_t* rgb,
-                                                   const unsigned* scode, const unsigned* sidx, const Counters* c,
-                                                   int depth, float* px, float* py, float* pz, float* nx, float* ny,
-                                                   float* nz, float* cr, float* cg, float* cb, unsigned* head) {
-    PSR_CLOUD(xyz, nrm, rgb, scode, sidx, c, px, py, pz, nx, ny, nz, cr, cg, cb, head);
-    const int n = c->n_points;
-    const float c0 = c->center[0], c1 = c->center[1], c2 = c->center[2], e = c->max_edge;
-    const float nscale = (float)(2 << depth);
-    PSR_GRID_STRIDE(i, n) {
+// Gathers the sorted points, scales the normals to 2^(D+1) (mesh/BuildOctree.cu:152-164) and
+// flags the first point of every unique leaf; the scan over the flags gives point -> unique leaf
+// id and unique leaf -> code, first point.
+struct GatherLoad {
+    const InputRef* in;
+    const unsigned* scode;
+    const unsigned* sidx;
+    const Counters* c;
+    int depth;
+    float *px, *py, *pz, *nx, *ny, *nz, *cr, *cg, *cb;
+    __device__ unsigned operator()(int i) const {
+        const float* xyz = in->xyz;
+        const float* nrm = in->nrm;
+        const uint8_t* rgb = in->rgb;
+        const float c0 = c->center[0], c1 = c->center[1], c2 = c->center[2], e = c->max_edge;
+        const float nscale = (float)(2 << depth);
         const size_t o = sidx[i];
         px[i] = normalise_coord(xyz[3 * o], c0, e);
         py[i] = normalise_coord(xyz[3 * o + 1], c1, e);
@@ -154,13 +172,13 @@ __global__ void __launch_bounds__(kBlock) k_gather(const float* xyz, const float
         } else {
             cr[i] = cg[i] = cb[i] = 0.0f;
         }
-        head[i] = (i == 0 || scode[i] != scode[i - 1]) ? 1u : 0u;
+        return (i == 0 || scode[i] != scode[i - 1]) ? 1u : 0u;
     }
-}
-
-// scan over leaf heads: point -> unique leaf id, unique leaf -> code / first point
+    __device__ void rebase() { PSR_CLOUD(in, scode, sidx, c, px, py, pz, nx, ny, nz, cr, cg, cb); }   // to cloud blockIdx.y
+};
 struct HeadStore {
     const unsigned* scode;
+    Counters* c;
     int* puid;
     unsigned* ucode;
     int* ufirst;
@@ -169,16 +187,26 @@ struct HeadStore {
         puid[i] = u;
         if (v) { ucode[u] = scode[i]; ufirst[u] = i; }
     }
-    __device__ void rebase() { PSR_CLOUD(scode, puid, ucode, ufirst); }   // to cloud blockIdx.y
+    __device__ void done(unsigned total) const {
+        c->n_unique = (int)total;
+        ufirst[total] = c->n_points;
+    }
+    __device__ void rebase() { PSR_CLOUD(scode, c, puid, ucode, ufirst); }   // to cloud blockIdx.y
 };
 
-__global__ void k_after_unique(Counters* c, int* ufirst, const unsigned* total) {
-    PSR_CLOUD(c, ufirst, total);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        c->n_unique = (int)*total;
-        ufirst[c->n_unique] = c->n_points;
+// Level staging arrays: one record per slot of a level being built.
+struct LevelArrays {
+    int *key, *pidx, *pnum, *didx, *dnum, *child;
+    __device__ void put(int t, int k, int pi, int pn, int di, int dn, int ch) const {
+        key[t] = k;
+        pidx[t] = pi;
+        pnum[t] = pn;
+        didx[t] = di;
+        dnum[t] = dn;
+        child[t] = ch;
     }
-}
+    __device__ void rebase() { PSR_CLOUD(key, pidx, pnum, didx, dnum, child); }   // to cloud blockIdx.y
+};
 
 // D-level groups: 8 slots for every new parent code (mesh/BuildOctree.cu:267-280)
 struct LeafGroupLoad {
@@ -188,79 +216,77 @@ struct LeafGroupLoad {
     }
     __device__ void rebase() { PSR_CLOUD(ucode); }   // to cloud blockIdx.y
 };
-
-__global__ void k_after_leaf_groups(Counters* c, const unsigned* total, int depth, int node_cap) {
-    PSR_CLOUD(c, total);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int md = (int)*total + 8;
+// Places every unique leaf in its group's slot (:282-292), with the empty slots up to the next
+// leaf's (each slot is written once; D level: dnum = 1, didx = slot, :294-300).
+struct LeafPlaceStore {
+    const unsigned* ucode;
+    const int* ufirst;
+    Counters* c;
+    int depth, cap;
+    int* uslot;
+    LevelArrays T;
+    unsigned* err;
+    __device__ void operator()(int u, unsigned pre, unsigned v) const {
+        const int n = c->n_unique;
+        const unsigned code = ucode[u];
+        const int addr = (int)(pre + v), s = addr + (int)(code & 7u);
+        uslot[u] = s;
+        int end = addr + 8;   // first slot past the empty ones behind this leaf
+        if (u + 1 < n) {
+            const unsigned nc = ucode[u + 1];
+            end = addr + (((nc >> 3) != (code >> 3)) ? 8 : 0) + (int)(nc & 7u);
+        }
+        if (end > cap) end = cap;   // capacity overflow (flagged by done())
+        if (u == 0)
+            for (int q = 0; q < s; ++q) T.put(q, 0, 0, 0, q, 1, -1);
+        if (s < cap) T.put(s, (int)code, ufirst[u], ufirst[u + 1] - ufirst[u], s, 1, -1);
+        for (int q = s + 1; q < end; ++q) T.put(q, 0, 0, 0, q, 1, -1);
+    }
+    __device__ void done(unsigned total) const {
+        int md = (int)total + 8;
         if (c->n_unique == 0) md = 0;
         c->level_tmp_off[depth] = 0;
-        if (md > node_cap) { atomicOr(&c->error, kErrCapacity); md = 0; }
+        if (md > cap) { atomicOr(err, kErrCapacity); md = 0; }
         c->level_count[depth] = md;
-        c->n_groups = md;   // bound for the leaf placement
+        c->level_groups[depth] = md / 8;
     }
-}
+    __device__ void rebase() { PSR_CLOUD(ucode, ufirst, c, uslot, T, err); }   // to cloud blockIdx.y
+};
 
-// level initialisation: D level gets dnum = 1, didx = slot (:294-300), others zero
-__global__ void __launch_bounds__(kBlock) k_init_level(const Counters* c, int d, int depth, int* tkey, int* tpidx,
-                                                       int* tpnum, int* tdidx, int* tdnum, int* tchild) {
-    PSR_CLOUD(c, tkey, tpidx, tpnum, tdidx, tdnum, tchild);
-    const int m = c->level_count[d];
-    const int off = c->level_tmp_off[d];
-    PSR_GRID_STRIDE(i, m) {
-        tkey[off + i] = 0;
-        tpidx[off + i] = 0;
-        tpnum[off + i] = 0;
-        tdidx[off + i] = (d == depth) ? i : 0;
-        tdnum[off + i] = (d == depth) ? 1 : 0;
-        tchild[off + i] = -1;
-    }
+// One level of the build: the sibling groups of level d aggregate into their fathers
+// (mesh/BuildOctree.cu:323-357), a scan over the groups that start a new father group gives the
+// father groups' addresses one level up (:359-375, :796-799), and every father goes to its slot
+// with the empty slots up to the next father's (:377-390).
+// first non-empty slot of group g's 8 (the father's key is its key without the sibling bits)
+__device__ __forceinline__ int group_father_key(const LevelArrays& T, int base, int sh) {
+    int pn[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) pn[j] = T.pnum[base + j];
+    int at = -1;
+#pragma unroll
+    for (int j = 7; j >= 0; --j)
+        if (pn[j] != 0) at = j;
+    return at < 0 ? 0 : T.key[base + at] & ~(7 << sh);
 }
-
-// place unique leaves in their groups (:282-292) and map points to leaves (:302-313)
-__global__ void __launch_bounds__(kBlock) k_place_leaves(const Counters* c, const unsigned* ucode, const int* ufirst,
-                                                         const unsigned* uaddr, int* uslot, int* tkey, int* tpidx,
-                                                         int* tpnum) {
-    PSR_CLOUD(c, ucode, ufirst, uaddr, uslot, tkey, tpidx, tpnum);
-    const int u_n = c->n_unique;
-    PSR_GRID_STRIDE(u, u_n) {
-        int s = (int)uaddr[u] + (int)(ucode[u] & 7u);
-        uslot[u] = s;
-        if (s >= c->n_groups) continue;   // capacity overflow (flagged); n_groups holds M_D here
-        tkey[s] = (int)ucode[u];
-        tpidx[s] = ufirst[u];
-        tpnum[s] = ufirst[u + 1] - ufirst[u];
-    }
-}
-__global__ void __launch_bounds__(kBlock) k_point2node(const Counters* c, const int* puid, const int* uslot,
-                                                       int* point2node) {
-    PSR_CLOUD(c, puid, uslot, point2node);
-    const int n = c->n_points;
-    PSR_GRID_STRIDE(i, n) point2node[i] = uslot[puid[i]];
-}
-
-// per-group aggregation into the father (mesh/BuildOctree.cu:323-357)
-__global__ void __launch_bounds__(kBlock) k_group_aggregate(Counters* c, int d, int depth, const int* tkey,
-                                                            const int* tpidx, const int* tpnum, const int* tdidx,
-                                                            const int* tdnum, int* gkey, int* gpidx, int* gpnum,
-                                                            int* gdidx, int* gdnum) {
-    PSR_CLOUD(c, tkey, tpidx, tpnum, tdidx, tdnum, gkey, gpidx, gpnum, gdidx, gdnum);
-    const int m = c->level_count[d];
-    const int off = c->level_tmp_off[d];
-    const int G = m / 8;
-    if (blockIdx.x == 0 && threadIdx.x == 0) c->n_groups = G;
-    const int sh = 3 * (depth - d);
-    PSR_GRID_STRIDE(g, G) {
+struct LevelLoad {
+    const Counters* c;
+    int d, depth;
+    LevelArrays T;
+    int *gkey, *gpidx, *gpnum, *gdidx, *gdnum;
+    __device__ unsigned operator()(int g) const {
+        const int off = c->level_tmp_off[d];
+        const int sh = 3 * (depth - d), sh2 = 3 * (depth - d + 2);
         int fk = 0, pn = 0, pi = 0x7fffffff, dn = 0, di = 0x7fffffff;
+#pragma unroll
         for (int j = 0; j < 8; ++j) {
-            int t = off + 8 * g + j;
-            int pnum = tpnum[t], dnum = tdnum[t], didx = tdidx[t];
+            const int t = off + 8 * g + j;
+            const int pnum = T.pnum[t], dnum = T.dnum[t], didx = T.didx[t], key = T.key[t], pidx = T.pidx[t];
             if (pnum == 0) {
                 if (dnum != 0) { dn += dnum; di = min(di, didx); }
             } else {
-                fk = tkey[t] & ~(7 << sh);
+                fk = key & ~(7 << sh);
                 pn += pnum;
-                pi = min(pi, tpidx[t]);
+                pi = min(pi, pidx);
                 dn += dnum;
                 di = min(di, didx);
             }
@@ -270,54 +296,46 @@ __global__ void __launch_bounds__(kBlock) k_group_aggregate(Counters* c, int d, 
         gpnum[g] = pn;
         gdidx[g] = di;
         gdnum[g] = dn;
+        if (g == 0) return 0u;
+        return ((group_father_key(T, off + 8 * (g - 1), sh) >> sh2) != (fk >> sh2)) ? 8u : 0u;
     }
-}
-
-// father groups one level up (mesh/BuildOctree.cu:359-375, scan :796-799)
-struct FatherGroupLoad {
-    const int* gkey;
-    int sh2;
-    __device__ unsigned operator()(int g) const {
-        return (g == 0) ? 0u : (((gkey[g - 1] >> sh2) != (gkey[g] >> sh2)) ? 8u : 0u);
-    }
-    __device__ void rebase() { PSR_CLOUD(gkey); }   // to cloud blockIdx.y
+    __device__ void rebase() { PSR_CLOUD(c, T, gkey, gpidx, gpnum, gdidx, gdnum); }   // to cloud blockIdx.y
 };
-
-__global__ void k_after_father_groups(Counters* c, int d, const unsigned* total, int node_cap) {
-    PSR_CLOUD(c, total);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int m = (d > 1) ? (int)*total + 8 : 1;
-        int off = c->level_tmp_off[d] + c->level_count[d];
-        c->level_count[d - 1] = m;
+struct LevelStore {
+    Counters* c;
+    int d, depth, cap;
+    LevelArrays T;
+    const int *gkey, *gpidx, *gpnum, *gdidx, *gdnum;   // group g's entries: written by the same thread's load
+    int* tparent_slot;
+    unsigned* err;
+    __device__ void operator()(int g, unsigned pre, unsigned v) const {
+        const int off = c->level_tmp_off[d], m = c->level_count[d];
+        const int sh = 3 * (depth - d), sh2 = 3 * (depth - d + 2), sh3 = 3 * (depth - d + 1);
+        const int off1 = off + m;   // first slot of level d - 1
+        const int fk = gkey[g];
+        const int addr = (int)(pre + v), s = addr + ((fk >> sh3) & 7);
+        int end = d > 1 ? addr + 8 : 1;
+        if (8 * (g + 1) < m) {
+            const int nk = group_father_key(T, off + 8 * (g + 1), sh);
+            end = addr + (((nk >> sh2) != (fk >> sh2)) ? 8 : 0) + ((nk >> sh3) & 7);
+        }
+        if (off1 + end > cap) end = cap - off1;   // capacity overflow (flagged by done())
+        if (g == 0)
+            for (int q = 0; q < s && off1 + q < cap; ++q) T.put(off1 + q, 0, 0, 0, 0, 0, -1);
+        if (off1 + s < cap) T.put(off1 + s, fk, gpidx[g], gpnum[g], gdidx[g], gdnum[g], 8 * g);
+        for (int q = s + 1; q < end; ++q) T.put(off1 + q, 0, 0, 0, 0, 0, -1);
+        tparent_slot[off / 8 + g] = s;
+    }
+    __device__ void done(unsigned total) const {
+        int m = (d > 1) ? (int)total + 8 : 1;
+        const int off = c->level_tmp_off[d] + c->level_count[d];
         c->level_tmp_off[d - 1] = off;
-        if (off + m > node_cap) { atomicOr(&c->error, kErrCapacity); c->level_count[d - 1] = 0; }
+        if (off + m > cap) { atomicOr(err, kErrCapacity); m = 0; }
+        c->level_count[d - 1] = m;
+        c->level_groups[d - 1] = m / 8;
     }
-}
-
-// place fathers (mesh/BuildOctree.cu:377-390): record the father slot of every group
-__global__ void __launch_bounds__(kBlock) k_place_fathers(const Counters* c, int d, int depth, const int* gkey,
-                                                          const int* gpidx, const int* gpnum, const int* gdidx,
-                                                          const int* gdnum, const unsigned* gaddr, int* tkey,
-                                                          int* tpidx, int* tpnum, int* tdidx, int* tdnum, int* tchild,
-                                                          int* tparent_slot) {
-    PSR_CLOUD(c, gkey, gpidx, gpnum, gdidx, gdnum, gaddr, tkey, tpidx, tpnum, tdidx, tdnum, tchild, tparent_slot);
-    const int G = c->n_groups;
-    const int off_parent = c->level_tmp_off[d - 1];
-    const int off_group = c->level_tmp_off[d] / 8;
-    const int sh3 = 3 * (depth - d + 1);
-    PSR_GRID_STRIDE(g, G) {
-        int s = (int)gaddr[g] + ((gkey[g] >> sh3) & 7);
-        if (s >= c->level_count[d - 1]) continue;   // capacity overflow (flagged)
-        int t = off_parent + s;
-        tkey[t] = gkey[g];
-        tpidx[t] = gpidx[g];
-        tpnum[t] = gpnum[g];
-        tdidx[t] = gdidx[g];
-        tdnum[t] = gdnum[g];
-        tchild[t] = 8 * g;   // level-local address of the child group
-        tparent_slot[off_group + g] = s;
-    }
-}
+    __device__ void rebase() { PSR_CLOUD(c, T, gkey, gpidx, gpnum, gdidx, gdnum, tparent_slot, err); }   // to cloud blockIdx.y
+};
 
 // ---- coarse levels in one CTA --------------------------------------------------------
 // The levels near the root hold few nodes, so their per-level passes (group aggregate,
@@ -325,6 +343,7 @@ __global__ void __launch_bounds__(kBlock) k_place_fathers(const Counters* c, int
 // block barriers between steps instead of five launches per level.  Same arithmetic as
 // the per-level kernels above.
 constexpr int kLevelBlock = 1024;
+constexpr int kCoarseLevels = 4;   // levels up to this one: at most 4096 nodes, 4 rounds of the CTA
 
 // inclusive block scan of one value per thread (1024 threads); returns the block total
 __device__ __forceinline__ unsigned block_inclusive_scan_1024(unsigned v, unsigned* s_warp) {
@@ -351,6 +370,16 @@ __device__ __forceinline__ unsigned block_inclusive_scan_1024(unsigned v, unsign
     __syncthreads();
     s_warp[32] = total;
     return r;
+}
+
+// every level is counted: their places in the node arrays
+__device__ __forceinline__ void levels_done(Counters* c, int depth) {
+    int b = 0;
+    for (int d = 0; d <= depth; ++d) {
+        c->level_base[d] = b;
+        b += c->level_count[d];
+    }
+    c->n_nodes = b;
 }
 
 __global__ void __launch_bounds__(kLevelBlock) k_levels_block(Counters* c, int dtop, int depth, int* tkey, int* tpidx,
@@ -437,6 +466,7 @@ __global__ void __launch_bounds__(kLevelBlock) k_levels_block(Counters* c, int d
         }
         __syncthreads();
     }
+    if (t == 0) levels_done(c, depth);
 }
 
 // 27-neighbour tables of levels 1..dmax in one CTA (levels in order: a level reads its
@@ -465,24 +495,23 @@ __global__ void __launch_bounds__(kLevelBlock) k_neighbours_block(const Counters
 
 __global__ void k_levels_done(Counters* c, int depth) {
     PSR_CLOUD(c);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int b = 0;
-        for (int d = 0; d <= depth; ++d) {
-            c->level_base[d] = b;
-            b += c->level_count[d];
-        }
-        c->n_nodes = b;
-    }
+    if (threadIdx.x == 0 && blockIdx.x == 0) levels_done(c, depth);
 }
 
-// Final node records (mesh/BuildOctree.cu:392-488, :552-586, :514-550).
+// Final node records (mesh/BuildOctree.cu:392-488, :552-586, :514-550), the root's neighbour row
+// and the points' leaves (:302-313).
 __global__ void __launch_bounds__(kBlock) k_finalize_nodes(const Counters* c, int depth, const int* tkey,
                                                            const int* tpidx, const int* tpnum, const int* tdidx,
                                                            const int* tdnum, const int* tchild,
                                                            const int* tparent_slot, int* key, int* pidx, int* pnum,
                                                            int* parent, int* first_child, int* didx, int* dnum,
-                                                           int* ndepth, int* enc, float* cx, float* cy, float* cz) {
-    PSR_CLOUD(c, tkey, tpidx, tpnum, tdidx, tdnum, tchild, tparent_slot, key, pidx, pnum, parent, first_child, didx, dnum, ndepth, enc, cx, cy, cz);
+                                                           int* ndepth, int* enc, float* cx, float* cy, float* cz,
+                                                           int* neigh, size_t stride, const int* puid, const int* uslot,
+                                                           int* point2node) {
+    PSR_CLOUD(c, tkey, tpidx, tpnum, tdidx, tdnum, tchild, tparent_slot, key, pidx, pnum, parent, first_child, didx, dnum, ndepth, enc, cx, cy, cz, neigh, puid, uslot, point2node);
+    const int np = c->n_points;
+    PSR_GRID_STRIDE(i, np) point2node[i] = uslot[puid[i]];
+    if (blockIdx.x == 0 && threadIdx.x < 27) neigh[(size_t)threadIdx.x * stride] = (threadIdx.x == 13) ? 0 : -1;
     const int M = c->n_nodes;
     PSR_GRID_STRIDE(i, M) {
         int d = 0;
@@ -569,23 +598,16 @@ __global__ void __launch_bounds__(kBlock) k_neighbours(const Counters* c, int d,
     }
 }
 
-__global__ void k_root_neighbours(int* neigh, size_t stride) {
-    PSR_CLOUD(neigh);
-    int k = threadIdx.x;
-    if (k < 27) neigh[(size_t)k * stride] = (k == 13) ? 0 : -1;
-}
-
 // points -> Morton codes of the reference's normalised coordinates at `depth`, sorted with
 // their input indices (the octree's first steps; the normal estimation stage uses them on
-// their own).  n_points and the bounding-box seeds must be set.
-cudaError_t encode_sort_points(Workspace& ws, const float* xyz, int depth, const unsigned** scode,
-                               const unsigned** sidx) {
+// their own).  The input reference, n_points, the bounding-box seeds and the sort's bins must be
+// set.
+cudaError_t encode_sort_points(Workspace& ws, int depth, const unsigned** scode, const unsigned** sidx) {
     cudaStream_t s = ws.stream;
     Counters* c = ws.cnt;
     const int gp = grid_for(ws, ws.cap.points);
-    k_bbox<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(xyz, xyz, c);
-    k_bbox_finalize<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, 1.25f);
-    k_encode<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(xyz, c, depth, ws.code, ws.sidx);
+    k_bbox<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(ws.d_params, c, 1.25f);
+    k_encode<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(ws.d_params, c, depth, ws.code, ws.sort, sort_passes(3 * depth));
     bool alt = false;
     cudaError_t e = radix_sort_pairs(ws.code, ws.sidx, &c->n_points, 3 * depth, ws.sort, &c->error, s, &alt);
     if (e != cudaSuccess) return e;
@@ -600,58 +622,40 @@ cudaError_t octree_build(Workspace& ws) {
     Counters* c = ws.cnt;
     unsigned* err = &c->error;
     unsigned* total = (unsigned*)&c->scan_total;
-    const int gp = grid_for(ws, ws.cap.points);
-    k_reset_counters<<<PSR_GRID(ws, 1), 256, 0, s>>>(c, ws.d_params);
-    k_bbox<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(ws.in_xyz, ws.in_nrm, c);
-    k_bbox_finalize<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, 1.25f);
-    k_encode<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(ws.in_xyz, c, D, ws.code, ws.sidx);
-    bool alt = false;
-    cudaError_t e = radix_sort_pairs(ws.code, ws.sidx, &c->n_points, 3 * D, ws.sort, err, s, &alt);
+    k_reset_counters<<<PSR_GRID(ws, 1), 256, 0, s>>>(c, ws.d_params, ws.sort.bins);
+    const unsigned *scode = nullptr, *sidx = nullptr;
+    cudaError_t e = encode_sort_points(ws, D, &scode, &sidx);
     if (e != cudaSuccess) return e;
-    const unsigned* scode = alt ? ws.sort.keys_alt : ws.code;
-    const unsigned* sidx = alt ? ws.sort.vals_alt : ws.sidx;
-    unsigned* head = alt ? ws.code : ws.sort.keys_alt;   // free buffer of N words
-    k_gather<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(ws.in_xyz, ws.in_nrm, ws.in_rgb, scode, sidx, c, D, ws.px, ws.py, ws.pz, ws.nx,
-                                   ws.ny, ws.nz, ws.cr, ws.cg, ws.cb, head);
-    e = launch_scan(LoadArray{head}, HeadStore{scode, ws.puid, ws.ucode, ws.ufirst}, &c->n_points, 0, ws.scan, total,
-                    err, s, ScanCount{}, 1);
+    e = launch_scan<2>(GatherLoad{ws.d_params, scode, sidx, c, D, ws.px, ws.py, ws.pz, ws.nx, ws.ny, ws.nz, ws.cr, ws.cg, ws.cb},
+                       HeadStore{scode, c, ws.puid, ws.ucode, ws.ufirst}, &c->n_points, 0, ws.scan, total, err, s);
     if (e != cudaSuccess) return e;
-    k_after_unique<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, ws.ufirst, total);
-    e = launch_scan(LeafGroupLoad{ws.ucode}, StoreInclusive{ws.uaddr}, &c->n_unique, 0, ws.scan, total, err, s,
-                    ScanCount{}, 1);
+    const LevelArrays T{ws.tkey, ws.tpidx, ws.tpnum, ws.tdidx, ws.tdnum, ws.tchild};
+    e = launch_scan<2>(LeafGroupLoad{ws.ucode},
+                       LeafPlaceStore{ws.ucode, ws.ufirst, c, D, ws.cap.dnodes, ws.uslot, T, err}, &c->n_unique, 0,
+                       ws.scan, total, err, s, ScanCount{}, 2);
     if (e != cudaSuccess) return e;
-    k_after_leaf_groups<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, total, D, ws.cap.dnodes);
-    const int gn = grid_for(ws, ws.cap.dnodes);
-    k_init_level<<<PSR_GRID(ws, gn), kBlock, 0, s>>>(c, D, D, ws.tkey, ws.tpidx, ws.tpnum, ws.tdidx, ws.tdnum, ws.tchild);
-    k_place_leaves<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(c, ws.ucode, ws.ufirst, ws.uaddr, ws.uslot, ws.tkey, ws.tpidx, ws.tpnum);
-    k_point2node<<<PSR_GRID(ws, gp), kBlock, 0, s>>>(c, ws.puid, ws.uslot, ws.point2node);
-    // levels D .. dfuse+1 level by level across the GPU, the small levels near the root in
-    // one CTA
-    const int dfuse = D - 3;
-    for (int d = D; d >= 1 && d > dfuse; --d) {
-        const int gg = grid_for(ws, ws.cap.dnodes / 8 + 1);
-        k_group_aggregate<<<PSR_GRID(ws, gg), kBlock, 0, s>>>(c, d, D, ws.tkey, ws.tpidx, ws.tpnum, ws.tdidx, ws.tdnum, ws.gkey,
-                                                ws.gpidx, ws.gpnum, ws.gdidx, ws.gdnum);
-        e = launch_scan(FatherGroupLoad{ws.gkey, 3 * (D - d + 2)}, StoreInclusive{ws.gaddr}, &c->n_groups, 0, ws.scan,
-                        total, err, s, ScanCount{}, 1);
+    // levels D .. dfuse+1 level by level across the GPU, the levels near the root (at most 4096
+    // nodes each) in one CTA
+    const int dfuse = D - 1 < kCoarseLevels ? D - 1 : kCoarseLevels;
+    for (int d = D; d > dfuse; --d) {
+        e = launch_scan<1>(LevelLoad{c, d, D, T, ws.gkey, ws.gpidx, ws.gpnum, ws.gdidx, ws.gdnum},
+                           LevelStore{c, d, D, ws.cap.nodes, T, ws.gkey, ws.gpidx, ws.gpnum, ws.gdidx, ws.gdnum,
+                                      ws.tparent_slot, err},
+                           &c->level_groups[d], 0, ws.scan, total, err, s, ScanCount{}, 2);
         if (e != cudaSuccess) return e;
-        k_after_father_groups<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, d, total, ws.cap.nodes);
-        k_init_level<<<PSR_GRID(ws, gg), kBlock, 0, s>>>(c, d - 1, D, ws.tkey, ws.tpidx, ws.tpnum, ws.tdidx, ws.tdnum, ws.tchild);
-        k_place_fathers<<<PSR_GRID(ws, gg), kBlock, 0, s>>>(c, d, D, ws.gkey, ws.gpidx, ws.gpnum, ws.gdidx, ws.gdnum, ws.gaddr,
-                                              ws.tkey, ws.tpidx, ws.tpnum, ws.tdidx, ws.tdnum, ws.tchild,
-                                              ws.tparent_slot);
     }
     if (dfuse >= 1)
         k_levels_block<<<PSR_GRID(ws, 1), kLevelBlock, 0, s>>>(c, dfuse, D, ws.tkey, ws.tpidx, ws.tpnum, ws.tdidx, ws.tdnum, ws.tchild,
                                                  ws.tparent_slot, ws.gkey, ws.gpidx, ws.gpnum, ws.gdidx, ws.gdnum,
                                                  ws.gaddr, ws.cap.nodes);
-    k_levels_done<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, D);
+    else
+        k_levels_done<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, D);
     const int gm = grid_for(ws, ws.cap.nodes);
+    const size_t stride = (size_t)ws.cap.nodes;
     k_finalize_nodes<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, D, ws.tkey, ws.tpidx, ws.tpnum, ws.tdidx, ws.tdnum, ws.tchild,
                                            ws.tparent_slot, ws.key, ws.pidx, ws.pnum, ws.parent, ws.first_child,
-                                           ws.didx, ws.dnum, ws.ndepth, ws.enc, ws.ctr_x, ws.ctr_y, ws.ctr_z);
-    const size_t stride = (size_t)ws.cap.nodes;
-    k_root_neighbours<<<PSR_GRID(ws, 1), 32, 0, s>>>(ws.neigh, stride);
+                                           ws.didx, ws.dnum, ws.ndepth, ws.enc, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.neigh,
+                                           stride, ws.puid, ws.uslot, ws.point2node);
     if (dfuse >= 1)
         k_neighbours_block<<<PSR_GRID(ws, 1), kLevelBlock, 0, s>>>(c, dfuse, D, ws.key, ws.parent, ws.first_child, ws.neigh, stride);
     for (int d = (dfuse >= 1 ? dfuse + 1 : 1); d <= D; ++d)

@@ -239,18 +239,77 @@ constexpr int kRadix = 1 << kRadixBits;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kBlock * kSortItems;   // 2048 keys per tile
 
+constexpr int kSortMaxPasses = 4;
+
+// Scratch of the radix sort.  bins: [kSortMaxPasses][kRadix] digit counts of the whole input, then
+// their exclusive prefixes; [kSortMaxPasses * kRadix + p]: the next tile of pass p.  The caller's
+// first kernel zeroes it (kSortBinWords words).  status: [pass][tile][digit] words of the passes'
+// look-back, cleared by the kernel that counts the digits.
 struct SortScratch {
-    unsigned* hist;          // [kRadix][max_tiles]
+    unsigned* bins;
+    unsigned* status;
     unsigned* keys_alt;
     unsigned* vals_alt;
     int max_tiles;
-    ScanScratch scan;
+    int batch = 1;   // clouds of the launch (host side: the grid's y extent)
+    __device__ void rebase() { PSR_CLOUD(bins, status, keys_alt, vals_alt); }   // to cloud blockIdx.y
 };
+constexpr int kSortBinWords = kSortMaxPasses * (kRadix + 1);
+inline int sort_passes(int key_bits) { return (key_bits + kRadixBits - 1) / kRadixBits; }
 
 // n 32-bit words at p set to v, in each of `clouds` clouds (a memset that multi-cloud
 // launches can take: every cloud's copy of the buffer)
 cudaError_t fill_words(unsigned* p, unsigned v, long long n, int clouds, cudaStream_t stream);
 
+// Counting side of the sort, inside the kernel that makes the keys (kBlock threads a block):
+// count() the digits of every key of the block, then finish() in every block of the cloud.
+struct SortCounter {
+    unsigned (*s_h)[kRadix];   // [kSortMaxPasses][kRadix] shared
+    int passes;
+    __device__ void clear() const {
+        for (int d = threadIdx.x; d < passes * kRadix; d += kBlock) (&s_h[0][0])[d] = 0u;
+        __syncthreads();
+    }
+    __device__ void count(unsigned key) const {
+        for (int p = 0; p < passes; ++p) atomicAdd(&s_h[p][(key >> (kRadixBits * p)) & (kRadix - 1)], 1u);
+    }
+    // adds the block's counts to the bins; the last block to finish turns them into exclusive
+    // prefixes.  Also clears the passes' look-back words of n keys.
+    __device__ void finish(const SortScratch& sc, int n, unsigned* ticket, unsigned* err) const {
+        const int ntiles = (n + kSortTile - 1) / kSortTile;
+        if (ntiles > sc.max_tiles) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, kErrCapacity);
+            return;
+        }
+        for (int p = 0; p < passes; ++p) {
+            unsigned* st = sc.status + (size_t)p * sc.max_tiles * kRadix;
+            PSR_GRID_STRIDE(i, ntiles * kRadix) st[i] = 0u;
+        }
+        __syncthreads();
+        for (int d = threadIdx.x; d < passes * kRadix; d += kBlock) {
+            const unsigned v = (&s_h[0][0])[d];
+            if (v) atomicAdd(&sc.bins[d], v);
+        }
+        __shared__ unsigned s_warp[kBlock / 32 + 1];
+        __shared__ int s_last;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        static_assert(kRadix == kBlock, "a thread per digit");
+        for (int p = 0; p < passes; ++p) {
+            unsigned* b = sc.bins + p * kRadix;
+            unsigned excl;
+            block_exclusive_scan(__ldcg(b + threadIdx.x), excl, s_warp);
+            b[threadIdx.x] = excl;
+        }
+    }
+};
+
+// The passes: a stable sort of the n = *count_ptr (key, index) pairs whose digits were counted;
+// vals_in of the first pass is the input index.  *result_in_alt: where they end.
 cudaError_t radix_sort_pairs(unsigned* keys, unsigned* vals, const int* count_ptr, int key_bits, SortScratch sc,
                              unsigned* err, cudaStream_t stream, bool* result_in_alt);
 

@@ -26,6 +26,8 @@ struct Counters {
     int level_count[kMaxDepth + 1];
     int level_base[kMaxDepth + 1];
     int level_tmp_off[kMaxDepth + 1];   // offset of each level inside the build buffer
+    int level_groups[kMaxDepth + 1];    // sibling groups of each level (level_count / 8)
+    unsigned ticket[2];           // blocks done of the bounding box and the encoder
     int n_nodes;
     int n_vertices, n_edges, n_faces;
     int n_cross, n_tri;
@@ -56,6 +58,15 @@ struct Counters {
     int cg_checks[kMaxDepth + 1];     // true-residual evaluations of each depth's CG
     int cg_restarts[kMaxDepth + 1];   // refinement restarts from the true residual
     unsigned long long cg_depth_ns[kMaxDepth + 1];   // device time of each depth's CG
+};
+
+// The input arrays of one call, written by the host before each run: the caller's device
+// arrays, or the workspace's staged copies.  (Not moved by PSR_CLOUD: absolute addresses.)
+struct InputRef {
+    const float* xyz;
+    const float* nrm;
+    const uint8_t* rgb;    // null: no colours
+    int n;
 };
 
 // State of one depth's CG when it runs as a device loop (a CUDA-graph while node whose

@@ -74,7 +74,6 @@ struct Workspace {
     unsigned* ucode;        // unique leaf codes
     int* ufirst;            // first sorted point of each unique leaf (+ sentinel)
     int* uslot;             // D-level slot of each unique leaf
-    unsigned* uaddr;        // group address of each unique leaf
 
     // level build staging (levels D, D-1, ..., 0 appended in that order)
     int *tkey, *tpidx, *tpnum, *tdidx, *tdnum, *tchild;
@@ -174,7 +173,7 @@ struct Workspace {
     int* part_t;
     int part_cap_v, part_cap_t;
 
-    int* d_params;          // [0] point count of the current call (written before each run)
+    InputRef* d_params;     // the current call's input (written before each run)
 
     cudaStream_t stream;
     cudaStream_t aux = nullptr;         // second stream for work forked off `stream`
@@ -201,7 +200,7 @@ inline void set_batch(Workspace& ws, int clouds) {
     ws.batch = clouds;
     ws.scan.batch = clouds;
     ws.scan_aux.batch = clouds;
-    ws.sort.scan.batch = clouds;
+    ws.sort.batch = clouds;
 }
 
 // grid of a grid-stride kernel over `work` items: enough blocks, at most 8 per SM
