@@ -576,6 +576,7 @@ static cudaError_t issue_pipeline(psr_handle* h, cudaStream_t qs, int cg_iters, 
     // octree-only work on a third stream, beside the divergence and the solve: the
     // vertex / edge / face records and the colour search grid (own scan scratch)
     const bool overlap = h->cfg.concurrent_stages != 0;
+    ws.chain = !overlap;
     if (overlap) {
         if (q == cudaSuccess) q = cudaEventRecord(ws.ev_fork2, qs);
         if (q == cudaSuccess) q = cudaStreamWaitEvent(ws.aux2, ws.ev_fork2, 0);

@@ -323,10 +323,12 @@ cudaError_t field_build(Workspace& ws) {
         // The coarse depths' chunked divergence runs on the second stream beside k_div_fine
         // (both only read the vector field); it issues the only scan meanwhile.
         // item_start / n_items / partial live in the (otherwise idle) CG scratch.
-        cudaStream_t a2 = ws.aux;
-        e = cudaEventRecord(ws.ev_fork, s);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(a2, ws.ev_fork, 0);
-        if (e != cudaSuccess) return e;
+        cudaStream_t a2 = ws.chain ? s : ws.aux;
+        if (!ws.chain) {
+            e = cudaEventRecord(ws.ev_fork, s);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(a2, ws.ev_fork, 0);
+            if (e != cudaSuccess) return e;
+        }
         unsigned* item_start = (unsigned*)ws.cg_r;
         int* n_items = (int*)&c->n_groups;
         unsigned* total = (unsigned*)&c->scan_total;
@@ -340,13 +342,13 @@ cudaError_t field_build(Workspace& ws) {
                                                         ws.dnum, ws.neigh, stride, vx, vy, vz, ws.dff, partial);
         k_div_coarse_reduce<<<PSR_GRID(ws, grid_for(ws, 1 << 16)), kBlock, 0, a2>>>(c, dsplit, item_start, n_items, partial,
                                                                      ws.divg);
-        e = cudaEventRecord(ws.ev_join, a2);
+        if (!ws.chain) e = cudaEventRecord(ws.ev_join, a2);
         if (e != cudaSuccess) return e;
     }
     k_div_fine<<<PSR_GRID(ws, ws.num_sms * 8), kBlock, 0, s>>>(c, D, dsplit, ws.res, ws.enc, ws.didx, ws.dnum, ws.neigh, stride, vx,
                                                  vy, vz, ws.dff, ws.divg);
     k_div_leaf<<<PSR_GRID(ws, ws.num_sms * 8), kBlock, 0, s>>>(c, D, ws.res, ws.enc, ws.neigh, stride, vx, vy, vz, ws.dff, ws.divg);
-    if (dsplit > 0) {
+    if (dsplit > 0 && !ws.chain) {
         e = cudaStreamWaitEvent(s, ws.ev_join, 0);
         if (e != cudaSuccess) return e;
     }

@@ -27,7 +27,7 @@ struct Counters {
     int level_base[kMaxDepth + 1];
     int level_tmp_off[kMaxDepth + 1];   // offset of each level inside the build buffer
     int level_groups[kMaxDepth + 1];    // sibling groups of each level (level_count / 8)
-    unsigned ticket[2];           // blocks done of the bounding box and the encoder
+    unsigned ticket[3];           // blocks done of the bounding box, the encoder, the sample values
     int n_nodes;
     int n_vertices, n_edges, n_faces;
     int n_cross, n_tri;

@@ -142,6 +142,8 @@ struct CgcArgs {
     int res_period;     // > 0: true residual every res_period iterations; 0: only at
                         // convergence; < 0: never (the recursive residual alone)
     unsigned loop_mask; // depths the device loop solves when they do not fit the cluster
+    int clusters;       // units solved by a whole cluster; the CTAs of the clusters behind them
+                        // solve a coarser depth each
 };
 
 // The resident path holds a depth when its cluster's chunk of groups fits a CTA's shared
@@ -485,6 +487,8 @@ __global__ void __launch_bounds__(kBlock) k_cg_blocks(const Counters* c, const i
 
 struct CgUnit {
     int d, row0, row1;
+    unsigned me, nb;    // this CTA among those that solve the unit
+    unsigned rank0;     // cluster rank of the first of them
 };
 
 __device__ __forceinline__ float2 cg_ld2(unsigned a) {
@@ -558,7 +562,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     float* sap = sx + 8 * GP;
     constexpr int kDescPitch = kMode == kCgOne ? kCgcBlock : kCgRowGroups;
     unsigned* sdesc = reinterpret_cast<unsigned*>(sap + 8 * GP);   // [kCgDescWords][kDescPitch]
-    const unsigned me = cl.block_rank(), nb = cl.num_blocks();
+    const unsigned me = u.me, nb = u.nb;
     unsigned* err = &v.cw->error;
     const int tid = threadIdx.x;
     const int ngroups = (u.row1 - u.row0) >> 3;
@@ -573,9 +577,9 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     // rank << 11 | local group of global group G (absent or outside the unit: the zero group)
     auto locate = [&](int G) -> unsigned {
         const unsigned q = (unsigned)(G - ((u.row0 - 1) >> 3));
-        if (G < 0 || q >= (unsigned)ngroups) return (me << 11) | (unsigned)(GP - 1);
+        if (G < 0 || q >= (unsigned)ngroups) return ((u.rank0 + me) << 11) | (unsigned)(GP - 1);
         const unsigned own = chunk > 1 ? __umulhi(q, magic) : q;   // q / chunk
-        return (own << 11) | (q - own * (unsigned)chunk);
+        return ((u.rank0 + own) << 11) | (q - own * (unsigned)chunk);
     };
     auto base_of = [&](unsigned d, unsigned sa, unsigned elem) { return cg_map(sa + (d & 2047u) * elem, d >> 11); };
 
@@ -775,7 +779,9 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
             cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_true(sh, a, t, it); });
             if (sh.replace) {   // refinement restart: CG continues from the true residual
                 for_rows([&](int e) { rp[e].x = sap[e]; });
-                cl.sync();      // before any CTA reads a neighbour's new r
+                // before any CTA reads a neighbour's new r
+                if (nb > 1) cl.sync();
+                else __syncthreads();
             }
         }
     }
@@ -792,10 +798,10 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
 // published step also passes the cluster barrier.
 __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh, const CgcArgs& a,
                                            const CgcVec& v, const CgUnit& u) {
-    const unsigned me = cl.block_rank(), nb = cl.num_blocks();
+    const unsigned me = u.me, nb = u.nb;
     unsigned* err = &v.cw->error;
-    const int tid = cl.block_rank() * blockDim.x + threadIdx.x;
-    const int nthr = cl.num_blocks() * blockDim.x;
+    const int tid = me * blockDim.x + threadIdx.x;
+    const int nthr = nb * blockDim.x;
     FF acc = ff_zero();
     for (int i = u.row0 + tid; i < u.row1; i += nthr) {
         const float bi = v.b[i];
@@ -859,47 +865,51 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
             if (nb > 1) cl.sync();
             if (sh.replace) {   // refinement restart: CG continues from the true residual
                 for (int i = u.row0 + tid; i < u.row1; i += nthr) v.r[i] = v.ap[i];
-                cl.sync();
+                if (nb > 1) cl.sync();
+                else __syncthreads();
             }
         }
     }
-    if (ran && cl.block_rank() == 0 && threadIdx.x == 0) cgc_report(v, u.d, sh, it - 1);
+    if (ran && me == 0 && threadIdx.x == 0) cgc_report(v, u.d, sh, it - 1);
 }
 
-// one depth per cluster (a CTA when the launch has no cluster dimension)
-__device__ __forceinline__ void cg_unit_body(const CgcArgs& a, const CgcVec& v, int unit) {
-    cg::cluster_group cl = cg::this_cluster();
-    __shared__ CgcShared sh;
-    extern __shared__ float4 cg_dyn[];
-    const unsigned long long t_start = global_ns();
-    CgUnit u;
-    u.d = a.first - unit;
-    u.row0 = v.c->level_base[u.d];
-    u.row1 = (u.d < a.depth) ? v.c->level_base[u.d + 1] : v.c->n_nodes;
-    if (threadIdx.x < 27) sh.st[threadIdx.x] = v.stencil[u.d * 27 + threadIdx.x];
-    const int nblk = (int)cl.num_blocks();
-    cgc_barriers_init(sh);
-    cl.sync();   // the barriers are up before a peer arrives at them
-    const int m = u.row1 - u.row0;
-    const int chunk = cg_chunk_groups(m, nblk);
-    const bool fits = cg_fits_resident(u.d, m, nblk);   // uniform over the cluster
-    if (!fits && ((a.loop_mask >> u.d) & 1u)) return;    // the device loop solves this depth
-    if (fits) {
-        if (chunk <= kCgRowGroups) cgc_resident<kCgRows>(cl, sh, a, v, u, chunk, cg_dyn);
-        else if (chunk <= kCgcBlock) cgc_resident<kCgOne>(cl, sh, a, v, u, chunk, cg_dyn);
-        else cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);
-    } else {
-        cgc_global(cl, sh, a, v, u);
-    }
-    cl.sync();   // no CTA exits while others may still read its shared memory
-    if (cl.block_rank() == 0 && threadIdx.x == 0) v.cw->cg_depth_ns[u.d] = global_ns() - t_start;
-}
-
+// One depth per cluster; behind the first a.clusters clusters, one depth per CTA.  Cluster
+// barriers are passed by every CTA the same number of times only where a whole cluster solves.
 __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
     cg::cluster_group cl = cg::this_cluster();
     CgcVec v = a.v;
     v.rebase();
-    cg_unit_body(a, v, (int)(blockIdx.x / cl.num_blocks()));
+    __shared__ CgcShared sh;
+    extern __shared__ float4 cg_dyn[];
+    const unsigned long long t_start = global_ns();
+    const unsigned size = cl.num_blocks(), rank = cl.block_rank();
+    const int cluster = (int)(blockIdx.x / size);
+    const bool whole = cluster < a.clusters;
+    CgUnit u;
+    u.d = whole ? a.first - cluster : a.first - a.clusters - ((cluster - a.clusters) * (int)size + (int)rank);
+    u.me = whole ? rank : 0u;
+    u.nb = whole ? size : 1u;
+    u.rank0 = whole ? 0u : rank;
+    cgc_barriers_init(sh);
+    if (u.d >= 0) {
+        u.row0 = v.c->level_base[u.d];
+        u.row1 = (u.d < a.depth) ? v.c->level_base[u.d + 1] : v.c->n_nodes;
+        if (threadIdx.x < 27) sh.st[threadIdx.x] = v.stencil[u.d * 27 + threadIdx.x];
+    }
+    cl.sync();   // the barriers are up before a peer arrives at them
+    if (u.d >= 0) {
+        const int m = u.row1 - u.row0;
+        const int chunk = cg_chunk_groups(m, (int)u.nb);
+        const bool fits = cg_fits_resident(u.d, m, (int)u.nb);   // the same in all CTAs of the unit
+        if (fits || !((a.loop_mask >> u.d) & 1u)) {   // else the device loop solves this depth
+            if (!fits) cgc_global(cl, sh, a, v, u);
+            else if (chunk <= kCgRowGroups) cgc_resident<kCgRows>(cl, sh, a, v, u, chunk, cg_dyn);
+            else if (chunk <= kCgcBlock) cgc_resident<kCgOne>(cl, sh, a, v, u, chunk, cg_dyn);
+            else cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);
+            if (u.me == 0 && threadIdx.x == 0) v.cw->cg_depth_ns[u.d] = global_ns() - t_start;
+        }
+    }
+    cl.sync();   // no CTA exits while others may still read its shared memory
 }
 
 // ---- device-loop CG: the depths too large for a cluster's shared memory -----------------
@@ -1315,25 +1325,21 @@ __global__ void __launch_bounds__(kBlock) k_point_poly(const Counters* c, int de
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_point_values_coarse(const Counters* c, int depth, const float* px,
-                                                                const float* py, const float* pz,
-                                                                const int* point2node, const int* parent,
-                                                                const float* ctr_x, const float* ctr_y,
-                                                                const float* ctr_z, const float* coef,
-                                                                size_t cstride, float* out) {
-    PSR_CLOUD(c, px, py, pz, point2node, parent, ctr_x, ctr_y, ctr_z, coef, out);
-    const int n = c->n_points;
-    const int bD = c->level_base[depth];
-    const int b1 = c->level_base[depth - 1];
-    const float inv2h = (float)(1 << (depth - 1));   // 1 / (2 h) of a depth-(D-1) cell
-    PSR_GRID_STRIDE(i, n) {
-        const int node = parent[bD + point2node[i]];
+// the levels up to D-1 at sample i (u in [0, 1] per axis of the sample's depth-(D-1) cell)
+struct PointCoarse {
+    const int* parent;
+    const float *ctr_x, *ctr_y, *ctr_z;
+    const float* coef;
+    size_t cstride;
+    __device__ float operator()(int depth, int bD, int b1, int leaf, float x, float y, float z) const {
+        const float inv2h = (float)(1 << (depth - 1));   // 1 / (2 h) of a depth-(D-1) cell
+        const int node = parent[bD + leaf];
         const int a = node - b1;
-        // position in the cell, u in [0, 1] per axis (cell from centre - h to centre + h)
+        // cell from centre - h to centre + h
         const float hh = 0.5f / inv2h;
-        const float ux = (px[i] - (ctr_x[node] - hh)) * inv2h;
-        const float uy = (py[i] - (ctr_y[node] - hh)) * inv2h;
-        const float uz = (pz[i] - (ctr_z[node] - hh)) * inv2h;
+        const float ux = (x - (ctr_x[node] - hh)) * inv2h;
+        const float uy = (y - (ctr_y[node] - hh)) * inv2h;
+        const float uz = (z - (ctr_z[node] - hh)) * inv2h;
         const float wx[3] = {(1.0f - ux) * (1.0f - ux), 2.0f * ux * (1.0f - ux), ux * ux};
         const float wy[3] = {(1.0f - uy) * (1.0f - uy), 2.0f * uy * (1.0f - uy), uy * uy};
         const float wz[3] = {(1.0f - uz) * (1.0f - uz), 2.0f * uz * (1.0f - uz), uz * uz};
@@ -1341,27 +1347,46 @@ __global__ void __launch_bounds__(kBlock) k_point_values_coarse(const Counters* 
 #pragma unroll
         for (int k = 0; k < 27; ++k)
             val = fmaf(wx[k / 9] * wy[(k / 3) % 3] * wz[k % 3], coef[(size_t)k * cstride + a], val);
-        out[i] = val;
+        return val;
     }
+    __device__ void rebase() { PSR_CLOUD(parent, ctr_x, ctr_y, ctr_z, coef); }   // to cloud blockIdx.y
+};
+
+__global__ void __launch_bounds__(kBlock) k_point_values_coarse(const Counters* c, int depth, const float* px,
+                                                                const float* py, const float* pz,
+                                                                const int* point2node, PointCoarse coarse, float* out) {
+    PSR_CLOUD(c, px, py, pz, point2node, coarse, out);
+    const int n = c->n_points;
+    const int bD = c->level_base[depth];
+    const int b1 = c->level_base[depth - 1];
+    PSR_GRID_STRIDE(i, n) out[i] = coarse(depth, bD, b1, point2node[i], px[i], py[i], pz[i]);
 }
 
 // The sample values are summed in chunks of kBlock points (chunk_sums[chunk]), then the
 // chunks in order: the iso-value's summation order depends only on the point count, not on
 // the launch's grid, so a cloud gets the same iso-value alone and in a multi-cloud launch.
-__global__ void __launch_bounds__(kBlock) k_point_values(const Counters* c, int depth, const float* px,
-                                                         const float* py, const float* pz, const int* point2node,
-                                                         const int* neigh, size_t stride, const int* enc,
-                                                         const float* x, float* out, double* chunk_sums) {
-    PSR_CLOUD(c, px, py, pz, point2node, neigh, enc, x, out, chunk_sums);
+// The last block to finish adds the chunks.  kWithCoarse: the levels up to D-1 are evaluated
+// here too instead of by a launch beside the depth-D solve.
+template <bool kWithCoarse>
+__global__ void __launch_bounds__(kBlock) k_point_values(Counters* c, int depth, const float* px, const float* py,
+                                                         const float* pz, const int* point2node, const int* neigh,
+                                                         size_t stride, const int* enc, const float* x,
+                                                         PointCoarse coarse, float* out, double* chunk_sums) {
+    PSR_CLOUD(c, px, py, pz, point2node, neigh, enc, x, coarse, out, chunk_sums);
     __shared__ double s_w[kBlock / 32];
+    __shared__ int s_last;
     const int n = c->n_points;
     const int bD = c->level_base[depth];
+    const int b1 = c->level_base[depth - 1];
     const int nchunks = (n + kBlock - 1) / kBlock;
     for (int ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         const int i = ch * kBlock + threadIdx.x;
         double acc = 0.0;
         if (i < n) {
-            const float v = level_terms(bD + point2node[i], out[i], px[i], py[i], pz[i], depth, neigh, stride, enc, x);
+            const int leaf = point2node[i];
+            const float qx = px[i], qy = py[i], qz = pz[i];
+            const float v0 = kWithCoarse ? coarse(depth, bD, b1, leaf, qx, qy, qz) : out[i];
+            const float v = level_terms(bD + leaf, v0, qx, qy, qz, depth, neigh, stride, enc, x);
             out[i] = v;
             acc = (double)v;
         }
@@ -1372,17 +1397,16 @@ __global__ void __launch_bounds__(kBlock) k_point_values(const Counters* c, int 
             double sum = 0.0;
             for (int w = 0; w < kBlock / 32; ++w) sum += s_w[w];
             chunk_sums[ch] = sum;
+            __threadfence();
         }
         __syncthreads();
     }
-}
-
-__global__ void k_iso_finalize(Counters* c, const double* chunk_sums) {
-    PSR_CLOUD(c, chunk_sums);
-    __shared__ double s_w[32];
-    const int nchunks = (c->n_points + kBlock - 1) / kBlock;
+    if (threadIdx.x == 0) s_last = atomicAdd(&c->ticket[2], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
     double s = 0.0;
-    for (int b = threadIdx.x; b < nchunks; b += blockDim.x) s += chunk_sums[b];
+    for (int b = threadIdx.x; b < nchunks; b += blockDim.x) s += __ldcg(chunk_sums + b);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane_id() == 0) s_w[threadIdx.x >> 5] = s;
     __syncthreads();
@@ -1544,6 +1568,33 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     const int loop_units = (ws.ev_flags == cudaEventRecordExternal && D >= 8) ? D - 4 : 0;
     a.loop_mask = 0u;
     for (int z = 0; z < loop_units; ++z) a.loop_mask |= 1u << (D - z);
+    const size_t cstride = (size_t)ws.cap.dnodes / 8 + 64;
+    const PointCoarse coarse{ws.parent, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.pv_coef, cstride};
+    const int nb = ws.num_sms * 4;
+    if (ws.chain && loop_units == 0) {
+        // One launch for every depth: clusters of at most 8 CTAs for the two finest, a CTA each for
+        // the rest in the clusters behind them.  A chain without forks takes one hardware queue,
+        // so that the resident slots of a server run side by side (the driver has 8 by default:
+        // with three branches a graph, eight depth-5 clouds took 245 us each, 158 with 32 queues).
+        const int cs = ws.cg_ctas > 0 ? cl1 : (g_cg_cluster < 8 ? g_cg_cluster : 8);
+        CgcArgs b = a;
+        b.first = D;
+        b.clusters = D < 2 ? D : 2;
+        const int singles = D + 1 - b.clusters;
+        e = launch_cg(k_cg_cluster, b, (b.clusters + (singles + cs - 1) / cs) * cs, cs, ws.batch, s);
+        if (e != cudaSuccess) return e;
+        if (ws.ev_cg) {
+            e = cudaEventRecordWithFlags(ws.ev_cg, s, ws.ev_flags);
+            if (e != cudaSuccess) return e;
+        }
+        k_point_poly<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, s>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.neigh,
+                                                                     (size_t)ws.cap.nodes, ws.parent, ws.enc, ws.xsol,
+                                                                     ws.pv_coef, cstride);
+        k_point_values<true><<<PSR_GRID(ws, nb), kBlock, 0, s>>>(ws.cnt, ws.depth, ws.px, ws.py, ws.pz, ws.point2node,
+                                                                 ws.neigh, (size_t)ws.cap.nodes, ws.enc, ws.xsol, coarse,
+                                                                 ws.point_val, ws.iso_partial);
+        return cudaGetLastError();
+    }
     e = cudaEventRecord(ws.ev_fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ws.aux, ws.ev_fork, 0);
     if (e == cudaSuccess && ncl > 1) e = cudaStreamWaitEvent(ws.aux3, ws.ev_fork, 0);
@@ -1570,6 +1621,7 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     if (e == cudaSuccess && ncta > 0) {
         CgcArgs b = a;
         b.first = D - ncl;
+        b.clusters = ncta;
         e = launch_cg(k_cg_cluster, b, ncta, 1, ws.batch, ws.aux);   // clusters of one CTA
     }
     // the coarse sample values and the depth-D terms wait for every depth's solution
@@ -1578,6 +1630,7 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     if (ncl > 1) {
         CgcArgs b = a;
         b.first = D - 1;
+        b.clusters = ncl - 1;
         e = launch_cg(k_cg_cluster, b, (ncl - 1) * cl2, cl2, ws.batch, ws.aux3);
         if (e == cudaSuccess) e = cudaEventRecord(ws.ev_join3, ws.aux3);
         if (e != cudaSuccess) return e;
@@ -1586,18 +1639,17 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     // solved, beside the depth-D CG
     if (ncl > 1) e = cudaStreamWaitEvent(ws.aux, ws.ev_join3, 0);
     if (e == cudaSuccess) {
-        const size_t cstride = (size_t)ws.cap.dnodes / 8 + 64;
         k_point_poly<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, ws.aux>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.neigh,
                                                             (size_t)ws.cap.nodes, ws.parent, ws.enc, ws.xsol,
                                                             ws.pv_coef, cstride);
-        k_point_values_coarse<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, ws.aux>>>(ws.cnt, D, ws.px, ws.py, ws.pz, ws.point2node,
-                                                                     ws.parent, ws.ctr_x, ws.ctr_y, ws.ctr_z,
-                                                                     ws.pv_coef, cstride, ws.point_val);
+        k_point_values_coarse<<<PSR_GRID(ws, nb), kBlock, 0, ws.aux>>>(ws.cnt, D, ws.px, ws.py, ws.pz, ws.point2node, coarse,
+                                                                       ws.point_val);
         e = cudaEventRecord(ws.ev_join, ws.aux);
     }
     if (e != cudaSuccess) return e;
     if (ncl > 0) {
         a.first = D;
+        a.clusters = 1;
         e = launch_cg(k_cg_cluster, a, cl1, cl1, ws.batch, s);
         if (e != cudaSuccess) return e;
     }
@@ -1608,10 +1660,9 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     e = cudaStreamWaitEvent(s, ws.ev_join, 0);
     if (e != cudaSuccess) return e;
     // iso-value: the depth-D terms complete the sample values
-    const int nb = ws.num_sms * 4;
-    k_point_values<<<PSR_GRID(ws, nb), kBlock, 0, s>>>(ws.cnt, ws.depth, ws.px, ws.py, ws.pz, ws.point2node, ws.neigh,
-                                         (size_t)ws.cap.nodes, ws.enc, ws.xsol, ws.point_val, ws.iso_partial);
-    k_iso_finalize<<<PSR_GRID(ws, 1), 256, 0, s>>>(ws.cnt, ws.iso_partial);
+    k_point_values<false><<<PSR_GRID(ws, nb), kBlock, 0, s>>>(ws.cnt, ws.depth, ws.px, ws.py, ws.pz, ws.point2node,
+                                                              ws.neigh, (size_t)ws.cap.nodes, ws.enc, ws.xsol, coarse,
+                                                              ws.point_val, ws.iso_partial);
     return cudaGetLastError();
 }
 
