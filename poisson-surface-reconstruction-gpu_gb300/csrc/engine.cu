@@ -303,6 +303,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.cnt, 1);
     A.add(ws.scan.words, (size_t)cap.scan_tiles + kScanHeader);
     A.add(ws.scan_aux.words, (size_t)cap.scan_tiles + kScanHeader);
+    for (auto& sc : ws.scan_side) A.add(sc.words, (size_t)cap.scan_tiles + kScanHeader);
     A.add(ws.sort.bins, (size_t)kSortBinWords);
     A.add(ws.sort.status, (size_t)kSortMaxPasses * kRadix * sort_tiles);
     A.add(ws.sort.keys_alt, (size_t)N);
@@ -362,7 +363,6 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.cube_class, (size_t)dnodes);
     A.add(ws.face_hit, (size_t)cap.faces);
     A.add(ws.sub_root, (size_t)nodes);
-    A.add(ws.sub_root_depth, (size_t)nodes);
     A.add(ws.root_group, (size_t)nodes);
     A.add(ws.root_self, (size_t)nodes);
     // roots beyond this capacity take the walk over their octree chain in the subdivision
@@ -411,7 +411,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.mb.groups, 8 * (size_t)nodes);
     A.add(ws.mb.edge_of_dnode, (size_t)subd);
     A.add(ws.mb.tri_of_dnode, (size_t)subd);
-    A.add(ws.mb.group_cross0, (size_t)nodes);
+    A.add(ws.mb.group_live, (size_t)nodes);
     A.add(ws.mb.parts, 4 * (size_t)nodes + 8);
     A.add(ws.mb.kept_prefix, (size_t)ws.part_cap_v);
     A.add(ws.mb.misc, 16);
@@ -442,6 +442,11 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     ws.scan_aux.max_tiles = cap.scan_tiles;
     if (e == cudaSuccess)
         e = cudaMemset(ws.scan_aux.words, 0, sizeof(unsigned long long) * ((size_t)cap.scan_tiles + kScanHeader));
+    for (auto& sc : ws.scan_side) {
+        sc.max_tiles = cap.scan_tiles;
+        if (e == cudaSuccess)
+            e = cudaMemset(sc.words, 0, sizeof(unsigned long long) * ((size_t)cap.scan_tiles + kScanHeader));
+    }
     // the device-loop CG's block tickets start at zero; each reduction leaves them at zero
     if (e == cudaSuccess) e = cudaMemset(ws.cg_loop, 0, sizeof(CgLoopState) * (kMaxDepth + 1));
     ws.sort.max_tiles = sort_tiles;
@@ -457,6 +462,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws.aux2, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws.ev_fork2, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws.ev_join2, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws.ev_geo, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws.aux3, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws.ev_join3, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws.aux4, cudaStreamNonBlocking);
@@ -474,7 +480,11 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
         build_dff_table(D, dff);
         std::vector<float> st;
         build_stencil(kMaxDepth, st, (double)cfg.laplacian_epsilon);
-        std::vector<float> dff32(dff.begin(), dff.end());   // the kernels use float entries
+        // the kernels use float entries, row by row of the function the node carries: the leaves of
+        // a node's neighbourhood then read neighbouring entries
+        std::vector<float> dff32(dff.size());
+        for (int i = 0; i < ws.res; ++i)
+            for (int j = 0; j < ws.res; ++j) dff32[(size_t)i * ws.res + j] = (float)dff[(size_t)i + (size_t)ws.res * j];
         e = cudaMemcpy(ws.dff, dff32.data(), dff32.size() * sizeof(float), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(ws.stencil, st.data(), st.size() * sizeof(float), cudaMemcpyHostToDevice);
         // the CG takes four values per depth: an entry depends only on the axes its offset moves on
@@ -522,6 +532,7 @@ psr_status psr_destroy(psr_handle* h) {
     if (h->ws.ev_join) cudaEventDestroy(h->ws.ev_join);
     if (h->ws.ev_fork2) cudaEventDestroy(h->ws.ev_fork2);
     if (h->ws.ev_join2) cudaEventDestroy(h->ws.ev_join2);
+    if (h->ws.ev_geo) cudaEventDestroy(h->ws.ev_geo);
     if (h->ws.ev_join3) cudaEventDestroy(h->ws.ev_join3);
     if (h->ws.ev_join4) cudaEventDestroy(h->ws.ev_join4);
     if (h->ws.aux4) cudaStreamDestroy(h->ws.aux4);
@@ -577,6 +588,7 @@ static cudaError_t issue_pipeline(psr_handle* h, cudaStream_t qs, int cg_iters, 
     // vertex / edge / face records and the colour search grid (own scan scratch)
     const bool overlap = h->cfg.concurrent_stages != 0;
     ws.chain = !overlap;
+    ws.want_normals = want_normals != 0;
     if (overlap) {
         if (q == cudaSuccess) q = cudaEventRecord(ws.ev_fork2, qs);
         if (q == cudaSuccess) q = cudaStreamWaitEvent(ws.aux2, ws.ev_fork2, 0);
@@ -584,14 +596,14 @@ static cudaError_t issue_pipeline(psr_handle* h, cudaStream_t qs, int cg_iters, 
             const ScanScratch main_scan = ws.scan;
             ws.stream = ws.aux2;
             ws.scan = ws.scan_aux;
-            q = mesh_geometry(ws);
+            q = mesh_geometry(ws, want_colour);
             if (q == cudaSuccess) q = transfer_prepare(ws, want_colour); PSR_TRACE(q, "mesh_geometry/transfer_prepare");
             ws.stream = qs;
             ws.scan = main_scan;
         }
         if (q == cudaSuccess) q = cudaEventRecord(ws.ev_join2, ws.aux2);
     } else {
-        if (q == cudaSuccess) q = mesh_geometry(ws);
+        if (q == cudaSuccess) q = mesh_geometry(ws, want_colour);
         if (q == cudaSuccess) q = transfer_prepare(ws, want_colour);
     }
     if (q == cudaSuccess) q = field_build(ws); PSR_TRACE(q, "field_build");

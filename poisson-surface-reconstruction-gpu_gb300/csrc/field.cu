@@ -114,12 +114,12 @@ __device__ __forceinline__ FF div_terms(int l0, int l1, int step, int ox, int oy
                                         int bD, const int* enc, const float* vx, const float* vy, const float* vz,
                                         const float* dff) {
     FF acc = ff_zero();
+    const float *rx = dff + (size_t)res * ox, *ry = dff + (size_t)res * oy, *rz = dff + (size_t)res * oz;
+#pragma unroll 4
     for (int l = l0; l < l1; l += step) {
         int lx, ly, lz;
         decode3(enc[bD + l], depth, lx, ly, lz);
-        const float ux = dff[(size_t)ox + (size_t)res * lx];
-        const float uy = dff[(size_t)oy + (size_t)res * ly];
-        const float uz = dff[(size_t)oz + (size_t)res * lz];
+        const float ux = rx[lx], uy = ry[ly], uz = rz[lz];
         float t = __fmul_rn(vx[l], ux);
         t = fmaf(vy[l], uy, t);
         t = fmaf(vz[l], uz, t);
@@ -128,65 +128,65 @@ __device__ __forceinline__ FF div_terms(int l0, int l1, int step, int ox, int oy
     return acc;
 }
 
+// Divergence arguments of a launch (the three parts below run side by side).
+struct DivArgs {
+    const Counters* c;
+    int depth, dsplit, res;
+    const int *enc, *didx, *dnum, *neigh;
+    size_t stride;
+    const float *vx, *vy, *vz, *dff;
+    const unsigned* item_start;
+    FF* partial;
+    float* divg;
+    __device__ void rebase() { PSR_CLOUD(c, enc, didx, dnum, neigh, vx, vy, vz, dff, item_start, partial, divg); }
+};
+
 // Depth-D nodes: every neighbour holds exactly one depth-D leaf (itself), so a node's
 // divergence has at most 27 terms; one thread per node sums them in slot order.
-__global__ void __launch_bounds__(kBlock) k_div_leaf(const Counters* c, int depth, int res, const int* enc,
-                                                     const int* neigh, size_t stride, const float* vx,
-                                                     const float* vy, const float* vz, const float* dff,
-                                                     float* divg) {
-    PSR_CLOUD(c, enc, neigh, vx, vy, vz, dff, divg);
-    const int bD = c->level_base[depth];
-    const int MD = c->level_count[depth];
+__device__ __forceinline__ void div_leaf(const DivArgs& a) {
+    const int bD = a.c->level_base[a.depth];
+    const int MD = a.c->level_count[a.depth];
     PSR_GRID_STRIDE(o, MD) {
         const int i = bD + o;
         int ox, oy, oz;
-        decode3(enc[i], depth, ox, oy, oz);
+        decode3(a.enc[i], a.depth, ox, oy, oz);
+        const float *rx = a.dff + (size_t)a.res * ox, *ry = a.dff + (size_t)a.res * oy, *rz = a.dff + (size_t)a.res * oz;
         FF acc = ff_zero();
 #pragma unroll 9
         for (int k = 0; k < 27; ++k) {
-            const int nb = neigh[(size_t)k * stride + i];
+            const int nb = a.neigh[(size_t)k * a.stride + i];
             if (nb < 0) continue;
             int lx, ly, lz;
-            decode3(enc[nb], depth, lx, ly, lz);
+            decode3(a.enc[nb], a.depth, lx, ly, lz);
             const int l = nb - bD;
-            const float ux = dff[(size_t)ox + (size_t)res * lx];
-            const float uy = dff[(size_t)oy + (size_t)res * ly];
-            const float uz = dff[(size_t)oz + (size_t)res * lz];
-            float t = __fmul_rn(vx[l], ux);
-            t = fmaf(vy[l], uy, t);
-            t = fmaf(vz[l], uz, t);
+            float t = __fmul_rn(a.vx[l], rx[lx]);
+            t = fmaf(a.vy[l], ry[ly], t);
+            t = fmaf(a.vz[l], rz[lz], t);
             acc = ff_add_float(acc, t);
         }
-        divg[i] = ff_to_float(acc);
+        a.divg[i] = ff_to_float(acc);
     }
 }
 
 // One warp per node for depths dsplit .. D-1.  The (neighbour, leaf) pairs of the node are
 // flattened over the lanes: lane k < 27 holds neighbour k's leaf range, a warp scan gives
-// the range offsets, and term t belongs to the last neighbour whose offset is <= t.  A
-// depth-D node has at most 27 terms (one leaf per neighbour): one pass, 27 lanes busy.
-__global__ void __launch_bounds__(kBlock) k_div_fine(const Counters* c, int depth, int dsplit, int res,
-                                                     const int* enc, const int* didx, const int* dnum,
-                                                     const int* neigh, size_t stride, const float* vx,
-                                                     const float* vy, const float* vz, const float* dff,
-                                                     float* divg) {
-    PSR_CLOUD(c, enc, didx, dnum, neigh, vx, vy, vz, dff, divg);
-    __shared__ int s_off[kBlock / 32][33];
-    __shared__ int s_base[kBlock / 32][32];
-    const int b0 = c->level_base[dsplit];
-    const int bD = c->level_base[depth];
-    const int M = bD;   // depth-D nodes: k_div_leaf
+// the range offsets, and term t belongs to the last neighbour whose offset is <= t.
+__device__ __forceinline__ void div_fine(const DivArgs& a, int (*s_off)[33], int (*s_base)[32]) {
+    const int b0 = a.c->level_base[a.dsplit];
+    const int bD = a.c->level_base[a.depth];
+    const int M = bD;   // depth-D nodes: div_leaf
     const int lane = lane_id();
     const int wib = threadIdx.x >> 5;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int i = b0 + warp; i < M; i += nwarps) {
         int ox, oy, oz;
-        decode3(enc[i], depth, ox, oy, oz);
+        decode3(a.enc[i], a.depth, ox, oy, oz);
+        const float *rx = a.dff + (size_t)a.res * ox, *ry = a.dff + (size_t)a.res * oy, *rz = a.dff + (size_t)a.res * oz;
         int cnt = 0, base = 0;
         if (lane < 27) {
-            const int nb = neigh[(size_t)lane * stride + i];
-            if (nb >= 0) { cnt = dnum[nb]; base = didx[nb]; }
+            const int nb = a.neigh[(size_t)lane * a.stride + i];
+            if (nb >= 0) { cnt = a.dnum[nb]; base = a.didx[nb]; }
         }
         int incl = cnt;
 #pragma unroll
@@ -204,105 +204,96 @@ __global__ void __launch_bounds__(kBlock) k_div_fine(const Counters* c, int dept
             while (k < 26 && s_off[wib][k + 1] <= t) ++k;   // terms are visited in increasing order
             const int l = s_base[wib][k] + (t - s_off[wib][k]);
             int lx, ly, lz;
-            decode3(enc[bD + l], depth, lx, ly, lz);
-            const float ux = dff[(size_t)ox + (size_t)res * lx];
-            const float uy = dff[(size_t)oy + (size_t)res * ly];
-            const float uz = dff[(size_t)oz + (size_t)res * lz];
-            float tt = __fmul_rn(vx[l], ux);
-            tt = fmaf(vy[l], uy, tt);
-            tt = fmaf(vz[l], uz, tt);
+            decode3(a.enc[bD + l], a.depth, lx, ly, lz);
+            float tt = __fmul_rn(a.vx[l], rx[lx]);
+            tt = fmaf(a.vy[l], ry[ly], tt);
+            tt = fmaf(a.vz[l], rz[lz], tt);
             acc = ff_add_float(acc, tt);
         }
         acc = ff_warp_sum(acc);
-        if (lane == 0) divg[i] = ff_to_float(acc);
+        if (lane == 0) a.divg[i] = ff_to_float(acc);
         __syncwarp();
     }
 }
 
-constexpr int kDivChunk = 512;
-
-// chunk count of every coarse node (depth < dsplit)
-struct DivChunkLoad {
-    const int* neigh;
-    size_t stride;
-    const int* dnum;
-    __device__ unsigned operator()(int i) const {
-        unsigned n = 0;
-        for (int k = 0; k < 27; ++k) {
-            int nb = neigh[(size_t)k * stride + i];
-            if (nb >= 0) n += (unsigned)((dnum[nb] + kDivChunk - 1) / kDivChunk);
-        }
-        return n;
-    }
-    __device__ void rebase() { PSR_CLOUD(neigh, dnum); }   // to cloud blockIdx.y
-};
-
-__global__ void k_div_chunk_count(Counters* c, int dsplit, const unsigned* total, int cap, int* n_items) {
-    PSR_CLOUD(c, total, n_items);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int n = (int)*total;
-        if (n > cap) { atomicOr(&c->error, kErrCapacity); n = 0; }
-        *n_items = n;
-    }
-}
-
-// one warp per chunk: partial sum of up to kDivChunk leaves of one neighbour of one node
-__global__ void __launch_bounds__(kBlock) k_div_chunks(const Counters* c, int depth, int dsplit, int res,
-                                                       const int* n_items_ptr, const unsigned* item_start,
-                                                       const int* enc, const int* didx, const int* dnum,
-                                                       const int* neigh, size_t stride, const float* vx,
-                                                       const float* vy, const float* vz, const float* dff,
-                                                       FF* partial) {
-    PSR_CLOUD(c, n_items_ptr, item_start, enc, didx, dnum, neigh, vx, vy, vz, dff, partial);
-    const int n_nodes = c->level_base[dsplit];
-    const int n_items = *n_items_ptr;
-    const int bD = c->level_base[depth];
+// Coarse depths (< dsplit), one warp per chunk: partial sum of up to kDivChunk leaves of one
+// neighbour of one node
+__device__ __forceinline__ void div_chunks(const DivArgs& a) {
+    const int n_nodes = a.c->level_base[a.dsplit];
+    const int n_items = a.c->n_div_items;
+    const int bD = a.c->level_base[a.depth];
     const int lane = lane_id();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int it = warp; it < n_items; it += nwarps) {
-        // node owning this item: last node with item_start <= it
-        int lo = 0, hi = n_nodes - 1;
-        while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if ((int)item_start[mid] <= it) lo = mid;
-            else hi = mid - 1;
+        // node owning this item: last node with item_start <= it; each step the lanes probe 32
+        // places of the range at once
+        int lo = 0, hi = n_nodes;   // item_start[lo] <= it < item_start[hi]
+        while (hi - lo > 1) {
+            const int step = (hi - lo + 31) >> 5;
+            const int at = lo + lane * step;
+            const unsigned m = __ballot_sync(0xffffffffu, at < hi && (int)a.item_start[at < hi ? at : lo] <= it);
+            const int last = 31 - __clz(m);   // lane 0 always holds
+            lo += last * step;
+            hi = min(hi, lo + step);
         }
         const int i = lo;
-        int rem = it - (int)item_start[i];
-        int nb = -1, ch = 0;
-        for (int k = 0; k < 27; ++k) {
-            int q = neigh[(size_t)k * stride + i];
-            if (q < 0) continue;
-            int nc = (dnum[q] + kDivChunk - 1) / kDivChunk;
-            if (rem < nc) { nb = q; ch = rem; break; }
-            rem -= nc;
+        // the chunk's neighbour: lane k counts neighbour k's chunks
+        const int rem = it - (int)a.item_start[i];
+        int q = -1, dn = 0, di = 0;
+        if (lane < 27) {
+            q = a.neigh[(size_t)lane * a.stride + i];
+            if (q >= 0) { dn = a.dnum[q]; di = a.didx[q]; }
         }
+        const int nc = (dn + kDivChunk - 1) / kDivChunk;
+        int incl = nc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const unsigned own = __ballot_sync(0xffffffffu, rem < incl);
         FF acc = ff_zero();
-        if (nb >= 0) {
+        if (own) {   // always
+            const int k = __ffs(own) - 1;
+            const int ch = rem - __shfl_sync(0xffffffffu, incl - nc, k);
+            const int d0 = __shfl_sync(0xffffffffu, di, k), d1 = d0 + __shfl_sync(0xffffffffu, dn, k);
             int ox, oy, oz;
-            decode3(enc[i], depth, ox, oy, oz);
-            const int l0 = didx[nb] + ch * kDivChunk;
-            const int l1 = min(didx[nb] + dnum[nb], l0 + kDivChunk);
-            acc = div_terms(l0 + lane, l1, 32, ox, oy, oz, depth, res, bD, enc, vx, vy, vz, dff);
+            decode3(a.enc[i], a.depth, ox, oy, oz);
+            const int l0 = d0 + ch * kDivChunk;
+            const int l1 = min(d1, l0 + kDivChunk);
+            acc = div_terms(l0 + lane, l1, 32, ox, oy, oz, a.depth, a.res, bD, a.enc, a.vx, a.vy, a.vz, a.dff);
         }
         acc = ff_warp_sum(acc);
-        if (lane == 0) partial[it] = acc;
+        if (lane == 0) a.partial[it] = acc;
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_div_coarse_reduce(const Counters* c, int dsplit, const unsigned* item_start,
-                                                              const int* n_items_ptr, const FF* partial,
-                                                              float* divg) {
-    PSR_CLOUD(c, item_start, n_items_ptr, partial, divg);
-    const int n_nodes = c->level_base[dsplit];
-    const int n_items = *n_items_ptr;
-    PSR_GRID_STRIDE(i, n_nodes) {
-        int a = (int)item_start[i];
-        int b = (i + 1 < n_nodes) ? (int)item_start[i + 1] : n_items;
+// The three parts only read the vector field: one launch, blockIdx.z a part (the longest first).
+__global__ void __launch_bounds__(kBlock) k_divergence(DivArgs a) {
+    __shared__ int s_off[kBlock / 32][33];
+    __shared__ int s_base[kBlock / 32][32];
+    a.rebase();
+    const int part = (int)blockIdx.z + (a.dsplit > 0 ? 0 : 1);
+    if (part == 0) div_chunks(a);
+    else if (part == 1) div_fine(a, s_off, s_base);
+    else div_leaf(a);
+}
+
+// a warp per coarse node adds its chunks (the root has one per 512 leaves)
+__global__ void __launch_bounds__(kBlock) k_div_coarse_reduce(DivArgs a) {
+    a.rebase();
+    const int n_nodes = a.c->level_base[a.dsplit];
+    const int n_items = a.c->n_div_items;
+    const int lane = lane_id();
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n_nodes; i += nwarps) {
+        const int t0 = (int)a.item_start[i];
+        const int t1 = (i + 1 < n_nodes) ? (int)a.item_start[i + 1] : n_items;
         FF s = ff_zero();
-        for (int t = a; t < b; ++t) s = ff_add(s, partial[t]);
-        divg[i] = ff_to_float(s);
+        for (int t = t0 + lane; t < t1; t += 32) s = ff_add(s, a.partial[t]);
+        s = ff_warp_sum(s);
+        if (lane == 0) a.divg[i] = ff_to_float(s);
     }
 }
 
@@ -317,41 +308,18 @@ cudaError_t field_build(Workspace& ws) {
     k_vector_field<<<PSR_GRID(ws, ws.num_sms * 8), kBlock, 0, s>>>(c, D, ws.px, ws.py, ws.pz, ws.nx, ws.ny, ws.nz,
                                                                     ws.pidx, ws.pnum, ws.ctr_x, ws.ctr_y, ws.ctr_z,
                                                                     ws.neigh, stride, vx, vy, vz);
-    const int dsplit = D >= 2 ? D - 2 : 0;
-    cudaError_t e = cudaSuccess;
-    if (dsplit > 0) {
-        // The coarse depths' chunked divergence runs on the second stream beside k_div_fine
-        // (both only read the vector field); it issues the only scan meanwhile.
-        // item_start / n_items / partial live in the (otherwise idle) CG scratch.
-        cudaStream_t a2 = ws.chain ? s : ws.aux;
-        if (!ws.chain) {
-            e = cudaEventRecord(ws.ev_fork, s);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(a2, ws.ev_fork, 0);
-            if (e != cudaSuccess) return e;
-        }
-        unsigned* item_start = (unsigned*)ws.cg_r;
-        int* n_items = (int*)&c->n_groups;
-        unsigned* total = (unsigned*)&c->scan_total;
-        e = launch_scan(DivChunkLoad{ws.neigh, stride, ws.dnum}, StoreExclusive{item_start}, &c->level_base[dsplit],
-                        0, ws.scan, total, &c->error, a2, ScanCount{}, 1);
-        if (e != cudaSuccess) return e;
-        const int item_cap = ws.cap.nodes;   // partial buffer holds cap.nodes float pairs
-        k_div_chunk_count<<<PSR_GRID(ws, 1), 1, 0, a2>>>(c, dsplit, total, item_cap, n_items);
-        FF* partial = reinterpret_cast<FF*>(ws.cg_partial);
-        k_div_chunks<<<PSR_GRID(ws, ws.num_sms * 8), kBlock, 0, a2>>>(c, D, dsplit, ws.res, n_items, item_start, ws.enc, ws.didx,
-                                                        ws.dnum, ws.neigh, stride, vx, vy, vz, ws.dff, partial);
-        k_div_coarse_reduce<<<PSR_GRID(ws, grid_for(ws, 1 << 16)), kBlock, 0, a2>>>(c, dsplit, item_start, n_items, partial,
-                                                                     ws.divg);
-        if (!ws.chain) e = cudaEventRecord(ws.ev_join, a2);
+    // item_start / partial live in the (otherwise idle) CG scratch; the chunks were counted and
+    // numbered beside the mesh records
+    const int dsplit = div_split(D);
+    const DivArgs a{c, D, dsplit, ws.res, ws.enc, ws.didx, ws.dnum, ws.neigh, stride, vx, vy, vz, ws.dff,
+                    (const unsigned*)ws.cg_r, reinterpret_cast<FF*>(ws.cg_partial), ws.divg};
+    if (!ws.chain) {
+        const cudaError_t e = cudaStreamWaitEvent(s, ws.ev_geo, 0);
         if (e != cudaSuccess) return e;
     }
-    k_div_fine<<<PSR_GRID(ws, ws.num_sms * 8), kBlock, 0, s>>>(c, D, dsplit, ws.res, ws.enc, ws.didx, ws.dnum, ws.neigh, stride, vx,
-                                                 vy, vz, ws.dff, ws.divg);
-    k_div_leaf<<<PSR_GRID(ws, ws.num_sms * 8), kBlock, 0, s>>>(c, D, ws.res, ws.enc, ws.neigh, stride, vx, vy, vz, ws.dff, ws.divg);
-    if (dsplit > 0 && !ws.chain) {
-        e = cudaStreamWaitEvent(s, ws.ev_join, 0);
-        if (e != cudaSuccess) return e;
-    }
+    const dim3 g = PSR_GRID(ws, ws.num_sms * 8);
+    k_divergence<<<dim3(g.x, g.y, dsplit > 0 ? 3 : 2), kBlock, 0, s>>>(a);
+    if (dsplit > 0) k_div_coarse_reduce<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -135,24 +135,22 @@ __device__ __forceinline__ int edge_slot_of(int e, const int a[3]) {
 // ------------------------------------------------------------------------------------
 // octree vertex / edge / face records
 // ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_mesh_reset(const Counters* c, int* node_vtx, int* node_edge,
-                                                       int* node_face, int* ov_group, int* ov_sub, size_t stride) {
-    PSR_CLOUD(c, node_vtx, node_edge, node_face, ov_group, ov_sub);
-    const int M = c->n_nodes;
-    PSR_GRID_STRIDE(i, M) {
-        for (int k = 0; k < 8; ++k) node_vtx[(size_t)k * stride + i] = 0;
-        for (int k = 0; k < 12; ++k) node_edge[(size_t)k * stride + i] = 0;
-        for (int k = 0; k < 6; ++k) node_face[(size_t)k * stride + i] = 0;
-        for (int k = 0; k < 8; ++k) { ov_group[(size_t)k * stride + i] = -1; ov_sub[(size_t)k * stride + i] = -1; }
+// Ownership of a node's corners, edges (depth D) and faces from its neighbours' keys
+// (initVertexOwner, initEdgeArray, initFaceArray, mesh/BuildMeshGeometry.cu:42-101, :149-220,
+// :282-354): a node owns an element when no other cell around it has a smaller key.  Also clears
+// the back-pointers and overlays of the node; blockIdx.z = 1 clears the colour cell table.
+__global__ void __launch_bounds__(kBlock) k_mesh_owners(const Counters* c, int depth, const int* key, const int* neigh,
+                                                        size_t stride, unsigned char* vmask, unsigned short* emask,
+                                                        unsigned char* fmask, int* node_vtx, int* node_edge,
+                                                        int* node_face, int* ov_group, int* ov_sub, int* cell_table,
+                                                        int cells) {
+    PSR_CLOUD(c, key, neigh, vmask, emask, fmask, node_vtx, node_edge, node_face, ov_group, ov_sub, cell_table);
+    if (blockIdx.z == 1) {
+        PSR_GRID_STRIDE(i, cells) cell_table[i] = 0;
+        return;
     }
-}
-
-// vertex ownership (initVertexOwner, mesh/BuildMeshGeometry.cu:42-101): a node owns a
-// corner when no other cell around it has a smaller key
-__global__ void __launch_bounds__(kBlock) k_vertex_owner(const Counters* c, const int* key, const int* neigh,
-                                                         size_t stride, unsigned char* vmask) {
-    PSR_CLOUD(c, key, neigh, vmask);
     const int M = c->n_nodes;
+    const int bD = c->level_base[depth], mD = c->level_count[depth];
     PSR_GRID_STRIDE(i, M) {
         const int myk = key[i];
         unsigned smaller = 0;
@@ -166,6 +164,24 @@ __global__ void __launch_bounds__(kBlock) k_vertex_owner(const Counters* c, cons
 #pragma unroll
         for (int q = 0; q < 8; ++q) if (!(smaller & vertex_cells(q))) m |= 1u << q;
         vmask[i] = (unsigned char)m;
+        m = 0;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) if (!(smaller & face_cells(f))) m |= 1u << f;
+        fmask[i] = (unsigned char)m;
+        if ((unsigned)(i - bD) < (unsigned)mD) {
+            m = 0;
+#pragma unroll
+            for (int e = 0; e < 12; ++e) if (!(smaller & edge_cells(e))) m |= 1u << e;
+            emask[i - bD] = (unsigned short)m;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) node_vtx[(size_t)k * stride + i] = 0;
+#pragma unroll
+        for (int k = 0; k < 12; ++k) node_edge[(size_t)k * stride + i] = 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) node_face[(size_t)k * stride + i] = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { ov_group[(size_t)k * stride + i] = -1; ov_sub[(size_t)k * stride + i] = -1; }
     }
 }
 
@@ -204,48 +220,6 @@ struct VertexStore {
     __device__ void rebase() { PSR_CLOUD(vmask, ndepth, cx, cy, cz, vx, vy, vz, vowner, vkind, vdepth, err); }   // to cloud blockIdx.y
 };
 
-// maintainVertexNodePointer (mesh/BuildMeshGeometry.cu:108-147)
-__global__ void __launch_bounds__(kBlock) k_vertex_maintain(const Counters* c, const int* neigh, size_t stride,
-                                                            const int* vowner, const int* vkind, int* node_vtx) {
-    PSR_CLOUD(c, neigh, vowner, vkind, node_vtx);
-    const int V = c->n_vertices;
-    PSR_GRID_STRIDE(v, V) {
-        const int ow = vowner[v];
-        int mx, my, mz;
-        corner_sides(vkind[v], mx, my, mz);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int ax = (j & 1) ? mx : 0, ay = (j & 2) ? my : 0, az = (j & 4) ? mz : 0;
-            const int nb = neigh[(size_t)nslot(ax, ay, az) * stride + ow];
-            if (nb != -1) node_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * stride + nb] = v + 1;
-        }
-    }
-}
-
-// edge ownership for D-level nodes (initEdgeArray, mesh/BuildMeshGeometry.cu:149-220)
-__global__ void __launch_bounds__(kBlock) k_edge_owner(const Counters* c, int depth, const int* key, const int* neigh,
-                                                       size_t stride, unsigned short* emask) {
-    PSR_CLOUD(c, key, neigh, emask);
-    const int md = c->level_count[depth];
-    const int b = c->level_base[depth];
-    PSR_GRID_STRIDE(o, md) {
-        const int i = b + o;
-        const int myk = key[i];
-        unsigned smaller = 0;
-#pragma unroll
-        for (int k = 0; k < 27; ++k) {
-            if (k == 13 || k == 0 || k == 2 || k == 6 || k == 8 || k == 18 || k == 20 || k == 24 || k == 26)
-                continue;   // corner-diagonal cells touch no edge
-            const int nb = neigh[(size_t)k * stride + i];
-            if (nb != -1 && key[nb] < myk) smaller |= 1u << k;
-        }
-        unsigned m = 0;
-#pragma unroll
-        for (int e = 0; e < 12; ++e) if (!(smaller & edge_cells(e))) m |= 1u << e;
-        emask[o] = (unsigned short)m;
-    }
-}
-
 struct PopcLoad16 {
     const unsigned short* m;
     __device__ unsigned operator()(int i) const { return __popc((unsigned)m[i]); }
@@ -270,42 +244,6 @@ struct EdgeStore {
     __device__ void rebase() { PSR_CLOUD(emask, base_ptr, eowner, ekind, err); }   // to cloud blockIdx.y
 };
 
-// maintainEdgeNodePointer (mesh/BuildMeshGeometry.cu:222-280)
-__global__ void __launch_bounds__(kBlock) k_edge_maintain(const Counters* c, const int* neigh, size_t stride,
-                                                          const int* eowner, const int* ekind, int* node_edge) {
-    PSR_CLOUD(c, neigh, eowner, ekind, node_edge);
-    const int E = c->n_edges;
-    PSR_GRID_STRIDE(ei, E) {
-        const int ow = eowner[ei], kind = ekind[ei];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int a[3];
-            edge_offset(kind, j, a);
-            const int nb = neigh[(size_t)nslot(a[0], a[1], a[2]) * stride + ow];
-            if (nb != -1) node_edge[(size_t)edge_slot_of(kind, a) * stride + nb] = ei + 1;
-        }
-    }
-}
-
-// face ownership (initFaceArray, mesh/BuildMeshGeometry.cu:282-354)
-__global__ void __launch_bounds__(kBlock) k_face_owner(const Counters* c, const int* key, const int* neigh,
-                                                       size_t stride, unsigned char* fmask) {
-    PSR_CLOUD(c, key, neigh, fmask);
-    const int M = c->n_nodes;
-    PSR_GRID_STRIDE(i, M) {
-        const int myk = key[i];
-        unsigned m = 0;
-#pragma unroll
-        for (int f = 0; f < 6; ++f) {
-            int a[3] = {0, 0, 0};
-            a[f >> 1] = 2 * (f & 1) - 1;
-            const int nb = neigh[(size_t)nslot(a[0], a[1], a[2]) * stride + i];
-            if (!(nb != -1 && key[nb] < myk)) m |= 1u << f;
-        }
-        fmask[i] = (unsigned char)m;
-    }
-}
-
 struct FaceStore {
     const unsigned char* fmask;
     const int* key;
@@ -313,6 +251,7 @@ struct FaceStore {
     const int* parent;
     int depth;
     int *fowner, *fkind, *fhas;
+    int* face_hit;   // starts cleared
     int cap;
     unsigned* err;
     __device__ void operator()(int i, unsigned pre, unsigned cnt) const {
@@ -326,27 +265,111 @@ struct FaceStore {
             if (!((m >> f) & 1)) continue;
             fowner[q] = i;
             fkind[q] = f;
+            face_hit[q] = 0;
             fhas[q] = (parent[i] == -1) ? -1 : ((__ldg(&g_tab.parent_face_kind[son][f]) != -1) ? 1 : -1);
             ++q;
         }
     }
-    __device__ void rebase() { PSR_CLOUD(fmask, key, ndepth, parent, fowner, fkind, fhas, err); }   // to cloud blockIdx.y
+    __device__ void rebase() { PSR_CLOUD(fmask, key, ndepth, parent, fowner, fkind, fhas, face_hit, err); }   // to cloud blockIdx.y
 };
 
-// maintainFaceNodePointer (mesh/BuildMeshGeometry.cu:356-400)
-__global__ void __launch_bounds__(kBlock) k_face_maintain(const Counters* c, const int* neigh, size_t stride,
-                                                          const int* fowner, const int* fkind, int* node_face) {
-    PSR_CLOUD(c, neigh, fowner, fkind, node_face);
-    const int F = c->n_faces;
-    PSR_GRID_STRIDE(fi, F) {
-        const int ow = fowner[fi], kind = fkind[fi];
-        const int orient = kind >> 1, m = 2 * (kind & 1) - 1;
+// chunk count of every coarse node (depth < dsplit) of the divergence
+struct DivChunkLoad {
+    const int* neigh;
+    size_t stride;
+    const int* dnum;
+    __device__ unsigned operator()(int i) const {
+        int nb[27], dn[27];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            int a[3] = {0, 0, 0};
-            a[orient] = j ? m : 0;
-            const int nb = neigh[(size_t)nslot(a[0], a[1], a[2]) * stride + ow];
-            if (nb != -1) node_face[(size_t)((orient << 1) + (2 * a[orient] - m < 0 ? 1 : 0)) * stride + nb] = fi + 1;
+        for (int k = 0; k < 27; ++k) nb[k] = neigh[(size_t)k * stride + i];
+#pragma unroll
+        for (int k = 0; k < 27; ++k) dn[k] = dnum[nb[k] >= 0 ? nb[k] : 0];
+        unsigned n = 0;
+#pragma unroll
+        for (int k = 0; k < 27; ++k)
+            if (nb[k] >= 0) n += (unsigned)((dn[k] + kDivChunk - 1) / kDivChunk);
+        return n;
+    }
+    __device__ void rebase() { PSR_CLOUD(neigh, dnum); }   // to cloud blockIdx.y
+};
+struct DivChunkStore {
+    unsigned* item_start;
+    Counters* c;
+    int cap;
+    __device__ void operator()(int i, unsigned pre, unsigned) const { item_start[i] = pre; }
+    __device__ void done(unsigned total) const {
+        int n = (int)total;
+        if (n > cap) { atomicOr(&c->error, kErrCapacity); n = 0; }
+        c->n_div_items = n;
+    }
+    __device__ void rebase() { PSR_CLOUD(item_start, c); }   // to cloud blockIdx.y
+};
+
+// Back-pointers of the nodes around every vertex, edge and face (maintainVertexNodePointer,
+// maintainEdgeNodePointer, maintainFaceNodePointer, mesh/BuildMeshGeometry.cu:108-147, :222-280,
+// :356-400), blockIdx.z an element kind each; blockIdx.z = 3 counts the samples of the colour cells.
+__global__ void __launch_bounds__(kBlock) k_mesh_maintain(Counters* c, int depth, const int* neigh, size_t stride,
+                                                          const int* vowner, const int* vkind, int* node_vtx,
+                                                          const int* eowner, const int* ekind, int* node_edge,
+                                                          const int* fowner, const int* fkind, int* node_face, int g,
+                                                          const int* key, const int* point2node, int* cell_table) {
+    PSR_CLOUD(c, neigh, vowner, vkind, node_vtx, eowner, ekind, node_edge, fowner, fkind, node_face, key, point2node, cell_table);
+    if (blockIdx.z == 0) {
+        const int V = c->n_vertices;
+        PSR_GRID_STRIDE(v, V) {
+            const int ow = vowner[v];
+            int mx, my, mz;
+            corner_sides(vkind[v], mx, my, mz);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int ax = (j & 1) ? mx : 0, ay = (j & 2) ? my : 0, az = (j & 4) ? mz : 0;
+                const int nb = neigh[(size_t)nslot(ax, ay, az) * stride + ow];
+                if (nb != -1) node_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * stride + nb] = v + 1;
+            }
+        }
+    } else if (blockIdx.z == 1) {
+        const int E = c->n_edges;
+        PSR_GRID_STRIDE(ei, E) {
+            const int ow = eowner[ei], kind = ekind[ei];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                int a[3];
+                edge_offset(kind, j, a);
+                const int nb = neigh[(size_t)nslot(a[0], a[1], a[2]) * stride + ow];
+                if (nb != -1) node_edge[(size_t)edge_slot_of(kind, a) * stride + nb] = ei + 1;
+            }
+        }
+    } else if (blockIdx.z == 2) {
+        const int F = c->n_faces;
+        PSR_GRID_STRIDE(fi, F) {
+            const int ow = fowner[fi], kind = fkind[fi];
+            const int orient = kind >> 1, m = 2 * (kind & 1) - 1;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                int a[3] = {0, 0, 0};
+                a[orient] = j ? m : 0;
+                const int nb = neigh[(size_t)nslot(a[0], a[1], a[2]) * stride + ow];
+                if (nb != -1) node_face[(size_t)((orient << 1) + (2 * a[orient] - m < 0 ? 1 : 0)) * stride + nb] = fi + 1;
+            }
+        }
+    } else {
+        // run length of every occupied cell of level g at the last sample of its run (the samples are
+        // Morton-sorted)
+        const int n = c->n_points;
+        const int bD = c->level_base[depth];
+        const int sh = 3 * (depth - g);
+        auto cell = [&](int i) { return (unsigned)key[bD + point2node[i]] >> sh; };
+        if (blockIdx.x == 0 && threadIdx.x == 0) c->n_colour_cells = (1 << (3 * g)) + 1;
+        PSR_GRID_STRIDE(i, n) {
+            const unsigned m = cell(i);
+            if (i + 1 < n && cell(i + 1) == m) continue;
+            int lo = 0, hi = i;   // first sample of the run ending at i
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (cell(mid) < m) lo = mid + 1;
+                else hi = mid;
+            }
+            cell_table[m] = i + 1 - lo;
         }
     }
 }
@@ -620,6 +643,7 @@ struct GroupFlagLoad {
     __device__ void rebase() { PSR_CLOUD(sub_root, ndepth); }   // to cloud blockIdx.y
 };
 struct GroupFlagStore {
+    Counters* c;
     int* root_group;
     int* groups;
     int max_groups;
@@ -632,25 +656,23 @@ struct GroupFlagStore {
             groups[(size_t)g * kGroupRec + 1] = r;
         }
     }
-    __device__ void rebase() { PSR_CLOUD(root_group, groups, err); }   // to cloud blockIdx.y
+    __device__ void done(unsigned total) const {
+        int ng = (int)total;
+        if (ng > max_groups) { atomicOr(err, kErrCapacity); ng = 0; }
+        c->n_group_flags = ng;
+    }
+    __device__ void rebase() { PSR_CLOUD(c, root_group, groups, err); }   // to cloud blockIdx.y
 };
 
-__global__ void k_group_count(Counters* c, const unsigned* total, int max_groups) {
-    PSR_CLOUD(c, total);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int ng = (int)*total;
-        if (ng > max_groups) { atomicOr(&c->error, kErrCapacity); ng = 0; }
-        c->n_groups = ng;
-    }
-}
-
-// per-group sizes (thread per group)
-__global__ void __launch_bounds__(kBlock) k_group_sizes(Counters* c, int depth, const int* sub_root,
-                                                        const int* ndepth, int* groups) {
-    PSR_CLOUD(c, sub_root, ndepth, groups);
-    const int ng = c->n_groups;
-    const int R = c->n_subroots;
-    PSR_GRID_STRIDE(g, ng) {
+// per-group sizes; their prefixes number the groups' virtual nodes
+struct GroupSizeLoad {
+    Counters* c;
+    int depth;
+    const int* sub_root;
+    const int* ndepth;
+    int* groups;
+    __device__ unsigned operator()(int g) const {
+        const int ng = c->n_group_flags, R = c->n_subroots;
         int* G = groups + (size_t)g * kGroupRec;
         const int first = G[1];
         const int next = (g + 1 < ng) ? groups[(size_t)(g + 1) * kGroupRec + 1] : R;
@@ -663,61 +685,26 @@ __global__ void __launch_bounds__(kBlock) k_group_sizes(Counters* c, int depth, 
         G[2] = (int)n;
         if (nodes > 0x3fffffffLL) atomicOr(&c->error, kErrCapacity);
         G[4] = nodes > 0x3fffffffLL ? 0x3fffffff : (int)nodes;
+        return (unsigned)G[4];
     }
-}
-
-struct GroupFieldLoad {
-    const int* groups;
-    int field;
-    __device__ unsigned operator()(int g) const { return (unsigned)groups[(size_t)g * kGroupRec + field]; }
-    __device__ void rebase() { PSR_CLOUD(groups); }   // to cloud blockIdx.y
+    __device__ void rebase() { PSR_CLOUD(c, sub_root, ndepth, groups); }   // to cloud blockIdx.y
 };
-struct GroupFieldStore {
+struct GroupSizeStore {
+    Counters* c;
     int* groups;
-    int field;
-    __device__ void operator()(int g, unsigned pre, unsigned) const { groups[(size_t)g * kGroupRec + field] = (int)pre; }
-    __device__ void rebase() { PSR_CLOUD(groups); }   // to cloud blockIdx.y
-};
-
-// the virtual numbering of all groups must fit beside the octree indices (na + index)
-__global__ void k_group_totals(Counters* c, const unsigned* node_total, int na) {
-    PSR_CLOUD(c, node_total);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const unsigned nt = *node_total;
-        if (nt > 0x7fffffffu - (unsigned)na) {
+    int na;
+    __device__ void operator()(int g, unsigned pre, unsigned) const { groups[(size_t)g * kGroupRec + 3] = (int)pre; }
+    // the virtual numbering of all groups must fit beside the octree indices (na + index)
+    __device__ void done(unsigned total) const {
+        int ng = c->n_group_flags;
+        if (total > 0x7fffffffu - (unsigned)na) {
             atomicOr(&c->error, kErrCapacity);
-            c->n_groups = 0;
+            ng = 0;
         }
+        c->n_groups = ng;
     }
-}
-
-// per root: its depth, the octree node it stands for, and the redirected child slot of
-// its parent (overlay)
-__global__ void __launch_bounds__(kBlock) k_root_overlay(const Counters* c, int depth, const int* sub_root,
-                                                         const int* ndepth, const int* key, const int* parent,
-                                                         const int* neigh, const int* root_group, const int* groups,
-                                                         int* sub_root_depth, int* root_self, int* ov_group,
-                                                         int* ov_sub, size_t stride) {
-    PSR_CLOUD(c, sub_root, ndepth, key, parent, neigh, root_group, groups, sub_root_depth, root_self, ov_group, ov_sub);
-    const int R = c->n_subroots;
-    const int ng = c->n_groups;
-    PSR_GRID_STRIDE(r, R) {
-        const int node = sub_root[r];
-        const int rd = ndepth[node];
-        sub_root_depth[r] = rd;
-        const int self = neigh[(size_t)13 * stride + node];   // its neighs[13] in the reference
-        root_self[r] = (self == -1) ? node : self;
-        const int g = root_group[r];
-        if (g < 0 || g >= ng) continue;
-        const int q = r - groups[(size_t)g * kGroupRec + 1];
-        const int son = (key[node] >> (3 * (depth - rd))) & 7;
-        const int pa = parent[node];
-        if (pa >= 0) {
-            ov_group[(size_t)son * stride + pa] = g;
-            ov_sub[(size_t)son * stride + pa] = q;
-        }
-    }
-}
+    __device__ void rebase() { PSR_CLOUD(c, groups); }   // to cloud blockIdx.y
+};
 
 // ---- subdivision, breadth-first over live nodes ----------------------------------------
 // Virtual numbering (singleRebuildArray :599-635 / wholeRebuildArray :1110-1168): group g
@@ -734,9 +721,9 @@ __device__ __forceinline__ int sub_level_off(int rd, int n, int d) {
     return off;
 }
 
-// per-depth candidate bookkeeping (Counters::sub_*): [d] for depth d; one lane per depth
-__global__ void k_sub_setup(Counters* c, int depth, const int* sub_root_depth, int cap_nodes) {
-    PSR_CLOUD(c, sub_root_depth);
+// per-depth candidate bookkeeping (Counters::sub_*): [d] for depth d; one thread per depth
+__device__ __forceinline__ void sub_setup(Counters* c, int depth, const int* sub_root, const int* ndepth,
+                                          int cap_nodes) {
     const int d = threadIdx.x;
     const int R = c->n_subroots;
     __shared__ int s_end[kMaxDepth + 2];
@@ -744,7 +731,7 @@ __global__ void k_sub_setup(Counters* c, int depth, const int* sub_root_depth, i
         int lo = 0, hi = R;   // first root deeper than d (roots are in depth order)
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (sub_root_depth[mid] <= d) lo = mid + 1;
+            if (ndepth[sub_root[mid]] <= d) lo = mid + 1;
             else hi = mid;
         }
         s_end[d] = lo;
@@ -752,19 +739,19 @@ __global__ void k_sub_setup(Counters* c, int depth, const int* sub_root_depth, i
     __syncthreads();
     if (d <= depth + 1) {
         const int start = (d > 0) ? s_end[d - 1] : 0;
+        const int n = (c->n_groups > 0) ? s_end[d] - start : 0;
         c->sub_rstart[d] = start;
-        c->sub_nroots[d] = (c->n_groups > 0) ? s_end[d] - start : 0;
-        c->sub_cand[d] = 0;
+        c->sub_nroots[d] = n;
         c->sub_cbase[d] = 0;
         c->sub_lbase[d] = 0;
         c->sub_nlive[d] = 0;
-    }
-    __syncthreads();
-    if (d == 0) {
-        if (c->sub_nroots[1] > cap_nodes) atomicOr(&c->error, kErrCapacity);
-        else c->sub_cand[1] = c->sub_nroots[1];
-        c->n_sub_nodes = 0;
-        c->n_sub_dnodes = 0;
+        c->sub_cand[d] = 0;
+        if (d == 1) {
+            if (n > cap_nodes) atomicOr(&c->error, kErrCapacity);
+            else c->sub_cand[1] = n;
+            c->n_sub_nodes = 0;
+            c->n_sub_dnodes = 0;
+        }
     }
 }
 
@@ -812,20 +799,35 @@ __device__ __forceinline__ int sub_value_node(int v, int na, const int* G, const
 
 // Levels up to a root's depth are the same for every cell below that root: their sum is one
 // tensor-product quadratic on the root's cell, kept as its 27 Bernstein coefficients
-// (root_poly[k][r], k < 27; [27][r]: sum |y| of those levels).  A cell inside it takes
+// (k_root_setup: root_poly[k][r], k < 27; [27][r]: sum |y| of those levels).  A cell inside it takes
 // them by Bernstein subdivision: with the cell at [a, b] of the root's unit interval, the
 // new coefficients are the blossom values P(a, a), P(a, b), P(b, b) -- convex weights, exact
 // for these dyadic a, b.
-__global__ void __launch_bounds__(kBlock) k_root_poly(const Counters* c, int depth, const int* sub_root,
-                                                      const int* ndepth, const float* ctr_x, const float* ctr_y,
-                                                      const float* ctr_z, const int* neigh, size_t stride,
-                                                      const int* parent, const int* enc, const float* x,
-                                                      float* root_poly, int cap_poly) {
-    PSR_CLOUD(c, sub_root, ndepth, ctr_x, ctr_y, ctr_z, neigh, parent, enc, x, root_poly);
-    const int R = c->n_subroots < cap_poly ? c->n_subroots : cap_poly;
+// Per root: the octree node it stands for, the redirected child slot of its parent (overlay) and
+// its polynomial; block 0 also sets up the per-depth bookkeeping.
+__global__ void __launch_bounds__(kBlock) k_root_setup(Counters* c, int depth, const int* sub_root, const int* ndepth,
+                                                       const int* key, const int* root_group, const int* groups,
+                                                       int* root_self, int* ov_group, int* ov_sub, const float* ctr_x,
+                                                       const float* ctr_y, const float* ctr_z, const int* neigh,
+                                                       size_t stride, const int* parent, const int* enc, const float* x,
+                                                       float* root_poly, int cap_poly, int cap_nodes) {
+    PSR_CLOUD(c, sub_root, ndepth, key, root_group, groups, root_self, ov_group, ov_sub, ctr_x, ctr_y, ctr_z, neigh, parent, enc, x, root_poly);
+    if (blockIdx.x == 0) sub_setup(c, depth, sub_root, ndepth, cap_nodes);
+    const int R = c->n_subroots;
+    const int ng = c->n_groups;
     PSR_GRID_STRIDE(r, R) {
         const int node = sub_root[r];
         const int rd = ndepth[node];
+        const int self = neigh[(size_t)13 * stride + node];   // its neighs[13] in the reference
+        root_self[r] = (self == -1) ? node : self;
+        const int g = root_group[r];
+        const int pa = parent[node];
+        if (g >= 0 && g < ng && pa >= 0) {
+            const int son = (key[node] >> (3 * (depth - rd))) & 7;
+            ov_group[(size_t)son * stride + pa] = g;
+            ov_sub[(size_t)son * stride + pa] = r - groups[(size_t)g * kGroupRec + 1];
+        }
+        if (r >= cap_poly) continue;
         const float qx = ctr_x[node], qy = ctr_y[node], qz = ctr_z[node];
         float C[27];
 #pragma unroll
@@ -857,6 +859,7 @@ __device__ __forceinline__ void blossom3(float a, float b, float (&M)[3][3]) {
 }
 
 // C += the root polynomial P subdivided to the cell at Morton code rel (m levels below it)
+template <bool kReadOnly>
 __device__ __forceinline__ void add_subdivided(const float* P, size_t pstride, unsigned rel, int m, float (&C)[27]) {
     int i3[3] = {0, 0, 0};
     for (int j = 0; j < m; ++j)
@@ -869,7 +872,7 @@ __device__ __forceinline__ void add_subdivided(const float* P, size_t pstride, u
     blossom3((float)i3[2] * inv, (float)(i3[2] + 1) * inv, Mz);
     float p[27];
 #pragma unroll
-    for (int k = 0; k < 27; ++k) p[k] = __ldg(P + (size_t)k * pstride);   // written by an earlier launch
+    for (int k = 0; k < 27; ++k) p[k] = kReadOnly ? __ldg(P + (size_t)k * pstride) : P[(size_t)k * pstride];
     float T1[27], T2[27];
 #pragma unroll
     for (int a = 0; a < 3; ++a)
@@ -939,6 +942,9 @@ __device__ __forceinline__ unsigned child_touch(unsigned pt, int ch) {
 
 // One candidate of depth d (computeRebuildNeighbor :669-696 for its neighbours): its record,
 // its neighbours and its sign test; returns 1 when it stays live.
+// kShared: several depths in one launch, so what an earlier depth wrote may not be read through the
+// read-only path.
+template <bool kShared>
 struct SubLevelLoad {
     const Counters* c;
     int d, depth, na;
@@ -958,6 +964,8 @@ struct SubLevelLoad {
     const float* root_poly;
     int cap_poly;
     SubArrays A;
+    template <class T>
+    static __device__ T rd(const T* p) { return kShared ? *p : __ldg(p); }
     __device__ unsigned operator()(int i) const {
         const int nl_prev = c->sub_nlive[d - 1];
         if (i < 8 * nl_prev) {
@@ -969,7 +977,7 @@ struct SubLevelLoad {
                 float C[27];
 #pragma unroll
                 for (int kk = 0; kk < 27; ++kk) C[kk] = 0.0f;
-                add_subdivided(A.poly + pl, (size_t)A.cap_live, (unsigned)(i & 7), 1, C);
+                add_subdivided<!kShared>(A.poly + pl, (size_t)A.cap_live, (unsigned)(i & 7), 1, C);
                 const float mag = A.poly[(size_t)27 * A.cap_live + pl];
                 float lo = C[0], hi = C[0];
 #pragma unroll
@@ -1074,7 +1082,7 @@ struct SubLevelLoad {
                     const int kk = 9 * ix + q;
                     int lp, lc;
                     nb_lut(son, kk, lp, lc);
-                    const int t = __ldg(rowp + (size_t)lp * rstride);
+                    const int t = rd(rowp + (size_t)lp * rstride);
                     np[q] = has_row ? t : -1;
                 }
                 int og[9], fc[9], os[9];
@@ -1143,7 +1151,7 @@ struct SubLevelLoad {
         const int prec = (pslot >= 0) ? pslot : -2 - pa;
         // nearest contributing node on the path to the root (itself when it contributes;
         // roots always do): lets the value chains skip non-contributing levels in one hop
-        const int jump = contrib ? slot : ((pslot >= 0) ? __ldg(A.jump + pslot) : slot);
+        const int jump = contrib ? slot : ((pslot >= 0) ? rd(A.jump + pslot) : slot);
         // Bernstein coefficients of the levels up to d on the node's cell
         float C[27], mag;
         if (at_root_depth) {
@@ -1153,8 +1161,8 @@ struct SubLevelLoad {
             const int pl = c->sub_lbase[d - 1] + (i >> 3);   // the parent's live entry
 #pragma unroll
             for (int kk = 0; kk < 27; ++kk) C[kk] = 0.0f;
-            add_subdivided(A.poly + pl, (size_t)A.cap_live, (unsigned)(i & 7), 1, C);
-            mag = __ldg(A.poly + (size_t)27 * A.cap_live + pl);
+            add_subdivided<!kShared>(A.poly + pl, (size_t)A.cap_live, (unsigned)(i & 7), 1, C);
+            mag = rd(A.poly + (size_t)27 * A.cap_live + pl);
             if (contrib) {   // its own level (octree neighbours; never for an interior node)
                 const float sc = (float)(1 << d);
                 const int base = (1 << d) - 1;
@@ -1175,7 +1183,7 @@ struct SubLevelLoad {
         for (int kk = 0; kk < 27; ++kk) stash[kk * kBlock + threadIdx.x] = C[kk];
         stash[27 * kBlock + threadIdx.x] = mag;
         const unsigned touch = at_root_depth ? 0x3fu
-                                             : child_touch(__ldg(A.touch + c->sub_lbase[d - 1] + (i >> 3)), i & 7);
+                                             : child_touch(rd(A.touch + c->sub_lbase[d - 1] + (i >> 3)), i & 7);
         stash[28 * kBlock + threadIdx.x] = __uint_as_float(touch);
         stash[29 * kBlock + threadIdx.x] = __int_as_float(vnode);
         if (interior) {
@@ -1246,6 +1254,29 @@ struct SubLevelStore {
     __device__ void rebase() { PSR_CLOUD(c, A, err); }   // to cloud blockIdx.y
 };
 
+// The depths 1 .. dmax (at most 8 + 64 + 512 candidates) in one CTA: the scans of so few elements
+// cost a launch each otherwise.
+__global__ void __launch_bounds__(kBlock) k_sub_coarse(SubLevelLoad<true> load, SubLevelStore store, int dmax) {
+    PSR_CLOUD(load, store);
+    __shared__ unsigned s_warp[kBlock / 32 + 1];
+    for (int d = 1; d <= dmax; ++d) {
+        load.d = d;
+        store.d = d;
+        const int n = *(volatile const int*)&load.c->sub_cand[d];
+        unsigned run = 0;
+        for (int base = 0; base < n; base += kBlock) {
+            const int i = base + (int)threadIdx.x;
+            const unsigned v = i < n ? load(i) : 0u;
+            unsigned excl;
+            const unsigned sum = block_exclusive_scan(v, excl, s_warp);
+            if (i < n) store(i, run + excl, v);
+            run += sum;
+        }
+        if (threadIdx.x == 0) store.done(run);
+        __syncthreads();   // the depth's records and counts before the next depth reads them
+    }
+}
+
 // index of virtual node v among the live depth-D cells (sorted), or -1
 __device__ __forceinline__ int live_index(const int* lv_vnode, int n, int v) {
     int lo = 0, hi = n;
@@ -1260,8 +1291,8 @@ __device__ __forceinline__ int live_index(const int* lv_vnode, int n, int v) {
 // per live depth-D cell: the live index of each same-depth sub neighbour (-1: none, an
 // octree node, or a cell with a certain sign); one thread per (cell, slot)
 __global__ void __launch_bounds__(kBlock) k_sub_live_neigh(const Counters* c, int depth, SubArrays A,
-                                                           int* lv_nb, size_t dstride, int na) {
-    PSR_CLOUD(c, A, lv_nb);
+                                                           int* lv_nb, size_t dstride, int na, int* group_live) {
+    PSR_CLOUD(c, A, lv_nb, group_live);
     const int nl = c->n_sub_dnodes;
     const int lb = c->sub_lbase[depth];
     const long long n = 27LL * nl;
@@ -1269,6 +1300,10 @@ __global__ void __launch_bounds__(kBlock) k_sub_live_neigh(const Counters* c, in
         const int L = (int)(t / 27), k = (int)(t - 27LL * L);
         const int v = A.neigh[(size_t)k * A.cstride + A.live[lb + L]];
         lv_nb[(size_t)k * dstride + L] = (k == 13) ? L : ((v >= na) ? live_index(A.lv_vnode, nl, v - na) : -1);
+        if (k == 13) {   // a group's live cells are consecutive
+            const int g = A.group[A.live[lb + L]];
+            if (L == 0 || A.group[A.live[lb + L - 1]] != g) group_live[g] = L;
+        }
     }
 }
 
@@ -1278,10 +1313,11 @@ __global__ void __launch_bounds__(kBlock) k_sub_live_neigh(const Counters* c, in
 // keep their owners (every cell around a crossing edge has a sign change, so is live), and a
 // vertex value does not depend on the cell that evaluates it (the same nonzero terms in the
 // same order), so the mesh is unchanged.
-__global__ void __launch_bounds__(kBlock) k_sub_vertex_owner(const Counters* c, int depth, SubArrays A,
-                                                             const int* lv_nb, size_t dstride,
-                                                             unsigned char* s_vmask) {
-    PSR_CLOUD(c, A, lv_nb, s_vmask);
+// Edges likewise (initSubdivideEdgeArray :812-886).
+__global__ void __launch_bounds__(kBlock) k_sub_owners(const Counters* c, int depth, SubArrays A, const int* lv_nb,
+                                                       size_t dstride, unsigned char* s_vmask,
+                                                       unsigned short* s_emask) {
+    PSR_CLOUD(c, A, lv_nb, s_vmask, s_emask);
     const int nl = c->n_sub_dnodes;
     const int lb = c->sub_lbase[depth];
     PSR_GRID_STRIDE(L, nl) {
@@ -1297,6 +1333,10 @@ __global__ void __launch_bounds__(kBlock) k_sub_vertex_owner(const Counters* c, 
 #pragma unroll
         for (int q = 0; q < 8; ++q) if (!(smaller & vertex_cells(q))) m |= 1u << q;
         s_vmask[L] = (unsigned char)m;
+        m = 0;
+#pragma unroll
+        for (int e = 0; e < 12; ++e) if (!(smaller & edge_cells(e))) m |= 1u << e;
+        s_emask[L] = (unsigned short)m;
     }
 }
 
@@ -1329,49 +1369,6 @@ struct SubVertexStore {
     __device__ void rebase() { PSR_CLOUD(vmask, c, A, vx, vy, vz, vowner, vkind, err); }   // to cloud blockIdx.y
 };
 
-// maintainSubdivideVertexNodePointer (:765-810): s_vtx indexed by live cell
-__global__ void __launch_bounds__(kBlock) k_sub_vertex_maintain(const Counters* c, const int* lv_nb,
-                                                                size_t dstride, const int* vowner, const int* vkind,
-                                                                int* s_vtx) {
-    PSR_CLOUD(c, lv_nb, vowner, vkind, s_vtx);
-    const int V = c->n_sub_vertices;
-    PSR_GRID_STRIDE(v, V) {
-        const int ow = vowner[v];
-        int mx, my, mz;
-        corner_sides(vkind[v], mx, my, mz);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int ax = (j & 1) ? mx : 0, ay = (j & 2) ? my : 0, az = (j & 4) ? mz : 0;
-            const int nb = lv_nb[(size_t)nslot(ax, ay, az) * dstride + ow];
-            if (nb >= 0) s_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * dstride + nb] = v + 1;
-        }
-    }
-}
-
-// edge ownership among the live depth-D cells (initSubdivideEdgeArray :812-886)
-__global__ void __launch_bounds__(kBlock) k_sub_edge_owner(const Counters* c, int depth, SubArrays A,
-                                                           const int* lv_nb, size_t dstride,
-                                                           unsigned short* s_emask) {
-    PSR_CLOUD(c, A, lv_nb, s_emask);
-    const int nl = c->n_sub_dnodes;
-    const int lb = c->sub_lbase[depth];
-    PSR_GRID_STRIDE(L, nl) {
-        const int myk = A.key[A.live[lb + L]];
-        unsigned smaller = 0;
-#pragma unroll
-        for (int k = 0; k < 27; ++k) {
-            if (k == 13 || k == 0 || k == 2 || k == 6 || k == 8 || k == 18 || k == 20 || k == 24 || k == 26)
-                continue;   // corner-diagonal cells touch no edge
-            const int nb = lv_nb[(size_t)k * dstride + L];
-            if (nb >= 0 && A.key[A.live[lb + nb]] < myk) smaller |= 1u << k;
-        }
-        unsigned m = 0;
-#pragma unroll
-        for (int e = 0; e < 12; ++e) if (!(smaller & edge_cells(e))) m |= 1u << e;
-        s_emask[L] = (unsigned short)m;
-    }
-}
-
 struct SubEdgeStore {
     const unsigned short* emask;
     int *eowner, *ekind;
@@ -1390,19 +1387,37 @@ struct SubEdgeStore {
     __device__ void rebase() { PSR_CLOUD(emask, eowner, ekind, edge_of_live, err); }   // to cloud blockIdx.y
 };
 
-// maintainSubdivideEdgeNodePointer (:888-949)
-__global__ void __launch_bounds__(kBlock) k_sub_edge_maintain(const Counters* c, const int* lv_nb, size_t dstride,
-                                                              const int* eowner, const int* ekind, int* s_edge) {
-    PSR_CLOUD(c, lv_nb, eowner, ekind, s_edge);
-    const int E = c->n_sub_edges;
-    PSR_GRID_STRIDE(ei, E) {
-        const int ow = eowner[ei], kind = ekind[ei];
+// maintainSubdivideVertexNodePointer (:765-810) and maintainSubdivideEdgeNodePointer (:888-949), an
+// element kind per blockIdx.z: s_vtx, s_edge indexed by live cell.  They need no clearing: every
+// slot of a live cell is written by the owner of that vertex / edge.
+__global__ void __launch_bounds__(kBlock) k_sub_maintain(const Counters* c, const int* lv_nb, size_t dstride,
+                                                         const int* vowner, const int* vkind, int* s_vtx,
+                                                         const int* eowner, const int* ekind, int* s_edge) {
+    PSR_CLOUD(c, lv_nb, vowner, vkind, s_vtx, eowner, ekind, s_edge);
+    if (blockIdx.z == 0) {
+        const int V = c->n_sub_vertices;
+        PSR_GRID_STRIDE(v, V) {
+            const int ow = vowner[v];
+            int mx, my, mz;
+            corner_sides(vkind[v], mx, my, mz);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int a[3];
-            edge_offset(kind, j, a);
-            const int nb = lv_nb[(size_t)nslot(a[0], a[1], a[2]) * dstride + ow];
-            if (nb >= 0) s_edge[(size_t)edge_slot_of(kind, a) * dstride + nb] = ei + 1;
+            for (int j = 0; j < 8; ++j) {
+                const int ax = (j & 1) ? mx : 0, ay = (j & 2) ? my : 0, az = (j & 4) ? mz : 0;
+                const int nb = lv_nb[(size_t)nslot(ax, ay, az) * dstride + ow];
+                if (nb >= 0) s_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * dstride + nb] = v + 1;
+            }
+        }
+    } else {
+        const int E = c->n_sub_edges;
+        PSR_GRID_STRIDE(ei, E) {
+            const int ow = eowner[ei], kind = ekind[ei];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                int a[3];
+                edge_offset(kind, j, a);
+                const int nb = lv_nb[(size_t)nslot(a[0], a[1], a[2]) * dstride + ow];
+                if (nb >= 0) s_edge[(size_t)edge_slot_of(kind, a) * dstride + nb] = ei + 1;
+            }
         }
     }
 }
@@ -1579,24 +1594,30 @@ struct SubCubeLoad {
     __device__ void rebase() { PSR_CLOUD(s_vtx, vvalue, cube_class, err); }   // to cloud blockIdx.y
 };
 
-// triangles of a live cell; indices relative to its group's first crossing
+// triangles of a live cell; indices relative to its group's first crossing (the crossing prefix at
+// the first edge of the group's first live cell).  The last element fixes the staged counts.
 struct SubCubeStore {
     const int* cube_class;
     const int* s_edge;
     size_t dstride;
     const unsigned* ecross;
-    const unsigned* group_cross0;   // per group: crossing prefix at its first edge
-    const Counters* c;
+    const unsigned* edge_of_live;
+    const int* group_live;
+    unsigned* tri_of_live;   // sub-triangle prefix per live cell (for the part table)
+    Counters* c;
     int depth;
     SubArrays A;
     int* part_t;
     const int* toff_ptr;
-    int cap;
+    int cap, cap_v;
+    int *n_parts, *n_staged_v, *n_staged_t;
     unsigned* err;
     __device__ void operator()(int L, unsigned pre, unsigned cnt) const {
+        tri_of_live[L] = pre;
         if (!cnt) return;
         const int g = A.group[A.live[c->sub_lbase[depth] + L]];
-        const unsigned base = group_cross0[g];
+        const unsigned e0 = edge_of_live[group_live[g]];
+        const unsigned base = ((int)e0 < c->n_sub_edges) ? ecross[e0] : (unsigned)c->n_sub_cross;
         const int cls = cube_class[L];
         const unsigned long long tri = __ldg(&g_tab.mc_tri[cls]);
         for (int t = 0; t < (int)cnt; ++t) {
@@ -1609,7 +1630,15 @@ struct SubCubeStore {
             }
         }
     }
-    __device__ void rebase() { PSR_CLOUD(cube_class, s_edge, ecross, group_cross0, c, A, part_t, toff_ptr, err); }   // to cloud blockIdx.y
+    __device__ void done(unsigned total) const {
+        *n_parts = 1 + c->n_groups;
+        const int nv = c->n_cross + c->n_sub_cross;
+        const int nt = c->n_tri + ((int)total < cap ? (int)total : cap);
+        if (nv > cap_v || nt > cap) atomicOr(&c->error, kErrCapacity);
+        *n_staged_v = nv < cap_v ? nv : cap_v;
+        *n_staged_t = nt < cap ? nt : cap;
+    }
+    __device__ void rebase() { PSR_CLOUD(cube_class, s_edge, ecross, edge_of_live, group_live, tri_of_live, c, A, part_t, toff_ptr, n_parts, n_staged_v, n_staged_t, err); }   // to cloud blockIdx.y
 };
 
 // first live index at or after virtual node v
@@ -1624,41 +1653,48 @@ __device__ __forceinline__ int live_lower_bound(const int* lv_vnode, int n, int 
 }
 
 // per-group first sub edge / first crossing / first triangle -> part table
-// parts: [0] main, [1 + g] group g.  part record: vstart, vcount, tstart, tcount
-__global__ void k_part_table(Counters* c, int depth, const int* groups, const int* lv_vnode,
-                             const unsigned* edge_of_live, const unsigned* ecross_sub, const unsigned* tri_of_live,
-                             unsigned* group_cross0, int* parts) {
-    PSR_CLOUD(c, groups, lv_vnode, edge_of_live, ecross_sub, tri_of_live, group_cross0, parts);
-    const int ng = c->n_groups;
-    const int nE = c->n_sub_edges;
-    const int nl = c->n_sub_dnodes;
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        parts[0] = 0;
-        parts[1] = c->n_cross;
-        parts[2] = 0;
-        parts[3] = c->n_tri;
+// parts: [0] main, [1 + g] group g.  part record: vstart, vcount, tstart, tcount.
+// A job of the launch that scans the staged vertices.
+struct PartTableJob {
+    const Counters* c;
+    int depth;
+    const int* groups;
+    const int* lv_vnode;
+    const unsigned *edge_of_live, *ecross_sub, *tri_of_live;
+    int* parts;
+    static constexpr bool kUsed = true;
+    __device__ void run(unsigned*) {
+        PSR_CLOUD(c, groups, lv_vnode, edge_of_live, ecross_sub, tri_of_live, parts);
+        const int ng = c->n_groups;
+        const int nE = c->n_sub_edges;
+        const int nl = c->n_sub_dnodes;
+        if (threadIdx.x == 0 && blockIdx.x == 0) {
+            parts[0] = 0;
+            parts[1] = c->n_cross;
+            parts[2] = 0;
+            parts[3] = c->n_tri;
+        }
+        PSR_GRID_STRIDE(g, ng) {   // one thread per group (independent entries)
+            const int* G = groups + (size_t)g * kGroupRec;
+            const int v0 = G[3] + sub_level_off(G[0], G[2], depth);
+            const int v1 = G[3] + G[4];
+            // first sub edge of the group = edge prefix at its first live cell
+            const int L0 = live_lower_bound(lv_vnode, nl, v0);
+            const int L1 = live_lower_bound(lv_vnode, nl, v1);
+            const int e0 = (L0 < nl) ? (int)edge_of_live[L0] : nE;
+            const int e1 = (L1 < nl) ? (int)edge_of_live[L1] : nE;
+            const unsigned x0 = (e0 < nE) ? ecross_sub[e0] : (unsigned)c->n_sub_cross;
+            const unsigned x1 = (e1 < nE) ? ecross_sub[e1] : (unsigned)c->n_sub_cross;
+            const unsigned t0 = (L0 < nl) ? tri_of_live[L0] : (unsigned)c->n_sub_tri;
+            const unsigned t1 = (L1 < nl) ? tri_of_live[L1] : (unsigned)c->n_sub_tri;
+            int* P = parts + 4 * (size_t)(g + 1);
+            P[0] = c->n_cross + (int)x0;
+            P[1] = (int)(x1 - x0);
+            P[2] = c->n_tri + (int)t0;
+            P[3] = (int)(t1 - t0);
+        }
     }
-    PSR_GRID_STRIDE(g, ng) {   // one thread per group (independent entries)
-        const int* G = groups + (size_t)g * kGroupRec;
-        const int v0 = G[3] + sub_level_off(G[0], G[2], depth);
-        const int v1 = G[3] + G[4];
-        // first sub edge of the group = edge prefix at its first live cell
-        const int L0 = live_lower_bound(lv_vnode, nl, v0);
-        const int L1 = live_lower_bound(lv_vnode, nl, v1);
-        const int e0 = (L0 < nl) ? (int)edge_of_live[L0] : nE;
-        const int e1 = (L1 < nl) ? (int)edge_of_live[L1] : nE;
-        const unsigned x0 = (e0 < nE) ? ecross_sub[e0] : (unsigned)c->n_sub_cross;
-        const unsigned x1 = (e1 < nE) ? ecross_sub[e1] : (unsigned)c->n_sub_cross;
-        const unsigned t0 = (L0 < nl) ? tri_of_live[L0] : (unsigned)c->n_sub_tri;
-        const unsigned t1 = (L1 < nl) ? tri_of_live[L1] : (unsigned)c->n_sub_tri;
-        group_cross0[g] = x0;
-        int* P = parts + 4 * (size_t)(g + 1);
-        P[0] = c->n_cross + (int)x0;
-        P[1] = (int)(x1 - x0);
-        P[2] = c->n_tri + (int)t0;
-        P[3] = (int)(t1 - t0);
-    }
-}
+};
 
 // ------------------------------------------------------------------------------------
 // insertion (insertTriangle :1247-1282): drop vertices with |x| < 1e-6, offset triangle
@@ -1673,17 +1709,23 @@ struct KeepVertexStore {
     const float* part_v;
     float* mesh_v;
     unsigned* kept_prefix;
+    double* nacc;   // normal accumulators, cleared for the transfer (null: no normals)
+    int* vcount;
     int cap;
     unsigned* err;
     __device__ void operator()(int v, unsigned pre, unsigned keep) const {
         kept_prefix[v] = pre;
         if (!keep) return;
         if ((int)pre >= cap) { atomicOr(err, kErrCapacity); return; }
+        if (nacc) {
+            nacc[3 * (size_t)pre] = nacc[3 * (size_t)pre + 1] = nacc[3 * (size_t)pre + 2] = 0.0;
+            vcount[pre] = 0;
+        }
         mesh_v[3 * (size_t)pre] = part_v[3 * (size_t)v];
         mesh_v[3 * (size_t)pre + 1] = part_v[3 * (size_t)v + 1];
         mesh_v[3 * (size_t)pre + 2] = part_v[3 * (size_t)v + 2];
     }
-    __device__ void rebase() { PSR_CLOUD(part_v, mesh_v, kept_prefix, err); }   // to cloud blockIdx.y
+    __device__ void rebase() { PSR_CLOUD(part_v, mesh_v, kept_prefix, nacc, vcount, err); }   // to cloud blockIdx.y
 };
 
 __device__ __forceinline__ int find_part(const int* parts, int np, int t) {
@@ -1732,52 +1774,47 @@ struct KeepTriStore {
     __device__ void rebase() { PSR_CLOUD(part_t, parts, np_ptr, kept_prefix, n_staged_v, n_kept_v, mesh_t, err); }   // to cloud blockIdx.y
 };
 
-__global__ void k_count_parts(Counters* c, int* n_parts, int* n_staged_v, int* n_staged_t, int cap_v, int cap_t) {
-    PSR_CLOUD(c, n_parts, n_staged_v, n_staged_t);
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        *n_parts = 1 + c->n_groups;
-        int nv = c->n_cross + c->n_sub_cross, nt = c->n_tri + c->n_sub_tri;
-        if (nv > cap_v || nt > cap_t) atomicOr(&c->error, kErrCapacity);
-        *n_staged_v = nv < cap_v ? nv : cap_v;
-        *n_staged_t = nt < cap_t ? nt : cap_t;
-    }
-}
-
 // Vertex, edge and face records of the octree: they need only the octree, so they are
 // issued on their own stream beside the divergence and the solve (ws.stream, ws.scan and
-// the scan total are the caller's for that stream).
-cudaError_t mesh_geometry_impl(Workspace& ws, const MeshBufs& mb, unsigned* total) {
+// the scan total are the caller's for that stream).  The chunks of the coarse divergence and the
+// colour cells are counted in the same launches.
+cudaError_t mesh_geometry_impl(Workspace& ws, const MeshBufs& mb, unsigned* total, int with_colour) {
     cudaStream_t s = ws.stream;
     const int D = ws.depth;
     Counters* c = ws.cnt;
     unsigned* err = &c->error;
+    unsigned* side = (unsigned*)c->scan_total_side;
     const size_t stride = (size_t)ws.cap.nodes;
-    const int gm = grid_for(ws, ws.cap.nodes);
+    const dim3 gm = PSR_GRID(ws, grid_for(ws, ws.cap.nodes));
+    const int g = D < kColourGridLevel ? D : kColourGridLevel;
+    const int dsplit = div_split(D);
+    k_mesh_owners<<<dim3(gm.x, gm.y, with_colour ? 2 : 1), kBlock, 0, s>>>(
+        c, D, ws.key, ws.neigh, stride, ws.vmask, ws.emask16, ws.fmask, ws.node_vtx, ws.node_edge, ws.node_face,
+        mb.ov_group, mb.ov_sub, ws.cell_start, (1 << (3 * g)) + 1);
+    auto vertices = scan_job<1>(PopcLoad8{ws.vmask},
+                                VertexStore{ws.vmask, ws.ndepth, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.v_x, ws.v_y, ws.v_z,
+                                            ws.v_owner, ws.v_kind, ws.v_depth, ws.cap.vertices, err},
+                                &c->n_nodes, ws.scan, total, ScanCount{&c->n_vertices, ws.cap.vertices});
+    auto faces = scan_job<1>(PopcLoad8{ws.fmask},
+                             FaceStore{ws.fmask, ws.key, ws.ndepth, ws.parent, D, ws.f_owner, ws.f_kind, ws.f_hasparent,
+                                       ws.face_hit, ws.cap.faces, err},
+                             &c->n_nodes, ws.scan_side[0], side, ScanCount{&c->n_faces, ws.cap.faces});
+    auto edges = scan_job<1>(PopcLoad16{ws.emask16},
+                             EdgeStore{ws.emask16, &c->level_base[D], ws.e_owner, ws.e_kind, ws.cap.edges, err},
+                             &c->level_count[D], ws.scan_side[1], side + 1, ScanCount{&c->n_edges, ws.cap.edges});
     cudaError_t e;
-    k_mesh_reset<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, ws.node_vtx, ws.node_edge, ws.node_face, mb.ov_group, mb.ov_sub, stride);
-    // vertices
-    k_vertex_owner<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, ws.key, ws.neigh, stride, ws.vmask);
-    e = launch_scan<1>(PopcLoad8{ws.vmask},
-                    VertexStore{ws.vmask, ws.ndepth, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.v_x, ws.v_y, ws.v_z, ws.v_owner,
-                                ws.v_kind, ws.v_depth, ws.cap.vertices, err},
-                    &c->n_nodes, 0, ws.scan, total, err, s, ScanCount{&c->n_vertices, ws.cap.vertices});
+    if (dsplit > 0)
+        e = launch_scans(scan_job<1>(DivChunkLoad{ws.neigh, stride, ws.dnum},
+                                     DivChunkStore{(unsigned*)ws.cg_r, c, ws.cap.nodes},   // as many float pairs
+                                     &c->level_base[dsplit], ws.scan_side[2], side + 2),
+                         vertices, faces, edges, err, s);
+    else
+        e = launch_scans(vertices, faces, edges, NoScan{}, err, s);
+    if (e == cudaSuccess && !ws.chain) e = cudaEventRecord(ws.ev_geo, s);
     if (e != cudaSuccess) return e;
-    k_vertex_maintain<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, ws.neigh, stride, ws.v_owner, ws.v_kind, ws.node_vtx);
-    // edges (D level)
-    k_edge_owner<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, D, ws.key, ws.neigh, stride, ws.emask16);
-    e = launch_scan<1>(PopcLoad16{ws.emask16},
-                    EdgeStore{ws.emask16, &c->level_base[D], ws.e_owner, ws.e_kind, ws.cap.edges, err},
-                    &c->level_count[D], 0, ws.scan, total, err, s, ScanCount{&c->n_edges, ws.cap.edges});
-    if (e != cudaSuccess) return e;
-    k_edge_maintain<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, ws.neigh, stride, ws.e_owner, ws.e_kind, ws.node_edge);
-    // faces
-    k_face_owner<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, ws.key, ws.neigh, stride, ws.fmask);
-    e = launch_scan<1>(PopcLoad8{ws.fmask},
-                    FaceStore{ws.fmask, ws.key, ws.ndepth, ws.parent, D, ws.f_owner, ws.f_kind, ws.f_hasparent,
-                              ws.cap.faces, err},
-                    &c->n_nodes, 0, ws.scan, total, err, s, ScanCount{&c->n_faces, ws.cap.faces});
-    if (e != cudaSuccess) return e;
-    k_face_maintain<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, ws.neigh, stride, ws.f_owner, ws.f_kind, ws.node_face);
+    k_mesh_maintain<<<dim3(gm.x, gm.y, with_colour ? 4 : 3), kBlock, 0, s>>>(
+        c, D, ws.neigh, stride, ws.v_owner, ws.v_kind, ws.node_vtx, ws.e_owner, ws.e_kind, ws.node_edge, ws.f_owner,
+        ws.f_kind, ws.node_face, g, ws.key, ws.point2node, ws.cell_start);
     return cudaGetLastError();
 }
 
@@ -1799,8 +1836,6 @@ cudaError_t mesh_build_impl(Workspace& ws, const MeshBufs& mb) {
                                ws.e_cross, ws.part_v, 0, ws.part_cap_v, err},
                     &c->n_edges, 0, ws.scan, total, err, s, ScanCount{&c->n_cross, ws.part_cap_v});
     if (e != cudaSuccess) return e;
-    // face hits must start cleared
-    fill_words((unsigned*)ws.face_hit, 0u, ws.cap.faces, ws.batch, s);
     e = launch_scan<1>(CubeLoad{ws.node_vtx, stride, &c->level_base[D], ws.vvalue, ws.cube_class, err},
                     CubeStore{ws.cube_class, &c->level_base[D], ws.node_edge, ws.node_face, stride, ws.e_cross,
                               ws.parent, ws.f_hasparent, ws.face_hit, ws.part_t, 0, ws.part_cap_t, err},
@@ -1811,18 +1846,16 @@ cudaError_t mesh_build_impl(Workspace& ws, const MeshBufs& mb) {
                     RootStore{ws.sub_root, ws.cap.nodes, err}, &c->level_base[D], 0, ws.scan, total, err, s, ScanCount{&c->n_subroots, ws.cap.nodes});
     if (e != cudaSuccess) return e;
     // subdivision groups
-    e = launch_scan(GroupFlagLoad{ws.sub_root, ws.ndepth, D - 4},
-                    GroupFlagStore{ws.root_group, mb.groups, mb.max_groups, err}, &c->n_subroots, 0, ws.scan,
-                    total, err, s, ScanCount{}, 1);
+    e = launch_scan<1>(GroupFlagLoad{ws.sub_root, ws.ndepth, D - 4},
+                       GroupFlagStore{c, ws.root_group, mb.groups, mb.max_groups, err}, &c->n_subroots, 0, ws.scan, total,
+                       err, s, ScanCount{}, 1);
     if (e != cudaSuccess) return e;
-    k_group_count<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, total, mb.max_groups);
-    k_group_sizes<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, D, ws.sub_root, ws.ndepth, mb.groups);
-    e = launch_scan(GroupFieldLoad{mb.groups, 4}, GroupFieldStore{mb.groups, 3}, &c->n_groups, 0, ws.scan, total, err,
-                    s, ScanCount{}, 1);
+    e = launch_scan<1>(GroupSizeLoad{c, D, ws.sub_root, ws.ndepth, mb.groups}, GroupSizeStore{c, mb.groups, ws.cap.nodes},
+                       &c->n_group_flags, 0, ws.scan, total, err, s, ScanCount{}, 1);
     if (e != cudaSuccess) return e;
-    k_group_totals<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, total, ws.cap.nodes);
-    k_root_overlay<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, D, ws.sub_root, ws.ndepth, ws.key, ws.parent, ws.neigh, ws.root_group,
-                                         mb.groups, ws.sub_root_depth, ws.root_self, mb.ov_group, mb.ov_sub, stride);
+    k_root_setup<<<PSR_GRID(ws, 4 * ws.num_sms), kBlock, 0, s>>>(
+        c, D, ws.sub_root, ws.ndepth, ws.key, ws.root_group, mb.groups, ws.root_self, mb.ov_group, mb.ov_sub, ws.ctr_x,
+        ws.ctr_y, ws.ctr_z, ws.neigh, stride, ws.parent, ws.enc, ws.xsol, ws.root_poly, ws.cap_poly, ws.cap.sub_nodes);
     return cudaGetLastError();
 }
 
@@ -1834,6 +1867,7 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
     Counters* c = ws.cnt;
     unsigned* err = &c->error;
     unsigned* total = (unsigned*)&c->scan_total;
+    unsigned* side = (unsigned*)c->scan_total_side;
     const size_t stride = (size_t)ws.cap.nodes;
     const size_t dstride = (size_t)ws.cap.sub_dnodes;
     const int na = ws.cap.nodes;
@@ -1846,39 +1880,40 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
     SubArrays A{ws.c_vnode, ws.c_key, ws.c_group, ws.c_parent, ws.c_jump, ws.c_depth, ws.c_cx, ws.c_cy, ws.c_cz,
                 ws.c_neigh, (size_t)ws.cap.sub_nodes, ws.c_live, ws.c_poly, ws.c_touch, ws.lv_vnode,
                 ws.cap.sub_nodes, ws.cap.sub_live, ws.cap.sub_dnodes};
-    k_sub_setup<<<PSR_GRID(ws, 1), 32, 0, s>>>(c, D, ws.sub_root_depth, ws.cap.sub_nodes);   // kMaxDepth + 2 <= 32 lanes
-    k_root_poly<<<PSR_GRID(ws, grid_for(ws, ws.cap_poly)), kBlock, 0, s>>>(c, D, ws.sub_root, ws.ndepth, ws.ctr_x, ws.ctr_y,
-                                                             ws.ctr_z, ws.neigh, stride, ws.parent, ws.enc, ws.xsol,
-                                                             ws.root_poly, ws.cap_poly);
     // depth after depth: candidates (children of the live nodes above, then the roots of this
     // depth), their neighbours and sign tests; the live ones are compacted in order
-    for (int d = 1; d <= D; ++d) {
-        e = launch_scan<1>(SubLevelLoad{c, d, D, na, mb.groups, ws.sub_root, ws.root_group, ws.root_self, ws.key,
-                                        ws.neigh, stride, ws.first_child, ws.parent, mb.ov_group, mb.ov_sub, ws.enc,
-                                        ws.xsol, ws.root_poly, ws.cap_poly, A},
-                           SubLevelStore{c, d, D, A, err}, &c->sub_cand[d], 0, ws.scan, total, err, s, ScanCount{},
-                           sbps);
+    auto level = [&](auto load, int d) {
+        load.c = c; load.d = d; load.depth = D; load.na = na; load.groups = mb.groups; load.sub_root = ws.sub_root;
+        load.root_group = ws.root_group; load.root_self = ws.root_self; load.key = ws.key; load.neigh = ws.neigh;
+        load.stride = stride; load.first_child = ws.first_child; load.parent = ws.parent; load.ov_group = mb.ov_group;
+        load.ov_sub = mb.ov_sub; load.enc = ws.enc; load.x = ws.xsol; load.root_poly = ws.root_poly;
+        load.cap_poly = ws.cap_poly; load.A = A;
+        return load;
+    };
+    const int dcoarse = D < 3 ? D : 3;
+    k_sub_coarse<<<PSR_GRID(ws, 1), kBlock, 0, s>>>(level(SubLevelLoad<true>{}, 1), SubLevelStore{c, 1, D, A, err}, dcoarse);
+    for (int d = dcoarse + 1; d <= D; ++d) {
+        e = launch_scan<1>(level(SubLevelLoad<false>{}, d), SubLevelStore{c, d, D, A, err}, &c->sub_cand[d], 0, ws.scan,
+                           total, err, s, ScanCount{}, sbps);
         if (e != cudaSuccess) return e;
     }
     // the live depth-D cells carry every record from here on, indexed by their live index
-    k_sub_live_neigh<<<PSR_GRID(ws, 2 * gl), kBlock, 0, s>>>(c, D, A, ws.lv_nb, dstride, na);
-    // s_vtx / s_edge need no clearing: every slot of a live cell is written by the owner of
-    // that vertex / edge
-    k_sub_vertex_owner<<<PSR_GRID(ws, gl), kBlock, 0, s>>>(c, D, A, ws.lv_nb, dstride, ws.s_vmask);
-    e = launch_scan<2>(PopcLoad8{ws.s_vmask},
-                       SubVertexStore{ws.s_vmask, c, D, A, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.sv_kind,
-                                      8 * ws.cap.sub_dnodes, err},
-                       &c->n_sub_dnodes, 0, ws.scan, total, err, s, ScanCount{&c->n_sub_vertices, 8 * ws.cap.sub_dnodes},
-                       sbps);
+    k_sub_live_neigh<<<PSR_GRID(ws, 2 * gl), kBlock, 0, s>>>(c, D, A, ws.lv_nb, dstride, na, mb.group_live);
+    k_sub_owners<<<PSR_GRID(ws, gl), kBlock, 0, s>>>(c, D, A, ws.lv_nb, dstride, ws.s_vmask, ws.s_emask);
+    e = launch_scans(scan_job<2>(PopcLoad8{ws.s_vmask},
+                                 SubVertexStore{ws.s_vmask, c, D, A, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.sv_kind,
+                                                8 * ws.cap.sub_dnodes, err},
+                                 &c->n_sub_dnodes, ws.scan, total, ScanCount{&c->n_sub_vertices, 8 * ws.cap.sub_dnodes}),
+                     scan_job<2>(PopcLoad16{ws.s_emask},
+                                 SubEdgeStore{ws.s_emask, ws.se_owner, ws.se_kind, mb.edge_of_dnode,
+                                              12 * ws.cap.sub_dnodes, err},
+                                 &c->n_sub_dnodes, ws.scan_side[0], side,
+                                 ScanCount{&c->n_sub_edges, 12 * ws.cap.sub_dnodes}),
+                     NoScan{}, NoScan{}, err, s, sbps);
     if (e != cudaSuccess) return e;
-    k_sub_vertex_maintain<<<PSR_GRID(ws, gl), kBlock, 0, s>>>(c, ws.lv_nb, dstride, ws.sv_owner, ws.sv_kind, ws.s_vtx);
-    k_sub_edge_owner<<<PSR_GRID(ws, gl), kBlock, 0, s>>>(c, D, A, ws.lv_nb, dstride, ws.s_emask);
-    e = launch_scan<2>(PopcLoad16{ws.s_emask},
-                       SubEdgeStore{ws.s_emask, ws.se_owner, ws.se_kind, mb.edge_of_dnode, 12 * ws.cap.sub_dnodes, err},
-                       &c->n_sub_dnodes, 0, ws.scan, total, err, s, ScanCount{&c->n_sub_edges, 12 * ws.cap.sub_dnodes},
-                       sbps);
-    if (e != cudaSuccess) return e;
-    k_sub_edge_maintain<<<PSR_GRID(ws, gl), kBlock, 0, s>>>(c, ws.lv_nb, dstride, ws.se_owner, ws.se_kind, ws.s_edge);
+    const dim3 g2 = PSR_GRID(ws, gl);
+    k_sub_maintain<<<dim3(g2.x, g2.y, 2), kBlock, 0, s>>>(c, ws.lv_nb, dstride, ws.sv_owner, ws.sv_kind, ws.s_vtx,
+                                                          ws.se_owner, ws.se_kind, ws.s_edge);
     k_sub_vertex_values<<<PSR_GRID(ws, 16 * ws.num_sms), kSvBlock, 0, s>>>(
         c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, mb.groups, ws.root_self, A, ws.enc,
         ws.xsol, ws.sv_value, na);
@@ -1888,26 +1923,22 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
                                      ws.sv_z, ws.se_cross, ws.part_v, &c->n_cross, ws.part_cap_v, err},
                        &c->n_sub_edges, 0, ws.scan, total, err, s, ScanCount{&c->n_sub_cross, ws.part_cap_v}, sbps);
     if (e != cudaSuccess) return e;
-    // triangle prefix per live cell
-    e = launch_scan<2>(SubCubeLoad{ws.s_vtx, dstride, ws.sv_value, ws.s_cube_class, err},
-                       StoreExclusive{mb.tri_of_dnode}, &c->n_sub_dnodes, 0, ws.scan, total, err, s,
-                       ScanCount{&c->n_sub_tri, ws.part_cap_t}, sbps);
-    if (e != cudaSuccess) return e;
-    k_part_table<<<PSR_GRID(ws, grid_for(ws, 1 << 16)), kBlock, 0, s>>>(c, D, mb.groups, ws.lv_vnode, mb.edge_of_dnode, ws.se_cross,
-                                                          mb.tri_of_dnode, mb.group_cross0, mb.parts);
-    e = launch_scan<2>(SubCubeLoad{ws.s_vtx, dstride, ws.sv_value, ws.s_cube_class, err},
-                       SubCubeStore{ws.s_cube_class, ws.s_edge, dstride, ws.se_cross, mb.group_cross0, c, D, A,
-                                    ws.part_t, &c->n_tri, ws.part_cap_t, err},
-                       &c->n_sub_dnodes, 0, ws.scan, total, err, s, ScanCount{}, sbps);
-    if (e != cudaSuccess) return e;
-    // insertion of all parts
     int* n_parts = mb.misc;
     int* n_staged_v = mb.misc + 1;
     int* n_staged_t = mb.misc + 2;
-    k_count_parts<<<PSR_GRID(ws, 1), 1, 0, s>>>(c, n_parts, n_staged_v, n_staged_t, ws.part_cap_v, ws.part_cap_t);
-    e = launch_scan(KeepVertexLoad{ws.part_v},
-                    KeepVertexStore{ws.part_v, ws.mesh_v, mb.kept_prefix, ws.cap.mesh_vertices, err}, n_staged_v, 0,
-                    ws.scan, total, err, s, ScanCount{&c->n_mesh_vertices, ws.cap.mesh_vertices}, sbps);
+    e = launch_scan<2>(SubCubeLoad{ws.s_vtx, dstride, ws.sv_value, ws.s_cube_class, err},
+                       SubCubeStore{ws.s_cube_class, ws.s_edge, dstride, ws.se_cross, mb.edge_of_dnode, mb.group_live,
+                                    mb.tri_of_dnode, c, D, A, ws.part_t, &c->n_tri, ws.part_cap_t, ws.part_cap_v, n_parts,
+                                    n_staged_v, n_staged_t, err},
+                       &c->n_sub_dnodes, 0, ws.scan, total, err, s, ScanCount{&c->n_sub_tri, ws.part_cap_t}, sbps);
+    if (e != cudaSuccess) return e;
+    // insertion of all parts
+    e = launch_scans(scan_job<2>(KeepVertexLoad{ws.part_v},
+                                 KeepVertexStore{ws.part_v, ws.mesh_v, mb.kept_prefix,
+                                                 ws.want_normals ? ws.nacc : nullptr, ws.vcount, ws.cap.mesh_vertices, err},
+                                 n_staged_v, ws.scan, total, ScanCount{&c->n_mesh_vertices, ws.cap.mesh_vertices}),
+                     PartTableJob{c, D, mb.groups, ws.lv_vnode, mb.edge_of_dnode, ws.se_cross, mb.tri_of_dnode, mb.parts},
+                     NoScan{}, NoScan{}, err, s, sbps);
     if (e != cudaSuccess) return e;
     e = launch_scan<1>(KeepTriLoad{ws.part_t, mb.parts, n_parts},
                     KeepTriStore{ws.part_t, mb.parts, n_parts, mb.kept_prefix, n_staged_v, &c->n_mesh_vertices,
@@ -1920,8 +1951,8 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
 }  // namespace psr
 
 namespace psr {
-cudaError_t mesh_geometry(Workspace& ws) {
-    return mesh_geometry_impl(ws, ws.mb, (unsigned*)&ws.cnt->scan_total_aux);
+cudaError_t mesh_geometry(Workspace& ws, int with_colour) {
+    return mesh_geometry_impl(ws, ws.mb, (unsigned*)&ws.cnt->scan_total_aux, with_colour);
 }
 
 cudaError_t mesh_build(Workspace& ws) {

@@ -81,14 +81,12 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned& e
 // elements per thread: 8 for light functors, 1 or 2 where Load / Store do enough work per
 // element that more, smaller tiles (more blocks in flight) pay.
 template <int kItems, class Load, class Store>
-__global__ void __launch_bounds__(kBlock) k_scan(Load load, Store store, const int* count_ptr, int count_add,
-                                                 ScanScratch sc, unsigned* total, unsigned* err, ScanCount cnt) {
-    PSR_CLOUD(load, store, count_ptr, sc, total, err, cnt);
+__device__ __forceinline__ void scan_body(Load load, Store store, int n, ScanScratch sc, unsigned* total, unsigned* err,
+                                          ScanCount cnt) {
     constexpr int kTile = kBlock * kItems;
     __shared__ unsigned s_warp[kBlock / 32 + 1];
     __shared__ int s_tile;
     __shared__ unsigned s_prefix;
-    const int n = *count_ptr + count_add;
     const int ntiles = (n + kTile - 1) / kTile;
     if (n <= 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -201,6 +199,47 @@ __global__ void __launch_bounds__(kBlock) k_scan(Load load, Store store, const i
     }
 }
 
+template <int kItems, class Load, class Store>
+__global__ void __launch_bounds__(kBlock) k_scan(Load load, Store store, const int* count_ptr, int count_add,
+                                                 ScanScratch sc, unsigned* total, unsigned* err, ScanCount cnt) {
+    PSR_CLOUD(load, store, count_ptr, sc, total, err, cnt);
+    scan_body<kItems>(load, store, *count_ptr + count_add, sc, total, err, cnt);
+}
+
+// One scan of a launch of several: scans that only read what earlier launches wrote run side by
+// side, blockIdx.z taking one each, with a scratch of its own.
+template <int kItems, class Load, class Store>
+struct ScanJob {
+    Load load;
+    Store store;
+    const int* count_ptr;
+    ScanScratch sc;
+    unsigned* total;
+    ScanCount cnt;
+    static constexpr bool kUsed = true;
+    __device__ void run(unsigned* err) {
+        PSR_CLOUD(load, store, count_ptr, sc, total, cnt);
+        scan_body<kItems>(load, store, *count_ptr, sc, total, err, cnt);
+    }
+};
+struct NoScan {
+    static constexpr bool kUsed = false;
+    __device__ void run(unsigned*) {}
+};
+template <int kItems, class Load, class Store>
+ScanJob<kItems, Load, Store> scan_job(Load load, Store store, const int* count_ptr, ScanScratch sc, unsigned* total,
+                                      ScanCount cnt = ScanCount{}) {
+    return ScanJob<kItems, Load, Store>{load, store, count_ptr, sc, total, cnt};
+}
+template <class A, class B, class C, class D>
+__global__ void __launch_bounds__(kBlock) k_scans(A a, B b, C c, D d, unsigned* err) {
+    PSR_CLOUD(err);
+    if (blockIdx.z == 0) a.run(err);
+    else if (blockIdx.z == 1) b.run(err);
+    else if (blockIdx.z == 2) c.run(err);
+    else d.run(err);
+}
+
 // blocks of a scan launch: blocks_per_sm per SM, at most max_tiles
 int scan_grid(int max_tiles, int blocks_per_sm = 4);
 
@@ -213,6 +252,14 @@ inline cudaError_t launch_scan(Load load, Store store, const int* count_ptr, int
                                int blocks_per_sm = 4) {
     const dim3 grid(cloud_blocks(sc.batch, scan_grid(sc.max_tiles, blocks_per_sm)), sc.batch);
     k_scan<kItems, Load, Store><<<grid, kBlock, 0, stream>>>(load, store, count_ptr, count_add, sc, total, err, cnt);
+    return cudaGetLastError();
+}
+
+template <class A, class B, class C = NoScan, class D = NoScan>
+inline cudaError_t launch_scans(A a, B b, C c, D d, unsigned* err, cudaStream_t stream, int blocks_per_sm = 4) {
+    const int jobs = 2 + (C::kUsed ? 1 : 0) + (D::kUsed ? 1 : 0);
+    const dim3 grid(cloud_blocks(a.sc.batch, scan_grid(a.sc.max_tiles, blocks_per_sm)), a.sc.batch, jobs);
+    k_scans<A, B, C, D><<<grid, kBlock, 0, stream>>>(a, b, c, d, err);
     return cudaGetLastError();
 }
 

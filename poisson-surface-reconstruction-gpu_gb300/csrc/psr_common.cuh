@@ -32,6 +32,8 @@ struct Counters {
     int n_vertices, n_edges, n_faces;
     int n_cross, n_tri;
     int n_subroots;
+    int n_group_flags;            // subdivision groups before the check of their numbering
+    int n_div_items;              // chunks of the coarse divergence
     // subdivision, per depth d: candidates, their first compact slot, the first entry of
     // the depth's live list, live nodes, first root index and roots of depth d
     int sub_cand[kMaxDepth + 2], sub_cbase[kMaxDepth + 2], sub_lbase[kMaxDepth + 2];
@@ -46,6 +48,7 @@ struct Counters {
     int n_weld;                   // mesh vertices left by welding
     int scan_total;               // scratch total written by scans
     int scan_total_aux;           // the same for scans issued on the geometry stream
+    int scan_total_side[3];       // and for the scans beside another one in its launch
     unsigned error;
     float bbox_min[3], bbox_max[3];
     float center[3];

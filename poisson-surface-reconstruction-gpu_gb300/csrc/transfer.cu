@@ -22,34 +22,6 @@ __device__ __forceinline__ unsigned morton3(int x, int y, int z, int g) {
     return m;
 }
 
-__device__ __forceinline__ unsigned point_cell(int i, int depth, int g, int bD, const int* key,
-                                               const int* point2node) {
-    return (unsigned)key[bD + point2node[i]] >> (3 * (depth - g));
-}
-
-// cell_start[m] = first sorted sample whose cell code is >= m, for m in [0, 8^g]: the
-// exclusive prefix sum of the samples per cell.  k_cell_count counts them (the table
-// starts zeroed; the samples are Morton-sorted, so the last sample of a cell's run adds
-// the run's length), then one scan turns the counts into starts in place.
-__global__ void __launch_bounds__(kBlock) k_cell_count(Counters* c, int depth, int g, const int* key,
-                                                       const int* point2node, int* count) {
-    PSR_CLOUD(c, key, point2node, count);
-    const int n = c->n_points;
-    const int bD = c->level_base[depth];
-    if (blockIdx.x == 0 && threadIdx.x == 0) c->n_colour_cells = (1 << (3 * g)) + 1;
-    PSR_GRID_STRIDE(i, n) {
-        const unsigned m = point_cell(i, depth, g, bD, key, point2node);
-        if (i + 1 < n && point_cell(i + 1, depth, g, bD, key, point2node) == m) continue;
-        int lo = 0, hi = i;   // first sample of the run ending at i
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (point_cell(mid, depth, g, bD, key, point2node) < m) lo = mid + 1;
-            else hi = mid;
-        }
-        count[m] = i + 1 - lo;
-    }
-}
-
 // (d, i) lexicographic order: smaller squared distance first, then lower sample index
 __device__ __forceinline__ bool knn_less(float da, int ia, float db, int ib) {
     return da < db || (da == db && ia < ib);
@@ -442,15 +414,6 @@ __global__ void __launch_bounds__(kBlock) k_colour_far(const Counters* c, int gm
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_normals_zero(const Counters* c, double* acc, int* cnt) {
-    PSR_CLOUD(c, acc, cnt);
-    const int V = c->n_mesh_vertices;
-    PSR_GRID_STRIDE(v, V) {
-        acc[3 * (size_t)v] = acc[3 * (size_t)v + 1] = acc[3 * (size_t)v + 2] = 0.0;
-        cnt[v] = 0;
-    }
-}
-
 // a b - c d within 1.5 ulp (Kahan's difference of products: fma recovers the rounding error
 // of c d), so a sliver triangle's cross product keeps its direction instead of cancelling
 __device__ __forceinline__ float diff_of_products(float a, float b, float c, float d) {
@@ -507,14 +470,11 @@ __global__ void __launch_bounds__(kBlock) k_vertex_normals(const Counters* c, co
     }
 }
 
-// sample grid of the colour search: needs only the sorted samples, so it runs beside the solve
+// cell_start[m] = first sorted sample whose cell code is >= m, for m in [0, 8^g]: the exclusive
+// prefix sum, in place, of the samples per cell that the mesh geometry's launches counted.  It
+// needs only the sorted samples, so it runs beside the solve.
 cudaError_t transfer_prepare(Workspace& ws, int with_colour) {
     if (!with_colour) return cudaSuccess;
-    const int D = ws.depth;
-    const int g = D < kColourGridLevel ? D : kColourGridLevel;
-    cudaError_t e = fill_words((unsigned*)ws.cell_start, 0u, ((long long)1 << (3 * g)) + 1, ws.batch, ws.stream);
-    if (e != cudaSuccess) return e;
-    k_cell_count<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, ws.stream>>>(ws.cnt, D, g, ws.key, ws.point2node, ws.cell_start);
     unsigned* table = reinterpret_cast<unsigned*>(ws.cell_start);
     Counters* c = ws.cnt;
     return launch_scan(LoadArray{table}, StoreExclusive{table}, &c->n_colour_cells, 0, ws.scan,
@@ -549,7 +509,6 @@ cudaError_t transfer_build(Workspace& ws, int with_colour, int with_normals) {
     }
     if (with_normals) {
         double* acc = ws.nacc;
-        k_normals_zero<<<PSR_GRID(ws, grid), kBlock, 0, s>>>(ws.cnt, acc, ws.vcount);
         k_triangle_normals<<<PSR_GRID(ws, grid), kBlock, 0, s>>>(ws.cnt, ws.mesh_v, ws.mesh_t, acc, ws.vcount);
         k_vertex_normals<<<PSR_GRID(ws, grid), kBlock, 0, s>>>(ws.cnt, acc, ws.vcount, ws.mesh_n);
     }

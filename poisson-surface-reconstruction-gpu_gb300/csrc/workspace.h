@@ -39,7 +39,7 @@ struct MeshBufs {
     int max_groups;
     unsigned* edge_of_dnode;   // sub-edge prefix per live depth-D cell
     unsigned* tri_of_dnode;    // sub-triangle prefix per live depth-D cell
-    unsigned* group_cross0;    // per group: crossing prefix at its first sub edge
+    int* group_live;           // per group: its first live depth-D cell
     int* parts;                // per output part: vertex start / count, triangle start / count
     unsigned* kept_prefix;     // per staged vertex: kept vertices before it
     int* misc;                 // [0] parts, [1] staged vertices, [2] staged triangles
@@ -47,6 +47,7 @@ struct MeshBufs {
 
 struct Workspace {
     int batch = 1;          // clouds of the launches being issued (the grids' y extent)
+    bool want_normals = false;   // the call's mesh gets vertex normals
     bool chain = false;     // the pipeline is issued as one chain, without forks (depths up to 7)
     int cg_ctas = 0;        // CTAs of the depth-D CG cluster (0: the largest the device runs, 16)
     int cg_ctas_fine = 0;   // CTAs of each depth-(D-1), (D-2) CG cluster (0: 8)
@@ -57,6 +58,7 @@ struct Workspace {
     Counters* cnt_host;     // pinned mirror for the final read-back
     ScanScratch scan;
     ScanScratch scan_aux;   // scans issued on the geometry stream (aux2) while `scan` is in use
+    ScanScratch scan_side[3];   // scans that run beside another one in its launch
     SortScratch sort;
     unsigned* scan_total;   // device scratch (points into cnt)
 
@@ -92,7 +94,7 @@ struct Workspace {
 
     // function tables (FP64, res x res) and per-depth stencil coefficients
     int res;
-    float* dff;             // d/dx F_i . F_j rounded to float (index i + res * j)
+    float* dff;             // d/dx F_i . F_j rounded to float (index res * i + j)
     float* stencil;         // [D+1][27] Laplacian coefficients (0 where dropped)
 
     // field / solve
@@ -127,7 +129,6 @@ struct Workspace {
 
     // subdivision
     int* sub_root;          // node index of each root (node order)
-    int* sub_root_depth;
     int* root_group;        // per subdivision root: its group
     int* root_self;         // per root: the octree node it stands for
     float* root_poly;       // [28][cap_poly]: per root, Bernstein coefficients of the levels up to it
@@ -181,6 +182,7 @@ struct Workspace {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t aux2 = nullptr;        // third stream: octree-only mesh records beside the solve
     cudaEvent_t ev_fork2 = nullptr, ev_join2 = nullptr;
+    cudaEvent_t ev_geo = nullptr;       // the mesh records' scans (and the divergence chunks') are done
     cudaStream_t aux3 = nullptr;        // fourth stream: the CG of depths D-1 and D-2
     cudaEvent_t ev_join3 = nullptr;
     cudaStream_t aux4 = nullptr;        // fifth stream: the device-loop CG of large depths
@@ -201,6 +203,7 @@ inline void set_batch(Workspace& ws, int clouds) {
     ws.batch = clouds;
     ws.scan.batch = clouds;
     ws.scan_aux.batch = clouds;
+    for (auto& sc : ws.scan_side) sc.batch = clouds;
     ws.sort.batch = clouds;
 }
 
@@ -212,6 +215,10 @@ inline int grid_for(const Workspace& ws, long long work) {
     return (int)(g < 1 ? 1 : g);
 }
 
+// coarse divergence: depths below div_split(D) are summed in chunks of kDivChunk leaves
+constexpr int kDivChunk = 512;
+inline int div_split(int D) { return D >= 2 ? D - 2 : 0; }
+
 // stage entry points (each issues kernels on ws.stream; no host synchronisation)
 cudaError_t octree_build(Workspace& ws);
 void prepare_launch_configs(Workspace& ws);
@@ -219,9 +226,11 @@ cudaError_t field_build(Workspace& ws);
 // res_period: true residual every res_period CG iterations and at convergence (0: only at
 // convergence, < 0: never)
 cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, int cg_max_iter, int res_period);
-cudaError_t mesh_geometry(Workspace& ws);   // vertex / edge / face records (octree only)
+// vertex / edge / face records, divergence chunks, and the colour search's sample grid (octree and
+// points only)
+cudaError_t mesh_geometry(Workspace& ws, int with_colour);
 cudaError_t mesh_build(Workspace& ws);      // values, marching cubes, subdivision, compaction
-cudaError_t transfer_prepare(Workspace& ws, int with_colour);   // sample grid (points only)
+cudaError_t transfer_prepare(Workspace& ws, int with_colour);   // last step of the sample grid
 cudaError_t transfer_build(Workspace& ws, int with_colour, int with_normals);
 
 }  // namespace psr
