@@ -132,17 +132,22 @@ __global__ void __launch_bounds__(kBlock) k_nrm_cells(Counters* c, const unsigne
     }
 }
 
-// Near pass, 8 lanes per point: the points of the 3x3x3 block of level-7 cells around the
-// point's cell; exact when K were found and the K-th is closer than one cell width (every
-// point outside the block is at least one width away), else the point goes to the far list
+// Near pass, 8 lanes per point: the points of the 3x3x3 block of cells around the point's cell,
+// at level 7 and, while that does not settle the point, at coarser levels (their cells are ranges
+// of the same table).  A level settles it when K points were found and the K-th is closer than one
+// cell width (every point outside the block is at least one width away).  A block with fewer than
+// K points is not scanned; one with more than kNrmNearCap, or a point that level kNrmNearCoarsest
+// leaves, goes to the far list.  Without the coarser levels a cloud whose spacing exceeds the level-7
+// cells went to the far pass point by point, a block each: 1.06 ms of 31k points, now part of the
+// 25 us of this pass.
+constexpr int kNrmNearCap = 1024;
+constexpr int kNrmNearCoarsest = 3;
 __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned* scode, const float* px,
                                                      const float* py, const float* pz, const int* cell_start,
                                                      int* nbr, int* far) {
     __shared__ int s_off[kNrmGroups][28];
     __shared__ int s_base[kNrmGroups][27];
     const int n = c->n_points;
-    const int G = 1 << kNrmGridLevel;
-    const float w = 1.0f / (float)G;
     const int lane = threadIdx.x & (kNrmLanes - 1);
     const int gib = threadIdx.x / kNrmLanes;
     const unsigned gmask = 0xffu << (threadIdx.x & 24);
@@ -157,56 +162,65 @@ __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned
         for (int l = 0; l < kNrmGridLevel; ++l)
 #pragma unroll
             for (int a = 0; a < 3; ++a) cxyz[a] |= (int)((code >> (3 * l + 2 - a)) & 1u) << l;
-        int running = 0;
+        bool settled = false;
+        for (int g = kNrmGridLevel; g >= kNrmNearCoarsest; --g) {   // uniform in the group
+            const int G = 1 << g, up = kNrmGridLevel - g;
+            const float w = 1.0f / (float)G;
+            int running = 0;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int k = lane + kNrmLanes * r;
-            int cnt = 0, base = 0;
-            if (k < 27) {
-                const int a = cxyz[0] + k / 9 - 1, b = cxyz[1] + (k / 3) % 3 - 1, z = cxyz[2] + k % 3 - 1;
-                if (a >= 0 && a < G && b >= 0 && b < G && z >= 0 && z < G) {
-                    const unsigned m = nrm_morton(a, b, z);
-                    base = cell_start[m];
-                    cnt = cell_start[m + 1] - base;
+            for (int r = 0; r < 4; ++r) {
+                const int k = lane + kNrmLanes * r;
+                int cnt = 0, base = 0;
+                if (k < 27) {
+                    const int a = (cxyz[0] >> up) + k / 9 - 1, b = (cxyz[1] >> up) + (k / 3) % 3 - 1,
+                              z = (cxyz[2] >> up) + k % 3 - 1;
+                    if (a >= 0 && a < G && b >= 0 && b < G && z >= 0 && z < G) {
+                        const unsigned m = nrm_morton(a, b, z);
+                        base = cell_start[(size_t)m << (3 * up)];
+                        cnt = cell_start[(size_t)(m + 1) << (3 * up)] - base;
+                    }
                 }
-            }
-            int incl = cnt;
+                int incl = cnt;
 #pragma unroll
-            for (int o = 1; o < kNrmLanes; o <<= 1) {
-                const int y = __shfl_up_sync(gmask, incl, o, kNrmLanes);
-                if (lane >= o) incl += y;
+                for (int o = 1; o < kNrmLanes; o <<= 1) {
+                    const int y = __shfl_up_sync(gmask, incl, o, kNrmLanes);
+                    if (lane >= o) incl += y;
+                }
+                if (k < 27) {
+                    s_off[gib][k] = running + incl - cnt;
+                    s_base[gib][k] = base;
+                }
+                running += __shfl_sync(gmask, incl, kNrmLanes - 1, kNrmLanes);
             }
-            if (k < 27) {
-                s_off[gib][k] = running + incl - cnt;
-                s_base[gib][k] = base;
-            }
-            running += __shfl_sync(gmask, incl, kNrmLanes - 1, kNrmLanes);
-        }
-        if (lane == 0) s_off[gib][27] = running;
-        __syncwarp(gmask);
-        float bd[kNrmK];
-        int bi[kNrmK];
+            if (lane == 0) s_off[gib][27] = running;
+            __syncwarp(gmask);
+            if (running > kNrmNearCap) break;
+            if (running < kNrmK && running < n) continue;   // the K-th is farther out
+            float bd[kNrmK];
+            int bi[kNrmK];
 #pragma unroll
-        for (int q = 0; q < kNrmK; ++q) { bd[q] = 1e30f; bi[q] = 0x7fffffff; }
-        int k = 0;
-        for (int t = lane; t < running; t += kNrmLanes) {
-            while (s_off[gib][k + 1] <= t) ++k;
-            nrm_visit(qx, qy, qz, px, py, pz, s_base[gib][k] + (t - s_off[gib][k]), bd, bi);
-        }
-        __syncwarp(gmask);
-        float md[kNrmK];
-        int mi[kNrmK];
-        nrm_group_merge<kNrmK>(bd, bi, md, mi, gmask, kNrmLanes);
-        if (lane == 0) {
+            for (int q = 0; q < kNrmK; ++q) { bd[q] = 1e30f; bi[q] = 0x7fffffff; }
+            int k = 0;
+            for (int t = lane; t < running; t += kNrmLanes) {
+                while (s_off[gib][k + 1] <= t) ++k;
+                nrm_visit(qx, qy, qz, px, py, pz, s_base[gib][k] + (t - s_off[gib][k]), bd, bi);
+            }
+            __syncwarp(gmask);
+            float md[kNrmK];
+            int mi[kNrmK];
+            nrm_group_merge<kNrmK>(bd, bi, md, mi, gmask, kNrmLanes);
             // fewer than K points in the whole cloud: all of them are the neighbours
-            const bool all_found = mi[kNrmK - 1] != 0x7fffffff || running == n;
-            if (all_found && (md[kNrmK - 1] < w * w || running == n)) {
+            if (md[kNrmK - 1] < w * w || running == n) {
+                if (lane == 0) {
 #pragma unroll
-                for (int q = 0; q < kNrmK; ++q) nbr[(size_t)p * kNrmK + q] = mi[q];
-            } else {
-                far[atomicAdd(&c->n_colour_far, 1)] = p;
+                    for (int q = 0; q < kNrmK; ++q) nbr[(size_t)p * kNrmK + q] = mi[q];
+                }
+                settled = true;
+                break;
             }
         }
+        if (!settled && lane == 0) far[atomicAdd(&c->n_colour_far, 1)] = p;
+        __syncwarp(gmask);
     }
 }
 
@@ -347,26 +361,50 @@ __global__ void __launch_bounds__(kBlock) k_nrm_far(const Counters* c, const flo
     }
 }
 
-// eigenvector of the smallest eigenvalue of the symmetric 3x3 matrix (a00 a01 a02; a11 a12;
-// a22): eigenvalues from the characteristic cubic (trigonometric form), the vector as the
-// longest cross product of two rows of A - lambda I
+// Eigenvector of the smallest eigenvalue of the symmetric 3x3 matrix (a00 a01 a02; a11 a12; a22).
+// The smallest root of the characteristic cubic: the trigonometric form in FP32, moved a little
+// towards minus infinity, then Newton steps on the cubic in FP64.  Left of its smallest root a
+// cubic with three real roots is concave and rising, so the steps approach the root from the left
+// without overshooting; near it they converge quadratically, and they stop when a step no longer
+// moves.  (The trigonometric form in FP64 alone cost a third of this pass: GB300 issues an FP64
+// warp instruction every 19 cycles per SM.)  The vector is the longest cross product of two rows of
+// A - lambda I.
 __device__ __forceinline__ void nrm_smallest_eigvec(double a00, double a01, double a02, double a11, double a12,
                                                     double a22, double (&v)[3]) {
-    const double scale = fmax(fmax(fmax(fabs(a00), fabs(a01)), fmax(fabs(a02), fabs(a11))), fmax(fabs(a12), fabs(a22)));
-    if (!(scale > 0.0)) { v[0] = v[1] = v[2] = 0.0; return; }
-    a00 /= scale; a01 /= scale; a02 /= scale; a11 /= scale; a12 /= scale; a22 /= scale;
-    const double q = (a00 + a11 + a22) / 3.0;
+    v[0] = v[1] = v[2] = 0.0;
+    const float big = fmaxf(fmaxf(fmaxf(fabsf((float)a00), fabsf((float)a01)), fmaxf(fabsf((float)a02), fabsf((float)a11))),
+                            fmaxf(fabsf((float)a12), fabsf((float)a22)));
+    if (!(big > 0.0f)) return;
+    // by a power of two (exact): the largest entry to [1, 2)
+    const double sc = __hiloint2double((1023 + 127 - (__float_as_int(big) >> 23)) << 20, 0);
+    a00 *= sc; a01 *= sc; a02 *= sc; a11 *= sc; a12 *= sc; a22 *= sc;
+    const double q = (a00 + a11 + a22) * (1.0 / 3.0);
     const double b00 = a00 - q, b11 = a11 - q, b22 = a22 - q;
-    const double p2 = (b00 * b00 + b11 * b11 + b22 * b22 + 2.0 * (a01 * a01 + a02 * a02 + a12 * a12)) / 6.0;
-    double lambda = q;
-    if (p2 > 0.0) {
-        const double p = sqrt(p2);
-        const double det = b00 * (b11 * b22 - a12 * a12) - a01 * (a01 * b22 - a12 * a02) + a02 * (a01 * a12 - b11 * a02);
-        double r = det / (2.0 * p * p2);
-        r = fmin(fmax(r, -1.0), 1.0);
-        const double phi = acos(r) / 3.0;
-        lambda = q + 2.0 * p * cos(phi + 2.0943951023931954923);   // the smallest root
+    // x^3 - 3 p2 x - det = 0 for x = lambda - q
+    const double s01 = a01 * a01, s02 = a02 * a02, s12 = a12 * a12;
+    const double p2 = (b00 * b00 + b11 * b11 + b22 * b22 + 2.0 * (s01 + s02 + s12)) * (1.0 / 6.0);
+    const double det = b00 * (b11 * b22 - s12) - a01 * (a01 * b22 - a12 * a02) + a02 * (a01 * a12 - b11 * a02);
+    double x = 0.0;
+    const float p2f = (float)p2;
+    if (p2f > 0.0f) {
+        const float pf = sqrtf(p2f);
+        const float r = fminf(fmaxf((float)det / (2.0f * pf * p2f), -1.0f), 1.0f);
+        // the smallest root is in [-2 p, -p]
+        x = (double)(2.0f * pf * cosf(acosf(r) * (1.0f / 3.0f) + 2.0943951024f));
+        x -= 1e-3 * (double)pf;
+        const double p3 = 3.0 * p2;
+        for (int it = 0; it < 40; ++it) {
+            const double x2 = x * x;
+            const double f = (x2 - p3) * x - det, d = 3.0 * (x2 - p2);
+            if (!(d > 0.0) || !(f < 0.0)) break;   // at the root (or a double one)
+            // the quotient to FP32 is enough for a step; its error is made up by the next one
+            const double step = (double)__fdividef((float)f, (float)d);
+            const double next = x - step;
+            if (next == x) break;
+            x = next;
+        }
     }
+    const double lambda = q + x;
     const double r0[3] = {a00 - lambda, a01, a02};
     const double r1[3] = {a01, a11 - lambda, a12};
     const double r2[3] = {a02, a12, a22 - lambda};
@@ -379,40 +417,77 @@ __device__ __forceinline__ void nrm_smallest_eigvec(double a00, double a01, doub
     double b0 = c01[0], b1 = c01[1], b2 = c01[2], nb = n01;
     if (n02 > nb) { b0 = c02[0]; b1 = c02[1]; b2 = c02[2]; nb = n02; }
     if (n12 > nb) { b0 = c12[0]; b1 = c12[1]; b2 = c12[2]; nb = n12; }
-    if (!(nb > 0.0)) { v[0] = v[1] = v[2] = 0.0; return; }
-    const double inv = 1.0 / sqrt(nb);
+    if (!(nb > 0.0)) return;
+    const double inv = rsqrt(nb);
     v[0] = b0 * inv;
     v[1] = b1 * inv;
     v[2] = b2 * inv;
 }
 
-// normal of every point: centroid and covariance of its neighbours (FP64), the smallest
-// eigenvector, flipped towards the viewpoint (in input coordinates), written in input order
+// Normal of every point: centroid and covariance of its neighbours, the smallest eigenvector,
+// flipped towards the viewpoint (in input coordinates), written in input order.  The moments are
+// those of the offsets from the first neighbour: an offset is a float pair (TwoDiff: exact),
+// their products and sums float pairs of about 44 bits, the rest FP64.  Offsets do not cancel
+// against the coordinates' squares, so the covariance is closer to the exact one than FP64 moments
+// of the coordinates (which lose the ratio of the squared coordinate to the squared spacing).
 __global__ void __launch_bounds__(kBlock) k_nrm_pca(const Counters* c, const float* px, const float* py,
                                                     const float* pz, const float* xyz, const unsigned* sidx,
                                                     const int* nbr, float vpx, float vpy, float vpz, float* out) {
     const int n = c->n_points;
     const float nan = __int_as_float(0x7fc00000);
     PSR_GRID_STRIDE(p, n) {
-        int cnt = 0;
-        double sx = 0, sy = 0, sz = 0, sxx = 0, sxy = 0, sxz = 0, syy = 0, syz = 0, szz = 0;
+        int id[kNrmK];
+#pragma unroll
+        for (int q = 0; q < kNrmK; ++q) id[q] = nbr[(size_t)p * kNrmK + q];
+        float nx[kNrmK], ny[kNrmK], nz[kNrmK];
 #pragma unroll
         for (int q = 0; q < kNrmK; ++q) {
-            const int j = nbr[(size_t)p * kNrmK + q];
-            if (j < 0 || j >= n) continue;
-            const double x = px[j], y = py[j], z = pz[j];
+            const int j = (id[q] >= 0 && id[q] < n) ? id[q] : 0;
+            nx[q] = px[j];
+            ny[q] = py[j];
+            nz[q] = pz[j];
+        }
+        int cnt = 0;
+        float o[3] = {0.0f, 0.0f, 0.0f};
+        FF s1[3] = {ff_zero(), ff_zero(), ff_zero()};
+        FF s2[6] = {ff_zero(), ff_zero(), ff_zero(), ff_zero(), ff_zero(), ff_zero()};
+#pragma unroll
+        for (int q = 0; q < kNrmK; ++q) {
+            if (id[q] < 0 || id[q] >= n) continue;
+            const float at[3] = {nx[q], ny[q], nz[q]};
+            if (cnt == 0) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a) o[a] = at[a];
+            }
             ++cnt;
-            sx += x; sy += y; sz += z;
-            sxx += x * x; sxy += x * y; sxz += x * z; syy += y * y; syz += y * z; szz += z * z;
+            FF d[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {   // at - o exactly (Knuth's TwoDiff)
+                const float t = __fsub_rn(at[a], o[a]);
+                const float bv = __fsub_rn(t, at[a]);
+                d[a] = FF{t, __fsub_rn(__fsub_rn(at[a], __fsub_rn(t, bv)), __fadd_rn(o[a], bv))};
+                s1[a] = ff_add(s1[a], d[a]);
+            }
+            int k = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = a; b < 3; ++b) {
+                    FF m = ff_prod(d[a].hi, d[b].hi);
+                    m.lo += fmaf(d[a].hi, d[b].lo, d[a].lo * d[b].hi);
+                    s2[k] = ff_add(s2[k], m);
+                    ++k;
+                }
         }
         const size_t s = sidx[p];
         float nv[3] = {nan, nan, nan};
         if (cnt >= 3) {
-            const double inv = 1.0 / cnt;
-            const double mx = sx * inv, my = sy * inv, mz = sz * inv;
+            const double inv = cnt == kNrmK ? 1.0 / kNrmK : 1.0 / cnt;
+            const double mx = ff_to_double(s1[0]) * inv, my = ff_to_double(s1[1]) * inv, mz = ff_to_double(s1[2]) * inv;
             double v[3];
-            nrm_smallest_eigvec(sxx * inv - mx * mx, sxy * inv - mx * my, sxz * inv - mx * mz, syy * inv - my * my,
-                                syz * inv - my * mz, szz * inv - mz * mz, v);
+            nrm_smallest_eigvec(ff_to_double(s2[0]) * inv - mx * mx, ff_to_double(s2[1]) * inv - mx * my,
+                                ff_to_double(s2[2]) * inv - mx * mz, ff_to_double(s2[3]) * inv - my * my,
+                                ff_to_double(s2[4]) * inv - my * mz, ff_to_double(s2[5]) * inv - mz * mz, v);
             if (v[0] != 0.0 || v[1] != 0.0 || v[2] != 0.0) {
                 const double cosv = (vpx - xyz[3 * s]) * v[0] + (vpy - xyz[3 * s + 1]) * v[1] + (vpz - xyz[3 * s + 2]) * v[2];
                 const double sg = (cosv < 0.0) ? -1.0 : 1.0;
