@@ -43,7 +43,6 @@ struct Counters {
     int n_sub_vertices, n_sub_edges, n_sub_cross, n_sub_tri;
     int n_mesh_vertices, n_mesh_triangles;
     int n_colour_far;             // mesh vertices whose 4 nearest samples the near pass left
-    int n_colour_far2;            //   and of those, the ones the coarser pass left
     int n_colour_cells;           // entries of the colour cell table
     int n_weld;                   // mesh vertices left by welding
     int scan_total;               // scratch total written by scans

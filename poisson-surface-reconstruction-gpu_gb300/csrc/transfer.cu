@@ -116,117 +116,118 @@ __device__ __forceinline__ unsigned spread3(unsigned v) {
     return v;
 }
 
-// Near pass, 8 lanes per mesh vertex: the samples of the 3x3x3 block of finest-level
-// cells around the vertex's cell (every sample outside it is at least one cell width
-// away), spread over the group's lanes (flattened over the 27 cell ranges), each lane
-// keeping a sorted 4-list, merged by warp-minimum rounds within the group.  When 4 were
-// found and the 4th is closer than one width they are the exact 4 nearest and the colour
-// is written; otherwise the vertex goes to the far list for the wide search (k_colour_far).
+// Near pass, 8 lanes per mesh vertex: the samples of the 3x3x3 block of cells around the vertex's
+// cell (every sample outside it is at least one cell width away), spread over the group's lanes
+// (flattened over the 27 cell ranges), each lane keeping a sorted 4-list, merged by warp-minimum
+// rounds within the group.  When 4 were found and the 4th is closer than one width they are the
+// exact 4 nearest and the colour is written.  A vertex that a level leaves goes on to the next
+// coarser one (its cells are ranges of the same table: cell m of level g is the entries
+// m << 3 (gt - g) .. (m + 1) << 3 (gt - g)): a sparse cloud's vertices find their samples there.
+// Coarser blocks of more than kNearCoarseCap samples, and what level kNearCoarsest leaves, go to the
+// far list with the smallest bound found, for the wide search (k_colour_far).  Blocks with fewer
+// than 4 samples are not scanned.  With the finest level alone below depth 8, a depth-7 cloud of
+// 61k points (96k mesh vertices) spent 458 us in the wide search.
 constexpr int kNearLanes = 8;
 constexpr int kNearGroups = kBlock / kNearLanes;
-constexpr int kNearCoarseCap = 512;   // samples the coarser pass scans per vertex at most
-// The same search one or two levels coarser (g < gt, the table's level: cell m of level g
-// is the range of table entries m << 3 (gt - g) .. (m + 1) << 3 (gt - g)) serves the vertices
-// a finer pass left (`in`: (vertex, bound) pairs, *in_count of them), when their block holds
-// at most `cap` samples; the ones it does not settle go on to `out` with the smaller bound.
-__global__ void __launch_bounds__(kBlock) k_colour_near(Counters* c, int g, int gt, const float* mv, const float* px,
+constexpr int kNearCoarseCap = 512;   // samples a coarser level scans per vertex at most
+constexpr int kNearCoarsest = 4;
+__global__ void __launch_bounds__(kBlock) k_colour_near(Counters* c, int gt, const float* mv, const float* px,
                                                         const float* py, const float* pz, const float* cr,
                                                         const float* cg, const float* cb, const int* cell_start,
-                                                        const int* in, const int* in_count, int cap, int* far,
-                                                        int* far_count, float* out) {
-    PSR_CLOUD(c, mv, px, py, pz, cr, cg, cb, cell_start, in, in_count, far, far_count, out);
+                                                        int* far, int* far_count, float* out) {
+    PSR_CLOUD(c, mv, px, py, pz, cr, cg, cb, cell_start, far, far_count, out);
     __shared__ int s_off[kNearGroups][28];
     __shared__ int s_base[kNearGroups][27];
-    const int V = in ? *in_count : c->n_mesh_vertices;
-    const int G = 1 << g;
-    const int shift = 3 * (gt - g);
-    const float w = 1.0f / (float)G;
+    const int V = c->n_mesh_vertices, n = c->n_points;
     const int lane = threadIdx.x & (kNearLanes - 1);
     const int gib = threadIdx.x / kNearLanes;
     const unsigned gmask = 0xffu << (threadIdx.x & 24);   // the group's lanes in its warp
     const int group = (blockIdx.x * blockDim.x + threadIdx.x) / kNearLanes;
     const int ngroups = (gridDim.x * blockDim.x) / kNearLanes;
-    for (int t = group; t < V; t += ngroups) {
-        const int v = in ? in[2 * (size_t)t] : t;
-        const float prev = in ? __int_as_float(in[2 * (size_t)t + 1]) : 1e6f;
+    for (int v = group; v < V; v += ngroups) {
         const float qx = mv[3 * (size_t)v], qy = mv[3 * (size_t)v + 1], qz = mv[3 * (size_t)v + 2];
-        const int cx = min(max((int)floorf(qx * G), 0), G - 1);
-        const int cy = min(max((int)floorf(qy * G), 0), G - 1);
-        const int cz = min(max((int)floorf(qz * G), 0), G - 1);
-        // cells k = lane + 8 r, offsets in k order
-        int running = 0;
+        float bound = 1e6f;   // the 4th squared distance found so far (1e6: none)
+        bool settled = false;
+        for (int g = gt; g == gt || g >= kNearCoarsest; --g) {   // uniform in the group
+            const int G = 1 << g, shift = 3 * (gt - g);
+            const float w = 1.0f / (float)G;
+            const int cx = min(max((int)floorf(qx * G), 0), G - 1);
+            const int cy = min(max((int)floorf(qy * G), 0), G - 1);
+            const int cz = min(max((int)floorf(qz * G), 0), G - 1);
+            // cells k = lane + 8 r, offsets in k order
+            int running = 0;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int k = lane + kNearLanes * r;
-            int cnt = 0, base = 0;
-            if (k < 27) {
-                const int a = cx + k / 9 - 1, b = cy + (k / 3) % 3 - 1, z = cz + k % 3 - 1;
-                if (a >= 0 && a < G && b >= 0 && b < G && z >= 0 && z < G) {
-                    const unsigned m = (spread3((unsigned)a) << 2) | (spread3((unsigned)b) << 1) | spread3((unsigned)z);
-                    base = cell_start[(size_t)m << shift];
-                    cnt = cell_start[(size_t)(m + 1) << shift] - base;
+            for (int r = 0; r < 4; ++r) {
+                const int k = lane + kNearLanes * r;
+                int cnt = 0, base = 0;
+                if (k < 27) {
+                    const int a = cx + k / 9 - 1, b = cy + (k / 3) % 3 - 1, z = cz + k % 3 - 1;
+                    if (a >= 0 && a < G && b >= 0 && b < G && z >= 0 && z < G) {
+                        const unsigned m = (spread3((unsigned)a) << 2) | (spread3((unsigned)b) << 1) | spread3((unsigned)z);
+                        base = cell_start[(size_t)m << shift];
+                        cnt = cell_start[(size_t)(m + 1) << shift] - base;
+                    }
+                }
+                int incl = cnt;
+#pragma unroll
+                for (int o = 1; o < kNearLanes; o <<= 1) {
+                    const int y = __shfl_up_sync(gmask, incl, o, kNearLanes);
+                    if (lane >= o) incl += y;
+                }
+                if (k < 27) {
+                    s_off[gib][k] = running + incl - cnt;
+                    s_base[gib][k] = base;
+                }
+                running += __shfl_sync(gmask, incl, kNearLanes - 1, kNearLanes);
+            }
+            if (lane == 0) s_off[gib][27] = running;
+            __syncwarp(gmask);
+            if (g < gt && running > kNearCoarseCap) break;   // a crowded block: left to the wide search
+            if (running < 4) continue;
+            float bd[4] = {1e6f, 1e6f, 1e6f, 1e6f};
+            int bi[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
+            int k = 0;
+            for (int t = lane; t < running; t += kNearLanes) {
+                while (s_off[gib][k + 1] <= t) ++k;   // flattened index -> cell (increasing)
+                knn_visit(qx, qy, qz, px, py, pz, s_base[gib][k] + (t - s_off[gib][k]), bd, bi);
+            }
+            __syncwarp(gmask);
+            // the group's 4 nearest: four rounds of the minimum head, its lane popping it
+            float md[4];
+            int mi[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                float d = bd[0];
+                int i = bi[0];
+#pragma unroll
+                for (int o = kNearLanes / 2; o > 0; o >>= 1) {
+                    const float od = __shfl_xor_sync(gmask, d, o);
+                    const int oi = __shfl_xor_sync(gmask, i, o);
+                    if (knn_less(od, oi, d, i)) { d = od; i = oi; }
+                }
+                md[r] = d;
+                mi[r] = i;
+                if (bd[0] == d && bi[0] == i) {
+                    bd[0] = bd[1]; bi[0] = bi[1];
+                    bd[1] = bd[2]; bi[1] = bi[2];
+                    bd[2] = bd[3]; bi[2] = bi[3];
+                    bd[3] = 1e6f; bi[3] = 0x7fffffff;
                 }
             }
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < kNearLanes; o <<= 1) {
-                const int y = __shfl_up_sync(gmask, incl, o, kNearLanes);
-                if (lane >= o) incl += y;
+            bound = fminf(bound, md[3]);
+            if (md[3] < w * w) {
+                if (lane == 0) colour_blend(md, mi, cr, cg, cb, &out[3 * (size_t)v]);
+                settled = true;
+                break;
             }
-            if (k < 27) {
-                s_off[gib][k] = running + incl - cnt;
-                s_base[gib][k] = base;
-            }
-            running += __shfl_sync(gmask, incl, kNearLanes - 1, kNearLanes);
+            if (running == n) break;   // every sample seen
         }
-        if (lane == 0) s_off[gib][27] = running;
-        __syncwarp(gmask);
-        if (cap > 0 && running > cap) {   // a crowded block: left to the wide search as it is
-            if (lane == 0) {
-                const int slot = atomicAdd(far_count, 1);
-                far[2 * (size_t)slot] = v;
-                far[2 * (size_t)slot + 1] = __float_as_int(prev);
-            }
-            continue;
-        }
-        float bd[4] = {1e6f, 1e6f, 1e6f, 1e6f};
-        int bi[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
-        int k = 0;
-        for (int t = lane; t < running; t += kNearLanes) {
-            while (s_off[gib][k + 1] <= t) ++k;   // flattened index -> cell (increasing)
-            knn_visit(qx, qy, qz, px, py, pz, s_base[gib][k] + (t - s_off[gib][k]), bd, bi);
+        if (!settled && lane == 0) {
+            const int slot = atomicAdd(far_count, 1);
+            far[2 * (size_t)slot] = v;
+            far[2 * (size_t)slot + 1] = __float_as_int(bound);
         }
         __syncwarp(gmask);
-        // the group's 4 nearest: four rounds of the minimum head, its lane popping it
-        float md[4];
-        int mi[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            float d = bd[0];
-            int i = bi[0];
-#pragma unroll
-            for (int o = kNearLanes / 2; o > 0; o >>= 1) {
-                const float od = __shfl_xor_sync(gmask, d, o);
-                const int oi = __shfl_xor_sync(gmask, i, o);
-                if (knn_less(od, oi, d, i)) { d = od; i = oi; }
-            }
-            md[r] = d;
-            mi[r] = i;
-            if (bd[0] == d && bi[0] == i) {
-                bd[0] = bd[1]; bi[0] = bi[1];
-                bd[1] = bd[2]; bi[1] = bi[2];
-                bd[2] = bd[3]; bi[2] = bi[3];
-                bd[3] = 1e6f; bi[3] = 0x7fffffff;
-            }
-        }
-        if (lane == 0) {
-            if (mi[3] != 0x7fffffff && md[3] < w * w) colour_blend(md, mi, cr, cg, cb, &out[3 * (size_t)v]);
-            else {   // (vertex, the 4th squared distance found so far: an upper bound, 1e6 if none)
-                const int slot = atomicAdd(far_count, 1);
-                far[2 * (size_t)slot] = v;
-                far[2 * (size_t)slot + 1] = __float_as_int(mi[3] != 0x7fffffff ? fminf(md[3], prev) : prev);
-            }
-        }
     }
 }
 
@@ -488,24 +489,11 @@ cudaError_t transfer_build(Workspace& ws, int with_colour, int with_normals) {
     if (with_colour) {
         const int g = D < kColourGridLevel ? D : kColourGridLevel;
         int* cell_start = ws.cell_start;   // (1 << 3g) + 1 entries, from transfer_prepare
-        k_colour_near<<<PSR_GRID(ws, grid), kBlock, 0, s>>>(ws.cnt, g, g, ws.mesh_v, ws.px, ws.py, ws.pz, ws.cr, ws.cg,
-                                                          ws.cb, cell_start, nullptr, nullptr, 0, ws.colour_far,
-                                                          &ws.cnt->n_colour_far, ws.mesh_c);
-        // the vertices it leaves: the same search two levels coarser (a sparse cloud's
-        // vertices find their 4 samples there), then the wide search for the rest
-        const int* far_list = ws.colour_far;
-        const int* far_count = &ws.cnt->n_colour_far;
-        if (D >= 8) {
-            k_colour_near<<<PSR_GRID(ws, grid), kBlock, 0, s>>>(ws.cnt, g - 2, g, ws.mesh_v, ws.px, ws.py, ws.pz, ws.cr,
-                                                              ws.cg, ws.cb, cell_start, ws.colour_far,
-                                                              &ws.cnt->n_colour_far, kNearCoarseCap, ws.colour_far2,
-                                                              &ws.cnt->n_colour_far2, ws.mesh_c);
-            far_list = ws.colour_far2;
-            far_count = &ws.cnt->n_colour_far2;
-        }
+        k_colour_near<<<PSR_GRID(ws, grid), kBlock, 0, s>>>(ws.cnt, g, ws.mesh_v, ws.px, ws.py, ws.pz, ws.cr, ws.cg, ws.cb,
+                                                          cell_start, ws.colour_far, &ws.cnt->n_colour_far, ws.mesh_c);
         k_colour_far<<<PSR_GRID(ws, ws.num_sms * 8), kBlock, 0, s>>>(ws.cnt, g, ws.mesh_v, ws.px, ws.py, ws.pz, ws.cr,
-                                                                   ws.cg, ws.cb, cell_start, far_list, far_count,
-                                                                   ws.mesh_c);
+                                                                   ws.cg, ws.cb, cell_start, ws.colour_far,
+                                                                   &ws.cnt->n_colour_far, ws.mesh_c);
     }
     if (with_normals) {
         double* acc = ws.nacc;
