@@ -340,13 +340,17 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.vfield, 3 * (size_t)dnodes);
     A.add(ws.divg, (size_t)nodes);
     A.add(ws.xsol, (size_t)nodes);
-    A.add(ws.cg_r, (size_t)nodes); A.add(ws.cg_p, (size_t)nodes); A.add(ws.cg_q, (size_t)nodes);
-    A.add(ws.cg_ap, (size_t)nodes);
-    A.add(ws.cg_blk, (size_t)nodes * 8 + 64);
+    const size_t pitch = (size_t)nodes / 8 + 8;   // sibling groups, and a zero group at the end
+    A.add(ws.cg_r, (size_t)nodes); A.add(ws.cg_p, (size_t)nodes); A.add(ws.cg_q, 8 * pitch);
+    A.add(ws.cg_ap, 8 * pitch);
+    if (cfg.max_depth >= 8) {   // the whole-GPU CG
+        A.add(ws.cg_nbg, 27 * pitch);
+        A.add(ws.cg_rp, 8 * pitch);
+        // virtual blocks of 256 groups; a cloud's depths leave at most one part-filled each
+        ws.cg_part_cap = (int)((pitch / 256 + 8) * (size_t)std::max(1, cfg.batch_clouds));
+        A.add(ws.cg_part, 2 * (size_t)ws.cg_part_cap);
+    }
     A.add(ws.cg_desc, 14 * ((size_t)nodes / 8 + 8));
-    A.add(ws.cg_loop, (size_t)kMaxDepth + 1);
-    A.add(ws.cg_loop_part, (size_t)(kMaxDepth + 1) * kLoopMaxBlocks);
-    A.add(ws.cg_loop_ctl, (size_t)kLoopControlWords);
     A.add(ws.cg_partial, std::max((size_t)nodes, (size_t)4096 * (kMaxDepth + 1)));
     A.add(ws.point_val, (size_t)N);
     A.add(ws.pv_coef, 27 * ((size_t)dnodes / 8 + 64));
@@ -446,8 +450,6 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
         if (e == cudaSuccess)
             e = cudaMemset(sc.words, 0, sizeof(unsigned long long) * ((size_t)cap.scan_tiles + kScanHeader));
     }
-    // the device-loop CG's block tickets start at zero; each reduction leaves them at zero
-    if (e == cudaSuccess) e = cudaMemset(ws.cg_loop, 0, sizeof(CgLoopState) * (kMaxDepth + 1));
     ws.sort.max_tiles = sort_tiles;
     e = cudaMallocHost(&h->cnt_host_all, sizeof(Counters) * (size_t)h->clouds);
     ws.cnt_host = h->cnt_host_all;
@@ -464,9 +466,6 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws.ev_geo, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws.aux3, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws.ev_join3, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws.aux4, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws.ev_join4, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws.loop_body, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming);
     // tables
     if (e == cudaSuccess) e = upload_tables_octree();
@@ -533,9 +532,6 @@ psr_status psr_destroy(psr_handle* h) {
     if (h->ws.ev_join2) cudaEventDestroy(h->ws.ev_join2);
     if (h->ws.ev_geo) cudaEventDestroy(h->ws.ev_geo);
     if (h->ws.ev_join3) cudaEventDestroy(h->ws.ev_join3);
-    if (h->ws.ev_join4) cudaEventDestroy(h->ws.ev_join4);
-    if (h->ws.aux4) cudaStreamDestroy(h->ws.aux4);
-    if (h->ws.loop_body) cudaStreamDestroy(h->ws.loop_body);
     if (h->ws.aux3) cudaStreamDestroy(h->ws.aux3);
     if (h->ws.aux2) cudaStreamDestroy(h->ws.aux2);
     if (h->ws.aux) cudaStreamDestroy(h->ws.aux);

@@ -27,6 +27,7 @@ struct Counters {
     int level_base[kMaxDepth + 1];
     int level_tmp_off[kMaxDepth + 1];   // offset of each level inside the build buffer
     int level_groups[kMaxDepth + 1];    // sibling groups of each level (level_count / 8)
+    unsigned long long grid_bar;  // arrivals of the whole-GPU solver's blocks
     unsigned ticket[3];           // blocks done of the bounding box, the encoder, the sample values
     int n_nodes;
     int n_vertices, n_edges, n_faces;
@@ -71,21 +72,6 @@ struct InputRef {
     int n;
 };
 
-// State of one depth's CG when it runs as a device loop (a CUDA-graph while node whose
-// body launches one kernel per step over the whole GPU): the scalars the cluster solver
-// keeps in shared memory, in global memory between the kernels of an iteration.
-struct CgLoopState {
-    double rr, rr_prev, pap, floor2, rr_true;
-    float alpha, beta;
-    int go, check, replace, checks, restarts;
-    int active;              // the depth runs in the device loop (else a cluster solves it)
-    int it;                  // iterations done
-    unsigned ticket;         // blocks of the current kernel done (last-block reductions)
-    unsigned long long t0;   // global timer at the start of the solve
-    unsigned long long t1;   // global timer at the end of its last step
-};
-constexpr int kLoopMaxBlocks = 2048;   // virtual blocks of one depth of the device loop (partials)
-
 // Look-up tables shared by the kernels (values derived in tables.cpp).
 struct ConstTables {
     int lut_parent[8][27];
@@ -109,10 +95,6 @@ struct ConstTables {
 // workspace address are its slot.
 constexpr unsigned long long kCloudStride = 1ull << 35;   // 32 GiB of address space per cloud
 constexpr int kMaxBatchClouds = 64;
-// words of the device loop's control block (pass and unit counts, the unit list, its
-// virtual-block offsets)
-constexpr int kLoopControlWords = 3 + 2 * kMaxBatchClouds * (kMaxDepth + 1);
-
 // blocks along x of a launch over `clouds` clouds whose one-cloud launch has gx blocks:
 // about twice the one-cloud grid in total (each cloud's blocks stride over its work), at
 // least one block per cloud

@@ -98,11 +98,6 @@ constexpr int kCgGroups = 1792;                   // local groups of a CTA's arr
 constexpr int kCgRowGroups = kCgcBlock / 8;       // at most this many groups: a thread per row
 constexpr int kCgDescWords = 14;                  // 27 neighbour groups, two per word
 constexpr size_t kCgSmemBytes = (size_t)kCgGroups * 8 * (sizeof(float2) + 2 * sizeof(float));   // (r, p), x, A p
-// per-warp shared block of 4 sibling groups (device loop): group gi at gi * 80 + {0, 18, 8,
-// 26}[gi] floats, so the 4 groups start in banks 0, 2, 8, 10 and the 32 lanes' stencil reads (at
-// sibling offsets {0,1,4,5,16,17,20,21} + a common neighbour offset) hit 32 distinct banks
-constexpr int kCgWarpBlockFloats = 352;
-
 constexpr int kCgMaxRefine = 4;
 
 // Workspace pointers of the CG; a multi-cloud launch moves them to the CTA's cloud (a
@@ -113,7 +108,6 @@ struct CgcVec {
     const int* neigh;
     const int* parent;
     const int* first_child;
-    const int* blk;     // device loop: 64 entries per sibling group of depth >= 1
     unsigned* desc;     // [kCgDescWords][dstride]: packed neighbour groups of CTAs with more than one group a thread
     const float* stencil;
     const float* b;
@@ -122,7 +116,7 @@ struct CgcVec {
     float* pa;
     float* pb;
     float* ap;
-    __device__ void rebase() { PSR_CLOUD(c, cw, neigh, parent, first_child, blk, desc, stencil, b, x, r, pa, pb, ap); }
+    __device__ void rebase() { PSR_CLOUD(c, cw, neigh, parent, first_child, desc, stencil, b, x, r, pa, pb, ap); }
 };
 
 // a workspace pointer of cloud 0 moved to cloud k (null stays null)
@@ -141,7 +135,6 @@ struct CgcArgs {
     int max_iter;
     int res_period;     // > 0: true residual every res_period iterations; 0: only at
                         // convergence; < 0: never (the recursive residual alone)
-    unsigned loop_mask; // depths the device loop solves when they do not fit the cluster
     int clusters;       // units solved by a whole cluster; the CTAs of the clusters behind them
                         // solve a coarser depth each
 };
@@ -338,68 +331,16 @@ __device__ __forceinline__ void cgc_allreduce(unsigned nb, unsigned me, CgcShare
 
 // After the r.r reduction of an iteration (thread 0): beta, the continue flag and whether
 // the true residual is due.  `it` is the iteration just completed.
-// The step scalars are quotients of the FP64 sums rounded to float and divided in FP32 (within
-// 1.5 ulp of the FP64 quotient rounded to float): an FP64 division on the one thread that
-// finishes the sums sits on every iteration's critical path, and GB300 divides in FP64
-// slowly.
-__device__ __forceinline__ float cg_quot(double num, double den) {
-    return den != 0.0 ? __fdiv_rn((float)num, (float)den) : 0.0f;
-}
-
-template <class St, class Ar>
-__device__ __forceinline__ void cg_after_rr(St& sh, const Ar& a, double w, int it) {
-    sh.beta = cg_quot(w, sh.rr);
-    sh.rr_prev = sh.rr;
-    sh.rr = w;
-    const bool conv = !((float)w > a.tol2);   // the reference compares a float r.r (CGAlgorithm.cu:36)
-    const bool more = sh.pap != 0.0 && it + 1 <= a.max_iter;
-    sh.go = !conv && more;
-    sh.check = a.res_period >= 0 && sh.pap != 0.0 &&
-               (conv || (a.res_period > 0 && it % a.res_period == 0 && more));
-}
-
-// After the true-residual reduction (thread 0).  The CG restarts from the true residual
-// (beta = 0: one cycle of iterative refinement) when that residual is above both the
-// tolerance and the floor an FP32 solution can reach, and either the recursive residual
-// has converged or has drifted more than 2x (in norm) below the true one; at most
-// kCgMaxRefine restarts, each one reducing the true r.r at least fourfold.  `it` is the
-// next iteration's number.
-template <class St, class Ar>
-__device__ __forceinline__ void cg_after_true(St& sh, const Ar& a, double w, int it) {
-    ++sh.checks;
-    const double target = fmax((double)a.tol2, sh.floor2);
-    const bool drift = w > 4.0 * fmax(sh.rr, sh.floor2);
-    const bool falling = sh.rr_true < 0.0 || w < 0.25 * sh.rr_true;
-    sh.replace = w > target && (!sh.go || drift) && sh.restarts < kCgMaxRefine && it <= a.max_iter && falling;
-    if (sh.replace) {
-        ++sh.restarts;
-        sh.beta = 0.0f;
-        sh.go = 1;
-        sh.rr = w;
-    }
-    sh.rr_true = w;
-}
-
-// Start of a solve (thread 0): r0 = b, so r.r is also ||b||^2.
-template <class St, class Ar>
-__device__ __forceinline__ void cg_start(St& sh, const Ar& a, double w) {
-    sh.rr = w;
-    sh.beta = 0.0f;
-    sh.go = ((float)w > a.tol2) && a.max_iter >= 1;
-    sh.floor2 = w * 0x1p-40;
-    sh.rr_true = -1.0;
-    sh.checks = 0;
-    sh.restarts = 0;
-    sh.replace = 0;
-}
-
-// The same decisions from fixed-point sums (the cluster solver)
-__device__ __forceinline__ void cgc_alpha(CgcShared& sh, const CgSum& t) {
+// The step scalars are quotients of the sums rounded to float and divided in FP32 (within 1.5 ulp of
+// the exact quotient rounded to float): an FP64 division on the one thread that finishes the sums
+// would sit on every iteration's critical path, and GB300 divides in FP64 slowly.
+template <class St>
+__device__ __forceinline__ void cgc_alpha(St& sh, const CgSum& t) {
     sh.pap = t;
     sh.alpha = t.m != 0 ? __fdiv_rn(sh.rrf, cgs_float(t)) : 0.0f;
 }
-template <class Ar>
-__device__ __forceinline__ void cgc_after_rr(CgcShared& sh, const Ar& a, const CgSum& t, int it) {
+template <class St, class Ar>
+__device__ __forceinline__ void cgc_after_rr(St& sh, const Ar& a, const CgSum& t, int it) {
     const float w = cgs_float(t);
     sh.beta = sh.rr.m != 0 ? __fdiv_rn(w, sh.rrf) : 0.0f;
     sh.rr = t;
@@ -411,8 +352,15 @@ __device__ __forceinline__ void cgc_after_rr(CgcShared& sh, const Ar& a, const C
     if (due) sh.until_check = a.res_period;
     sh.check = a.res_period >= 0 && sh.pap.m != 0 && (conv || (due && more));
 }
-template <class Ar>
-__device__ __forceinline__ void cgc_after_true(CgcShared& sh, const Ar& a, const CgSum& t, int it) {
+
+// After the true-residual reduction (thread 0).  The CG restarts from the true residual
+// (beta = 0: one cycle of iterative refinement) when that residual is above both the
+// tolerance and the floor an FP32 solution can reach, and either the recursive residual
+// has converged or has drifted more than 2x (in norm) below the true one; at most
+// kCgMaxRefine restarts, each one reducing the true r.r at least fourfold.  `it` is the
+// next iteration's number.
+template <class St, class Ar>
+__device__ __forceinline__ void cgc_after_true(St& sh, const Ar& a, const CgSum& t, int it) {
     ++sh.checks;
     const double w = cgs_double(t), rr = cgs_double(sh.rr);
     const double target = fmax((double)a.tol2, sh.floor2);
@@ -428,8 +376,10 @@ __device__ __forceinline__ void cgc_after_true(CgcShared& sh, const Ar& a, const
     }
     sh.rr_true = w;
 }
-template <class Ar>
-__device__ __forceinline__ void cgc_start(CgcShared& sh, const Ar& a, const CgSum& t) {
+
+// Start of a solve (thread 0): r0 = b, so r.r is also ||b||^2.
+template <class St, class Ar>
+__device__ __forceinline__ void cgc_start(St& sh, const Ar& a, const CgSum& t) {
     sh.rr = t;
     sh.rrf = cgs_float(t);
     sh.beta = 0.0f;
@@ -443,13 +393,6 @@ __device__ __forceinline__ void cgc_start(CgcShared& sh, const Ar& a, const CgSu
 }
 
 // Per-depth results of a finished solve (thread 0 of cluster CTA 0).
-template <class St>
-__device__ __forceinline__ void cg_report(const CgcVec& v, int d, const St& sh) {
-    v.cw->cg_rr[d] = sh.rr;
-    v.cw->cg_rr_true[d] = sh.rr_true;
-    v.cw->cg_checks[d] = sh.checks;
-    v.cw->cg_restarts[d] = sh.restarts;
-}
 // The iteration count goes out here and not per iteration: a global store in flight would hold
 // up the release at every reduction.
 __device__ __forceinline__ void cgc_report(const CgcVec& v, int d, const CgcShared& sh, int iterations) {
@@ -458,31 +401,6 @@ __device__ __forceinline__ void cgc_report(const CgcVec& v, int d, const CgcShar
     v.cw->cg_rr_true[d] = sh.rr_true;
     v.cw->cg_checks[d] = sh.checks;
     v.cw->cg_restarts[d] = sh.restarts;
-}
-
-// position of neighbour k (9 ox + 3 oy + oz) of sibling s (x = 4, y = 2, z = 1) in the
-// group's 4x4x4 block (16 bx + 4 by + bz)
-__host__ __device__ constexpr int cg_kpos(int k) { return 16 * (k / 9) + 4 * ((k / 3) % 3) + (k % 3); }
-__device__ __forceinline__ int cg_spos(int s) { return 16 * ((s >> 2) & 1) + 4 * ((s >> 1) & 1) + (s & 1); }
-
-// Block table of every sibling group (depth >= 1; group G = rows 1 + 8G .. 8 + 8G):
-// block position (bx, by, bz) holds neighbour (ox, oy, oz) of sibling (cx, cy, cz) with
-// b = c + o, taking c = 1 on an axis where b >= 2, else 0.  Stored transposed: table
-// entry j of a group is position (j & 7) * 8 + (j >> 3), so lane s of a group reads its
-// 8 positions s, s + 8, ... as two contiguous int4.
-__global__ void __launch_bounds__(kBlock) k_cg_blocks(const Counters* c, const int* neigh, size_t stride,
-                                                      int* blk) {
-    PSR_CLOUD(c, neigh, blk);
-    const int ngroups = (c->n_nodes - 1) >> 3;
-    PSR_GRID_STRIDE(t, ngroups * 64) {
-        const int G = t >> 6, j = t & 63;
-        const int pos = ((j & 7) << 3) | (j >> 3);
-        const int bx = pos >> 4, by = (pos >> 2) & 3, bz = pos & 3;
-        const int cx = bx >= 2, cy = by >= 2, cz = bz >= 2;
-        const int k = 9 * (bx - cx) + 3 * (by - cy) + (bz - cz);
-        const int sib = 4 * cx + 2 * cy + cz;
-        blk[t] = neigh[(size_t)k * stride + 1 + 8 * G + sib];
-    }
 }
 
 struct CgUnit {
@@ -901,382 +819,437 @@ __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
         const int m = u.row1 - u.row0;
         const int chunk = cg_chunk_groups(m, (int)u.nb);
         const bool fits = cg_fits_resident(u.d, m, (int)u.nb);   // the same in all CTAs of the unit
-        if (fits || !((a.loop_mask >> u.d) & 1u)) {   // else the device loop solves this depth
-            if (!fits) cgc_global(cl, sh, a, v, u);
-            else if (chunk <= kCgRowGroups) cgc_resident<kCgRows>(cl, sh, a, v, u, chunk, cg_dyn);
-            else if (chunk <= kCgcBlock) cgc_resident<kCgOne>(cl, sh, a, v, u, chunk, cg_dyn);
-            else cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);
-            if (u.me == 0 && threadIdx.x == 0) v.cw->cg_depth_ns[u.d] = global_ns() - t_start;
-        }
+        if (!fits) cgc_global(cl, sh, a, v, u);
+        else if (chunk <= kCgRowGroups) cgc_resident<kCgRows>(cl, sh, a, v, u, chunk, cg_dyn);
+        else if (chunk <= kCgcBlock) cgc_resident<kCgOne>(cl, sh, a, v, u, chunk, cg_dyn);
+        else cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);
+        if (u.me == 0 && threadIdx.x == 0) v.cw->cg_depth_ns[u.d] = global_ns() - t_start;
     }
     cl.sync();   // no CTA exits while others may still read its shared memory
 }
 
-// ---- device-loop CG: the depths too large for a cluster's shared memory -----------------
-// A depth whose cluster chunk does not fit shared memory (cg_fits_resident false) is solved
-// by a loop of whole-GPU kernels inside a CUDA-graph while node.  Body, per pass: twice the
-// true residual when it is due (k_cgl_true), p and A p with p.Ap (k_cgl_spmv), x and r with
-// r.r (k_cgl_update); then one thread lists the (depth, cloud) units that go on and ends
-// the loop when none does (k_cgl_control).  The iteration, the decisions after each
-// reduction and the precision (exact products, float-pair sums in a thread and a warp, FP64
-// across warps and blocks, in a fixed order) are the cluster solver's; the scalars live in
-// a CgLoopState per depth.  Each unit's work is split over virtual blocks, one per
-// kLoopRowsPerSplit rows, which the launch's blocks take in turn over the listed units, so
-// the sums keep one order whatever the number of clouds, and units that are done cost
-// nothing.  Every reduction
-// ends in the last virtual block to finish (a ticket counter after a fence), which sums the
-// virtual blocks' partials in order; every virtual block has read the state before it
-// takes its ticket, so the last one may clear a flag the kernel acted on.  The loop ends
-// after at most max_iter iterations per depth; no block waits on another.
-// Operator: the block-table gathers of the resident path (8 per row: each lane of a warp
-// loads its sibling group's 8 block entries, the group's 64 values go to a per-warp shared
-// block, the 27-point stencil reads them there), from global memory.
-constexpr int kLoopBlock = 256;
-constexpr int kLoopWarps = kLoopBlock / 32;
-constexpr int kLoopUnroll = 2;   // CG iterations per pass of the while node's body
-static_assert(kLoopMaxBlocks >= 1, "partials per unit");
+// ---- whole-GPU CG: the depths from 5 on of trees of depth 8 and 9 ------------------------
+// One cooperative launch (so all its blocks are resident) solves every unit -- a depth of a cloud
+// -- in lockstep rounds: A p with p.Ap, grid barrier, x and r with r.r, grid barrier.  A unit
+// whose true residual is due spends a round on it instead.  The arithmetic, the reductions'
+// precision and the decisions are the cluster solver's; the scalars of a unit are kept in the
+// shared memory of every block that works on it, each computing them from the same sums.
+// Work is dealt in virtual blocks of 256 sibling groups of one unit, a contiguous range of them
+// per block; a thread applies the operator to a group (cg_apply_group), from global memory with
+// sibling-major vectors (row `sib` of group G at sib * pitch + G), so that a warp's 32 consecutive
+// groups read consecutive words for their own rows and runs of them for their neighbours'.  The
+// neighbour groups (27 a group, 13.5 bytes a row) are looked up once per solve.  Each virtual
+// block's sum goes to global memory and every block adds a unit's sums in one order, which
+// depends on the unit's rows alone: a cloud's result is the same alone and in a batch.
+// A round of 1.2M rows takes 21 us, of 3.1M rows 50 us, bound by L2 traffic and the two grid
+// barriers (3.4k cycles each); the CUDA-graph while node over whole-GPU kernels before it took 43 and
+// 97 us (7 launches per two iterations).  Keeping the block's p in shared memory and reading only
+// other blocks' groups from L2 was slower (5.0 ms against 3.4 of 3.1M rows): the scattered remote
+// reads wait one by one.
+constexpr int kGridBlock = 512;    // 128 registers a thread: a group's 27 neighbours and 32 loads in flight
+constexpr int kVbGroups = 256;                       // groups of a virtual block
+constexpr int kGridSubs = kGridBlock / kVbGroups;    // virtual blocks a block works on at once
+constexpr int kGridDepth = 5;                        // depths below it: at most 4096 rows, one CTA each
+static_assert(sizeof(CgSum) == 16, "workspace.h: cg_part");
 
-struct CgLoopArgs {
-    CgcVec v;            // cloud 0's workspace
-    CgLoopState* st;     // per depth (cloud 0)
-    double* part;        // per depth: kLoopMaxBlocks partial sums (cloud 0)
-    unsigned* ctl;       // CgLoopControl (cloud 0 only)
-    int first;           // unit z solves depth first - z
-    int units, clouds;
-    int ctas[kMaxDepth + 1];   // CTAs of the cluster launch that owns each depth
-    unsigned loop_mask;
+struct CgGridArgs {
+    CgcVec v;             // cloud 0's workspace
+    int depth;
+    int first, last;      // depths first .. last (descending) of every cloud
+    int clouds;
+    size_t stride;
+    unsigned pitch;       // groups of the sibling-major arrays; the last one is the zero group (element
+                          // numbers up to 8 * pitch fit 32 bits)
+    int* nbg;             // [27][pitch]: neighbour groups
+    float2* rp;           // [8][pitch]: (r, p)
+    float* xs;            // [8][pitch]: x
+    float* ap;            // [8][pitch]: A p
+    CgSum* part;          // [2][part_cap]: sums of the virtual blocks (cloud 0)
+    int part_cap;
+    unsigned long long* bar;   // arrivals, and above 32 bits the blocks that had work (cloud 0; starts at 0)
     float tol2;
     int max_iter;
     int res_period;
 };
 
-// Loop control of a launch: body passes run so far, the units (cloud << 8 | z) the next
-// pass works on, and the first virtual block of each (vstart[count]: their total).
-struct CgLoopControl {
-    unsigned passes;
-    unsigned count;
-    unsigned list[kMaxBatchClouds * (kMaxDepth + 1)];
-    unsigned vstart[kMaxBatchClouds * (kMaxDepth + 1) + 1];
-};
-static_assert(sizeof(CgLoopControl) == sizeof(unsigned) * kLoopControlWords, "control block words");
-constexpr int kLoopRowsPerSplit = 1024;   // rows per virtual block (below 2M rows)
-
-// virtual blocks of a unit of m rows: one per kLoopRowsPerSplit rows, at most
-// kLoopMaxBlocks (the sums' order depends on m alone)
-__device__ __forceinline__ unsigned loop_split(int m) {
-    const int v = (m + kLoopRowsPerSplit - 1) / kLoopRowsPerSplit;
-    return (unsigned)(v < 1 ? 1 : (v > kLoopMaxBlocks ? kLoopMaxBlocks : v));
-}
-
-struct LoopUnit {
-    int d, row0, m, bx, split;
-    CgcVec v;
-    CgLoopState* st;
-    double* part;
+// State of one unit in a block's shared memory (the cluster solver's scalars).
+struct CgGridUnit {
+    CgSum rr, pap;
+    double floor2, rr_true;
+    float rrf, alpha, beta;
+    int go, check, replace, checks, restarts, until_check;
+    int it;               // iterations done
+    int resid;            // this round evaluated the true residual
+    int d, k;             // depth, cloud
+    int G0, ng;           // first group (global number), groups
+    int vb0, nvb;         // first virtual block of the launch, virtual blocks
+    float w[4];           // centre, face, edge, corner
+    float own[8];         // p of the first group's rows where its table does not name itself
 };
 
-// virtual block vb of the listed units: its unit (cloud's workspace) and index in the unit
-__device__ __forceinline__ LoopUnit loop_unit(const CgLoopArgs& a, const CgLoopControl* ctl, int vb) {
-    int lo = 0, hi = (int)ctl->count - 1;   // the unit i with vstart[i] <= vb < vstart[i + 1]
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if ((int)ctl->vstart[mid] <= vb) lo = mid;
-        else hi = mid - 1;
-    }
-    const unsigned e = ctl->list[lo];
-    const int k = (int)(e >> 8), z = (int)(e & 255u);
-    LoopUnit u;
-    u.bx = vb - (int)ctl->vstart[lo];
-    u.split = (int)(ctl->vstart[lo + 1] - ctl->vstart[lo]);
-    u.d = a.first - z;
-    u.v = a.v;
-    u.v.c = at_cloud(a.v.c, k); u.v.cw = at_cloud(a.v.cw, k); u.v.neigh = at_cloud(a.v.neigh, k);
-    u.v.blk = at_cloud(a.v.blk, k); u.v.stencil = at_cloud(a.v.stencil, k); u.v.b = at_cloud(a.v.b, k);
-    u.v.x = at_cloud(a.v.x, k); u.v.r = at_cloud(a.v.r, k); u.v.pa = at_cloud(a.v.pa, k);
-    u.v.pb = at_cloud(a.v.pb, k); u.v.ap = at_cloud(a.v.ap, k);
-    u.row0 = u.v.c->level_base[u.d];
-    u.m = u.v.c->level_count[u.d];
-    u.st = at_cloud(a.st, k) + u.d;
-    u.part = at_cloud(a.part, k) + (size_t)u.d * kLoopMaxBlocks;
-    return u;
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
 }
 
-// Sum of every thread's `v` over the unit's virtual blocks (FP64).  Returns true in the
-// block that finishes the sum, with the sum in `w` of thread 0 (the ticket is back at zero).
-__device__ __forceinline__ bool loop_reduce(FF v, const LoopUnit& u, double& w) {
-    const int split = u.split;
-    __shared__ double s_w[kLoopWarps];
-    __shared__ int s_last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v = ff_warp_sum(v);
-    if (lane == 0) s_w[warp] = ff_to_double(v);
+// Every block of the launch has arrived `round` times; `active` adds to the count above 32 bits.
+// Thread 0's fences make the block's writes visible to the others and theirs to the block (as a
+// cooperative-groups grid barrier does).  Bounded: false when the wait ran out.
+__device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned target, bool active,
+                                             unsigned long long& seen) {
+    __shared__ unsigned long long s_seen;
+    __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double b = 0.0;
-        for (int k = 0; k < kLoopWarps; ++k) b += s_w[k];
-        u.part[u.bx] = b;
         __threadfence();
-        s_last = atomicAdd(&u.st->ticket, 1u) == (unsigned)split - 1;
+        atomicAdd(bar, 1ull + (active ? 1ull << 32 : 0ull));
+        unsigned long long v = ld_acquire_u64(bar);
+        int spin = 0;
+        while ((int)((unsigned)v - target) < 0 && ++spin < kSpinLimit) v = ld_acquire_u64(bar);
+        __threadfence();
+        s_seen = v;
+        s_ok = (int)((unsigned)v - target) >= 0;
     }
     __syncthreads();
-    const bool last = s_last;
-    if (last) {
-        __threadfence();
-        if (warp == 0) {
-            double t = 0.0;
-            for (int k = lane; k < split; k += 32) t += __ldcg(&u.part[k]);
-            t = dbl_warp_sum(t);
-            if (lane == 0) {
-                w = t;
-                u.st->ticket = 0u;
+    seen = s_seen;
+    return s_ok != 0;
+}
+
+// a + b, aligned like the lanes of a warp sum
+__device__ __forceinline__ CgSum cgs_add(CgSum a, CgSum b) {
+    auto top_of = [](const CgSum& v) { return v.m != 0 ? (int)v.e + 64 - __clzll(v.m < 0 ? -v.m : v.m) : 0; };
+    const int e = max(top_of(a), top_of(b)) - 57;
+    auto to = [&](const CgSum& v) -> long long {
+        const int d = e - (int)v.e;
+        if (v.m == 0) return 0;
+        if (d <= 0) return d > -64 ? v.m << -d : 0;
+        return d < 63 ? ((v.m >> (d - 1)) + 1) >> 1 : 0;
+    };
+    return CgSum{to(a) + to(b), e};
+}
+
+__global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
+    extern __shared__ float4 cg_dyn[];
+    CgGridUnit* U = reinterpret_cast<CgGridUnit*>(cg_dyn);   // one per unit of the launch
+    __shared__ int4 s_w[2][kGridBlock / 32];
+    __shared__ CgSum s_sum[kGridBlock / 32];
+    __shared__ int s_total;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sub = tid / kVbGroups, subt = tid % kVbGroups;
+    const int per = a.first - a.last + 1, nu = per * a.clouds;
+    const unsigned long long t0 = global_ns();
+    unsigned* err = &a.v.cw->error;
+    // the units: cloud after cloud, depth after depth
+    for (int u = tid; u < nu; u += kGridBlock) {
+        CgGridUnit& q = U[u];
+        q.k = u / per;
+        q.d = a.first - (u - q.k * per);
+        const Counters* c = at_cloud(a.v.c, q.k);
+        q.G0 = (c->level_base[q.d] - 1) >> 3;
+        q.ng = c->level_count[q.d] >> 3;
+        q.nvb = (q.ng + kVbGroups - 1) / kVbGroups;
+        const float* st = at_cloud(a.v.stencil, q.k) + q.d * 27;
+        q.w[0] = st[13]; q.w[1] = st[14]; q.w[2] = st[17]; q.w[3] = st[26];
+        q.go = q.check = q.replace = q.resid = q.it = 0;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int v = 0;
+        for (int u = 0; u < nu; ++u) {
+            U[u].vb0 = v;
+            v += U[u].nvb;
+        }
+        s_total = v;
+    }
+    __syncthreads();
+    const int total = s_total;
+    if (total > a.part_cap) {   // uniform over the launch
+        if (blockIdx.x == 0 && tid == 0) atomicOr(err, kErrCapacity);
+        return;
+    }
+    // this block's virtual blocks, and the units they belong to
+    const int v0 = (int)((long long)total * blockIdx.x / gridDim.x);
+    const int v1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
+    const int npass = (v1 - v0 + kGridSubs - 1) / kGridSubs;
+    auto unit_of = [&](int v) {
+        int lo = 0, hi = nu - 1;   // the last unit with vb0 <= v
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (U[mid].vb0 <= v) lo = mid;
+            else hi = mid - 1;
+        }
+        return lo;
+    };
+    const int u0 = v0 < v1 ? unit_of(v0) : 0, u1 = v0 < v1 ? unit_of(v1 - 1) + 1 : 0;
+    unsigned target = 0;
+    unsigned long long seen = 0;
+    int buf = 0;
+
+    // one step over the block's virtual blocks: body(unit, first group thread's G, local group, on)
+    // returns the thread's contribution; `skip(unit)`: the unit takes no part.  Ends with the grid
+    // barrier; the sums of the units are then in part[buf].
+    auto step = [&](bool active, auto skip, auto body) -> bool {
+        for (int p = 0; p < npass; ++p) {
+            const int vb = v0 + p * kGridSubs + sub;
+            FF acc = ff_zero();
+            int u = -1;
+            if (vb < v1) {
+                u = unit_of(vb);
+                if (skip(U[u])) u = -1;
+            }
+            if (u >= 0) {
+                const int g = (vb - U[u].vb0) * kVbGroups + subt;
+                if (g < U[u].ng) acc = body(U[u], g);
+            }
+            int4 ws = make_int4(0, 0, 0, 0);
+            if (__any_sync(0xffffffffu, acc.hi != 0.0f)) ws = cgs_warp_sum(acc);
+            if (lane == 0) s_w[p & 1][warp] = ws;
+            __syncthreads();
+            if (u >= 0 && (warp & (kVbGroups / 32 - 1)) == 0) {
+                const CgSum t = cgs_warp_sum(cgs_join(lane < kVbGroups / 32 ? s_w[p & 1][warp + lane] : make_int4(0, 0, 0, 0)));
+                if (lane == 0) a.part[(size_t)buf * a.part_cap + vb] = t;
             }
         }
-    }
-    __syncthreads();   // s_w and s_last are reused by the next virtual block
-    return last;
-}
-
-// One thread, before the loop: which depths of which clouds the loop solves (the others
-// are marked inactive), listed for the first pass.
-__global__ void k_cgl_plan(CgLoopArgs a) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    CgLoopControl* ctl = reinterpret_cast<CgLoopControl*>(a.ctl);
-    unsigned n = 0;
-    ctl->vstart[0] = 0u;
-    for (int k = 0; k < a.clouds; ++k) {
-        const Counters* c = at_cloud(a.v.c, k);
-        CgLoopState* st = at_cloud(a.st, k);
-        for (int z = 0; z < a.units; ++z) {
-            const int d = a.first - z;
-            const bool active = ((a.loop_mask >> d) & 1u) && !cg_fits_resident(d, c->level_count[d], a.ctas[d]);
-            st[d].active = active;
-            st[d].go = 0;
-            st[d].check = 0;
-            st[d].replace = 0;
-            st[d].it = 0;
-            if (active) {
-                ctl->list[n] = ((unsigned)k << 8) | (unsigned)z;
-                ctl->vstart[n + 1] = ctl->vstart[n] + loop_split(c->level_count[d]);
-                ++n;
+        target += gridDim.x;
+        return grid_barrier(a.bar, target, active, seen);
+    };
+    // the units' sums: a warp a unit, or the block where there are many virtual blocks (the order
+    // depends on the unit alone); post(unit, sum) by one thread
+    auto sums = [&](auto skip, auto post) {
+        const CgSum* part = a.part + (size_t)buf * a.part_cap;
+        for (int u = u0 + warp; u < u1; u += kGridBlock / 32) {
+            if (U[u].nvb > 32 || skip(U[u])) continue;
+            const CgSum t = cgs_warp_sum(lane < U[u].nvb ? part[U[u].vb0 + lane] : CgSum{0, 0});
+            if (lane == 0) post(U[u], t);
+        }
+        for (int u = u0; u < u1; ++u) {
+            if (U[u].nvb <= 32 || skip(U[u])) continue;   // the same in all threads: flags change below only
+            CgSum t{0, 0};
+            for (int v = tid; v < U[u].nvb; v += kGridBlock) t = cgs_add(t, part[U[u].vb0 + v]);
+            t = cgs_warp_sum(t);
+            if (lane == 0) s_sum[warp] = t;
+            __syncthreads();
+            if (warp == 0) {
+                t = cgs_warp_sum(lane < kGridBlock / 32 ? s_sum[lane] : CgSum{0, 0});
+                if (lane == 0) post(U[u], t);
             }
+            __syncthreads();
         }
-    }
-    ctl->count = n;
-    ctl->passes = 0u;
-}
-
-// r0 = b, p_{-1} = 0 (buffer pa), x0 = 0 for the listed depths
-__global__ void __launch_bounds__(kLoopBlock) k_cgl_init(CgLoopArgs a) {
-    const CgLoopControl* ctl = reinterpret_cast<const CgLoopControl*>(a.ctl);
-    const int nv = (int)ctl->vstart[ctl->count];
-    for (int vb = blockIdx.x; vb < nv; vb += gridDim.x) {
-        const LoopUnit u = loop_unit(a, ctl, vb);
-        FF acc = ff_zero();
-        for (int i = u.bx * kLoopBlock + threadIdx.x; i < u.m; i += u.split * kLoopBlock) {
-            const float bi = u.v.b[u.row0 + i];
-            u.v.r[u.row0 + i] = bi;
-            u.v.pa[u.row0 + i] = 0.0f;
-            u.v.x[u.row0 + i] = 0.0f;
-            acc = ff_add(acc, ff_prod(bi, bi));
-        }
-        double w = 0.0;
-        if (loop_reduce(acc, u, w) && threadIdx.x == 0) {
-            cg_start(*u.st, a, w);
-            u.st->t0 = global_ns();
-            u.st->t1 = u.st->t0;
-        }
-    }
-}
-
-// the sibling group's block-table entries of lane (l, sib)
-__device__ __forceinline__ const int4* loop_blk(const LoopUnit& u, int l, int sib) {
-    return reinterpret_cast<const int4*>(u.v.blk + (size_t)(((u.row0 - 1) >> 3) + (l >> 3)) * 64 + sib * 8);
-}
-
-// True residual b - A x when due (exact products, float-pair sums), staged in the direction
-// buffer the next iteration writes, and the refinement decision.
-__global__ void __launch_bounds__(kLoopBlock) k_cgl_true(CgLoopArgs a) {
-    const CgLoopControl* ctl = reinterpret_cast<const CgLoopControl*>(a.ctl);
-    __shared__ float s_st[27];
-    __shared__ float sblk[kLoopWarps * kCgWarpBlockFloats];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gi = lane >> 3, sib = lane & 7;
-    const int spos = cg_spos(sib);
-    float* myblk = sblk + warp * kCgWarpBlockFloats + gi * 80 + ((0x1a081200 >> (gi * 8)) & 0xff);
-    const int nv = (int)ctl->vstart[ctl->count];
-    for (int vb = blockIdx.x; vb < nv; vb += gridDim.x) {
-        const LoopUnit u = loop_unit(a, ctl, vb);
-        if (!u.st->check) continue;   // uniform over the block
-        const int next = u.st->it + 1;
-        float* stage = (next & 1) ? u.v.pb : u.v.pa;
-        if (threadIdx.x < 27) s_st[threadIdx.x] = u.v.stencil[u.d * 27 + threadIdx.x];
+        buf ^= 1;
         __syncthreads();
-        const int nslot = (u.m + 31) >> 5;
-        FF acc = ff_zero();
-        for (int sl = u.bx * kLoopWarps + warp; sl < nslot; sl += u.split * kLoopWarps) {
-            const int l = sl * 32 + lane;
-            const bool mine = l < u.m;   // whole groups: a group is all in or all out
-            if (mine) {
-                const int4* bp = loop_blk(u, l, sib);
-                const int4 q0 = bp[0], q1 = bp[1];
-                const int ids[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-                float vals[8];
+    };
+
+    // neighbour groups; r0 = b, p_{-1} = 0, x0 = 0
+    if (blockIdx.x == 0 && tid < 8)
+        for (int k = 0; k < a.clouds; ++k) {
+            at_cloud(a.rp, k)[tid * a.pitch + a.pitch - 1] = make_float2(0.0f, 0.0f);
+            at_cloud(a.xs, k)[tid * a.pitch + a.pitch - 1] = 0.0f;
+        }
+    bool ok = step(
+        true, [](const CgGridUnit&) { return false; },
+        [&](const CgGridUnit& q, int g) {
+            const int G = q.G0 + g;
+            CgcVec v = a.v;
+            v.neigh = at_cloud(a.v.neigh, q.k);
+            v.first_child = at_cloud(a.v.first_child, q.k);
+            const int pa = at_cloud(a.v.parent, q.k)[1 + 8 * G];
+            int* nbg = at_cloud(a.nbg, q.k);
+            int H[27];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) vals[e] = ids[e] >= 0 ? u.v.x[ids[e]] : 0.0f;
+            for (int n = 0; n < 27; ++n) H[n] = cg_neighbour_group(v, a.stride, pa, n);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) myblk[e * 8 + sib] = vals[e];
+            for (int n = 0; n < 27; ++n)
+                nbg[n * a.pitch + G] = (unsigned)(H[n] - q.G0) < (unsigned)q.ng ? H[n] : (int)a.pitch - 1;
+            const float* b = at_cloud(a.v.b, q.k) + 1 + 8 * (size_t)G;
+            float2* rp = at_cloud(a.rp, q.k) + G;
+            float* xs = at_cloud(a.xs, q.k) + G;
+            FF acc = ff_zero();
+            float bi[8];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) bi[s] = b[s];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                rp[s * a.pitch] = make_float2(bi[s], 0.0f);
+                xs[s * a.pitch] = 0.0f;
+                acc = ff_add(acc, ff_prod(bi[s], bi[s]));
             }
-            __syncwarp();
-            if (mine) {
-                FF y = ff_zero();
+            return acc;
+        });
+    if (ok) sums([](const CgGridUnit&) { return false; }, [&](CgGridUnit& q, const CgSum& t) { cgc_start(q, a, t); q.check = 0; });
+    auto idle = [](const CgGridUnit& q) { return !q.go && !q.check; };
+    // a round per iteration and per true residual; two counts per round tell when none had work
+    const long long most = 2LL * a.max_iter + kCgMaxRefine + 8;
+    unsigned worked = (unsigned)(seen >> 32);
+    long long round = 0;
+    for (; ok && round < most; ++round) {
+        bool active = false;
+        for (int u = u0; u < u1; ++u) active |= !idle(U[u]);
+        // (A) A p_k from the neighbours' (r_k, p_{k-1}), p.Ap; or the true residual b - A x
+        ok = step(active, idle, [&](CgGridUnit& q, int g) {
+            const int G = q.G0 + g;
+            const int* nbg = at_cloud(a.nbg, q.k) + G;
+            float* ap = at_cloud(a.ap, q.k) + G;
+            FF acc = ff_zero();
+            if (q.check) {
+                const float* xs = at_cloud(a.xs, q.k);
+                const float* b = at_cloud(a.v.b, q.k) + 1 + 8 * (size_t)G;
+                FF y[8];
 #pragma unroll
-                for (int k = 0; k < 27; ++k) y = ff_add(y, ff_prod(s_st[k], myblk[spos + cg_kpos(k)]));
-                const float ri = ff_to_float(ff_add(FF{u.v.b[u.row0 + l], 0.0f}, FF{-y.hi, -y.lo}));
-                stage[u.row0 + l] = ri;
+                for (int s = 0; s < 8; ++s) y[s] = ff_zero();
+#pragma unroll 1
+                for (int z = 0; z < 16; ++z) {   // the z-lines of the block
+                    const int bx = z >> 2, by = z & 3;
+                    const int nxy = 9 * ((bx + 1) >> 1) + 3 * ((by + 1) >> 1);
+                    const int sxy = 4 * ((bx + 1) & 1) + 2 * ((by + 1) & 1);
+                    float xv[4];
+#pragma unroll
+                    for (int bz = 0; bz < 4; ++bz)
+                        xv[bz] = xs[(unsigned)(sxy + ((bz + 1) & 1)) * a.pitch +
+                                    (unsigned)nbg[(unsigned)(nxy + cg_pos_axis(bz)) * a.pitch]];
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const int ox = bx - (r >> 1), oy = by - (r & 1);
+                        if (ox < 0 || ox > 2 || oy < 0 || oy > 2) continue;
+                        const int axes = (ox != 1) + (oy != 1);
+#pragma unroll
+                        for (int sz = 0; sz < 2; ++sz)
+#pragma unroll
+                            for (int oz = 0; oz < 3; ++oz) {
+                                FF& t = y[2 * r + sz];
+                                t = ff_add(t, ff_prod(q.w[axes + (oz != 1)], xv[sz + oz]));
+                            }
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const float ri = ff_to_float(ff_add(FF{b[s], 0.0f}, FF{-y[s].hi, -y[s].lo}));
+                    ap[s * a.pitch] = ri;
+                    acc = ff_add(acc, ff_prod(ri, ri));
+                }
+                return acc;
+            }
+            const float beta = q.beta;
+            const float w[4] = {q.w[0], q.w[1], q.w[2], q.w[3]};
+            const float2* rp = at_cloud(a.rp, q.k);
+            // the table past L1 (read once a round), so that L1 keeps the pairs
+            unsigned nb[27];
+#pragma unroll
+            for (int n = 0; n < 27; ++n) nb[n] = (unsigned)__ldcg(nbg + (unsigned)n * a.pitch);
+            float y[8], pi[8];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) y[s] = 0.0f;
+#pragma unroll
+            for (int bx = 0; bx < 4; ++bx) {   // a plane's 16 positions are loaded together
+                float2 e[16];
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    e[q] = rp[(unsigned)cg_pos_sib(16 * bx + q) * a.pitch + nb[cg_pos_group(16 * bx + q)]];
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    const int p = 16 * bx + q;
+                    const float v = fmaf(beta, e[q].y, e[q].x);
+                    if (cg_pos_group(p) == 13) pi[cg_pos_sib(p)] = v;   // the group itself, as its table says
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        const int ox = (p >> 4) - (s >> 2), oy = ((p >> 2) & 3) - ((s >> 1) & 1), oz = (p & 3) - (s & 1);
+                        if (ox >= 0 && ox < 3 && oy >= 0 && oy < 3 && oz >= 0 && oz < 3)
+                            y[s] = fmaf(w[cg_class(9 * ox + 3 * oy + oz)], v, y[s]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                ap[s * a.pitch] = y[s];
+                acc = ff_add(acc, ff_prod(pi[s], y[s]));
+            }
+            // Only a unit's first group can have a table that does not name the group itself (its
+            // parent is recorded as the first node of the level above): its p is what the table says
+            if (g == 0 && nb[13] != (unsigned)G) {
+#pragma unroll
+                for (int s = 0; s < 8; ++s) q.own[s] = pi[s];
+            }
+            return acc;
+        });
+        if (!ok) break;
+        sums(idle, [&](CgGridUnit& q, const CgSum& t) {
+            q.resid = q.check;
+            if (q.check) {
+                cgc_after_true(q, a, t, q.it + 1);
+                q.check = 0;
+            } else {
+                cgc_alpha(q, t);
+            }
+        });
+        // (B) x and r, r.r; after a true residual: the restart's r
+        auto rest = [](const CgGridUnit& q) { return !q.go && !q.resid; };
+        ok = step(active, rest, [&](CgGridUnit& q, int g) {
+            const int G = q.G0 + g;
+            float2* rp = at_cloud(a.rp, q.k) + G;
+            const float* ap = at_cloud(a.ap, q.k) + G;
+            FF acc = ff_zero();
+            if (q.resid) {
+                if (q.replace)
+#pragma unroll
+                    for (int s = 0; s < 8; ++s) rp[s * a.pitch].x = ap[s * a.pitch];
+                return acc;
+            }
+            float* xs = at_cloud(a.xs, q.k) + G;
+            const float alpha = q.alpha, beta = q.beta;
+            const bool self = g != 0 || at_cloud(a.nbg, q.k)[13 * a.pitch + G] == G;
+            float2 own[8];
+            float xo[8], y[8];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {   // every load before the first store
+                own[s] = rp[s * a.pitch];
+                xo[s] = xs[s * a.pitch];
+                y[s] = ap[s * a.pitch];
+            }
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                const float pi = self ? fmaf(beta, own[s].y, own[s].x) : q.own[s];
+                xs[s * a.pitch] = fmaf(alpha, pi, xo[s]);
+                const float ri = fmaf(-alpha, y[s], own[s].x);
+                rp[s * a.pitch] = make_float2(ri, pi);
                 acc = ff_add(acc, ff_prod(ri, ri));
             }
-            __syncwarp();
-        }
-        double w = 0.0;
-        if (loop_reduce(acc, u, w) && threadIdx.x == 0) {
-            cg_after_true(*u.st, a, w, next);
-            u.st->check = 0;
-            u.st->t1 = global_ns();
-        }
-    }
-}
-
-// p_k = r + beta p_{k-1}, A p_k, p.Ap.  Iteration it = st->it + 1 takes p_{k-1} from pa when
-// it is odd, from pb when it is even, and writes p_k to the other buffer.  After a
-// refinement restart (beta = 0) r is the true residual staged in that other buffer: each row
-// takes it into r, and p_k = fma(0, p_{k-1}, r) is that residual itself, so the rows that
-// overwrite the staged values with their p_k write the values already there.
-__global__ void __launch_bounds__(kLoopBlock) k_cgl_spmv(CgLoopArgs a) {
-    const CgLoopControl* ctl = reinterpret_cast<const CgLoopControl*>(a.ctl);
-    __shared__ float s_st[27];
-    __shared__ float sblk[kLoopWarps * kCgWarpBlockFloats];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gi = lane >> 3, sib = lane & 7;
-    const int spos = cg_spos(sib);
-    float* myblk = sblk + warp * kCgWarpBlockFloats + gi * 80 + ((0x1a081200 >> (gi * 8)) & 0xff);
-    const int nv = (int)ctl->vstart[ctl->count];
-    for (int vb = blockIdx.x; vb < nv; vb += gridDim.x) {
-        const LoopUnit u = loop_unit(a, ctl, vb);
-        if (!u.st->go) continue;   // uniform over the block
-        const int it = u.st->it + 1;
-        const float beta = u.st->beta;
-        const bool restart = u.st->replace != 0;
-        const float* pprev = (it & 1) ? u.v.pa : u.v.pb;
-        float* pcur = (it & 1) ? u.v.pb : u.v.pa;
-        const float* rsrc = restart ? pcur : u.v.r;
-        if (threadIdx.x < 27) s_st[threadIdx.x] = u.v.stencil[u.d * 27 + threadIdx.x];
+            return acc;
+        });
+        if (!ok) break;
+        sums([](const CgGridUnit& q) { return !q.go || q.resid; }, [&](CgGridUnit& q, const CgSum& t) {
+            ++q.it;
+            cgc_after_rr(q, a, t, q.it);
+        });
+        for (int u = u0 + tid; u < u1; u += kGridBlock) U[u].resid = 0;
         __syncthreads();
-        const int nslot = (u.m + 31) >> 5;
-        FF acc = ff_zero();
-        for (int sl = u.bx * kLoopWarps + warp; sl < nslot; sl += u.split * kLoopWarps) {
-            const int l = sl * 32 + lane;
-            const bool mine = l < u.m;
-            if (mine) {
-                const int4* bp = loop_blk(u, l, sib);
-                const int4 q0 = bp[0], q1 = bp[1];
-                const int ids[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-                float vals[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) vals[e] = ids[e] >= 0 ? fmaf(beta, pprev[ids[e]], rsrc[ids[e]]) : 0.0f;
-#pragma unroll
-                for (int e = 0; e < 8; ++e) myblk[e * 8 + sib] = vals[e];
-            }
-            __syncwarp();
-            if (mine) {
-                float y = 0.0f;
-#pragma unroll
-                for (int k = 0; k < 27; ++k) y = fmaf(s_st[k], myblk[spos + cg_kpos(k)], y);
-                const float pi = myblk[spos + cg_kpos(13)];   // the row itself
-                if (restart) u.v.r[u.row0 + l] = pi;
-                pcur[u.row0 + l] = pi;
-                u.v.ap[u.row0 + l] = y;
-                acc = ff_add(acc, ff_prod(pi, y));
-            }
-            __syncwarp();
-        }
-        double w = 0.0;
-        if (loop_reduce(acc, u, w) && threadIdx.x == 0) {
-            u.st->pap = w;
-            u.st->alpha = cg_quot(u.st->rr, w);
-            u.st->replace = 0;
-        }
+        const unsigned w = (unsigned)(seen >> 32);
+        if (w == worked) break;   // no block had work in this round
+        worked = w;
     }
-}
-
-// x = x + alpha p, r = r - alpha A p, r.r and the decisions after it
-__global__ void __launch_bounds__(kLoopBlock) k_cgl_update(CgLoopArgs a) {
-    const CgLoopControl* ctl = reinterpret_cast<const CgLoopControl*>(a.ctl);
-    const int nv = (int)ctl->vstart[ctl->count];
-    for (int vb = blockIdx.x; vb < nv; vb += gridDim.x) {
-        const LoopUnit u = loop_unit(a, ctl, vb);
-        if (!u.st->go) continue;   // uniform over the block
-        const int it = u.st->it + 1;
-        const float alpha = u.st->alpha;
-        const float* pcur = (it & 1) ? u.v.pb : u.v.pa;
-        FF acc = ff_zero();
-        for (int i = u.bx * kLoopBlock + threadIdx.x; i < u.m; i += u.split * kLoopBlock) {
-            const int row = u.row0 + i;
-            u.v.x[row] = fmaf(alpha, pcur[row], u.v.x[row]);
-            const float ri = fmaf(-alpha, u.v.ap[row], u.v.r[row]);
-            u.v.r[row] = ri;
-            acc = ff_add(acc, ff_prod(ri, ri));
-        }
-        double w = 0.0;
-        if (loop_reduce(acc, u, w) && threadIdx.x == 0) {
-            cg_after_rr(*u.st, a, w, it);
-            u.st->it = it;
-            u.st->t1 = global_ns();
-            u.v.cw->cg_iters[u.d] = it;
-        }
+    if (tid == 0 && (!ok || round >= most)) atomicOr(err, kErrSpinTimeout);
+    // x in row order; the reports by the block that holds a unit's first virtual block
+    for (int p = 0; p < npass; ++p) {
+        const int vb = v0 + p * kGridSubs + sub;
+        if (vb >= v1) continue;
+        const CgGridUnit& q = U[unit_of(vb)];
+        const int g0 = (vb - q.vb0) * kVbGroups, n = 8 * min(kVbGroups, q.ng - g0);
+        const float* xs = at_cloud(a.xs, q.k) + q.G0 + g0;
+        float* x = at_cloud(a.v.x, q.k) + 1 + 8 * (size_t)(q.G0 + g0);
+        for (int l = subt; l < n; l += kVbGroups) x[l] = xs[(unsigned)(l & 7) * a.pitch + (unsigned)(l >> 3)];
     }
-}
-
-// One thread, last in the body: lists the units with an iteration or a true residual
-// pending for the next pass and continues the loop while there is one.  Whatever the states
-// say, it stops after max_iter + kCgMaxRefine + 2 passes (each depth iterates at most
-// max_iter times, at least once per pass while it goes on, and its checks ride on those
-// passes plus one after the last iteration) and then marks every cloud's counters as timed
-// out.
-__global__ void k_cgl_control(CgLoopArgs a, cudaGraphConditionalHandle cond) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    CgLoopControl* ctl = reinterpret_cast<CgLoopControl*>(a.ctl);
-    const unsigned n0 = ctl->count;
-    unsigned n = 0;
-    for (unsigned i = 0; i < n0; ++i) {   // in place: entry n <= i is written after i is read
-        const unsigned e = ctl->list[i];
-        const unsigned sp = ctl->vstart[i + 1] - ctl->vstart[i];
-        const CgLoopState& q = at_cloud(a.st, (int)(e >> 8))[a.first - (int)(e & 255u)];
-        if (q.go || q.check) {
-            ctl->list[n] = e;
-            ctl->vstart[n + 1] = ctl->vstart[n] + sp;
-            ++n;
+    for (int u = u0 + tid; u < u1; u += kGridBlock) {
+        const CgGridUnit& q = U[u];
+        if (q.vb0 < v0) continue;
+        Counters* c = at_cloud(a.v.cw, q.k);
+        if (q.it > 0) {
+            c->cg_iters[q.d] = q.it;
+            c->cg_rr[q.d] = cgs_double(q.rr);
+            c->cg_rr_true[q.d] = q.rr_true;
+            c->cg_checks[q.d] = q.checks;
+            c->cg_restarts[q.d] = q.restarts;
         }
+        c->cg_depth_ns[q.d] = global_ns() - t0;
     }
-    const unsigned passes = ++ctl->passes;
-    if (n > 0 && passes > (unsigned)a.max_iter + kCgMaxRefine + 2u) {
-        n = 0;
-        ctl->vstart[0] = 0u;
-        for (int k = 0; k < a.clouds; ++k) atomicOr(&at_cloud(a.v.cw, k)->error, kErrSpinTimeout);
-    }
-    ctl->count = n;
-    cudaGraphSetConditional(cond, n > 0 ? 1u : 0u);
-}
-
-// after the loop: the per-depth results the cluster solver reports (one thread per unit)
-__global__ void k_cgl_finish(CgLoopArgs a) {
-    if (threadIdx.x != 0) return;
-    const int k = (int)blockIdx.y, d = a.first - (int)blockIdx.z;
-    const CgLoopState& q = at_cloud(a.st, k)[d];
-    if (!q.active) return;
-    CgcVec v = a.v;
-    v.cw = at_cloud(a.v.cw, k);
-    if (q.it > 0) cg_report(v, d, q);
-    v.cw->cg_depth_ns[d] = q.t1 - q.t0;
 }
 
 // ---- implicit function at the sample points and the iso-value ----------------------
@@ -1426,7 +1399,9 @@ void prepare_launch_configs(Workspace& ws) {
     if (g_cg_cluster == 0) {
         int size = 8;
         if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgSmemBytes) !=
-            cudaSuccess)
+                cudaSuccess ||
+            cudaFuncSetAttribute(k_cg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(CgGridUnit) * kMaxBatchClouds * (kMaxDepth - kGridDepth + 1))) != cudaSuccess)
             return;   // left unset: the CG launch reports the error
         if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cudaLaunchConfig_t cfg = {};
@@ -1468,56 +1443,41 @@ static cudaError_t launch_cg(void (*kernel)(CgcArgs), CgcArgs& a, int grid, int 
     return cudaLaunchKernelExC(&cfg, (const void*)kernel, args);
 }
 
-// The device loop of the depths in L.loop_mask (units first .. first - units + 1), issued
-// on ws.aux4 while that stream is being captured: the initialisation kernel, then a while
-// node added to the captured graph, whose body is captured on ws.loop_body, then the report
-// kernel.  The body runs once even when no depth needs it (the control kernel then ends
-// the loop), so one graph serves every cloud size.
-static cudaError_t launch_cg_loop(Workspace& ws, CgLoopArgs& L) {
-    // the launches' blocks (8 resident blocks of 256 threads per SM) take the listed units'
-    // virtual blocks in turn
-    const int grid = 8 * ws.num_sms;
-    cudaStream_t s = ws.aux4;
-    k_cgl_plan<<<1, 32, 0, s>>>(L);
-    k_cgl_init<<<grid, kLoopBlock, 0, s>>>(L);
-    cudaError_t e = cudaGetLastError();
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaGraph_t graph = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    if (e == cudaSuccess) e = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, nullptr, &ndeps);
-    if (e == cudaSuccess && cs != cudaStreamCaptureStatusActive) e = cudaErrorStreamCaptureUnsupported;
-    if (e != cudaSuccess) return e;
-    std::vector<cudaGraphNode_t> dep(deps, deps + ndeps);
-    cudaGraphConditionalHandle cond = 0;
-    e = cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault);
-    if (e != cudaSuccess) return e;
-    cudaGraphNodeParams np = {};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = cond;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t loop = nullptr;
-    e = cudaGraphAddNode(&loop, graph, dep.data(), nullptr, dep.size(), &np);
-    if (e != cudaSuccess) return e;
-    cudaGraph_t body = np.conditional.phGraph_out[0];
-    cudaStream_t b = ws.loop_body;
-    e = cudaStreamBeginCaptureToGraph(b, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return e;
-    for (int rep = 0; rep < kLoopUnroll; ++rep) {   // a depth that is done skips the rest of the pass
-        k_cgl_true<<<grid, kLoopBlock, 0, b>>>(L);
-        k_cgl_spmv<<<grid, kLoopBlock, 0, b>>>(L);
-        k_cgl_update<<<grid, kLoopBlock, 0, b>>>(L);
-    }
-    k_cgl_control<<<1, 32, 0, b>>>(L, cond);
-    cudaError_t el = cudaGetLastError();
-    cudaGraph_t captured = nullptr;
-    e = cudaStreamEndCapture(b, &captured);
-    if (e == cudaSuccess) e = el;
-    if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(s, &loop, nullptr, 1, cudaStreamSetCaptureDependencies);
-    if (e != cudaSuccess) return e;
-    k_cgl_finish<<<dim3(1, ws.batch, L.units), 32, 0, s>>>(L);
-    return cudaGetLastError();
+// The whole-GPU solver of the depths from kGridDepth on: one block per SM except the SMs that the
+// coarser depths' CTAs take (a block and a CTA of theirs each need an SM's registers).
+static cudaError_t launch_cg_grid(Workspace& ws, const CgcArgs& a, cudaStream_t s) {
+    CgGridArgs L;
+    L.v = a.v;
+    L.depth = a.depth;
+    L.first = a.depth;
+    L.last = kGridDepth;
+    L.clouds = ws.batch;
+    L.stride = a.stride;
+    L.pitch = (unsigned)a.dstride;
+    L.nbg = ws.cg_nbg;
+    L.rp = ws.cg_rp;
+    L.xs = ws.cg_q;
+    L.ap = ws.cg_ap;
+    L.part = reinterpret_cast<CgSum*>(ws.cg_part);
+    L.part_cap = ws.cg_part_cap;
+    L.bar = &ws.cnt->grid_bar;
+    L.tol2 = a.tol2;
+    L.max_iter = a.max_iter;
+    L.res_period = a.res_period;
+    void* args[] = {&L};
+    cudaLaunchConfig_t cfg = {};
+    int grid = ws.num_sms - kGridDepth;
+    if (grid < 1) grid = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kGridBlock);
+    cfg.dynamicSmemBytes = sizeof(CgGridUnit) * (size_t)(L.first - L.last + 1) * L.clouds;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, (const void*)k_cg_grid, args);
 }
 
 cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, int cg_max_iter, int res_period) {
@@ -1531,7 +1491,6 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     a.v.neigh = ws.neigh;
     a.v.parent = ws.parent;
     a.v.first_child = ws.first_child;
-    a.v.blk = ws.cg_blk;
     a.v.desc = ws.cg_desc;
     a.dstride = (size_t)ws.cap.nodes / 8 + 8;
     a.stride = (size_t)ws.cap.nodes;
@@ -1548,30 +1507,33 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     a.max_iter = (cg_mode == 1 && cg_iters > 0) ? cg_iters : cg_max_iter;
     a.res_period = res_period;
     cudaError_t e = cudaSuccess;
-    // The finest depths (D, D-1, and D-2 from depth 5 on; never the root) on clusters: depth
-    // D on the widest cluster, D-1 and D-2 (fewer rows, done well before depth D) on clusters
-    // of at most 8 CTAs, on a third stream, so that they hold fewer SMs; the rest one CTA
-    // each, on the second stream.  All three run concurrently.
-    const int ncl = D < 2 ? D : (D >= 5 ? 3 : 2);
-    const int ncta = D - ncl + 1;
+    // Trees up to depth 7: the finest depths (D, D-1, and D-2 from depth 5 on; never the root) on
+    // clusters -- depth D on the widest cluster, D-1 and D-2 (fewer rows, done well before depth D)
+    // on clusters of at most 8 CTAs, on a third stream, so that they hold fewer SMs -- and the rest
+    // one CTA each, on the second stream.  Trees of depth 8 and 9, whose finest depths have hundreds
+    // of thousands of rows: depths 5 .. D on the whole GPU in one launch (208k + 53k + 14k + 4k rows:
+    // 0.61 ms against 0.81 ms with a 16-CTA cluster for the finest), the rest one CTA each.
+    const bool whole = D >= 8;
+    const int ncl = whole ? 0 : (D < 2 ? D : (D >= 5 ? 3 : 2));
+    const int ncta = whole ? kGridDepth : D - ncl + 1;
     int cl1 = ws.cg_ctas > 0 ? ws.cg_ctas : g_cg_cluster;
     if (cl1 > g_cg_cluster) cl1 = g_cg_cluster;
     int cl2 = ws.cg_ctas_fine > 0 ? ws.cg_ctas_fine : 8;
     if (cl2 > g_cg_cluster) cl2 = g_cg_cluster;
-    // Depths 5 .. D may outgrow their cluster's shared memory (depths up to 4 have at most
-    // 4,096 rows).  For trees of depth 8 and 9, whose finest depths usually do, a captured
-    // graph solves those depths by the device loop, which decides per run from the row
-    // counts.  Shallower trees, and pipelines issued directly (no graph), leave them to the
-    // global-memory path of their cluster: their depths fit the clusters up to dense clouds
-    // of millions of points, and a graph holding a while node cannot be profiled kernel by
-    // kernel (Nsight Compute profiles such a graph only as a whole).
-    const int loop_units = (ws.ev_flags == cudaEventRecordExternal && D >= 8) ? D - 4 : 0;
-    a.loop_mask = 0u;
-    for (int z = 0; z < loop_units; ++z) a.loop_mask |= 1u << (D - z);
     const size_t cstride = (size_t)ws.cap.dnodes / 8 + 64;
     const PointCoarse coarse{ws.parent, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.pv_coef, cstride};
     const int nb = ws.num_sms * 4;
-    if (ws.chain && loop_units == 0) {
+    // sample values of all levels and the iso-value, once every depth is solved
+    auto sample_values = [&]() {
+        k_point_poly<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, s>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.neigh,
+                                                                     (size_t)ws.cap.nodes, ws.parent, ws.enc, ws.xsol,
+                                                                     ws.pv_coef, cstride);
+        k_point_values<true><<<PSR_GRID(ws, nb), kBlock, 0, s>>>(ws.cnt, ws.depth, ws.px, ws.py, ws.pz, ws.point2node,
+                                                                 ws.neigh, (size_t)ws.cap.nodes, ws.enc, ws.xsol, coarse,
+                                                                 ws.point_val, ws.iso_partial);
+        return cudaGetLastError();
+    };
+    if (ws.chain && !whole) {
         // One launch for every depth: clusters of at most 8 CTAs for the two finest, a CTA each for
         // the rest in the clusters behind them.  A chain without forks takes one hardware queue,
         // so that the resident slots of a server run side by side (the driver has 8 by default:
@@ -1587,46 +1549,26 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
             e = cudaEventRecordWithFlags(ws.ev_cg, s, ws.ev_flags);
             if (e != cudaSuccess) return e;
         }
-        k_point_poly<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, s>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.neigh,
-                                                                     (size_t)ws.cap.nodes, ws.parent, ws.enc, ws.xsol,
-                                                                     ws.pv_coef, cstride);
-        k_point_values<true><<<PSR_GRID(ws, nb), kBlock, 0, s>>>(ws.cnt, ws.depth, ws.px, ws.py, ws.pz, ws.point2node,
-                                                                 ws.neigh, (size_t)ws.cap.nodes, ws.enc, ws.xsol, coarse,
-                                                                 ws.point_val, ws.iso_partial);
-        return cudaGetLastError();
+        return sample_values();
     }
     e = cudaEventRecord(ws.ev_fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ws.aux, ws.ev_fork, 0);
     if (e == cudaSuccess && ncl > 1) e = cudaStreamWaitEvent(ws.aux3, ws.ev_fork, 0);
-    if (e == cudaSuccess && loop_units > 0) {
-        e = cudaStreamWaitEvent(ws.aux4, ws.ev_fork, 0);
-        k_cg_blocks<<<PSR_GRID(ws, grid_for(ws, 1 << 20)), kBlock, 0, ws.aux4>>>(ws.cnt, ws.neigh, (size_t)ws.cap.nodes,
-                                                                                ws.cg_blk);
-        CgLoopArgs L;
-        L.v = a.v;
-        L.st = ws.cg_loop;
-        L.part = ws.cg_loop_part;
-        L.ctl = ws.cg_loop_ctl;
-        L.first = D;
-        L.units = loop_units;
-        L.clouds = ws.batch;
-        for (int d = 0; d <= kMaxDepth; ++d) L.ctas[d] = (d == D) ? cl1 : (d >= D - ncl + 1 ? cl2 : 1);
-        L.loop_mask = a.loop_mask;
-        L.tol2 = a.tol2;
-        L.max_iter = a.max_iter;
-        L.res_period = a.res_period;
-        if (e == cudaSuccess) e = launch_cg_loop(ws, L);
-        if (e == cudaSuccess) e = cudaEventRecord(ws.ev_join4, ws.aux4);
-    }
     if (e == cudaSuccess && ncta > 0) {
         CgcArgs b = a;
-        b.first = D - ncl;
+        b.first = ncta - 1;
         b.clusters = ncta;
         e = launch_cg(k_cg_cluster, b, ncta, 1, ws.batch, ws.aux);   // clusters of one CTA
     }
-    // the coarse sample values and the depth-D terms wait for every depth's solution
-    if (e == cudaSuccess && loop_units > 0) e = cudaStreamWaitEvent(ws.aux, ws.ev_join4, 0);
     if (e != cudaSuccess) return e;
+    if (whole) {
+        // every depth is needed before the sample values: both parts join first
+        e = launch_cg_grid(ws, a, s);
+        if (e == cudaSuccess && ws.ev_cg) e = cudaEventRecordWithFlags(ws.ev_cg, s, ws.ev_flags);
+        if (e == cudaSuccess) e = cudaEventRecord(ws.ev_join, ws.aux);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ws.ev_join, 0);
+        return e == cudaSuccess ? sample_values() : e;
+    }
     if (ncl > 1) {
         CgcArgs b = a;
         b.first = D - 1;

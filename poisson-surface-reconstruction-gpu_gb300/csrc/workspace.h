@@ -103,12 +103,12 @@ struct Workspace {
     float* xsol;            // M
     cudaEvent_t ev_cg = nullptr;   // recorded right after the CG kernel (stage timing)
     unsigned ev_flags = 0;         // flags of the stage-timing event records (external in a capture)
-    float *cg_r, *cg_p, *cg_q, *cg_ap;   // residual, two direction buffers, A p
-    int* cg_blk;            // CG block table: 64 same-depth nodes per sibling group
+    float *cg_r, *cg_p, *cg_q, *cg_ap;   // residual, two direction buffers, A p (whole-GPU CG: x in cg_q)
+    int* cg_nbg;            // [27][cap.nodes / 8 + 8]: neighbour groups of every sibling group (whole-GPU CG)
+    float2* cg_rp;          // [8][cap.nodes / 8 + 8]: (r, p), sibling-major
+    longlong2* cg_part;     // [2][cg_part_cap]: sums of its virtual blocks
+    int cg_part_cap;
     unsigned* cg_desc;      // [14][cap.nodes / 8 + 8]: packed neighbour groups (solver.cu)
-    CgLoopState* cg_loop;   // [D+1]: device-loop CG state per depth
-    double* cg_loop_part;   // [D+1][kLoopMaxBlocks]: its per-block partial sums
-    unsigned* cg_loop_ctl;  // loop control of a launch (passes, listed units; cloud 0's copy)
     double* cg_partial;     // scratch: divergence chunk sums (float pairs, 8 bytes each)
     float* point_val;       // N
     float* pv_coef;         // [27][cap.dnodes / 8 + 64]: per depth-(D-1) node, Bernstein coefficients
@@ -184,9 +184,6 @@ struct Workspace {
     cudaEvent_t ev_geo = nullptr;       // the mesh records' scans (and the divergence chunks') are done
     cudaStream_t aux3 = nullptr;        // fourth stream: the CG of depths D-1 and D-2
     cudaEvent_t ev_join3 = nullptr;
-    cudaStream_t aux4 = nullptr;        // fifth stream: the device-loop CG of large depths
-    cudaEvent_t ev_join4 = nullptr;
-    cudaStream_t loop_body = nullptr;   // captures the body graph of the device loop
     int num_sms;
 };
 
