@@ -339,7 +339,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.stencil, (size_t)(kMaxDepth + 1) * 27);
     A.add(ws.vfield, 3 * (size_t)dnodes);
     A.add(ws.divg, (size_t)nodes);
-    A.add(ws.xsol, (size_t)nodes);
+    A.add(ws.xsol, (size_t)nodes + 64);   // from entry 64 on: x[-1] = 0 stands for absent neighbours
     const size_t pitch = (size_t)nodes / 8 + 8;   // sibling groups, and a zero group at the end
     A.add(ws.cg_r, (size_t)nodes); A.add(ws.cg_p, (size_t)nodes); A.add(ws.cg_q, 8 * pitch);
     A.add(ws.cg_ap, 8 * pitch);
@@ -436,6 +436,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     }
     h->arena_bytes = A.bytes;
     A.assign((char*)h->arena);
+    ws.xsol += 64;
     set_batch(ws, 1);
     ws.cg_ctas = cfg.cg_cluster_ctas;
     ws.cg_ctas_fine = cfg.cg_cluster_ctas_fine;

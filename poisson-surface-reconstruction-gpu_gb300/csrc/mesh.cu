@@ -377,11 +377,6 @@ __global__ void __launch_bounds__(kBlock) k_mesh_maintain(Counters* c, int depth
 // ------------------------------------------------------------------------------------
 // implicit values at the octree vertices (mesh/ComputeTriangleIndices.cu:346-399)
 // ------------------------------------------------------------------------------------
-__device__ __forceinline__ float node_terms(int node, float val, float qx, float qy, float qz, int depth,
-                                            const int* neigh, size_t stride, const int* enc, const float* x) {
-    return level_terms(node, val, qx, qy, qz, depth, neigh, stride, enc, x);
-}
-
 __global__ void __launch_bounds__(kBlock) k_vertex_values(const Counters* c, int depth, const float* vx,
                                                           const float* vy, const float* vz, const int* vowner,
                                                           const int* vkind, const int* vdepth, const int* neigh,
@@ -410,7 +405,7 @@ __global__ void __launch_bounds__(kBlock) k_vertex_values(const Counters* c, int
             while (true) {
                 float xv[27];
 #pragma unroll
-                for (int k = 0; k < 27; ++k) xv[k] = x[nbs[k] >= 0 ? nbs[k] : 0];
+                for (int k = 0; k < 27; ++k) xv[k] = x[nbs[k]];
                 int nx;
                 if (up && par != -1) {
                     nx = par;
@@ -428,7 +423,7 @@ __global__ void __launch_bounds__(kBlock) k_vertex_values(const Counters* c, int
                 e2 = enc[n0];
                 par2 = parent[n0];
                 fc2 = first_child[n0];
-                val = terms_from(e, nbs, xv, val, qx, qy, qz, depth);
+                val = terms_from(e, xv, val, qx, qy, qz, depth);
                 if (nx == -1) break;
 #pragma unroll
                 for (int k = 0; k < 27; ++k) nbs[k] = nb2[k];
@@ -944,8 +939,13 @@ __device__ __forceinline__ unsigned child_touch(unsigned pt, int ch) {
 // its neighbours and its sign test; returns 1 when it stays live.
 // kShared: several depths in one launch, so what an earlier depth wrote may not be read through the
 // read-only path.
-template <bool kShared>
+// kBlocks: blocks per SM its registers leave room for.  Alone on an SM a block keeps every look-up
+// of a candidate in registers (255 of them), the shorter chain for the few thousand candidates of a
+// depth-7 tree; the hundreds of thousands of depth 8 and 9 want two (128 registers, 2M points: the
+// level scans 1.69 -> 1.25 ms; depth 7: 6 us slower).
+template <bool kShared, int kBlocks>
 struct SubLevelLoad {
+    static constexpr int kMinBlocks = kBlocks;
     const Counters* c;
     int d, depth, na;
     const int* groups;
@@ -1256,7 +1256,7 @@ struct SubLevelStore {
 
 // The depths 1 .. dmax (at most 8 + 64 + 512 candidates) in one CTA: the scans of so few elements
 // cost a launch each otherwise.
-__global__ void __launch_bounds__(kBlock) k_sub_coarse(SubLevelLoad<true> load, SubLevelStore store, int dmax) {
+__global__ void __launch_bounds__(kBlock) k_sub_coarse(SubLevelLoad<true, 1> load, SubLevelStore store, int dmax) {
     PSR_CLOUD(load, store);
     __shared__ unsigned s_warp[kBlock / 32 + 1];
     for (int d = 1; d <= dmax; ++d) {
@@ -1277,9 +1277,22 @@ __global__ void __launch_bounds__(kBlock) k_sub_coarse(SubLevelLoad<true> load, 
     }
 }
 
-// index of virtual node v among the live depth-D cells (sorted), or -1
-__device__ __forceinline__ int live_index(const int* lv_vnode, int n, int v) {
-    int lo = 0, hi = n;
+// index of virtual node v among the live depth-D cells (sorted), or -1; the search gallops from
+// cell L outwards, since a neighbour's number is near its own
+__device__ __forceinline__ int live_index(const int* lv_vnode, int n, int v, int L) {
+    const int at = lv_vnode[L];
+    int lo, hi;   // the place is in [lo, hi)
+    int step = 1;
+    if (v < at) {
+        hi = L;
+        while (hi - step >= 0 && lv_vnode[hi - step] >= v) { hi -= step; step <<= 1; }
+        lo = hi - step < 0 ? 0 : hi - step;
+        ++hi;
+    } else {
+        lo = L;
+        while (lo + step < n && lv_vnode[lo + step] <= v) { lo += step; step <<= 1; }
+        hi = lo + step > n ? n : lo + step;
+    }
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
         if (lv_vnode[mid] < v) lo = mid + 1;
@@ -1299,7 +1312,7 @@ __global__ void __launch_bounds__(kBlock) k_sub_live_neigh(const Counters* c, in
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         const int L = (int)(t / 27), k = (int)(t - 27LL * L);
         const int v = A.neigh[(size_t)k * A.cstride + A.live[lb + L]];
-        lv_nb[(size_t)k * dstride + L] = (k == 13) ? L : ((v >= na) ? live_index(A.lv_vnode, nl, v - na) : -1);
+        lv_nb[(size_t)k * dstride + L] = (k == 13) ? L : ((v >= na) ? live_index(A.lv_vnode, nl, v - na, L) : -1);
         if (k == 13) {   // a group's live cells are consecutive
             const int g = A.group[A.live[lb + L]];
             if (L == 0 || A.group[A.live[lb + L - 1]] != g) group_live[g] = L;
@@ -1522,6 +1535,71 @@ __global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* 
             vvalue[v] = __fsub_rn(val, iso);
         }
         __syncwarp(gmask);
+    }
+}
+
+// The same values, one thread per vertex: from depth 8 on there are hundreds of thousands of
+// vertices, whose own parallelism hides the chains' loads, and the eight-lane form leaves seven
+// lanes idle while the first adds the terms one by one (1.24 ms of 2M points, depth 9, against
+// 0.5 ms).  Software-pipelined like k_vertex_values: the next level's neighbour row is read while
+// the current one's values are in flight.
+__global__ void __launch_bounds__(kBlock) k_sub_vertex_values_wide(const Counters* c, int depth, const float* vx,
+                                                                   const float* vy, const float* vz, const int* vowner,
+                                                                   const int* neigh, size_t stride, const int* parent,
+                                                                   const int* groups, const int* root_self, SubArrays A,
+                                                                   const int* enc, const float* x, float* vvalue, int na) {
+    PSR_CLOUD(c, vx, vy, vz, vowner, neigh, parent, groups, root_self, A, enc, x, vvalue);
+    const int V = c->n_sub_vertices;
+    const float iso = c->iso;
+    const int lb = c->sub_lbase[depth];
+    PSR_GRID_STRIDE(v, V) {
+        const float qx = vx[v], qy = vy[v], qz = vz[v];
+        const int own = A.live[lb + vowner[v]];
+        const int* G = groups + (size_t)A.group[own] * kGroupRec;
+        // levels: subdivision nodes through the jump links, then the octree ancestors
+        int node = A.jump[own];
+        bool sub = true;
+        int nbs[27];
+#pragma unroll
+        for (int k = 0; k < 27; ++k) nbs[k] = A.neigh[(size_t)k * A.cstride + node];
+        float val = 0.0f;
+        for (int level = 0; level <= kMaxDepth; ++level) {
+            int ox, oy, oz, d, next;
+            bool next_sub = false;
+            if (sub) {
+#pragma unroll
+                for (int k = 0; k < 27; ++k)
+                    if (nbs[k] >= na) nbs[k] = sub_value_node(nbs[k], na, G, root_self);
+                d = A.depth[node];
+                const float sc = (float)(1 << d);
+                const int base = (1 << d) - 1;
+                ox = base + (int)__fmul_rn(A.cx[node], sc);
+                oy = base + (int)__fmul_rn(A.cy[node], sc);
+                oz = base + (int)__fmul_rn(A.cz[node], sc);
+                const int p = A.parent[node];
+                next_sub = p >= 0;
+                next = next_sub ? A.jump[p] : -2 - p;
+            } else {
+                decode_fn_index(enc[node], depth, ox, oy, oz);
+                d = ilog2_dev(ox + 1);
+                next = parent[node];
+            }
+            float xv[27];
+#pragma unroll
+            for (int k = 0; k < 27; ++k) xv[k] = x[nbs[k]];
+            int nb2[27];
+            const int* row = next_sub ? A.neigh + next : neigh + (next >= 0 ? next : 0);
+            const size_t rstride = next_sub ? A.cstride : stride;
+#pragma unroll
+            for (int k = 0; k < 27; ++k) nb2[k] = row[(size_t)k * rstride];
+            val = terms_at(ox, oy, oz, d, xv, val, qx, qy, qz);
+            if (next < 0) break;
+#pragma unroll
+            for (int k = 0; k < 27; ++k) nbs[k] = nb2[k];
+            node = next;
+            sub = next_sub;
+        }
+        vvalue[v] = __fsub_rn(val, iso);
     }
 }
 
@@ -1891,10 +1969,14 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
         return load;
     };
     const int dcoarse = D < 3 ? D : 3;
-    k_sub_coarse<<<PSR_GRID(ws, 1), kBlock, 0, s>>>(level(SubLevelLoad<true>{}, 1), SubLevelStore{c, 1, D, A, err}, dcoarse);
+    k_sub_coarse<<<PSR_GRID(ws, 1), kBlock, 0, s>>>(level(SubLevelLoad<true, 1>{}, 1), SubLevelStore{c, 1, D, A, err}, dcoarse);
     for (int d = dcoarse + 1; d <= D; ++d) {
-        e = launch_scan<1>(level(SubLevelLoad<false>{}, d), SubLevelStore{c, d, D, A, err}, &c->sub_cand[d], 0, ws.scan,
-                           total, err, s, ScanCount{}, sbps);
+        if (D >= 8)
+            e = launch_scan<1>(level(SubLevelLoad<false, 2>{}, d), SubLevelStore{c, d, D, A, err}, &c->sub_cand[d], 0,
+                               ws.scan, total, err, s, ScanCount{}, sbps);
+        else
+            e = launch_scan<1>(level(SubLevelLoad<false, 1>{}, d), SubLevelStore{c, d, D, A, err}, &c->sub_cand[d], 0,
+                               ws.scan, total, err, s, ScanCount{}, sbps);
         if (e != cudaSuccess) return e;
     }
     // the live depth-D cells carry every record from here on, indexed by their live index
@@ -1914,9 +1996,14 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
     const dim3 g2 = PSR_GRID(ws, gl);
     k_sub_maintain<<<dim3(g2.x, g2.y, 2), kBlock, 0, s>>>(c, ws.lv_nb, dstride, ws.sv_owner, ws.sv_kind, ws.s_vtx,
                                                           ws.se_owner, ws.se_kind, ws.s_edge);
-    k_sub_vertex_values<<<PSR_GRID(ws, 16 * ws.num_sms), kSvBlock, 0, s>>>(
-        c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, mb.groups, ws.root_self, A, ws.enc,
-        ws.xsol, ws.sv_value, na);
+    if (D >= 8)
+        k_sub_vertex_values_wide<<<PSR_GRID(ws, 8 * ws.num_sms), kBlock, 0, s>>>(
+            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, mb.groups, ws.root_self, A, ws.enc,
+            ws.xsol, ws.sv_value, na);
+    else
+        k_sub_vertex_values<<<PSR_GRID(ws, 16 * ws.num_sms), kSvBlock, 0, s>>>(
+            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, mb.groups, ws.root_self, A, ws.enc,
+            ws.xsol, ws.sv_value, na);
     // crossings: staged after the main part's vertices
     e = launch_scan<2>(SubCrossLoad{ws.se_owner, ws.se_kind, ws.s_vtx, dstride, ws.sv_value, err},
                        SubCrossStore{ws.se_owner, ws.se_kind, ws.s_vtx, dstride, ws.sv_value, ws.sv_x, ws.sv_y,

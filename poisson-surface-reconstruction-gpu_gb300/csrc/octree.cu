@@ -14,14 +14,15 @@ namespace psr {
 // bounding box (mesh/BuildOctree.cu:51-133) and normalisation parameters (:619-631)
 // ------------------------------------------------------------------------------------
 // the counters of a call, and the sort's
-__global__ void k_reset_counters(Counters* c, const InputRef* in, unsigned* sort_bins) {
-    PSR_CLOUD(c, in, sort_bins);
+__global__ void k_reset_counters(Counters* c, const InputRef* in, unsigned* sort_bins, float* x) {
+    PSR_CLOUD(c, in, sort_bins, x);
     static_assert(sizeof(Counters) % 4 == 0, "Counters is cleared word by word");
     unsigned* w = (unsigned*)c;
     for (int i = threadIdx.x; i < (int)(sizeof(Counters) / 4); i += blockDim.x) w[i] = 0u;
     for (int i = threadIdx.x; i < kSortBinWords; i += blockDim.x) sort_bins[i] = 0u;
     __syncthreads();
     if (threadIdx.x == 0) {
+        x[-1] = 0.0f;   // the value of absent neighbours
         c->n_points = in->n;
         for (int a = 0; a < 3; ++a) {
             // The reference seeds its reduction (padding threads, mesh/BuildOctree.cu:66-73)
@@ -622,7 +623,7 @@ cudaError_t octree_build(Workspace& ws) {
     Counters* c = ws.cnt;
     unsigned* err = &c->error;
     unsigned* total = (unsigned*)&c->scan_total;
-    k_reset_counters<<<PSR_GRID(ws, 1), 256, 0, s>>>(c, ws.d_params, ws.sort.bins);
+    k_reset_counters<<<PSR_GRID(ws, 1), 256, 0, s>>>(c, ws.d_params, ws.sort.bins, ws.xsol);
     const unsigned *scode = nullptr, *sidx = nullptr;
     cudaError_t e = encode_sort_points(ws, D, &scode, &sidx);
     if (e != cudaSuccess) return e;

@@ -223,8 +223,14 @@ __device__ __forceinline__ void scan_body(Load load, Store store, int n, ScanScr
     }
 }
 
+// blocks per SM the registers of a scan must leave room for (heavy functors define kMinBlocks)
+template <class L>
+constexpr auto scan_min_blocks(int) -> decltype(L::kMinBlocks) { return L::kMinBlocks; }
+template <class L>
+constexpr int scan_min_blocks(long) { return 1; }
+
 template <int kItems, class Load, class Store>
-__global__ void __launch_bounds__(kBlock) k_scan(Load load, Store store, const int* count_ptr, int count_add,
+__global__ void __launch_bounds__(kBlock, scan_min_blocks<Load>(0)) k_scan(Load load, Store store, const int* count_ptr, int count_add,
                                                  ScanScratch sc, unsigned* total, unsigned* err, ScanCount cnt) {
     PSR_CLOUD(load, store, count_ptr, sc, total, err, cnt);
     scan_body<kItems>(load, store, *count_ptr + count_add, sc, total, err, cnt);

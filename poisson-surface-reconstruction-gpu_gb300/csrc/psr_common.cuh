@@ -229,42 +229,59 @@ __device__ __forceinline__ void child_neighbours(int son, Row row, First first, 
     }
 }
 
-// Terms of one level of an implicit-function chain: the 27 same-depth neighbours nb of
-// `node`, each adding ((x[nb] * Fx) * Fy) * Fz in slot order.  A neighbour's function
-// index is the node's own plus the slot offset, so the 81 basis values come from 9.
-__device__ __forceinline__ float terms_from(int encv, const int (&nbs)[27], const float (&xv)[27], float val,
-                                            float qx, float qy, float qz, int depth) {
-    int ox, oy, oz;
-    decode_fn_index(encv, depth, ox, oy, oz);
-    float bx[3], by[3], bz[3];
+// basis32 of the function indices o - 1, o, o + 1 of level d (o = 2^d - 1 + offset): the level is
+// shared, so its scale and shift are too.  The indices beyond the ends of the level, which belong
+// to no node, get the value of the formula instead of another level's.
+__device__ __forceinline__ void basis3(int o, int d, float x, float (&b)[3]) {
+    const float kF43 = 1.33333337306976318359375f;
+    const float kF23 = 0.666666686534881591796875f;
+    const float s = (float)(1 << d), inv = __int_as_float((127 - d) << 23);
+    const float f = (float)(o - (1 << d));   // offset - 1
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-        bx[j] = basis32(ox - 1 + j, qx);
-        by[j] = basis32(oy - 1 + j, qy);
-        bz[j] = basis32(oz - 1 + j, qz);
+        const float c = __fmul_rn(__fadd_rn(__fadd_rn(f, (float)j), 0.5f), inv);
+        const float t = __fmul_rn(__fsub_rn(x, c), s);
+        const float a = fabsf(t), u = __fsub_rn(1.5f, a);
+        const float in = __fmul_rn(__fsub_rn(0.75f, __fmul_rn(t, t)), kF43);
+        const float out = __fmul_rn(__fmul_rn(u, u), kF23);
+        b[j] = a < 0.5f ? in : (a < 1.5f ? out : 0.0f);
     }
+}
+
+// Terms of one level of an implicit-function chain: the 27 same-depth neighbours of a node, each
+// adding ((x[nb] * Fx) * Fy) * Fz in slot order.  A neighbour's function index is the node's own
+// plus the slot offset, so the 81 basis values come from 9.  Absent neighbours carry x = 0 (the
+// entry before the first: x[-1] = 0, so a missing neighbour needs no test) and add a zero, which
+// leaves the sum as it is.
+__device__ __forceinline__ float terms_at(int ox, int oy, int oz, int d, const float (&xv)[27], float val, float qx,
+                                          float qy, float qz) {
+    float bx[3], by[3], bz[3];
+    basis3(ox, d, qx, bx);
+    basis3(oy, d, qy, by);
+    basis3(oz, d, qz, bz);
 #pragma unroll
-    for (int k = 0; k < 27; ++k) {
-        if (nbs[k] == -1) continue;
-        float t = __fmul_rn(xv[k], bx[k / 9]);
-        t = __fmul_rn(t, by[(k / 3) % 3]);
-        t = __fmul_rn(t, bz[k % 3]);
-        val = __fadd_rn(val, t);
-    }
+    for (int k = 0; k < 27; ++k)
+        val = __fadd_rn(val, __fmul_rn(__fmul_rn(__fmul_rn(xv[k], bx[k / 9]), by[(k / 3) % 3]), bz[k % 3]));
     return val;
+}
+__device__ __forceinline__ float terms_from(int encv, const float (&xv)[27], float val, float qx, float qy, float qz,
+                                            int depth) {
+    int ox, oy, oz;
+    decode_fn_index(encv, depth, ox, oy, oz);
+    return terms_at(ox, oy, oz, ilog2_dev(ox + 1), xv, val, qx, qy, qz);
 }
 
 __device__ __forceinline__ float level_terms(int node, float val, float qx, float qy, float qz, int depth,
                                              const int* neigh, size_t stride, const int* enc, const float* x) {
     const int e = enc[node];
+    const int* row = neigh + node;
     int nbs[27];
 #pragma unroll
-    for (int k = 0; k < 27; ++k) nbs[k] = neigh[(size_t)k * stride + node];
-    // every value read at once (a missing neighbour reads entry 0 and adds nothing)
+    for (int k = 0; k < 27; ++k) nbs[k] = row[(size_t)k * stride];
     float xv[27];
 #pragma unroll
-    for (int k = 0; k < 27; ++k) xv[k] = x[nbs[k] >= 0 ? nbs[k] : 0];
-    return terms_from(e, nbs, xv, val, qx, qy, qz, depth);
+    for (int k = 0; k < 27; ++k) xv[k] = x[nbs[k]];
+    return terms_from(e, xv, val, qx, qy, qz, depth);
 }
 
 // ---- Bernstein form of the implicit function on a cell --------------------------------

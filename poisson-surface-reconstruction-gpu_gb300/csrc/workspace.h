@@ -100,7 +100,7 @@ struct Workspace {
     // field / solve
     float* vfield;          // 3 x dnodes (SoA: x block, y block, z block)
     float* divg;            // M
-    float* xsol;            // M
+    float* xsol;            // M, with xsol[-1] = 0
     cudaEvent_t ev_cg = nullptr;   // recorded right after the CG kernel (stage timing)
     unsigned ev_flags = 0;         // flags of the stage-timing event records (external in a capture)
     float *cg_r, *cg_p, *cg_q, *cg_ap;   // residual, two direction buffers, A p (whole-GPU CG: x in cg_q)
