@@ -338,6 +338,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.dff, (size_t)ws.res * ws.res);
     A.add(ws.stencil, (size_t)(kMaxDepth + 1) * 27);
     A.add(ws.vfield, 3 * (size_t)dnodes);
+    A.add(ws.leaf, (size_t)dnodes);
     A.add(ws.divg, (size_t)nodes);
     A.add(ws.xsol, (size_t)nodes + 64);   // from entry 64 on: x[-1] = 0 stands for absent neighbours
     const size_t pitch = (size_t)nodes / 8 + 8;   // sibling groups, and a zero group at the end

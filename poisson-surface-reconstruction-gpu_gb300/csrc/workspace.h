@@ -99,6 +99,7 @@ struct Workspace {
 
     // field / solve
     float* vfield;          // 3 x dnodes (SoA: x block, y block, z block)
+    float4* leaf;           // dnodes: the field and the packed function index of each depth-D node
     float* divg;            // M
     float* xsol;            // M, with xsol[-1] = 0
     cudaEvent_t ev_cg = nullptr;   // recorded right after the CG kernel (stage timing)
