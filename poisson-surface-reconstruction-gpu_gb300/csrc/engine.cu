@@ -375,15 +375,11 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     ws.cap_poly = (int)std::max<long long>(65536, nodes / 16);
     if (cfg.root_poly_capacity > 0) ws.cap_poly = cfg.root_poly_capacity;
     A.add(ws.root_poly, 28 * (size_t)ws.cap_poly);
-    A.add(ws.c_vnode, (size_t)subn); A.add(ws.c_key, (size_t)subn); A.add(ws.c_group, (size_t)subn);
-    A.add(ws.c_parent, (size_t)subn); A.add(ws.c_jump, (size_t)subn); A.add(ws.c_depth, (size_t)subn);
-    A.add(ws.c_cx, (size_t)subn); A.add(ws.c_cy, (size_t)subn); A.add(ws.c_cz, (size_t)subn);
-    A.add(ws.c_neigh, 27 * (size_t)subn);
-    A.add(ws.c_live, (size_t)subd);
+    A.add(ws.c_rec, (size_t)subd); A.add(ws.c_pos, (size_t)subd);
+    A.add(ws.c_jump, (size_t)subd); A.add(ws.c_kids, (size_t)subd);
+    A.add(ws.c_neigh, 27 * (size_t)subd);
     A.add(ws.c_poly, 28 * (size_t)subd);
-    A.add(ws.c_touch, (size_t)subd);
     A.add(ws.lv_vnode, (size_t)subd);
-    A.add(ws.lv_nb, 27 * (size_t)subd);
     A.add(ws.s_vtx, 8 * (size_t)subd); A.add(ws.s_edge, 12 * (size_t)subd);
     A.add(ws.s_vmask, (size_t)subd); A.add(ws.s_emask, (size_t)subd);
     A.add(ws.sv_x, 8 * (size_t)subd); A.add(ws.sv_y, 8 * (size_t)subd); A.add(ws.sv_z, 8 * (size_t)subd);

@@ -705,11 +705,13 @@ struct GroupSizeStore {
 // Virtual numbering (singleRebuildArray :599-635 / wholeRebuildArray :1110-1168): group g
 // owns the virtual sub nodes G[3] .. G[3] + G[4] - 1, level by level from its root depth rd
 // (its n roots) to D; node (q, rel) of level d sits at G[3] + off_d + q 8^(d-rd) + rel (rel:
-// the Morton code below root q).  Neighbour tables hold octree nodes (< na), na + virtual
-// index for sub nodes, or -1.  Only candidates are stored, in compact slots: at depth d the
-// 8 children of every live node of depth d-1, in order, then the roots of depth d.  Both
-// parts are in virtual order (groups are ordered by root depth), so the live depth-D cells,
-// which carry all records from here on, come out in the reference's order.
+// the Morton code below root q).  Only live nodes are stored, in one list, depth after depth:
+// of depth d's candidates (the 8 children of every live node of depth d-1, in order, then the
+// roots of depth d) those that stay live.  Both parts are in virtual order (groups are ordered
+// by root depth), so the live depth-D cells, which carry all records from here on, come out in
+// the reference's order.  Neighbour rows hold octree nodes (< na), na + list entry for live sub
+// nodes, or -1 (nothing there, or a sub node that is not live: it carries no value, and neither
+// it nor anything below it is referred to again).
 __device__ __forceinline__ int sub_level_off(int rd, int n, int d) {
     int off = 0, cnt = n;
     for (int e = rd; e < d; ++e) { off += cnt; cnt *= 8; }
@@ -751,16 +753,15 @@ __device__ __forceinline__ void sub_setup(Counters* c, int depth, const int* sub
 }
 
 struct SubArrays {
-    int *vnode, *key, *group, *parent, *jump, *depth;   // parent: slot, or -2 - octree parent
-    float *cx, *cy, *cz;
-    int* neigh;   // [27][cap]
-    size_t cstride;
-    int* live;    // live slots, depth after depth
-    float* poly;  // [28][cap_live]: per live entry, Bernstein coefficients of its levels, sum |y|
-    unsigned char* touch;   // per live entry: faces of its root's cell it lies on (bits x-, x+, y-, y+, z-, z+)
-    int* lv_vnode;   // virtual index of each live depth-D cell
+    int4* rec;      // per live entry: parent (entry, or -2 - octree parent), group, key, virtual index
+    float4* pos;    // centre, depth (as bits)
+    int* jump;      // nearest contributing entry on the path to the root (itself when it contributes)
+    int2* kids;     // its live children: first entry, octant bits
+    int* neigh;     // [27][cap_live]: same-depth neighbours
+    float* poly;    // [28][cap_live]: Bernstein coefficients of its levels, sum |y|
+    int* lv_vnode;  // virtual index of each live depth-D cell
     int cap_nodes, cap_live, cap_live_d;
-    __device__ void rebase() { PSR_CLOUD(vnode, key, group, parent, jump, depth, cx, cy, cz, neigh, live, poly, touch, lv_vnode); }   // to cloud blockIdx.y
+    __device__ void rebase() { PSR_CLOUD(rec, pos, jump, kids, neigh, poly, lv_vnode); }   // to cloud blockIdx.y
 };
 
 // ---- certain-sign cells -------------------------------------------------------------
@@ -784,13 +785,6 @@ struct SubArrays {
 // Float vertex values are sums of the same nonzero terms (at most 27 (D+1)), within
 // ~1.7e-5 sum |y| of the exact value; the float coefficients here are as close; the test
 // keeps a margin of 1e-4 (sum |y| + |iso|).
-
-// value carried by a sub-node neighbour (na + virtual index) of group G: its root's octree
-// node for a root (it stands for that node), else nothing (x = 0 in subdivision space)
-__device__ __forceinline__ int sub_value_node(int v, int na, const int* G, const int* root_self) {
-    const int local = v - na - G[3];
-    return ((unsigned)local < (unsigned)G[2]) ? root_self[G[1] + local] : -1;
-}
 
 // Levels up to a root's depth are the same for every cell below that root: their sum is one
 // tensor-product quadratic on the root's cell, kept as its 27 Bernstein coefficients
@@ -853,21 +847,16 @@ __device__ __forceinline__ void blossom3(float a, float b, float (&M)[3][3]) {
     M[2][0] = b1 * b1; M[2][1] = 2.0f * b * b1;     M[2][2] = b * b;
 }
 
-// C += the root polynomial P subdivided to the cell at Morton code rel (m levels below it)
-template <bool kReadOnly>
-__device__ __forceinline__ void add_subdivided(const float* P, size_t pstride, unsigned rel, int m, float (&C)[27]) {
-    int i3[3] = {0, 0, 0};
-    for (int j = 0; j < m; ++j)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) i3[a] |= (int)((rel >> (3 * j + 2 - a)) & 1u) << j;
-    const float inv = __int_as_float((127 - m) << 23);   // 2^-m
+// polynomial P (27 coefficients, pstride apart) restricted to octant ch of its cell
+__device__ __forceinline__ void sub_octant(const float* P, size_t pstride, int ch, float (&C)[27]) {
     float Mx[3][3], My[3][3], Mz[3][3];
-    blossom3((float)i3[0] * inv, (float)(i3[0] + 1) * inv, Mx);
-    blossom3((float)i3[1] * inv, (float)(i3[1] + 1) * inv, My);
-    blossom3((float)i3[2] * inv, (float)(i3[2] + 1) * inv, Mz);
+    const float ax = 0.5f * (float)((ch >> 2) & 1), ay = 0.5f * (float)((ch >> 1) & 1), az = 0.5f * (float)(ch & 1);
+    blossom3(ax, ax + 0.5f, Mx);
+    blossom3(ay, ay + 0.5f, My);
+    blossom3(az, az + 0.5f, Mz);
     float p[27];
 #pragma unroll
-    for (int k = 0; k < 27; ++k) p[k] = kReadOnly ? __ldg(P + (size_t)k * pstride) : P[(size_t)k * pstride];
+    for (int k = 0; k < 27; ++k) p[k] = P[(size_t)k * pstride];
     float T1[27], T2[27];
 #pragma unroll
     for (int a = 0; a < 3; ++a)
@@ -886,7 +875,14 @@ __device__ __forceinline__ void add_subdivided(const float* P, size_t pstride, u
     for (int ab3 = 0; ab3 < 9; ++ab3)
 #pragma unroll
         for (int gg = 0; gg < 3; ++gg)
-            C[ab3 * 3 + gg] += fmaf(Mz[gg][0], T2[ab3 * 3], fmaf(Mz[gg][1], T2[ab3 * 3 + 1], Mz[gg][2] * T2[ab3 * 3 + 2]));
+            C[ab3 * 3 + gg] = fmaf(Mz[gg][0], T2[ab3 * 3], fmaf(Mz[gg][1], T2[ab3 * 3 + 1], Mz[gg][2] * T2[ab3 * 3 + 2]));
+}
+
+// centre and depth of child ch (depth d) of the cell at `p`
+__device__ __forceinline__ float4 sub_child_pos(const float4 p, int ch, int d) {
+    const float w = __int_as_float((126 - d) << 23);   // 2^-(d+1)
+    return make_float4((ch & 4) ? __fadd_rn(p.x, w) : __fsub_rn(p.x, w), (ch & 2) ? __fadd_rn(p.y, w) : __fsub_rn(p.y, w),
+                       (ch & 1) ? __fadd_rn(p.z, w) : __fsub_rn(p.z, w), __int_as_float(d));
 }
 
 // Coefficients of a live node are kept (per live entry): a child's levels above its own are
@@ -921,37 +917,17 @@ __device__ __forceinline__ void root_coefficients(int r, int root_node, int rd, 
     }
 }
 
-// per-thread hand-over of a candidate's coefficients (28), face bits and virtual index
-// from the scan's load to its store
+// per-thread hand-over of a candidate's coefficients (28) from the scan's load to its store
 __device__ __forceinline__ float* sub_poly_stash() {
-    __shared__ float s_stash[30 * kBlock];
+    __shared__ float s_stash[28 * kBlock];
     return s_stash;
 }
 
-// faces of the root's cell that child `ch` (x = 4, y = 2, z = 1) of a cell with face bits
-// pt lies on: a face its parent lies on, on the child's side
-__device__ __forceinline__ unsigned child_touch(unsigned pt, int ch) {
-    const unsigned side = ((ch & 4) ? 2u : 1u) | ((ch & 2) ? 8u : 4u) | ((ch & 1) ? 32u : 16u);
-    return pt & side;
-}
-
-// One candidate of depth d (computeRebuildNeighbor :669-696 for its neighbours): its record,
-// its neighbours and its sign test; returns 1 when it stays live.
-// kShared: several depths in one launch, so what an earlier depth wrote may not be read through the
-// read-only path.
-// kBlocks: blocks per SM its registers leave room for.  Alone on an SM a block keeps every look-up
-// of a candidate in registers (255 of them), the shorter chain for the few thousand candidates of a
-// depth-7 tree; the hundreds of thousands of depth 8 and 9 want two (128 registers, 2M points: the
-// level scans 1.69 -> 1.25 ms; depth 7: 6 us slower).
-template <bool kShared, int kBlocks>
-struct SubLevelLoad {
-    static constexpr int kMinBlocks = kBlocks;
-    const Counters* c;
-    int d, depth, na;
+// The octree's part of the subdivision's look-ups: written by earlier launches only.
+struct SubTree {
     const int* groups;
     const int* sub_root;
     const int* root_group;
-    const int* root_self;
     const int* key;
     const int* neigh;
     size_t stride;
@@ -963,269 +939,210 @@ struct SubLevelLoad {
     const float* x;
     const float* root_poly;
     int cap_poly;
+    int na;
+    __device__ void rebase() { PSR_CLOUD(groups, sub_root, root_group, key, neigh, first_child, parent, ov_group, ov_sub, enc, x, root_poly); }   // to cloud blockIdx.y
+};
+
+// first live entry of the roots of depth d (they follow the depth's live children)
+__device__ __forceinline__ int sub_first_root(const Counters* c, int d) {
+    return c->sub_lbase[d] + c->sub_nlive[d] - c->sub_nroots[d];
+}
+
+// a root's number less this is its index among the roots of depth d
+__device__ __forceinline__ int sub_root_shift(const Counters* c, int d) { return c->sub_rstart[d] - sub_first_root(c, d); }
+
+// Neighbour rows of the live entries e0 .. e0 + n - 1 (n <= 32) of depth d, whose depth is complete
+// (computeRebuildNeighbor :669-696): lane p of every warp works on entry e0 + p, the block's 8 warps
+// share the 27 slots, and found(slot, p, record, neighbour) gets each.  A neighbour is a child of one
+// of the parent's neighbours: of an octree node its octree child (or, for a root, the root of the
+// same group that replaces it), of a live entry its child entry if that is live.  The chain of a slot
+// is four dependent loads (record, parent's row, children, what `found` reads), and all rows of a
+// depth are in flight at once.
+template <class Found>
+__device__ __forceinline__ void sub_rows(const Counters* c, const SubTree& o, const SubArrays& A, int d, int depth,
+                                         int e0, int n, Found found) {
+    const int p = (int)lane_id();
+    if (p >= n) return;
+    const int e = e0 + p;
+    const int4 me = A.rec[e];
+    const int son = (me.z >> (3 * (depth - d))) & 7;
+    const bool root = me.x < 0;
+    const int pa = root ? -2 - me.x : me.x;
+    const int* row = root ? o.neigh + (pa >= 0 ? pa : 0) : A.neigh + pa;
+    const size_t rstride = root ? o.stride : (size_t)A.cap_live;
+    for (int k = threadIdx.x >> 5; k < 27; k += kBlock / 32) {
+        int lp, lc;
+        nb_lut(son, k, lp, lc);
+        int v = -1;
+        if (k == 13) {
+            v = o.na + e;
+        } else if (pa >= 0) {
+            const int nb = row[(size_t)lp * rstride];
+            if (nb >= o.na) {
+                const int2 kd = A.kids[nb - o.na];
+                if ((kd.y >> lc) & 1) v = o.na + kd.x + __popc(kd.y & ((1 << lc) - 1));
+            } else if (nb >= 0) {
+                const int fc = __ldg(o.first_child + nb);
+                v = fc < 0 ? -1 : fc + lc;
+                if (root && __ldg(o.ov_group + (size_t)lc * o.stride + nb) == me.y) {
+                    const int r = __ldg(o.groups + (size_t)me.y * kGroupRec + 1) +
+                                  __ldg(o.ov_sub + (size_t)lc * o.stride + nb);
+                    v = o.na + sub_first_root(c, d) + r - c->sub_rstart[d];
+                }
+            }
+        }
+        A.neigh[(size_t)k * A.cap_live + e] = v;
+        found(k, p, me, v);
+    }
+}
+
+// Sign test of one depth's candidates: the 8 children of every live entry of the depth above, then
+// the roots of this depth (always live).  A tile starts with the neighbour rows of its parents
+// (begin), which name the octree nodes whose values a child's own level can read: a child's
+// neighbours are children of its parent's, subdivision nodes below a root carry nothing, so a child
+// none of whose parent's outer neighbours has octree children takes its parent's polynomial as it
+// is.  Nothing else is built before the test; only live candidates get a record.
+// Latency-bound at depth 7 (a few thousand candidates a launch), bound by the polynomials' arithmetic
+// at depth 9 (3.1 million).  With a record of 27 neighbours built for every candidate the launches of
+// depths 4 to D took 131 us (200,000 samples, depth 7), 533 us (500,000, depth 9) and 1.22 ms
+// (2,000,000, depth 9); now 90, 327 and 768 us.  Two blocks per SM: 128 registers, nothing spilled.
+struct SubLevelLoad {
+    static constexpr int kMinBlocks = 2;
+    const Counters* c;
+    int d, depth;
+    SubTree o;
     SubArrays A;
-    template <class T>
-    static __device__ T rd(const T* p) { return kShared ? *p : __ldg(p); }
+    static __device__ int* first_children() {   // [32 parents][27]: first child of an octree neighbour, or -1
+        __shared__ int s_fc[32 * 27];
+        return s_fc;
+    }
+    // rows of the tile's parents; called by every thread of the block before the tile's loads
+    __device__ void begin(int base) const {
+        __shared__ unsigned s_con[32];
+        const int f0 = base >> 3;
+        const int nf = min(c->sub_nlive[d - 1] - f0, 32);   // parents of this tile
+        if (nf <= 0) return;
+        const int e0 = c->sub_lbase[d - 1] + f0;
+        int* s_fc = first_children();
+        if (threadIdx.x < 32) s_con[threadIdx.x] = 0u;
+        __syncthreads();
+        sub_rows(c, o, A, d - 1, depth, e0, nf, [&](int k, int p, const int4& me, int v) {
+            const bool oct = v >= 0 && v < o.na;
+            s_fc[p * 27 + k] = oct ? __ldg(o.first_child + v) : -1;
+            // a contributing level has an octree neighbour or is a root's
+            if (oct || me.x < 0) s_con[p] = 1u;
+        });
+        __syncthreads();
+        if ((int)threadIdx.x < nf) {
+            const int e = e0 + (int)threadIdx.x;
+            A.jump[e] = s_con[threadIdx.x] ? e : A.jump[A.rec[e].x];
+        }
+    }
     __device__ unsigned operator()(int i) const {
-        const int nl_prev = c->sub_nlive[d - 1];
-        if (i < 8 * nl_prev) {
-            // A child on no face of its root's cell is interior: its levels are its parent's,
-            // restricted to its octant, with nothing of its own or deeper; test that first
-            // (the same test as below, without touching any record)
-            const int pl = c->sub_lbase[d - 1] + (i >> 3);
-            if (child_touch(A.touch[pl], i & 7) == 0u) {
-                float C[27];
+        if (i >= 8 * c->sub_nlive[d - 1]) return 1u;   // a root
+        const int ch = i & 7, p = threadIdx.x >> 3;
+        const int pl = c->sub_lbase[d - 1] + (i >> 3);
+        float C[27];
+        sub_octant(A.poly + pl, (size_t)A.cap_live, ch, C);
+        float mag = A.poly[(size_t)27 * A.cap_live + pl];
+        const int* s_fc = first_children() + p * 27;
+        int fc[27];
+        bool contrib = false, deeper = false;   // deeper: an octree neighbour with children
 #pragma unroll
-                for (int kk = 0; kk < 27; ++kk) C[kk] = 0.0f;
-                add_subdivided<!kShared>(A.poly + pl, (size_t)A.cap_live, (unsigned)(i & 7), 1, C);
-                const float mag = A.poly[(size_t)27 * A.cap_live + pl];
-                float lo = C[0], hi = C[0];
-#pragma unroll
-                for (int kk = 1; kk < 27; ++kk) { lo = fminf(lo, C[kk]); hi = fmaxf(hi, C[kk]); }
-                const float iso = c->iso;
-                const float margin = 1e-4f * (mag + fabsf(iso));
-                if (lo - iso > margin || hi - iso < -margin) return 0u;   // certain sign
-            }
+        for (int k = 0; k < 27; ++k) {
+            int lp, lc;
+            nb_lut(ch, k, lp, lc);
+            fc[k] = s_fc[lp];
+            contrib |= fc[k] >= 0;
+            fc[k] = fc[k] >= 0 ? fc[k] + lc : -1;
         }
-        const int slot = c->sub_cbase[d] + i;
-        int g, vnode, k, pslot, pa;   // pa: parent as a neighbour-table entry
-        float cc[3];
-        if (i < 8 * nl_prev) {
-            pslot = A.live[c->sub_lbase[d - 1] + (i >> 3)];
-            const int ch = i & 7;
-            g = A.group[pslot];
-            const int* G = groups + (size_t)g * kGroupRec;
-            const int pl = A.vnode[pslot] - G[3] - sub_level_off(G[0], G[2], d - 1);
-            vnode = G[3] + sub_level_off(G[0], G[2], d) + 8 * pl + ch;
-            k = A.key[pslot] | (ch << (3 * (depth - d)));
-            const float w = __int_as_float((126 - d) << 23);   // 2^-(d+1)
-            cc[0] = (ch & 4) ? __fadd_rn(A.cx[pslot], w) : __fsub_rn(A.cx[pslot], w);
-            cc[1] = (ch & 2) ? __fadd_rn(A.cy[pslot], w) : __fsub_rn(A.cy[pslot], w);
-            cc[2] = (ch & 1) ? __fadd_rn(A.cz[pslot], w) : __fsub_rn(A.cz[pslot], w);
-            pa = na + A.vnode[pslot];
-        } else {
-            const int r = c->sub_rstart[d] + (i - 8 * nl_prev);
-            g = root_group[r];
-            const int* G = groups + (size_t)g * kGroupRec;
-            vnode = G[3] + (r - G[1]);
-            const int root_node = sub_root[r];
-            k = key[root_node];
-            cc[0] = cc[1] = cc[2] = 0.5f;
-            float w = 0.25f;
-            for (int l = depth - 1; l >= depth - d; --l) {
+        if (contrib) {   // its own level
+            float y[27];
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    if ((k >> (3 * l + 2 - a)) & 1) cc[a] = __fadd_rn(cc[a], w);
-                    else cc[a] = __fsub_rn(cc[a], w);
-                }
-                w = __fdiv_rn(w, 2.0f);
+            for (int k = 0; k < 27; ++k) {
+                y[k] = fc[k] >= 0 ? __ldg(o.x + fc[k]) : 0.0f;
+                if (fc[k] >= 0 && d < depth) deeper |= __ldg(o.first_child + fc[k]) != -1;
             }
-            pslot = -1;
-            pa = parent[root_node];
+            const float4 q = sub_child_pos(A.pos[pl], ch, d);
+            const float sc = (float)(1 << d);
+            const int b = (1 << d) - 1;
+            sign_level(y, b + (int)__fmul_rn(q.x, sc), b + (int)__fmul_rn(q.y, sc), b + (int)__fmul_rn(q.z, sc), q.x,
+                       q.y, q.z, 0.5f, C, mag);
         }
-        const int* G = groups + (size_t)g * kGroupRec;
-        const bool at_root_depth = (d == G[0]);
-        const int local = vnode - G[3] - sub_level_off(G[0], G[2], d);
-        const int off_prev = (d > G[0]) ? sub_level_off(G[0], G[2], d - 1) : 0;
-        const int off_cur = sub_level_off(G[0], G[2], d);
-        int contrib = 0;
-        bool deeper = false;   // an octree neighbour with children reaches below depth d
-        const int son = (k >> (3 * (depth - d))) & 7;
-        // Position inside the root's cell: rel = the Morton code of the node's L = d - rd
-        // levels below its root (x = bit 2, y = bit 1, z = bit 0 of every triple).  A
-        // neighbour inside the same root's cell is the node at the shifted code in the same
-        // root's block (dilated-integer +-1 per axis); only neighbours outside the root's
-        // cell need the parent-based look-up.
-        const unsigned lmask = (1u << (3 * (d - G[0]))) - 1u;
-        const unsigned rel = (unsigned)local & lmask;
-        unsigned cmp[3][3];
-        bool ok[3][3];
+        if (!deeper) {
+            float lo = C[0], hi = C[0];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const unsigned M = (0x24924924u >> a) & lmask;   // x, y, z bit positions
-            const unsigned u = 4u >> a;
-            const unsigned cm = rel & M;
-            cmp[a][0] = (cm - u) & M;
-            cmp[a][1] = cm;
-            cmp[a][2] = ((cm | ~M) + u) & M;
-            ok[a][0] = cm != 0u;
-            ok[a][1] = true;
-            ok[a][2] = cm != M;
-        }
-        const int r = G[1] + (int)((unsigned)local >> (3 * (d - G[0])));
-        // An interior node (below its root, all 27 neighbours inside the root's cell) has only
-        // zero-valued sub nodes around it and nothing deeper: it is tested before anything is
-        // built.  Other nodes are built first (the test may read their own level).  Only live
-        // nodes are referred to later (children, value chains), so a node dropped here needs
-        // nothing else.
-        const bool interior = ok[0][0] && ok[0][2] && ok[1][0] && ok[1][2] && ok[2][0] && ok[2][2];
-        // values of the own level's neighbours, read as each neighbour is found: below its
-        // root only octree neighbours carry one (deeper subdivision nodes are never roots).
-        // Every array read in the loop is written by earlier launches only: read-only loads
-        // let the 27 look-up chains overlap instead of waiting behind each A.neigh store
-        float y[27];
-#pragma unroll
-        for (int kk = 0; kk < 27; ++kk) y[kk] = 0.0f;
-        if (!interior) {
-            // Three slabs of 9 neighbours, each in three rounds of independent loads (all
-            // addresses clamped to valid entries, results selected afterwards): the parent's
-            // neighbour row; the redirect, child and first-child entries of those neighbours;
-            // the values and grandchildren of the neighbours found
-            const bool has_row = pslot >= 0 || pa >= 0;
-            const int* rowp = (pslot >= 0) ? A.neigh + pslot : neigh + (pa >= 0 ? pa : 0);
-            const size_t rstride = (pslot >= 0) ? A.cstride : stride;
-#pragma unroll
-            for (int ix = 0; ix < 3; ++ix) {
-                int np[9];
-#pragma unroll
-                for (int q = 0; q < 9; ++q) {
-                    const int kk = 9 * ix + q;
-                    int lp, lc;
-                    nb_lut(son, kk, lp, lc);
-                    const int t = rd(rowp + (size_t)lp * rstride);
-                    np[q] = has_row ? t : -1;
-                }
-                int og[9], fc[9], os[9];
-#pragma unroll
-                for (int q = 0; q < 9; ++q) {
-                    const int kk = 9 * ix + q;
-                    int lp, lc;
-                    nb_lut(son, kk, lp, lc);
-                    const int n0 = (np[q] >= 0 && np[q] < na) ? np[q] : 0;
-                    og[q] = __ldg(ov_group + (size_t)lc * stride + n0);
-                    os[q] = __ldg(ov_sub + (size_t)lc * stride + n0);
-                    fc[q] = __ldg(first_child + n0);
-                }
-                int vv[9];
-                bool plain_oct[9];
-#pragma unroll
-                for (int q = 0; q < 9; ++q) {
-                    const int kk = 9 * ix + q;
-                    const int iy = (kk / 3) % 3, iz = kk % 3;
-                    int lp, lc;
-                    nb_lut(son, kk, lp, lc);
-                    int v = -1;
-                    plain_oct[q] = false;
-                    if (ok[0][ix] && ok[1][iy] && ok[2][iz]) {
-                        const unsigned relk = cmp[0][ix] | cmp[1][iy] | cmp[2][iz];
-                        v = na + vnode + (int)relk - (int)rel;
-                        if (at_root_depth) contrib = 1;   // the node itself, a root
-                    } else {
-                        const int n = np[q];
-                        if (n != -1) {
-                            if (n < na) {
-                                if (og[q] == g) {
-                                    // redirected child pointer of this group's root
-                                    v = na + G[3] + os[q];
-                                } else {
-                                    v = (fc[q] == -1) ? -1 : fc[q] + lc;
-                                    plain_oct[q] = true;
-                                }
-                            } else {
-                                // a sub node of depth d - 1 in this group: its children are
-                                // at 8 x its index in level d
-                                v = na + G[3] + off_cur + 8 * (n - na - G[3] - off_prev) + lc;
-                            }
-                        }
-                        // a contributing neighbour is an octree node or a root; the subdivision
-                        // nodes at a group's root depth are exactly its roots, and deeper ones
-                        // are never roots
-                        if (v >= 0 && (v < na || at_root_depth)) contrib = 1;
-                    }
-                    vv[q] = v;
-                }
-#pragma unroll
-                for (int q = 0; q < 9; ++q) {
-                    const int v = vv[q];
-                    const bool oct = v >= 0 && v < na;
-                    const int v0 = oct ? v : 0;
-                    const float xv = __ldg(x + v0);
-                    const int gc = __ldg(first_child + v0);
-                    if (plain_oct[q] && v >= 0 && d < depth && gc != -1) deeper = true;
-                    if (oct && !at_root_depth) y[9 * ix + q] = xv;
-                }
-#pragma unroll
-                for (int q = 0; q < 9; ++q) A.neigh[(size_t)(9 * ix + q) * A.cstride + slot] = vv[q];
-            }
-        }
-        const int prec = (pslot >= 0) ? pslot : -2 - pa;
-        // nearest contributing node on the path to the root (itself when it contributes;
-        // roots always do): lets the value chains skip non-contributing levels in one hop
-        const int jump = contrib ? slot : ((pslot >= 0) ? rd(A.jump + pslot) : slot);
-        // Bernstein coefficients of the levels up to d on the node's cell
-        float C[27], mag;
-        if (at_root_depth) {
-            root_coefficients(r, sub_root[r], d, cc[0], cc[1], cc[2], depth, neigh, stride, parent, enc, x,
-                              root_poly, cap_poly, C, mag);
-        } else {
-            const int pl = c->sub_lbase[d - 1] + (i >> 3);   // the parent's live entry
-#pragma unroll
-            for (int kk = 0; kk < 27; ++kk) C[kk] = 0.0f;
-            add_subdivided<!kShared>(A.poly + pl, (size_t)A.cap_live, (unsigned)(i & 7), 1, C);
-            mag = rd(A.poly + (size_t)27 * A.cap_live + pl);
-            if (contrib) {   // its own level (octree neighbours; never for an interior node)
-                const float sc = (float)(1 << d);
-                const int base = (1 << d) - 1;
-                sign_level(y, base + (int)__fmul_rn(cc[0], sc), base + (int)__fmul_rn(cc[1], sc),
-                           base + (int)__fmul_rn(cc[2], sc), cc[0], cc[1], cc[2], 0.5f, C, mag);
-            }
-            if (!deeper) {
-                float lo = C[0], hi = C[0];
-#pragma unroll
-                for (int kk = 1; kk < 27; ++kk) { lo = fminf(lo, C[kk]); hi = fmaxf(hi, C[kk]); }
-                const float iso = c->iso;
-                const float margin = 1e-4f * (mag + fabsf(iso));
-                if (lo - iso > margin || hi - iso < -margin) return 0u;   // certain sign
-            }
+            for (int kk = 1; kk < 27; ++kk) { lo = fminf(lo, C[kk]); hi = fmaxf(hi, C[kk]); }
+            const float iso = c->iso;
+            const float margin = 1e-4f * (mag + fabsf(iso));
+            if (lo - iso > margin || hi - iso < -margin) return 0u;   // certain sign
         }
         float* stash = sub_poly_stash();
 #pragma unroll
         for (int kk = 0; kk < 27; ++kk) stash[kk * kBlock + threadIdx.x] = C[kk];
         stash[27 * kBlock + threadIdx.x] = mag;
-        const unsigned touch = at_root_depth ? 0x3fu
-                                             : child_touch(rd(A.touch + c->sub_lbase[d - 1] + (i >> 3)), i & 7);
-        stash[28 * kBlock + threadIdx.x] = __uint_as_float(touch);
-        stash[29 * kBlock + threadIdx.x] = __int_as_float(vnode);
-        if (interior) {
-#pragma unroll
-            for (int kk = 0; kk < 27; ++kk) {
-                const int ix = kk / 9, iy = (kk / 3) % 3, iz = kk % 3;
-                const unsigned relk = cmp[0][ix] | cmp[1][iy] | cmp[2][iz];
-                A.neigh[(size_t)kk * A.cstride + slot] = na + vnode + (int)relk - (int)rel;
-            }
-        }
-        A.depth[slot] = d;
-        A.cx[slot] = cc[0];
-        A.cy[slot] = cc[1];
-        A.cz[slot] = cc[2];
-        A.parent[slot] = prec;
-        A.jump[slot] = jump;
-        A.vnode[slot] = vnode;
-        A.key[slot] = k;
-        A.group[slot] = g;
         return 1u;
     }
-    __device__ void rebase() { PSR_CLOUD(c, groups, sub_root, root_group, root_self, key, neigh, first_child, parent, ov_group, ov_sub, enc, x, root_poly, A); }   // to cloud blockIdx.y
+    __device__ void rebase() { PSR_CLOUD(c, o, A); }   // to cloud blockIdx.y
 };
+// Records of the live candidates, at their place in the live list.
 struct SubLevelStore {
     Counters* c;
     int d, depth;
+    SubTree o;
     SubArrays A;
     unsigned* err;
     __device__ void operator()(int i, unsigned pre, unsigned live) const {
-        if (!live) return;
+        const int nchild = 8 * c->sub_nlive[d - 1];
         const int at = c->sub_lbase[d] + (int)pre;
-        if (at >= A.cap_live) { atomicOr(err, kErrCapacity); return; }
-        const int slot = c->sub_cbase[d] + i;
-        A.live[at] = slot;
-        const float* stash = sub_poly_stash();
-#pragma unroll
-        for (int k = 0; k < 28; ++k) A.poly[(size_t)k * A.cap_live + at] = stash[k * kBlock + threadIdx.x];
-        A.touch[at] = (unsigned char)__float_as_uint(stash[28 * kBlock + threadIdx.x]);
-        if (d == depth) {
-            if ((int)pre >= A.cap_live_d) { atomicOr(err, kErrCapacity); return; }
-            A.lv_vnode[pre] = __float_as_int(stash[29 * kBlock + threadIdx.x]);
+        const bool keep = live && at < A.cap_live && (d < depth || (int)pre < A.cap_live_d);
+        if (live && !keep) atomicOr(err, kErrCapacity);
+        const bool child = i < nchild;
+        const int pl = c->sub_lbase[d - 1] + (i >> 3);
+        if (child) {   // the family's eight lanes are all here
+            const unsigned fam = __ballot_sync(0xffu << (threadIdx.x & 24), keep) >> (threadIdx.x & 24);
+            if ((i & 7) == 0) A.kids[pl] = make_int2(at, (int)(fam & 0xffu));
         }
+        if (!keep) return;
+        int4 me;
+        if (child) {
+            const int ch = i & 7;
+            const int4 pr = A.rec[pl];
+            const int* G = o.groups + (size_t)pr.y * kGroupRec;
+            const int rd = __ldg(G), n = __ldg(G + 2), first = __ldg(G + 3);
+            me.x = pl;
+            me.y = pr.y;
+            me.z = pr.z | (ch << (3 * (depth - d)));
+            me.w = first + sub_level_off(rd, n, d) + 8 * (pr.w - first - sub_level_off(rd, n, d - 1)) + ch;
+            A.pos[at] = sub_child_pos(A.pos[pl], ch, d);
+            const float* stash = sub_poly_stash();
+#pragma unroll
+            for (int k = 0; k < 28; ++k) A.poly[(size_t)k * A.cap_live + at] = stash[k * kBlock + threadIdx.x];
+        } else {
+            const int r = c->sub_rstart[d] + (i - nchild);
+            const int node = __ldg(o.sub_root + r);
+            me.y = __ldg(o.root_group + r);
+            const int* G = o.groups + (size_t)me.y * kGroupRec;
+            me.x = -2 - __ldg(o.parent + node);
+            me.z = __ldg(o.key + node);
+            me.w = __ldg(G + 3) + (r - __ldg(G + 1));
+            float q[3] = {0.5f, 0.5f, 0.5f}, w = 0.25f;
+            for (int l = depth - 1; l >= depth - d; --l) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    q[a] = ((me.z >> (3 * l + 2 - a)) & 1) ? __fadd_rn(q[a], w) : __fsub_rn(q[a], w);
+                w = __fmul_rn(w, 0.5f);
+            }
+            A.pos[at] = make_float4(q[0], q[1], q[2], __int_as_float(d));
+            float C[27], mag;
+            root_coefficients(r, node, d, q[0], q[1], q[2], depth, o.neigh, o.stride, o.parent, o.enc, o.x,
+                              o.root_poly, o.cap_poly, C, mag);
+#pragma unroll
+            for (int k = 0; k < 27; ++k) A.poly[(size_t)k * A.cap_live + at] = C[k];
+            A.poly[(size_t)27 * A.cap_live + at] = mag;
+        }
+        A.rec[at] = me;
+        if (d == depth) A.lv_vnode[pre] = me.w;
     }
     // chains the counts: candidates of depth d + 1 = 8 x live of depth d + roots of d + 1
     __device__ void done(unsigned total) const {
@@ -1251,12 +1168,12 @@ struct SubLevelStore {
             c->n_sub_dnodes = n;
         }
     }
-    __device__ void rebase() { PSR_CLOUD(c, A, err); }   // to cloud blockIdx.y
+    __device__ void rebase() { PSR_CLOUD(c, o, A, err); }   // to cloud blockIdx.y
 };
 
 // The depths 1 .. dmax (at most 8 + 64 + 512 candidates) in one CTA: the scans of so few elements
 // cost a launch each otherwise.
-__global__ void __launch_bounds__(kBlock) k_sub_coarse(SubLevelLoad<true, 1> load, SubLevelStore store, int dmax) {
+__global__ void __launch_bounds__(kBlock) k_sub_coarse(SubLevelLoad load, SubLevelStore store, int dmax) {
     PSR_CLOUD(load, store);
     __shared__ unsigned s_warp[kBlock / 32 + 1];
     for (int d = 1; d <= dmax; ++d) {
@@ -1265,91 +1182,67 @@ __global__ void __launch_bounds__(kBlock) k_sub_coarse(SubLevelLoad<true, 1> loa
         const int n = *(volatile const int*)&load.c->sub_cand[d];
         unsigned run = 0;
         for (int base = 0; base < n; base += kBlock) {
+            load.begin(base);
+            __syncthreads();
             const int i = base + (int)threadIdx.x;
             const unsigned v = i < n ? load(i) : 0u;
             unsigned excl;
             const unsigned sum = block_exclusive_scan(v, excl, s_warp);
             if (i < n) store(i, run + excl, v);
             run += sum;
+            __syncthreads();
         }
         if (threadIdx.x == 0) store.done(run);
         __syncthreads();   // the depth's records and counts before the next depth reads them
     }
 }
 
-// index of virtual node v among the live depth-D cells (sorted), or -1; the search gallops from
-// cell L outwards, since a neighbour's number is near its own
-__device__ __forceinline__ int live_index(const int* lv_vnode, int n, int v, int L) {
-    const int at = lv_vnode[L];
-    int lo, hi;   // the place is in [lo, hi)
-    int step = 1;
-    if (v < at) {
-        hi = L;
-        while (hi - step >= 0 && lv_vnode[hi - step] >= v) { hi -= step; step <<= 1; }
-        lo = hi - step < 0 ? 0 : hi - step;
-        ++hi;
-    } else {
-        lo = L;
-        while (lo + step < n && lv_vnode[lo + step] <= v) { lo += step; step <<= 1; }
-        hi = lo + step > n ? n : lo + step;
-    }
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (lv_vnode[mid] < v) lo = mid + 1;
-        else hi = mid;
-    }
-    return (lo < n && lv_vnode[lo] == v) ? lo : -1;
-}
-
-// per live depth-D cell: the live index of each same-depth sub neighbour (-1: none, an
-// octree node, or a cell with a certain sign); one thread per (cell, slot)
-__global__ void __launch_bounds__(kBlock) k_sub_live_neigh(const Counters* c, int depth, SubArrays A,
-                                                           int* lv_nb, size_t dstride, int na, int* group_live) {
-    PSR_CLOUD(c, A, lv_nb, group_live);
-    const int nl = c->n_sub_dnodes;
-    const int lb = c->sub_lbase[depth];
-    const long long n = 27LL * nl;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int L = (int)(t / 27), k = (int)(t - 27LL * L);
-        const int v = A.neigh[(size_t)k * A.cstride + A.live[lb + L]];
-        lv_nb[(size_t)k * dstride + L] = (k == 13) ? L : ((v >= na) ? live_index(A.lv_vnode, nl, v - na, L) : -1);
-        if (k == 13) {   // a group's live cells are consecutive
-            const int g = A.group[A.live[lb + L]];
-            if (L == 0 || A.group[A.live[lb + L - 1]] != g) group_live[g] = L;
-        }
-    }
-}
-
-// vertex ownership among the live depth-D cells (initSubdivideVertexOwner :698-763): a corner
-// is owned by the smallest-key live cell around it.  Cells with a certain sign take no part:
+// Per live depth-D cell: its neighbour row and jump link, and which vertices and edges it owns.
+// A corner is owned by the smallest-key live cell around it (initSubdivideVertexOwner :698-763).
+// Cells with a certain sign take no part:
 // every corner of a live cell still gets exactly one record, the records of crossing edges
 // keep their owners (every cell around a crossing edge has a sign change, so is live), and a
 // vertex value does not depend on the cell that evaluates it (the same nonzero terms in the
 // same order), so the mesh is unchanged.
-// Edges likewise (initSubdivideEdgeArray :812-886).
-__global__ void __launch_bounds__(kBlock) k_sub_owners(const Counters* c, int depth, SubArrays A, const int* lv_nb,
-                                                       size_t dstride, unsigned char* s_vmask,
+// Edges likewise (initSubdivideEdgeArray :812-886).  32 cells per block, as in the level scans.  A
+// search of every neighbour's number in the live list took 585 us for 757,000 cells (2,000,000
+// samples, depth 9) and the owners another 31 us in a launch of their own; now 197 us.
+__global__ void __launch_bounds__(kBlock) k_sub_owners(const Counters* c, int depth, SubTree o, SubArrays A,
+                                                       int* group_live, unsigned char* s_vmask,
                                                        unsigned short* s_emask) {
-    PSR_CLOUD(c, A, lv_nb, s_vmask, s_emask);
+    PSR_CLOUD(c, o, A, group_live, s_vmask, s_emask);
+    __shared__ unsigned s_con[32], s_smaller[32];
     const int nl = c->n_sub_dnodes;
     const int lb = c->sub_lbase[depth];
-    PSR_GRID_STRIDE(L, nl) {
-        const int myk = A.key[A.live[lb + L]];
-        unsigned smaller = 0;
-#pragma unroll
-        for (int k = 0; k < 27; ++k) {
-            if (k == 13) continue;
-            const int nb = lv_nb[(size_t)k * dstride + L];
-            if (nb >= 0 && A.key[A.live[lb + nb]] < myk) smaller |= 1u << k;
+    const int q = threadIdx.x & 7, p = threadIdx.x >> 3;
+    for (int L0 = 32 * blockIdx.x; L0 < nl; L0 += 32 * gridDim.x) {
+        const int n = min(nl - L0, 32);
+        if (threadIdx.x < 32) s_con[threadIdx.x] = s_smaller[threadIdx.x] = 0u;
+        __syncthreads();
+        sub_rows(c, o, A, depth, depth, lb + L0, n, [&](int k, int pp, const int4& me, int v) {
+            if (v >= o.na) {
+                if (k != 13 && A.rec[v - o.na].z < me.z) atomicOr(&s_smaller[pp], 1u << k);
+            } else if (v >= 0) {
+                s_con[pp] = 1u;
+            }
+            if (k == 13) {   // a group's live cells are consecutive
+                if (L0 + pp == 0 || A.rec[lb + L0 + pp - 1].y != me.y) group_live[me.y] = L0 + pp;
+            }
+        });
+        __syncthreads();
+        // eight lanes per cell: a vertex each, then edges q and 8 + q
+        const unsigned smaller = s_smaller[p];
+        const int sh = threadIdx.x & 24;
+        const unsigned mv = __ballot_sync(0xffffffffu, !(smaller & vertex_cells(q))) >> sh;
+        const unsigned m0 = __ballot_sync(0xffffffffu, !(smaller & edge_cells(q))) >> sh;
+        const unsigned m1 = __ballot_sync(0xffffffffu, q < 4 && !(smaller & edge_cells(8 + (q & 3)))) >> sh;
+        if (p < n && q == 0) {
+            const int e = lb + L0 + p;
+            s_vmask[L0 + p] = (unsigned char)(mv & 0xffu);
+            s_emask[L0 + p] = (unsigned short)((m0 & 0xffu) | ((m1 & 0xfu) << 8));
+            A.jump[e] = s_con[p] ? e : A.jump[A.rec[e].x];
         }
-        unsigned m = 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) if (!(smaller & vertex_cells(q))) m |= 1u << q;
-        s_vmask[L] = (unsigned char)m;
-        m = 0;
-#pragma unroll
-        for (int e = 0; e < 12; ++e) if (!(smaller & edge_cells(e))) m |= 1u << e;
-        s_emask[L] = (unsigned short)m;
+        __syncthreads();
     }
 }
 
@@ -1365,15 +1258,15 @@ struct SubVertexStore {
     __device__ void operator()(int L, unsigned pre, unsigned cnt) const {
         if (!cnt) return;
         if ((int)(pre + cnt) > cap) { atomicOr(err, kErrCapacity); return; }
-        const int s = A.live[c->sub_lbase[depth] + L];
+        const float4 p = A.pos[c->sub_lbase[depth] + L];
         const unsigned m = vmask[L];
         const float hw = 1.0f / (float)(1 << (depth + 1));
         int q = (int)pre;
         for (int k = 0; k < 8; ++k) {
             if (!((m >> k) & 1)) continue;
-            vx[q] = __fadd_rn(A.cx[s], (float)(2 * (k & 1) - 1) * hw);
-            vy[q] = __fadd_rn(A.cy[s], (float)(2 * ((k >> 1) & 1) - 1) * hw);
-            vz[q] = __fadd_rn(A.cz[s], (float)(2 * ((k >> 2) & 1) - 1) * hw);
+            vx[q] = __fadd_rn(p.x, (float)(2 * (k & 1) - 1) * hw);
+            vy[q] = __fadd_rn(p.y, (float)(2 * ((k >> 1) & 1) - 1) * hw);
+            vz[q] = __fadd_rn(p.z, (float)(2 * ((k >> 2) & 1) - 1) * hw);
             vowner[q] = L;
             vkind[q] = k;
             ++q;
@@ -1403,10 +1296,11 @@ struct SubEdgeStore {
 // maintainSubdivideVertexNodePointer (:765-810) and maintainSubdivideEdgeNodePointer (:888-949), an
 // element kind per blockIdx.z: s_vtx, s_edge indexed by live cell.  They need no clearing: every
 // slot of a live cell is written by the owner of that vertex / edge.
-__global__ void __launch_bounds__(kBlock) k_sub_maintain(const Counters* c, const int* lv_nb, size_t dstride,
+__global__ void __launch_bounds__(kBlock) k_sub_maintain(const Counters* c, int depth, SubArrays A, int na, size_t dstride,
                                                          const int* vowner, const int* vkind, int* s_vtx,
                                                          const int* eowner, const int* ekind, int* s_edge) {
-    PSR_CLOUD(c, lv_nb, vowner, vkind, s_vtx, eowner, ekind, s_edge);
+    PSR_CLOUD(c, A, vowner, vkind, s_vtx, eowner, ekind, s_edge);
+    const int lb = c->sub_lbase[depth];   // a live neighbour's entry is lb + its live index
     if (blockIdx.z == 0) {
         const int V = c->n_sub_vertices;
         PSR_GRID_STRIDE(v, V) {
@@ -1416,7 +1310,7 @@ __global__ void __launch_bounds__(kBlock) k_sub_maintain(const Counters* c, cons
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int ax = (j & 1) ? mx : 0, ay = (j & 2) ? my : 0, az = (j & 4) ? mz : 0;
-                const int nb = lv_nb[(size_t)nslot(ax, ay, az) * dstride + ow];
+                const int nb = A.neigh[(size_t)nslot(ax, ay, az) * A.cap_live + lb + ow] - na - lb;
                 if (nb >= 0) s_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * dstride + nb] = v + 1;
             }
         }
@@ -1428,7 +1322,7 @@ __global__ void __launch_bounds__(kBlock) k_sub_maintain(const Counters* c, cons
             for (int j = 0; j < 4; ++j) {
                 int a[3];
                 edge_offset(kind, j, a);
-                const int nb = lv_nb[(size_t)nslot(a[0], a[1], a[2]) * dstride + ow];
+                const int nb = A.neigh[(size_t)nslot(a[0], a[1], a[2]) * A.cap_live + lb + ow] - na - lb;
                 if (nb >= 0) s_edge[(size_t)edge_slot_of(kind, a) * dstride + nb] = ei + 1;
             }
         }
@@ -1454,10 +1348,11 @@ constexpr int kSvMaxLevels = kMaxDepth + 1;
 __global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* c, int depth, const float* vx,
                                                                 const float* vy, const float* vz, const int* vowner,
                                                                 const int* neigh, size_t stride, const int* parent,
-                                                                const int* groups, const int* root_self, SubArrays A,
+                                                                const int* root_self, SubArrays A,
                                                                 const int* enc, const float* x, float* vvalue, int na) {
-    PSR_CLOUD(c, vx, vy, vz, vowner, neigh, parent, groups, root_self, A, enc, x, vvalue);
-    __shared__ int s_node[kSvGroups][kSvMaxLevels];   // slot (subdivision) or octree node
+    PSR_CLOUD(c, vx, vy, vz, vowner, neigh, parent, root_self, A, enc, x, vvalue);
+    __shared__ int s_node[kSvGroups][kSvMaxLevels];   // live entry (subdivision) or octree node
+    __shared__ int s_root[kSvGroups];                 // a root neighbour's number to its root index
     __shared__ int s_o[kSvGroups][kSvMaxLevels][3];   // function index of the level's node
     __shared__ float s_t[kSvGroups][kSvMaxLevels * 27];
     __shared__ float s_b[kSvGroups][kSvMaxLevels][9];  // a level's 3 basis values per axis
@@ -1468,8 +1363,7 @@ __global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* 
     const unsigned gmask = 0xffu << (threadIdx.x & 24);   // the group's lanes in its warp
     for (int v = blockIdx.x * kSvGroups + w; v < V; v += gridDim.x * kSvGroups) {
         const float qx = vx[v], qy = vy[v], qz = vz[v];
-        const int own = A.live[lb + vowner[v]];
-        const int* G = groups + (size_t)A.group[own] * kGroupRec;
+        const int own = lb + vowner[v];
         int nsub = 0, nlev = 0;
         if (gl == 0) {
             // levels whose 27 neighbours are all zero-valued subdivision nodes add nothing:
@@ -1477,7 +1371,7 @@ __global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* 
             int sn = A.jump[own], now = -1;
             while (nsub < kSvMaxLevels) {
                 s_node[w][nsub++] = sn;
-                const int p = A.parent[sn];
+                const int p = A.rec[sn].x;
                 if (p < 0) { now = -2 - p; break; }
                 sn = A.jump[p];
             }
@@ -1491,12 +1385,14 @@ __global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* 
             const int nd = s_node[w][l];
             int ox, oy, oz;
             if (l < nsub) {
-                const int d = A.depth[nd];
+                const float4 q = A.pos[nd];
+                const int d = __float_as_int(q.w);
                 const float sc = (float)(1 << d);
                 const int base = (1 << d) - 1;
-                ox = base + (int)__fmul_rn(A.cx[nd], sc);
-                oy = base + (int)__fmul_rn(A.cy[nd], sc);
-                oz = base + (int)__fmul_rn(A.cz[nd], sc);
+                ox = base + (int)__fmul_rn(q.x, sc);
+                oy = base + (int)__fmul_rn(q.y, sc);
+                oz = base + (int)__fmul_rn(q.z, sc);
+                if (l == nsub - 1) s_root[w] = sub_root_shift(c, d) - na;
             } else {
                 decode_fn_index(enc[nd], depth, ox, oy, oz);
             }
@@ -1514,8 +1410,8 @@ __global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* 
         for (int t = gl; t < nlev * 27; t += kSvLanes) {
             const int l = t / 27, k = t - 27 * l;
             const int nd = s_node[w][l];
-            int nb = (l < nsub) ? A.neigh[(size_t)k * A.cstride + nd] : neigh[(size_t)k * stride + nd];
-            if (nb >= na) nb = sub_value_node(nb, na, G, root_self);
+            int nb = (l < nsub) ? A.neigh[(size_t)k * A.cap_live + nd] : neigh[(size_t)k * stride + nd];
+            if (nb >= na) nb = (l == nsub - 1) ? root_self[nb + s_root[w]] : -1;
             float term = 0.0f;
             if (nb >= 0) {
                 const float bxk = s_b[w][l][k / 9];
@@ -1546,37 +1442,38 @@ __global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* 
 __global__ void __launch_bounds__(kBlock) k_sub_vertex_values_wide(const Counters* c, int depth, const float* vx,
                                                                    const float* vy, const float* vz, const int* vowner,
                                                                    const int* neigh, size_t stride, const int* parent,
-                                                                   const int* groups, const int* root_self, SubArrays A,
+                                                                   const int* root_self, SubArrays A,
                                                                    const int* enc, const float* x, float* vvalue, int na) {
-    PSR_CLOUD(c, vx, vy, vz, vowner, neigh, parent, groups, root_self, A, enc, x, vvalue);
+    PSR_CLOUD(c, vx, vy, vz, vowner, neigh, parent, root_self, A, enc, x, vvalue);
     const int V = c->n_sub_vertices;
     const float iso = c->iso;
     const int lb = c->sub_lbase[depth];
     PSR_GRID_STRIDE(v, V) {
         const float qx = vx[v], qy = vy[v], qz = vz[v];
-        const int own = A.live[lb + vowner[v]];
-        const int* G = groups + (size_t)A.group[own] * kGroupRec;
+        const int own = lb + vowner[v];
         // levels: subdivision nodes through the jump links, then the octree ancestors
         int node = A.jump[own];
         bool sub = true;
         int nbs[27];
 #pragma unroll
-        for (int k = 0; k < 27; ++k) nbs[k] = A.neigh[(size_t)k * A.cstride + node];
+        for (int k = 0; k < 27; ++k) nbs[k] = A.neigh[(size_t)k * A.cap_live + node];
         float val = 0.0f;
         for (int level = 0; level <= kMaxDepth; ++level) {
             int ox, oy, oz, d, next;
             bool next_sub = false;
             if (sub) {
-#pragma unroll
-                for (int k = 0; k < 27; ++k)
-                    if (nbs[k] >= na) nbs[k] = sub_value_node(nbs[k], na, G, root_self);
-                d = A.depth[node];
+                const float4 q = A.pos[node];
+                d = __float_as_int(q.w);
                 const float sc = (float)(1 << d);
                 const int base = (1 << d) - 1;
-                ox = base + (int)__fmul_rn(A.cx[node], sc);
-                oy = base + (int)__fmul_rn(A.cy[node], sc);
-                oz = base + (int)__fmul_rn(A.cz[node], sc);
-                const int p = A.parent[node];
+                ox = base + (int)__fmul_rn(q.x, sc);
+                oy = base + (int)__fmul_rn(q.y, sc);
+                oz = base + (int)__fmul_rn(q.z, sc);
+                const int p = A.rec[node].x;
+                const int shift = p < 0 ? sub_root_shift(c, d) - na : 0;
+#pragma unroll
+                for (int k = 0; k < 27; ++k)
+                    if (nbs[k] >= na) nbs[k] = p < 0 ? root_self[nbs[k] + shift] : -1;
                 next_sub = p >= 0;
                 next = next_sub ? A.jump[p] : -2 - p;
             } else {
@@ -1589,7 +1486,7 @@ __global__ void __launch_bounds__(kBlock) k_sub_vertex_values_wide(const Counter
             for (int k = 0; k < 27; ++k) xv[k] = x[nbs[k]];
             int nb2[27];
             const int* row = next_sub ? A.neigh + next : neigh + (next >= 0 ? next : 0);
-            const size_t rstride = next_sub ? A.cstride : stride;
+            const size_t rstride = next_sub ? (size_t)A.cap_live : stride;
 #pragma unroll
             for (int k = 0; k < 27; ++k) nb2[k] = row[(size_t)k * rstride];
             val = terms_at(ox, oy, oz, d, xv, val, qx, qy, qz);
@@ -1693,7 +1590,7 @@ struct SubCubeStore {
     __device__ void operator()(int L, unsigned pre, unsigned cnt) const {
         tri_of_live[L] = pre;
         if (!cnt) return;
-        const int g = A.group[A.live[c->sub_lbase[depth] + L]];
+        const int g = A.rec[c->sub_lbase[depth] + L].y;
         const unsigned e0 = edge_of_live[group_live[g]];
         const unsigned base = ((int)e0 < c->n_sub_edges) ? ecross[e0] : (unsigned)c->n_sub_cross;
         const int cls = cube_class[L];
@@ -1955,33 +1852,21 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
     const int gl = D >= 8 ? 4 * ws.num_sms : ws.num_sms;
     const int sbps = D >= 8 ? 4 : 1;
     cudaError_t e;
-    SubArrays A{ws.c_vnode, ws.c_key, ws.c_group, ws.c_parent, ws.c_jump, ws.c_depth, ws.c_cx, ws.c_cy, ws.c_cz,
-                ws.c_neigh, (size_t)ws.cap.sub_nodes, ws.c_live, ws.c_poly, ws.c_touch, ws.lv_vnode,
-                ws.cap.sub_nodes, ws.cap.sub_live, ws.cap.sub_dnodes};
+    const SubTree o{mb.groups, ws.sub_root, ws.root_group, ws.key, ws.neigh, stride, ws.first_child, ws.parent,
+                    mb.ov_group, mb.ov_sub, ws.enc, ws.xsol, ws.root_poly, ws.cap_poly, na};
+    const SubArrays A{ws.c_rec, ws.c_pos, ws.c_jump, ws.c_kids, ws.c_neigh, ws.c_poly, ws.lv_vnode,
+                      ws.cap.sub_nodes, ws.cap.sub_live, ws.cap.sub_dnodes};
     // depth after depth: candidates (children of the live nodes above, then the roots of this
-    // depth), their neighbours and sign tests; the live ones are compacted in order
-    auto level = [&](auto load, int d) {
-        load.c = c; load.d = d; load.depth = D; load.na = na; load.groups = mb.groups; load.sub_root = ws.sub_root;
-        load.root_group = ws.root_group; load.root_self = ws.root_self; load.key = ws.key; load.neigh = ws.neigh;
-        load.stride = stride; load.first_child = ws.first_child; load.parent = ws.parent; load.ov_group = mb.ov_group;
-        load.ov_sub = mb.ov_sub; load.enc = ws.enc; load.x = ws.xsol; load.root_poly = ws.root_poly;
-        load.cap_poly = ws.cap_poly; load.A = A;
-        return load;
-    };
+    // depth) and their sign tests; the live ones are compacted in order
     const int dcoarse = D < 3 ? D : 3;
-    k_sub_coarse<<<PSR_GRID(ws, 1), kBlock, 0, s>>>(level(SubLevelLoad<true, 1>{}, 1), SubLevelStore{c, 1, D, A, err}, dcoarse);
+    k_sub_coarse<<<PSR_GRID(ws, 1), kBlock, 0, s>>>(SubLevelLoad{c, 1, D, o, A}, SubLevelStore{c, 1, D, o, A, err}, dcoarse);
     for (int d = dcoarse + 1; d <= D; ++d) {
-        if (D >= 8)
-            e = launch_scan<1>(level(SubLevelLoad<false, 2>{}, d), SubLevelStore{c, d, D, A, err}, &c->sub_cand[d], 0,
-                               ws.scan, total, err, s, ScanCount{}, sbps);
-        else
-            e = launch_scan<1>(level(SubLevelLoad<false, 1>{}, d), SubLevelStore{c, d, D, A, err}, &c->sub_cand[d], 0,
-                               ws.scan, total, err, s, ScanCount{}, sbps);
+        e = launch_scan<1>(SubLevelLoad{c, d, D, o, A}, SubLevelStore{c, d, D, o, A, err}, &c->sub_cand[d], 0, ws.scan,
+                           total, err, s, ScanCount{}, sbps);
         if (e != cudaSuccess) return e;
     }
     // the live depth-D cells carry every record from here on, indexed by their live index
-    k_sub_live_neigh<<<PSR_GRID(ws, 2 * gl), kBlock, 0, s>>>(c, D, A, ws.lv_nb, dstride, na, mb.group_live);
-    k_sub_owners<<<PSR_GRID(ws, gl), kBlock, 0, s>>>(c, D, A, ws.lv_nb, dstride, ws.s_vmask, ws.s_emask);
+    k_sub_owners<<<PSR_GRID(ws, 2 * gl), kBlock, 0, s>>>(c, D, o, A, mb.group_live, ws.s_vmask, ws.s_emask);
     e = launch_scans(scan_job<2>(PopcLoad8{ws.s_vmask},
                                  SubVertexStore{ws.s_vmask, c, D, A, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.sv_kind,
                                                 8 * ws.cap.sub_dnodes, err},
@@ -1994,15 +1879,15 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
                      NoScan{}, NoScan{}, err, s, sbps);
     if (e != cudaSuccess) return e;
     const dim3 g2 = PSR_GRID(ws, gl);
-    k_sub_maintain<<<dim3(g2.x, g2.y, 2), kBlock, 0, s>>>(c, ws.lv_nb, dstride, ws.sv_owner, ws.sv_kind, ws.s_vtx,
+    k_sub_maintain<<<dim3(g2.x, g2.y, 2), kBlock, 0, s>>>(c, D, A, na, dstride, ws.sv_owner, ws.sv_kind, ws.s_vtx,
                                                           ws.se_owner, ws.se_kind, ws.s_edge);
     if (D >= 8)
         k_sub_vertex_values_wide<<<PSR_GRID(ws, 8 * ws.num_sms), kBlock, 0, s>>>(
-            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, mb.groups, ws.root_self, A, ws.enc,
+            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, ws.root_self, A, ws.enc,
             ws.xsol, ws.sv_value, na);
     else
         k_sub_vertex_values<<<PSR_GRID(ws, 16 * ws.num_sms), kSvBlock, 0, s>>>(
-            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, mb.groups, ws.root_self, A, ws.enc,
+            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, ws.root_self, A, ws.enc,
             ws.xsol, ws.sv_value, na);
     // crossings: staged after the main part's vertices
     e = launch_scan<2>(SubCrossLoad{ws.se_owner, ws.se_kind, ws.s_vtx, dstride, ws.sv_value, err},

@@ -39,6 +39,16 @@ __device__ __forceinline__ auto scan_done(const S& s, unsigned tot, int) -> decl
 template <class S>
 __device__ __forceinline__ void scan_done(const S&, unsigned, long) {}
 
+// Load functors may define `void begin(int base) const`: every thread of the block calls it before
+// the loads of the tile that starts at element `base`.
+template <class L>
+__device__ __forceinline__ auto scan_begin(const L& l, int base, int) -> decltype(l.begin(base), void()) {
+    l.begin(base);
+    __syncthreads();
+}
+template <class L>
+__device__ __forceinline__ void scan_begin(const L&, int, long) {}
+
 // Functors over plain arrays may define all(base, v): a thread's items in 16-byte accesses (its
 // items are consecutive, so one by one each access of a warp would touch 32 sectors: the 2.1M-entry
 // cell table took 21.8 us).
@@ -126,6 +136,7 @@ __device__ __forceinline__ void scan_body(Load load, Store store, int n, ScanScr
         const int t = s_tile;
         __syncthreads();
         if (t >= ntiles) break;
+        scan_begin(load, t * kTile, 0);
         const int base = t * kTile + threadIdx.x * kItems;
         unsigned v[kItems];
         unsigned sum = 0;

@@ -134,16 +134,15 @@ struct Workspace {
     int* root_self;         // per root: the octree node it stands for
     float* root_poly;       // [28][cap_poly]: per root, Bernstein coefficients of the levels up to it
     int cap_poly;
-    // subdivision candidates in compact slots (SoA, capacity cap.sub_nodes)
-    int *c_vnode, *c_key, *c_group, *c_parent, *c_jump, *c_depth;
-    float *c_cx, *c_cy, *c_cz;
-    int* c_neigh;           // [27][cap.sub_nodes]
-    int* c_live;            // live slots, depth after depth (capacity cap.sub_live)
-    float* c_poly;          // [28][cap.sub_live]: per live entry, its Bernstein coefficients, sum |y|
-    unsigned char* c_touch; // per live entry: faces of its root's cell its cell lies on
+    // live subdivision nodes, depth after depth (capacity cap.sub_live)
+    int4* c_rec;            // parent, group, key, virtual index
+    float4* c_pos;          // centre, depth
+    int* c_jump;            // nearest contributing node on the path to the root
+    int2* c_kids;           // live children: first entry, octant bits
+    int* c_neigh;           // [27][cap.sub_live]
+    float* c_poly;          // [28][cap.sub_live]: Bernstein coefficients, sum |y|
     // live depth-D cells (capacity cap.sub_dnodes)
     int* lv_vnode;          // virtual index, ascending
-    int* lv_nb;             // [27][cap.sub_dnodes]: live index of each same-depth neighbour
     int *s_vtx, *s_edge;    // [8|12][cap.sub_dnodes]
     unsigned char* s_vmask;
     unsigned short* s_emask;
