@@ -476,11 +476,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
         build_dff_table(D, dff);
         std::vector<float> st;
         build_stencil(kMaxDepth, st, (double)cfg.laplacian_epsilon);
-        // the kernels use float entries, row by row of the function the node carries: the leaves of
-        // a node's neighbourhood then read neighbouring entries
-        std::vector<float> dff32(dff.size());
-        for (int i = 0; i < ws.res; ++i)
-            for (int j = 0; j < ws.res; ++j) dff32[(size_t)i * ws.res + j] = (float)dff[(size_t)i + (size_t)ws.res * j];
+        std::vector<float> dff32(dff.begin(), dff.end());   // the kernels use float entries
         e = cudaMemcpy(ws.dff, dff32.data(), dff32.size() * sizeof(float), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(ws.stencil, st.data(), st.size() * sizeof(float), cudaMemcpyHostToDevice);
         // the CG takes four values per depth: an entry depends only on the axes its offset moves on

@@ -117,7 +117,9 @@ void integrals(const Fn& a, const Fn& b, double& ff, double& dff, double& d2) {
 
 }  // namespace
 
-// d/dx-product table (full res x res; only pairs with overlapping support are non-zero)
+// d/dx-product table (full res x res; only pairs with overlapping support are non-zero), row by row
+// of the differentiated function, which is the one a node carries: the leaves of a node's
+// neighbourhood then read neighbouring entries
 void build_dff_table(int depth, std::vector<double>& dff) {
     const int res = (1 << (depth + 1)) - 1;
     dff.assign((size_t)res * res, 0.0);
@@ -128,7 +130,7 @@ void build_dff_table(int depth, std::vector<double>& dff) {
             if (std::fabs(f[i].c - f[j].c) >= 1.5 * (f[i].w + f[j].w)) continue;
             double a, b, c;
             integrals(f[i], f[j], a, b, c);
-            dff[(size_t)i + (size_t)res * j] = b;
+            dff[(size_t)i * res + j] = b;
         }
 }
 
