@@ -349,7 +349,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
         A.add(ws.cg_rp, 8 * pitch);
         // virtual blocks of 256 groups; a cloud's depths leave at most one part-filled each
         ws.cg_part_cap = (int)((pitch / 256 + 8) * (size_t)std::max(1, cfg.batch_clouds));
-        A.add(ws.cg_part, 2 * (size_t)ws.cg_part_cap);
+        A.add(ws.cg_part, 2 * ((size_t)ws.cg_part_cap + kMaxBatchClouds * (kMaxDepth + 1)));   // and totals of units
     }
     A.add(ws.cg_desc, 14 * ((size_t)nodes / 8 + 8));
     A.add(ws.cg_partial, std::max((size_t)nodes, (size_t)4096 * (kMaxDepth + 1)));

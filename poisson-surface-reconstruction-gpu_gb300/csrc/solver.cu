@@ -830,8 +830,8 @@ __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
 
 // ---- whole-GPU CG: the depths from 5 on of trees of depth 8 and 9 ------------------------
 // One cooperative launch (so all its blocks are resident) solves every unit -- a depth of a cloud
-// -- in lockstep rounds: A p with p.Ap, grid barrier, x and r with r.r, grid barrier.  A unit
-// whose true residual is due spends a round on it instead.  The arithmetic, the reductions'
+// -- in rounds of two steps: A p with p.Ap, then x and r with r.r.  A unit whose true residual is due
+// spends a round on it instead.  The arithmetic, the reductions'
 // precision and the decisions are the cluster solver's; the scalars of a unit are kept in the
 // shared memory of every block that works on it, each computing them from the same sums.
 // Work is dealt in virtual blocks of 256 sibling groups of one unit, a contiguous range of them
@@ -841,16 +841,25 @@ __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
 // neighbour groups (27 a group, 13.5 bytes a row) are looked up once per solve.  Each virtual
 // block's sum goes to global memory and every block adds a unit's sums in one order, which
 // depends on the unit's rows alone: a cloud's result is the same alone and in a batch.
-// A round of 1.2M rows takes 21 us, of 3.1M rows 50 us, bound by L2 traffic and the two grid
-// barriers (3.4k cycles each); the CUDA-graph while node over whole-GPU kernels before it took 43 and
-// 97 us (7 launches per two iterations).  Keeping the block's p in shared memory and reading only
-// other blocks' groups from L2 was slower (5.0 ms against 3.4 of 3.1M rows): the scattered remote
-// reads wait one by one.
+// A step ends when a block has the sums of all virtual blocks of its units, which is the only barrier:
+// units run at their own pace.  A block's warps go through its passes without waiting for one
+// another, and A p, which only the thread that computed it reads, stays in shared memory.  A round of
+// 0.28M rows takes 10 us, of 1.2M 19 us and of 3.1M 41 us; with a whole-GPU barrier per step and the
+// sums read after it 11, 20 and 49 us, and as kernels in a CUDA-graph while node (7 launches per two
+// iterations) 27, 43 and 97 us.  What is left: 4k to 6k cycles per step for records to travel through
+// L2, and in A p the gather of 64 (r, p) pairs a group (8k cycles per 512 groups).  Keeping the
+// block's p in shared memory and reading only other blocks' groups from L2 was slower (5.0 ms a solve
+// against 3.4 of 3.1M rows): the scattered remote reads wait one by one.
 constexpr int kGridBlock = 512;    // 128 registers a thread: a group's 27 neighbours and 32 loads in flight
 constexpr int kVbGroups = 256;                       // groups of a virtual block
 constexpr int kGridSubs = kGridBlock / kVbGroups;    // virtual blocks a block works on at once
+constexpr int kGridPasses = 16;                      // passes over its virtual blocks between two block barriers
+// passes whose A p stays in shared memory: 96 KB for 3.6M rows on 147 SMs, more of which go to global
+// memory; the rest of the SM's 256 KB is L1 for the gather
+constexpr int kGridApPasses = 6;
+constexpr size_t kGridApBytes = sizeof(float) * 8 * kGridBlock * kGridApPasses;
+constexpr int kGridUnits = kMaxBatchClouds * (kMaxDepth - 4);   // most units of a launch
 constexpr int kGridDepth = 5;                        // depths below it: at most 4096 rows, one CTA each
-static_assert(sizeof(CgSum) == 16, "workspace.h: cg_part");
 
 struct CgGridArgs {
     CgcVec v;             // cloud 0's workspace
@@ -864,9 +873,9 @@ struct CgGridArgs {
     float2* rp;           // [8][pitch]: (r, p)
     float* xs;            // [8][pitch]: x
     float* ap;            // [8][pitch]: A p
-    CgSum* part;          // [2][part_cap]: sums of the virtual blocks (cloud 0)
+    ulonglong2* part;     // [2][part_cap + kGridUnits]: sums of the virtual blocks, of units (cloud 0)
     int part_cap;
-    unsigned long long* bar;   // arrivals, and above 32 bits the blocks that had work (cloud 0; starts at 0)
+    unsigned long long* bar;   // arrivals of the blocks (cloud 0; starts at 0)
     float tol2;
     int max_iter;
     int res_period;
@@ -893,27 +902,49 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
     return v;
 }
 
-// Every block of the launch has arrived `round` times; `active` adds to the count above 32 bits.
-// Thread 0's fences make the block's writes visible to the others and theirs to the block (as a
-// cooperative-groups grid barrier does).  Bounded: false when the wait ran out.
-__device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned target, bool active,
-                                             unsigned long long& seen) {
-    __shared__ unsigned long long s_seen;
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// Every block of the launch has arrived.  Thread 0's fences make the block's writes visible to the
+// others and theirs to the block.  Bounded: false when the wait ran out.
+__device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned target) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        atomicAdd(bar, 1ull + (active ? 1ull << 32 : 0ull));
+        atomicAdd(bar, 1ull);
         unsigned long long v = ld_acquire_u64(bar);
         int spin = 0;
-        while ((int)((unsigned)v - target) < 0 && ++spin < kSpinLimit) v = ld_acquire_u64(bar);
+        while (v < target && ++spin < kSpinLimit) v = ld_acquire_u64(bar);
         __threadfence();
-        s_seen = v;
-        s_ok = (int)((unsigned)v - target) >= 0;
+        s_ok = v >= target;
     }
     __syncthreads();
-    seen = s_seen;
     return s_ok != 0;
+}
+
+// A virtual block's sum of one step as a 16-byte record that carries the step's number in both
+// halves, so that a reader knows from the record alone that the sum is the step's and that what the
+// writing block wrote before it is visible (after a fence of the reader's).
+__device__ __forceinline__ void cgs_publish(ulonglong2* p, const CgSum& t, unsigned step) {
+    const unsigned long long lo = (unsigned)t.m | (unsigned long long)(unsigned short)t.e << 32 |
+                                  (unsigned long long)(step & 0xffffu) << 48;
+    const unsigned long long hi = (unsigned)(t.m >> 32) | (unsigned long long)step << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+// waits for the record of `step`; false when the wait ran out
+__device__ __forceinline__ bool cgs_collect(const ulonglong2* p, unsigned step, CgSum& t) {
+    unsigned long long lo, hi;
+    int spin = 0;
+    do {
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+        if ((unsigned)(hi >> 32) == step && (unsigned)(lo >> 48) == (step & 0xffffu)) {
+            t.m = (long long)((unsigned long long)(unsigned)hi << 32 | (unsigned)lo);
+            t.e = (short)(lo >> 32);
+            return true;
+        }
+    } while (++spin < kSpinLimit);
+    t = CgSum{0, 0};
+    return false;
 }
 
 // a + b, aligned like the lanes of a warp sum
@@ -932,9 +963,9 @@ __device__ __forceinline__ CgSum cgs_add(CgSum a, CgSum b) {
 __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
     extern __shared__ float4 cg_dyn[];
     CgGridUnit* U = reinterpret_cast<CgGridUnit*>(cg_dyn);   // one per unit of the launch
-    __shared__ int4 s_w[2][kGridBlock / 32];
+    __shared__ int4 s_w[kGridPasses][kGridBlock / 32];   // warp sums of a step's passes
     __shared__ CgSum s_sum[kGridBlock / 32];
-    __shared__ int s_total;
+    __shared__ int s_total, s_late;   // s_late: a wait ran out
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int sub = tid / kVbGroups, subt = tid % kVbGroups;
     const int per = a.first - a.last + 1, nu = per * a.clouds;
@@ -982,62 +1013,109 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
         return lo;
     };
     const int u0 = v0 < v1 ? unit_of(v0) : 0, u1 = v0 < v1 ? unit_of(v1 - 1) + 1 : 0;
-    unsigned target = 0;
-    unsigned long long seen = 0;
-    int buf = 0;
+    // The records of a step (its number from 1) alternate between two buffers.  A block publishes a
+    // step's records after it has read all of the step before, so a record is overwritten (two steps
+    // later) only when every block of its unit has read it.
+    unsigned nstep = 0;
+    if (tid == 0) s_late = 0;
+    const size_t part_stride = (size_t)a.part_cap + kGridUnits;   // then a total per unit
+    for (int v = v0 + tid; v < v1; v += kGridBlock) a.part[v] = a.part[part_stride + v] = make_ulonglong2(0ull, 0ull);
+    for (int u = u0 + tid; u < u1; u += kGridBlock)
+        if (U[u].vb0 >= v0) a.part[a.part_cap + u] = a.part[part_stride + a.part_cap + u] = make_ulonglong2(0ull, 0ull);
 
-    // one step over the block's virtual blocks: body(unit, first group thread's G, local group, on)
-    // returns the thread's contribution; `skip(unit)`: the unit takes no part.  Ends with the grid
-    // barrier; the sums of the units are then in part[buf].
-    auto step = [&](bool active, auto skip, auto body) -> bool {
-        for (int p = 0; p < npass; ++p) {
-            const int vb = v0 + p * kGridSubs + sub;
-            FF acc = ff_zero();
-            int u = -1;
-            if (vb < v1) {
-                u = unit_of(vb);
-                if (skip(U[u])) u = -1;
+    // one step over the block's virtual blocks: body(unit, local group, pass) returns the thread's
+    // contribution; `skip(unit)`: the unit takes no part.  Publishes the virtual blocks' sums.
+    // `writes`: the step leaves vectors for other blocks; only then the records need fences.  (A step
+    // that does not only reads what other blocks may overwrite in the next one, and a record depends
+    // on every value its block read.)
+    bool fenced = true;
+    auto step = [&](bool writes, auto skip, auto body) {
+        ++nstep;
+        fenced = writes;
+        for (int p0 = 0; p0 < npass; p0 += kGridPasses) {
+            const int np = min(npass - p0, kGridPasses);
+            if (p0) __syncthreads();
+            for (int p = 0; p < np; ++p) {
+                const int vb = v0 + (p0 + p) * kGridSubs + sub;
+                FF acc = ff_zero();
+                int u = vb < v1 ? unit_of(vb) : -1;
+                if (u >= 0 && skip(U[u])) u = -1;
+                if (u >= 0) {
+                    const int g = (vb - U[u].vb0) * kVbGroups + subt;
+                    if (g < U[u].ng) acc = body(U[u], g, p0 + p);
+                }
+                int4 ws = make_int4(0, 0, 0, 0);
+                if (__any_sync(0xffffffffu, acc.hi != 0.0f)) ws = cgs_warp_sum(acc);
+                if (lane == 0) s_w[p][warp] = ws;
             }
-            if (u >= 0) {
-                const int g = (vb - U[u].vb0) * kVbGroups + subt;
-                if (g < U[u].ng) acc = body(U[u], g);
-            }
-            int4 ws = make_int4(0, 0, 0, 0);
-            if (__any_sync(0xffffffffu, acc.hi != 0.0f)) ws = cgs_warp_sum(acc);
-            if (lane == 0) s_w[p & 1][warp] = ws;
             __syncthreads();
-            if (u >= 0 && (warp & (kVbGroups / 32 - 1)) == 0) {
-                const CgSum t = cgs_warp_sum(cgs_join(lane < kVbGroups / 32 ? s_w[p & 1][warp + lane] : make_int4(0, 0, 0, 0)));
-                if (lane == 0) a.part[(size_t)buf * a.part_cap + vb] = t;
+            for (int q = warp; q < np * kGridSubs; q += kGridBlock / 32) {
+                const int p = q / kGridSubs, sb = q % kGridSubs, vb = v0 + (p0 + p) * kGridSubs + sb;
+                if (vb >= v1 || skip(U[unit_of(vb)])) continue;
+                constexpr int kWarps = kVbGroups / 32;
+                const CgSum t = cgs_warp_sum(cgs_join(lane < kWarps ? s_w[p][sb * kWarps + lane] : make_int4(0, 0, 0, 0)));
+                if (lane == 0) {
+                    if (fenced) fence_gpu();   // the block's writes of the step before its records
+                    cgs_publish(a.part + (nstep & 1) * part_stride + vb, t, nstep);
+                }
             }
         }
-        target += gridDim.x;
-        return grid_barrier(a.bar, target, active, seen);
     };
-    // the units' sums: a warp a unit, or the block where there are many virtual blocks (the order
-    // depends on the unit alone); post(unit, sum) by one thread
-    auto sums = [&](auto skip, auto post) {
-        const CgSum* part = a.part + (size_t)buf * a.part_cap;
-        for (int u = u0 + warp; u < u1; u += kGridBlock / 32) {
-            if (U[u].nvb > 32 || skip(U[u])) continue;
-            const CgSum t = cgs_warp_sum(lane < U[u].nvb ? part[U[u].vb0 + lane] : CgSum{0, 0});
-            if (lane == 0) post(U[u], t);
-        }
+    // Waits for the records of the units that took part in the step, which is also the barrier between
+    // the blocks of a unit, and adds them (the order depends on the unit alone); post(unit, sum) by
+    // one thread.  Of a unit with up to 32 virtual blocks a warp of every block reads all records; of
+    // a larger one the block that holds its first virtual block does and publishes the total (with
+    // 106 blocks polling 106 records each the wait took 7k cycles, so 4k).  False when a wait ran out.
+    auto sums = [&](auto skip, auto post) -> bool {
+        ulonglong2* part = a.part + (nstep & 1) * part_stride;
+        bool late = false;
         for (int u = u0; u < u1; ++u) {
-            if (U[u].nvb <= 32 || skip(U[u])) continue;   // the same in all threads: flags change below only
-            CgSum t{0, 0};
-            for (int v = tid; v < U[u].nvb; v += kGridBlock) t = cgs_add(t, part[U[u].vb0 + v]);
+            if (U[u].nvb <= 32 || U[u].vb0 < v0 || skip(U[u])) continue;   // the same in all threads
+            CgSum t{0, 0}, r;
+            for (int v = tid; v < U[u].nvb; v += kGridBlock) {
+                late |= !cgs_collect(part + U[u].vb0 + v, nstep, r);
+                t = cgs_add(t, r);
+            }
+            if (fenced && tid < U[u].nvb) fence_gpu();
             t = cgs_warp_sum(t);
             if (lane == 0) s_sum[warp] = t;
             __syncthreads();
             if (warp == 0) {
                 t = cgs_warp_sum(lane < kGridBlock / 32 ? s_sum[lane] : CgSum{0, 0});
-                if (lane == 0) post(U[u], t);
+                if (lane == 0) {
+                    if (fenced) fence_gpu();
+                    cgs_publish(part + a.part_cap + u, t, nstep);
+                }
             }
             __syncthreads();
         }
-        buf ^= 1;
+        for (int u = u0 + warp; u < u1; u += kGridBlock / 32) {
+            if (skip(U[u])) continue;
+            CgSum t{0, 0};
+            if (U[u].nvb <= 32) {
+                if (lane < U[u].nvb) late |= !cgs_collect(part + U[u].vb0 + lane, nstep, t);
+                if (fenced) fence_gpu();   // what the unit's other blocks wrote before their records
+                t = cgs_warp_sum(t);
+            } else if (lane == 0) {
+                late |= !cgs_collect(part + a.part_cap + u, nstep, t);
+                if (fenced) fence_gpu();
+            }
+            if (lane == 0) post(U[u], t);
+        }
+        if (late) s_late = 1;
         __syncthreads();
+        return s_late == 0;
+    };
+
+    // A p of a group, its rows `aps` apart: in shared memory for the first kGridApPasses passes
+    float* s_ap = reinterpret_cast<float*>(U + nu);
+    auto ap_of = [&](const CgGridUnit& q, int G, int pass, unsigned& aps) -> float* {
+        if (pass < kGridApPasses) {
+            aps = kGridBlock;
+            return s_ap + pass * 8 * kGridBlock + tid;
+        }
+        aps = a.pitch;
+        return at_cloud(a.ap, q.k) + G;
     };
 
     // neighbour groups; r0 = b, p_{-1} = 0, x0 = 0
@@ -1046,9 +1124,10 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             at_cloud(a.rp, k)[tid * a.pitch + a.pitch - 1] = make_float2(0.0f, 0.0f);
             at_cloud(a.xs, k)[tid * a.pitch + a.pitch - 1] = 0.0f;
         }
-    bool ok = step(
+    bool ok = grid_barrier(a.bar, gridDim.x);   // the cleared records and the zero group
+    step(
         true, [](const CgGridUnit&) { return false; },
-        [&](const CgGridUnit& q, int g) {
+        [&](const CgGridUnit& q, int g, int) {
             const int G = q.G0 + g;
             CgcVec v = a.v;
             v.neigh = at_cloud(a.v.neigh, q.k);
@@ -1076,20 +1155,21 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             }
             return acc;
         });
-    if (ok) sums([](const CgGridUnit&) { return false; }, [&](CgGridUnit& q, const CgSum& t) { cgc_start(q, a, t); q.check = 0; });
+    ok &= sums([](const CgGridUnit&) { return false; }, [&](CgGridUnit& q, const CgSum& t) { cgc_start(q, a, t); q.check = 0; });
     auto idle = [](const CgGridUnit& q) { return !q.go && !q.check; };
-    // a round per iteration and per true residual; two counts per round tell when none had work
+    // a round per iteration and per true residual, until none of the block's units has work
     const long long most = 2LL * a.max_iter + kCgMaxRefine + 8;
-    unsigned worked = (unsigned)(seen >> 32);
     long long round = 0;
     for (; ok && round < most; ++round) {
         bool active = false;
         for (int u = u0; u < u1; ++u) active |= !idle(U[u]);
+        if (!active) break;
         // (A) A p_k from the neighbours' (r_k, p_{k-1}), p.Ap; or the true residual b - A x
-        ok = step(active, idle, [&](CgGridUnit& q, int g) {
+        step(false, idle, [&](CgGridUnit& q, int g, int pass) {
             const int G = q.G0 + g;
             const int* nbg = at_cloud(a.nbg, q.k) + G;
-            float* ap = at_cloud(a.ap, q.k) + G;
+            unsigned aps;
+            float* ap = ap_of(q, G, pass, aps);
             FF acc = ff_zero();
             if (q.check) {
                 const float* xs = at_cloud(a.xs, q.k);
@@ -1124,7 +1204,7 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
 #pragma unroll
                 for (int s = 0; s < 8; ++s) {
                     const float ri = ff_to_float(ff_add(FF{b[s], 0.0f}, FF{-y[s].hi, -y[s].lo}));
-                    ap[s * a.pitch] = ri;
+                    ap[s * aps] = ri;
                     acc = ff_add(acc, ff_prod(ri, ri));
                 }
                 return acc;
@@ -1160,7 +1240,7 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             }
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
-                ap[s * a.pitch] = y[s];
+                ap[s * aps] = y[s];
                 acc = ff_add(acc, ff_prod(pi[s], y[s]));
             }
             // Only a unit's first group can have a table that does not name the group itself (its
@@ -1171,8 +1251,7 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             }
             return acc;
         });
-        if (!ok) break;
-        sums(idle, [&](CgGridUnit& q, const CgSum& t) {
+        ok = sums(idle, [&](CgGridUnit& q, const CgSum& t) {
             q.resid = q.check;
             if (q.check) {
                 cgc_after_true(q, a, t, q.it + 1);
@@ -1181,17 +1260,19 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
                 cgc_alpha(q, t);
             }
         });
+        if (!ok) break;
         // (B) x and r, r.r; after a true residual: the restart's r
         auto rest = [](const CgGridUnit& q) { return !q.go && !q.resid; };
-        ok = step(active, rest, [&](CgGridUnit& q, int g) {
+        step(true, rest, [&](CgGridUnit& q, int g, int pass) {
             const int G = q.G0 + g;
             float2* rp = at_cloud(a.rp, q.k) + G;
-            const float* ap = at_cloud(a.ap, q.k) + G;
+            unsigned aps;
+            const float* ap = ap_of(q, G, pass, aps);
             FF acc = ff_zero();
             if (q.resid) {
                 if (q.replace)
 #pragma unroll
-                    for (int s = 0; s < 8; ++s) rp[s * a.pitch].x = ap[s * a.pitch];
+                    for (int s = 0; s < 8; ++s) rp[s * a.pitch].x = ap[s * aps];
                 return acc;
             }
             float* xs = at_cloud(a.xs, q.k) + G;
@@ -1203,7 +1284,7 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             for (int s = 0; s < 8; ++s) {   // every load before the first store
                 own[s] = rp[s * a.pitch];
                 xo[s] = xs[s * a.pitch];
-                y[s] = ap[s * a.pitch];
+                y[s] = ap[s * aps];
             }
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
@@ -1215,16 +1296,13 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             }
             return acc;
         });
-        if (!ok) break;
-        sums([](const CgGridUnit& q) { return !q.go || q.resid; }, [&](CgGridUnit& q, const CgSum& t) {
-            ++q.it;
-            cgc_after_rr(q, a, t, q.it);
+        ok = sums(rest, [&](CgGridUnit& q, const CgSum& t) {
+            if (!q.resid) {
+                ++q.it;
+                cgc_after_rr(q, a, t, q.it);
+            }
+            q.resid = 0;
         });
-        for (int u = u0 + tid; u < u1; u += kGridBlock) U[u].resid = 0;
-        __syncthreads();
-        const unsigned w = (unsigned)(seen >> 32);
-        if (w == worked) break;   // no block had work in this round
-        worked = w;
     }
     if (tid == 0 && (!ok || round >= most)) atomicOr(err, kErrSpinTimeout);
     // x in row order; the reports by the block that holds a unit's first virtual block
@@ -1401,7 +1479,8 @@ void prepare_launch_configs(Workspace& ws) {
         if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgSmemBytes) !=
                 cudaSuccess ||
             cudaFuncSetAttribute(k_cg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(CgGridUnit) * kMaxBatchClouds * (kMaxDepth - kGridDepth + 1))) != cudaSuccess)
+                                 (int)(sizeof(CgGridUnit) * kMaxBatchClouds * (kMaxDepth - kGridDepth + 1) + kGridApBytes)) !=
+                cudaSuccess)
             return;   // left unset: the CG launch reports the error
         if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cudaLaunchConfig_t cfg = {};
@@ -1458,7 +1537,7 @@ static cudaError_t launch_cg_grid(Workspace& ws, const CgcArgs& a, cudaStream_t 
     L.rp = ws.cg_rp;
     L.xs = ws.cg_q;
     L.ap = ws.cg_ap;
-    L.part = reinterpret_cast<CgSum*>(ws.cg_part);
+    L.part = ws.cg_part;
     L.part_cap = ws.cg_part_cap;
     L.bar = &ws.cnt->grid_bar;
     L.tol2 = a.tol2;
@@ -1470,7 +1549,7 @@ static cudaError_t launch_cg_grid(Workspace& ws, const CgcArgs& a, cudaStream_t 
     if (grid < 1) grid = 1;
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kGridBlock);
-    cfg.dynamicSmemBytes = sizeof(CgGridUnit) * (size_t)(L.first - L.last + 1) * L.clouds;
+    cfg.dynamicSmemBytes = sizeof(CgGridUnit) * (size_t)(L.first - L.last + 1) * L.clouds + kGridApBytes;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

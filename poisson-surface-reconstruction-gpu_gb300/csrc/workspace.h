@@ -107,7 +107,7 @@ struct Workspace {
     float *cg_r, *cg_p, *cg_q, *cg_ap;   // residual, two direction buffers, A p (whole-GPU CG: x in cg_q)
     int* cg_nbg;            // [27][cap.nodes / 8 + 8]: neighbour groups of every sibling group (whole-GPU CG)
     float2* cg_rp;          // [8][cap.nodes / 8 + 8]: (r, p), sibling-major
-    longlong2* cg_part;     // [2][cg_part_cap]: sums of its virtual blocks
+    ulonglong2* cg_part;    // [2][cg_part_cap]: sums of its virtual blocks
     int cg_part_cap;
     unsigned* cg_desc;      // [14][cap.nodes / 8 + 8]: packed neighbour groups (solver.cu)
     double* cg_partial;     // scratch: divergence chunk sums (float pairs, 8 bytes each)
