@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kBlock) k_vector_field(const Counters* c, int 
     for (int o = group; o < md; o += ngroups) {
         const int i = b + o;
         const float ox = cx[i], oy = cy[i], oz = cz[i];
-        int running = 0;
+        int running = 0, used = 0;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int k = lane + kVfLanes * r;
@@ -69,19 +69,24 @@ __global__ void __launch_bounds__(kBlock) k_vector_field(const Counters* c, int 
                 const int y = __shfl_up_sync(gmask, incl, q, kVfLanes);
                 if (lane >= q) incl += y;
             }
-            if (k < 27) {
-                s_off[gib][k] = running + incl - cnt;
-                s_base[gib][k] = base;
+            // only neighbours with samples (a third of them), in slot order: where their samples start,
+            // and sample t is t + s_base
+            const unsigned some = __ballot_sync(gmask, cnt > 0) >> (threadIdx.x & 24);
+            if (cnt > 0) {
+                const int at = used + __popc(some & ((1u << lane) - 1u));
+                s_off[gib][at] = running + incl - cnt;
+                s_base[gib][at] = base - (running + incl - cnt);
             }
+            used += __popc(some & 0xffu);
             running += __shfl_sync(gmask, incl, kVfLanes - 1, kVfLanes);
         }
-        if (lane == 0) s_off[gib][27] = running;
+        if (lane == 0) s_off[gib][used] = 0x7fffffff;
         __syncwarp(gmask);
         float ax = 0.f, ay = 0.f, az = 0.f;
         int k = 0;
         for (int t = lane; t < running; t += kVfLanes) {
             while (s_off[gib][k + 1] <= t) ++k;
-            const int p = s_base[gib][k] + (t - s_off[gib][k]);
+            const int p = t + s_base[gib][k];
             const float w = bspline32((px[p] - ox) * s) * bspline32((py[p] - oy) * s) * bspline32((pz[p] - oz) * s);
             ax = fmaf(w, nx[p], ax);
             ay = fmaf(w, ny[p], ay);
@@ -160,7 +165,8 @@ __device__ __forceinline__ void div_leaf(const DivArgs& a) {
 
 // One warp per node for depths dsplit .. D-1.  The (neighbour, leaf) pairs of the node are
 // flattened over the lanes: lane k < 27 holds neighbour k's leaf range, a warp scan gives
-// the range offsets, and term t belongs to the last neighbour whose offset is <= t.
+// the range offsets, and term t belongs to the last neighbour whose offset is <= t.  Two thirds of
+// the neighbours have no leaves; the list leaves them out, since every lane walks all of it.
 __device__ __forceinline__ void div_fine(const DivArgs& a, int (*s_off)[33], int (*s_base)[32]) {
     const int b0 = a.c->level_base[a.dsplit];
     const int bD = a.c->level_base[a.depth];
@@ -184,15 +190,22 @@ __device__ __forceinline__ void div_fine(const DivArgs& a, int (*s_off)[33], int
             int y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += y;
         }
-        s_off[wib][lane] = incl - cnt;   // exclusive offset of neighbour `lane`
-        s_base[wib][lane] = base;
+        // only neighbours with leaves, in slot order: where their terms start, and the leaf of term t
+        // is t + s_base
+        const unsigned some = __ballot_sync(0xffffffffu, cnt > 0);
+        if (cnt > 0) {
+            const int at = __popc(some & ((1u << lane) - 1u));
+            s_off[wib][at] = incl - cnt;
+            s_base[wib][at] = base - (incl - cnt);
+        }
+        if (lane == 0) s_off[wib][__popc(some)] = 0x7fffffff;
         const int total = __shfl_sync(0xffffffffu, incl, 31);
         __syncwarp();
         FF sum = ff_zero();
         int k = 0;
         for (int t = lane; t < total; t += 32) {
-            while (k < 26 && s_off[wib][k + 1] <= t) ++k;   // terms are visited in increasing order
-            sum = ff_add_float(sum, div_term(a.leaf[s_base[wib][k] + (t - s_off[wib][k])], a.depth, rx, ry, rz));
+            while (s_off[wib][k + 1] <= t) ++k;   // terms are visited in increasing order
+            sum = ff_add_float(sum, div_term(a.leaf[t + s_base[wib][k]], a.depth, rx, ry, rz));
         }
         const FF acc = ff_warp_sum(sum);
         if (lane == 0) a.divg[i] = ff_to_float(acc);
@@ -208,44 +221,66 @@ __device__ __forceinline__ void div_chunks(const DivArgs& a) {
     const int lane = lane_id();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int it = warp; it < n_items; it += nwarps) {
-        // node owning this item: last node with item_start <= it; each step the lanes probe 32
-        // places of the range at once
-        int lo = 0, hi = n_nodes;   // item_start[lo] <= it < item_start[hi]
-        while (hi - lo > 1) {
-            const int step = (hi - lo + 31) >> 5;
-            const int at = lo + lane * step;
-            const unsigned m = __ballot_sync(0xffffffffu, at < hi && (int)a.item_start[at < hi ? at : lo] <= it);
-            const int last = 31 - __clz(m);   // lane 0 always holds
-            lo += last * step;
-            hi = min(hi, lo + step);
-        }
-        const int i = lo;
-        // the chunk's neighbour: lane k counts neighbour k's chunks
-        const int rem = it - (int)a.item_start[i];
-        int q = -1, dn = 0, di = 0;
-        if (lane < 27) {
-            q = a.neigh[(size_t)lane * a.stride + i];
-            if (q >= 0) { dn = a.dnum[q]; di = a.didx[q]; }
-        }
-        const int nc = (dn + kDivChunk - 1) / kDivChunk;
-        int incl = nc;
+    // a warp takes consecutive items: it looks for a node once and keeps its neighbours' ranges until
+    // the next node's items begin
+    const int per = (n_items + nwarps - 1) / nwarps;
+    const int it1 = min(n_items, (warp + 1) * per);
+    int i = -1, start = 0, next = 0;   // the node and its items
+    int dn = 0, di = 0, nc = 0, incl = 0;
+    const float *rx = a.dff, *ry = a.dff, *rz = a.dff;
+    for (int it = warp * per; it < it1; ++it) {
+        if (i < 0 || it >= next) {
+            int lo = 0, hi = n_nodes;   // item_start[lo] <= it < item_start[hi]
+            if (i >= 0) {   // the next nodes, 32 at once
+                while (true) {
+                    const int at = i + 1 + lane;
+                    const unsigned m = __ballot_sync(0xffffffffu, at < n_nodes && (int)a.item_start[at < n_nodes ? at : i] <= it);
+                    lo = i + __popc(m);
+                    if (m != 0xffffffffu) break;
+                    i += 32;
+                }
+                hi = lo + 1;
+            }
+            while (hi - lo > 1) {   // each step the lanes probe 32 places of the range at once
+                const int step = (hi - lo + 31) >> 5;
+                const int at = lo + lane * step;
+                const unsigned m = __ballot_sync(0xffffffffu, at < hi && (int)a.item_start[at < hi ? at : lo] <= it);
+                const int last = 31 - __clz(m);   // lane 0 always holds
+                lo += last * step;
+                hi = min(hi, lo + step);
+            }
+            i = lo;
+            start = (int)a.item_start[i];
+            next = i + 1 < n_nodes ? (int)a.item_start[i + 1] : n_items;
+            // lane k counts neighbour k's chunks
+            int q = -1;
+            dn = di = 0;
+            if (lane < 27) {
+                q = a.neigh[(size_t)lane * a.stride + i];
+                if (q >= 0) { dn = a.dnum[q]; di = a.didx[q]; }
+            }
+            nc = (dn + kDivChunk - 1) / kDivChunk;
+            incl = nc;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            int ox, oy, oz;
+            decode3(a.enc[i], a.depth, ox, oy, oz);
+            rx = a.dff + (size_t)a.res * ox;
+            ry = a.dff + (size_t)a.res * oy;
+            rz = a.dff + (size_t)a.res * oz;
         }
+        const int rem = it - start;
         const unsigned own = __ballot_sync(0xffffffffu, rem < incl);
         FF acc = ff_zero();
         if (own) {   // always
             const int k = __ffs(own) - 1;
             const int ch = rem - __shfl_sync(0xffffffffu, incl - nc, k);
             const int d0 = __shfl_sync(0xffffffffu, di, k), d1 = d0 + __shfl_sync(0xffffffffu, dn, k);
-            int ox, oy, oz;
-            decode3(a.enc[i], a.depth, ox, oy, oz);
             const int l0 = d0 + ch * kDivChunk;
             const int l1 = min(d1, l0 + kDivChunk);
-            const float *rx = a.dff + (size_t)a.res * ox, *ry = a.dff + (size_t)a.res * oy, *rz = a.dff + (size_t)a.res * oz;
             FF sum = ff_zero();
 #pragma unroll 4
             for (int l = l0 + lane; l < l1; l += 32) sum = ff_add_float(sum, div_term(a.leaf[l], a.depth, rx, ry, rz));

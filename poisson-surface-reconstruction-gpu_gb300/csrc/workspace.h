@@ -213,7 +213,7 @@ inline int grid_for(const Workspace& ws, long long work) {
 
 // coarse divergence: depths below div_split(D) are summed in chunks of kDivChunk leaves
 constexpr int kDivChunk = 512;
-inline int div_split(int D) { return D >= 2 ? D - 2 : 0; }
+inline int div_split(int D) { return D >= 8 ? 5 : (D >= 2 ? D - 2 : 0); }
 
 // stage entry points (each issues kernels on ws.stream; no host synchronisation)
 cudaError_t octree_build(Workspace& ws);
