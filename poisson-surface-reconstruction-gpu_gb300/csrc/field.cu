@@ -118,7 +118,8 @@ __device__ __forceinline__ void decode3(int e, int depth, int& ix, int& iy, int&
 // Term of a leaf (its field and its packed function index, one 16-byte record) for a node whose
 // rows of the function table are rx, ry, rz.  The parts below are bound by the latency of these
 // dependent loads: with the record one load instead of four separate ones, field and divergence
-// of a 2,000,000-sample depth-9 cloud take 2.49 ms instead of 2.62.
+// of a 2,000,000-sample depth-9 cloud take 2.49 ms instead of 2.62 (2.23 with the
+// empty neighbours left out and the chunks in runs, below).
 __device__ __forceinline__ float div_term(const float4 leaf, int depth, const float* rx, const float* ry,
                                           const float* rz) {
     int lx, ly, lz;
@@ -292,7 +293,9 @@ __device__ __forceinline__ void div_chunks(const DivArgs& a) {
 }
 
 // The three parts only read the vector field: one launch, blockIdx.z a part (the longest first).
-__global__ void __launch_bounds__(kBlock) k_divergence(DivArgs a) {
+// Bound by instruction issue (two thirds of the slots) once enough warps hide the table look-ups:
+// five blocks per SM, 48 registers (four: 2% slower at 500,000 samples, depth 9).
+__global__ void __launch_bounds__(kBlock, 5) k_divergence(DivArgs a) {
     __shared__ int s_off[kBlock / 32][33];
     __shared__ int s_base[kBlock / 32][32];
     a.rebase();

@@ -211,7 +211,11 @@ inline int grid_for(const Workspace& ws, long long work) {
     return (int)(g < 1 ? 1 : g);
 }
 
-// coarse divergence: depths below div_split(D) are summed in chunks of kDivChunk leaves
+// coarse divergence: depths below div_split(D) are summed in chunks of kDivChunk leaves, the others a
+// warp per node.  A chunk ends with its neighbour, so at depth 9 those of depth 6 hold 77 leaves each
+// (2,000,000 samples) and cost more to find than to add: from depth 8 on the line is at depth 5 (field
+// and divergence 2.45 ms; with it at D - 2 = 7 2.55 ms, at 4 2.64 ms, where a node's 12,000 terms take a
+// warp too long).  Trees of depth 7 keep D - 2 = 5 by the same measure.
 constexpr int kDivChunk = 512;
 inline int div_split(int D) { return D >= 8 ? 5 : (D >= 2 ? D - 2 : 0); }
 
