@@ -32,7 +32,7 @@ __device__ __forceinline__ float bspline32(float t) {
 // flattened over the group's lanes (a group scan gives the range offsets), every lane
 // accumulates its samples' weighted normals and a butterfly over the group combines the
 // lanes (fixed order).
-constexpr int kVfLanes = 8;
+constexpr int kVfLanes = 8;   // list_range8
 constexpr int kVfGroups = kBlock / kVfLanes;
 __global__ void __launch_bounds__(kBlock) k_vector_field(const Counters* c, int depth, const float* px, const float* py,
                                                          const float* pz, const float* nx, const float* ny,
@@ -63,22 +63,7 @@ __global__ void __launch_bounds__(kBlock) k_vector_field(const Counters* c, int 
                 const int nb = neigh[(size_t)k * stride + i];
                 if (nb >= 0) { base = pidx[nb]; cnt = pnum[nb]; }
             }
-            int incl = cnt;
-#pragma unroll
-            for (int q = 1; q < kVfLanes; q <<= 1) {
-                const int y = __shfl_up_sync(gmask, incl, q, kVfLanes);
-                if (lane >= q) incl += y;
-            }
-            // only neighbours with samples (a third of them), in slot order: where their samples start,
-            // and sample t is t + s_base
-            const unsigned some = __ballot_sync(gmask, cnt > 0) >> (threadIdx.x & 24);
-            if (cnt > 0) {
-                const int at = used + __popc(some & ((1u << lane) - 1u));
-                s_off[gib][at] = running + incl - cnt;
-                s_base[gib][at] = base - (running + incl - cnt);
-            }
-            used += __popc(some & 0xffu);
-            running += __shfl_sync(gmask, incl, kVfLanes - 1, kVfLanes);
+            list_range8(gmask, cnt, base, s_off[gib], s_base[gib], used, running);
         }
         if (lane == 0) s_off[gib][used] = 0x7fffffff;
         __syncwarp(gmask);

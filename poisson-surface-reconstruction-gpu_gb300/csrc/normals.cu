@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned
         for (int g = kNrmGridLevel; g >= kNrmNearCoarsest; --g) {   // uniform in the group
             const int G = 1 << g, up = kNrmGridLevel - g;
             const float w = 1.0f / (float)G;
-            int running = 0;
+            int running = 0, used = 0;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int k = lane + kNrmLanes * r;
@@ -180,19 +180,9 @@ __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned
                         cnt = cell_start[(size_t)(m + 1) << (3 * up)] - base;
                     }
                 }
-                int incl = cnt;
-#pragma unroll
-                for (int o = 1; o < kNrmLanes; o <<= 1) {
-                    const int y = __shfl_up_sync(gmask, incl, o, kNrmLanes);
-                    if (lane >= o) incl += y;
-                }
-                if (k < 27) {
-                    s_off[gib][k] = running + incl - cnt;
-                    s_base[gib][k] = base;
-                }
-                running += __shfl_sync(gmask, incl, kNrmLanes - 1, kNrmLanes);
+                list_range8(gmask, cnt, base, s_off[gib], s_base[gib], used, running);
             }
-            if (lane == 0) s_off[gib][27] = running;
+            if (lane == 0) s_off[gib][used] = 0x7fffffff;
             __syncwarp(gmask);
             if (running > kNrmNearCap) break;
             if (running < kNrmK && running < n) continue;   // the K-th is farther out
@@ -203,7 +193,7 @@ __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned
             int k = 0;
             for (int t = lane; t < running; t += kNrmLanes) {
                 while (s_off[gib][k + 1] <= t) ++k;
-                nrm_visit(qx, qy, qz, px, py, pz, s_base[gib][k] + (t - s_off[gib][k]), bd, bi);
+                nrm_visit(qx, qy, qz, px, py, pz, t + s_base[gib][k], bd, bi);
             }
             __syncwarp(gmask);
             float md[kNrmK];
