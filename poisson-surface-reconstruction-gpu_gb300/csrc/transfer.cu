@@ -116,6 +116,39 @@ __device__ __forceinline__ unsigned spread3(unsigned v) {
     return v;
 }
 
+// the 4 nearest of a group's 8 lanes (mask gmask): four rounds of the minimum head, its lane popping it
+__device__ __forceinline__ void knn_group_merge(float (&bd)[4], int (&bi)[4], float (&md)[4], int (&mi)[4],
+                                                unsigned gmask) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        float d = bd[0];
+        int i = bi[0];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            const float od = __shfl_xor_sync(gmask, d, o);
+            const int oi = __shfl_xor_sync(gmask, i, o);
+            if (knn_less(od, oi, d, i)) { d = od; i = oi; }
+        }
+        md[r] = d;
+        mi[r] = i;
+        if (bd[0] == d && bi[0] == i) {
+            bd[0] = bd[1]; bi[0] = bi[1];
+            bd[1] = bd[2]; bi[1] = bi[2];
+            bd[2] = bd[3]; bi[2] = bi[3];
+            bd[3] = 1e6f; bi[3] = 0x7fffffff;
+        }
+    }
+}
+
+// Squared distance from q to the cell from (lx, ly, lz) to (lx + w, ..), in the operations of a
+// sample's distance: rounding is monotone, so no sample of the closed cell has a smaller one.
+__device__ __forceinline__ float box_distance2(float qx, float qy, float qz, float lx, float ly, float lz, float w) {
+    const float dx = fmaxf(fmaxf(__fsub_rn(lx, qx), __fsub_rn(qx, lx + w)), 0.0f);
+    const float dy = fmaxf(fmaxf(__fsub_rn(ly, qy), __fsub_rn(qy, ly + w)), 0.0f);
+    const float dz = fmaxf(fmaxf(__fsub_rn(lz, qz), __fsub_rn(qz, lz + w)), 0.0f);
+    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+}
+
 // Near pass, 8 lanes per mesh vertex: the samples of the 3x3x3 block of cells around the vertex's
 // cell (every sample outside it is at least one cell width away), spread over the group's lanes
 // (flattened over the 27 cell ranges), each lane keeping a sorted 4-list, merged by warp-minimum
@@ -125,12 +158,17 @@ __device__ __forceinline__ unsigned spread3(unsigned v) {
 // m << 3 (gt - g) .. (m + 1) << 3 (gt - g)): a sparse cloud's vertices find their samples there.
 // Coarser blocks of more than kNearCoarseCap samples, and what level kNearCoarsest leaves, go to the
 // far list with the smallest bound found, for the wide search (k_colour_far).  Blocks with fewer
-// than 4 samples are not scanned.  With the finest level alone below depth 8, a depth-7 cloud of
+// than 4 samples are not scanned.  A block of more than kNearPruneMin is searched from the inside:
+// the vertex's own cell first, then the cells whose box is not farther than the 4th nearest found
+// there (500,000 samples, depth 9, about 400 in a block: transfer 552 -> 401 us; issue-bound, so
+// visits saved count; below the line the second merge costs what the visits give: 200,000 samples,
+// depth 7, 71 us without, 75 with the line at 64, 72 at 128).  With the finest level alone below depth 8, a depth-7 cloud of
 // 61k points (96k mesh vertices) spent 458 us in the wide search.
 constexpr int kNearLanes = 8;
 constexpr int kNearGroups = kBlock / kNearLanes;
 constexpr int kNearCoarseCap = 512;   // samples a coarser level scans per vertex at most
 constexpr int kNearCoarsest = 4;
+constexpr int kNearPruneMin = 128;
 __global__ void __launch_bounds__(kBlock) k_colour_near(Counters* c, int gt, const float* mv, const float* px,
                                                         const float* py, const float* pz, const float* cr,
                                                         const float* cg, const float* cb, const int* cell_start,
@@ -154,73 +192,72 @@ __global__ void __launch_bounds__(kBlock) k_colour_near(Counters* c, int gt, con
             const int cx = min(max((int)floorf(qx * G), 0), G - 1);
             const int cy = min(max((int)floorf(qy * G), 0), G - 1);
             const int cz = min(max((int)floorf(qz * G), 0), G - 1);
-            // cells k = lane + 8 r, offsets in k order
-            int running = 0;
+            // cells k = lane + 8 r
+            int cnt[4], base[4], total = 0;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int k = lane + kNearLanes * r;
-                int cnt = 0, base = 0;
+                cnt[r] = base[r] = 0;
                 if (k < 27) {
                     const int a = cx + k / 9 - 1, b = cy + (k / 3) % 3 - 1, z = cz + k % 3 - 1;
                     if (a >= 0 && a < G && b >= 0 && b < G && z >= 0 && z < G) {
                         const unsigned m = (spread3((unsigned)a) << 2) | (spread3((unsigned)b) << 1) | spread3((unsigned)z);
-                        base = cell_start[(size_t)m << shift];
-                        cnt = cell_start[(size_t)(m + 1) << shift] - base;
+                        base[r] = cell_start[(size_t)m << shift];
+                        cnt[r] = cell_start[(size_t)(m + 1) << shift] - base[r];
                     }
                 }
-                int incl = cnt;
-#pragma unroll
-                for (int o = 1; o < kNearLanes; o <<= 1) {
-                    const int y = __shfl_up_sync(gmask, incl, o, kNearLanes);
-                    if (lane >= o) incl += y;
-                }
-                if (k < 27) {
-                    s_off[gib][k] = running + incl - cnt;
-                    s_base[gib][k] = base;
-                }
-                running += __shfl_sync(gmask, incl, kNearLanes - 1, kNearLanes);
+                total += cnt[r];
             }
-            if (lane == 0) s_off[gib][27] = running;
-            __syncwarp(gmask);
-            if (g < gt && running > kNearCoarseCap) break;   // a crowded block: left to the wide search
-            if (running < 4) continue;
+#pragma unroll
+            for (int o = kNearLanes / 2; o > 0; o >>= 1) total += __shfl_xor_sync(gmask, total, o);
+            if (g < gt && total > kNearCoarseCap) break;   // a crowded block: left to the wide search
+            if (total < 4) continue;
             float bd[4] = {1e6f, 1e6f, 1e6f, 1e6f};
             int bi[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
-            int k = 0;
-            for (int t = lane; t < running; t += kNearLanes) {
-                while (s_off[gib][k + 1] <= t) ++k;   // flattened index -> cell (increasing)
-                knn_visit(qx, qy, qz, px, py, pz, s_base[gib][k] + (t - s_off[gib][k]), bd, bi);
+            float md[4] = {1e6f, 1e6f, 1e6f, 1e6f};
+            int mi[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
+            const bool prune = total > kNearPruneMin;
+            if (prune) {
+                // the vertex's own cell first: its 4 nearest bound the others
+                const int c0 = __shfl_sync(gmask, cnt[1], 13 - kNearLanes, kNearLanes);
+                const int b0 = __shfl_sync(gmask, base[1], 13 - kNearLanes, kNearLanes);
+                for (int t = lane; t < c0; t += kNearLanes) knn_visit(qx, qy, qz, px, py, pz, b0 + t, bd, bi);
+                knn_group_merge(bd, bi, md, mi, gmask);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {   // one lane keeps them, the others start again
+                    bd[q] = lane == 0 ? md[q] : 1e6f;
+                    bi[q] = lane == 0 ? mi[q] : 0x7fffffff;
+                }
             }
-            __syncwarp(gmask);
-            // the group's 4 nearest: four rounds of the minimum head, its lane popping it
-            float md[4];
-            int mi[4];
+            int running = 0, used = 0;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                float d = bd[0];
-                int i = bi[0];
-#pragma unroll
-                for (int o = kNearLanes / 2; o > 0; o >>= 1) {
-                    const float od = __shfl_xor_sync(gmask, d, o);
-                    const int oi = __shfl_xor_sync(gmask, i, o);
-                    if (knn_less(od, oi, d, i)) { d = od; i = oi; }
+                const int k = lane + kNearLanes * r;
+                if (prune && cnt[r] > 0) {
+                    const float d2 = box_distance2(qx, qy, qz, (float)(cx + k / 9 - 1) * w, (float)(cy + (k / 3) % 3 - 1) * w,
+                                                   (float)(cz + k % 3 - 1) * w, w);
+                    if (k == 13 || d2 > md[3]) cnt[r] = 0;
                 }
-                md[r] = d;
-                mi[r] = i;
-                if (bd[0] == d && bi[0] == i) {
-                    bd[0] = bd[1]; bi[0] = bi[1];
-                    bd[1] = bd[2]; bi[1] = bi[2];
-                    bd[2] = bd[3]; bi[2] = bi[3];
-                    bd[3] = 1e6f; bi[3] = 0x7fffffff;
-                }
+                list_range8(gmask, cnt[r], base[r], s_off[gib], s_base[gib], used, running);
             }
+            if (lane == 0) s_off[gib][used] = 0x7fffffff;
+            __syncwarp(gmask);
+            int k = 0;
+            const float d4 = md[3];
+            const int i4 = mi[3];
+            for (int t = lane; t < running; t += kNearLanes) {
+                while (s_off[gib][k + 1] <= t) ++k;   // flattened index -> cell (increasing)
+                knn_visit_below(qx, qy, qz, px, py, pz, t + s_base[gib][k], d4, i4, bd, bi);
+            }
+            __syncwarp(gmask);
+            if (running > 0) knn_group_merge(bd, bi, md, mi, gmask);
             bound = fminf(bound, md[3]);
             if (md[3] < w * w) {
                 if (lane == 0) colour_blend(md, mi, cr, cg, cb, &out[3 * (size_t)v]);
                 settled = true;
                 break;
             }
-            if (running == n) break;   // every sample seen
+            if (total == n) break;   // every sample seen
         }
         if (!settled && lane == 0) {
             const int slot = atomicAdd(far_count, 1);
