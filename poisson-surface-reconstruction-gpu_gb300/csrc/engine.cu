@@ -433,6 +433,10 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     }
     h->arena_bytes = A.bytes;
     A.assign((char*)h->arena);
+    if (cfg.max_depth >= 8) {   // from cg_r to cg_rp: free once the CG is done
+        ws.value_rows = (float4*)ws.cg_r;
+        ws.cap_rows = (int)(((char*)ws.cg_part - (char*)ws.cg_r) / (8 * sizeof(float4)));
+    }
     ws.xsol += 64;
     set_batch(ws, 1);
     ws.cg_ctas = cfg.cg_cluster_ctas;

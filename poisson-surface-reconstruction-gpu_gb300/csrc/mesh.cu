@@ -436,6 +436,47 @@ __global__ void __launch_bounds__(kBlock) k_vertex_values(const Counters* c, int
     }
 }
 
+// The same for trees of depth 8 and 9, where the kernel is bound by instruction issue: the chain's
+// nodes above depth D come from their value rows.
+__global__ void __launch_bounds__(kBlock, 3) k_vertex_values_rows(const Counters* c, int depth, const float* vx,
+                                                                  const float* vy, const float* vz, const int* vowner,
+                                                                  const int* vkind, const int* vdepth, ValueRows R,
+                                                                  float* vvalue) {
+    PSR_CLOUD(c, vx, vy, vz, vowner, vkind, vdepth, R, vvalue);
+    R.n = min(c->level_base[depth], R.n);
+    const int V = c->n_vertices;
+    const float iso = c->iso;
+    PSR_GRID_STRIDE(v, V) {
+        float val = 0.0f;
+        const int ow = vowner[v];
+        if (ow > 0) {
+            const float qx = vx[v], qy = vy[v], qz = vz[v];
+            const int ec = __ldg(&g_tab.children_vertex_kind[vkind[v]]);
+            int d = vdepth[v];
+            bool up = true;
+            ValueRow cur, nxt;
+            load_row(R, ow, cur);
+            const int fc_ow = cur.first_child;
+            while (true) {
+                int nx;
+                if (up && cur.parent != -1) {
+                    nx = cur.parent;
+                } else {
+                    const int f = up ? fc_ow : cur.first_child;
+                    up = false;
+                    nx = (d < depth && f != -1) ? f + ec : -1;
+                    if (nx != -1) ++d;
+                }
+                load_row(R, nx != -1 ? nx : 0, nxt);   // in flight during the terms
+                val = terms_from(cur.enc, cur.x, val, qx, qy, qz, depth);
+                if (nx == -1) break;
+                cur = nxt;
+            }
+        }
+        vvalue[v] = __fsub_rn(val, iso);
+    }
+}
+
 // ------------------------------------------------------------------------------------
 // marching cubes at depth D (mesh/ComputeTriangleIndices.cu:401-526)
 // ------------------------------------------------------------------------------------
@@ -1441,60 +1482,51 @@ __global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* 
 // the current one's values are in flight.
 __global__ void __launch_bounds__(kBlock) k_sub_vertex_values_wide(const Counters* c, int depth, const float* vx,
                                                                    const float* vy, const float* vz, const int* vowner,
-                                                                   const int* neigh, size_t stride, const int* parent,
-                                                                   const int* root_self, SubArrays A,
-                                                                   const int* enc, const float* x, float* vvalue, int na) {
-    PSR_CLOUD(c, vx, vy, vz, vowner, neigh, parent, root_self, A, enc, x, vvalue);
+                                                                   const int* root_self, SubArrays A, ValueRows R,
+                                                                   float* vvalue, int na) {
+    PSR_CLOUD(c, vx, vy, vz, vowner, root_self, A, R, vvalue);
+    R.n = min(c->level_base[depth], R.n);
     const int V = c->n_sub_vertices;
     const float iso = c->iso;
     const int lb = c->sub_lbase[depth];
     PSR_GRID_STRIDE(v, V) {
         const float qx = vx[v], qy = vy[v], qz = vz[v];
-        const int own = lb + vowner[v];
-        // levels: subdivision nodes through the jump links, then the octree ancestors
-        int node = A.jump[own];
-        bool sub = true;
-        int nbs[27];
-#pragma unroll
-        for (int k = 0; k < 27; ++k) nbs[k] = A.neigh[(size_t)k * A.cap_live + node];
+        // subdivision nodes through the jump links
         float val = 0.0f;
-        for (int level = 0; level <= kMaxDepth; ++level) {
-            int ox, oy, oz, d, next;
-            bool next_sub = false;
-            if (sub) {
-                const float4 q = A.pos[node];
-                d = __float_as_int(q.w);
-                const float sc = (float)(1 << d);
-                const int base = (1 << d) - 1;
-                ox = base + (int)__fmul_rn(q.x, sc);
-                oy = base + (int)__fmul_rn(q.y, sc);
-                oz = base + (int)__fmul_rn(q.z, sc);
-                const int p = A.rec[node].x;
-                const int shift = p < 0 ? sub_root_shift(c, d) - na : 0;
+        int node = A.jump[lb + vowner[v]], now;
+        while (true) {
+            int nbs[27];
 #pragma unroll
-                for (int k = 0; k < 27; ++k)
-                    if (nbs[k] >= na) nbs[k] = p < 0 ? root_self[nbs[k] + shift] : -1;
-                next_sub = p >= 0;
-                next = next_sub ? A.jump[p] : -2 - p;
-            } else {
-                decode_fn_index(enc[node], depth, ox, oy, oz);
-                d = ilog2_dev(ox + 1);
-                next = parent[node];
-            }
+            for (int k = 0; k < 27; ++k) nbs[k] = A.neigh[(size_t)k * A.cap_live + node];
+            const float4 q = A.pos[node];
+            const int p = A.rec[node].x;
+            const int next = p >= 0 ? A.jump[p] : 0;
+            const int d = __float_as_int(q.w);
+            const float sc = (float)(1 << d);
+            const int base = (1 << d) - 1;
+            const int shift = p < 0 ? sub_root_shift(c, d) - na : 0;
+#pragma unroll
+            for (int k = 0; k < 27; ++k)
+                if (nbs[k] >= na) nbs[k] = p < 0 ? root_self[nbs[k] + shift] : -1;
             float xv[27];
 #pragma unroll
-            for (int k = 0; k < 27; ++k) xv[k] = x[nbs[k]];
-            int nb2[27];
-            const int* row = next_sub ? A.neigh + next : neigh + (next >= 0 ? next : 0);
-            const size_t rstride = next_sub ? (size_t)A.cap_live : stride;
-#pragma unroll
-            for (int k = 0; k < 27; ++k) nb2[k] = row[(size_t)k * rstride];
-            val = terms_at(ox, oy, oz, d, xv, val, qx, qy, qz);
-            if (next < 0) break;
-#pragma unroll
-            for (int k = 0; k < 27; ++k) nbs[k] = nb2[k];
+            for (int k = 0; k < 27; ++k) xv[k] = R.x[nbs[k]];
+            val = terms_at(base + (int)__fmul_rn(q.x, sc), base + (int)__fmul_rn(q.y, sc), base + (int)__fmul_rn(q.z, sc),
+                           d, xv, val, qx, qy, qz);
+            now = -2 - p;
+            if (p < 0) break;
             node = next;
-            sub = next_sub;
+        }
+        // then the octree ancestors
+        if (now >= 0) {
+            ValueRow cur, nxt;
+            load_row(R, now, cur);
+            while (true) {
+                load_row(R, cur.parent >= 0 ? cur.parent : 0, nxt);
+                val = terms_from(cur.enc, cur.x, val, qx, qy, qz, depth);
+                if (cur.parent < 0) break;
+                cur = nxt;
+            }
         }
         vvalue[v] = __fsub_rn(val, iso);
     }
@@ -1803,8 +1835,12 @@ cudaError_t mesh_build_impl(Workspace& ws, const MeshBufs& mb) {
     const int gm = grid_for(ws, ws.cap.nodes);
     cudaError_t e;
     // implicit values
-    k_vertex_values<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, D, ws.v_x, ws.v_y, ws.v_z, ws.v_owner, ws.v_kind, ws.v_depth, ws.neigh,
-                                          stride, ws.parent, ws.first_child, ws.enc, ws.xsol, ws.vvalue);
+    if (D >= 8)
+        k_vertex_values_rows<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, D, ws.v_x, ws.v_y, ws.v_z, ws.v_owner, ws.v_kind,
+                                                                 ws.v_depth, value_rows(ws), ws.vvalue);
+    else
+        k_vertex_values<<<PSR_GRID(ws, gm), kBlock, 0, s>>>(c, D, ws.v_x, ws.v_y, ws.v_z, ws.v_owner, ws.v_kind, ws.v_depth, ws.neigh,
+                                              stride, ws.parent, ws.first_child, ws.enc, ws.xsol, ws.vvalue);
     // crossings -> staged vertices of the main part
     e = launch_scan<1>(CrossLoad{ws.e_owner, ws.e_kind, ws.node_vtx, stride, ws.vvalue, err},
                     CrossStore{ws.e_owner, ws.e_kind, ws.node_vtx, stride, ws.vvalue, ws.v_x, ws.v_y, ws.v_z,
@@ -1883,8 +1919,7 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
                                                           ws.se_owner, ws.se_kind, ws.s_edge);
     if (D >= 8)
         k_sub_vertex_values_wide<<<PSR_GRID(ws, 8 * ws.num_sms), kBlock, 0, s>>>(
-            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, ws.root_self, A, ws.enc,
-            ws.xsol, ws.sv_value, na);
+            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.root_self, A, value_rows(ws), ws.sv_value, na);
     else
         k_sub_vertex_values<<<PSR_GRID(ws, 16 * ws.num_sms), kSvBlock, 0, s>>>(
             c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, ws.root_self, A, ws.enc,

@@ -284,6 +284,48 @@ __device__ __forceinline__ float level_terms(int node, float val, float qx, floa
     return terms_from(e, xv, val, qx, qy, qz, depth);
 }
 
+// Value rows (trees of depth 8 and 9): per node above the finest depth one 128-byte line with the 27
+// values of its neighbourhood, its function index, parent and first child.  A chain of ancestors then
+// costs 8 loads a level instead of 54 and their addresses.
+struct ValueRows {
+    const float4* rows;   // 8 per node
+    int n;                // nodes 0 .. n - 1 have one
+    const int* neigh;     // the tables the others are read from
+    size_t stride;
+    const int *parent, *first_child, *enc;
+    const float* x;
+    __device__ void rebase() { PSR_CLOUD(rows, neigh, parent, first_child, enc, x); }   // to cloud blockIdx.y
+};
+struct ValueRow {
+    float x[27];
+    int enc, parent, first_child;
+};
+__device__ __forceinline__ void load_row(const ValueRows& R, int node, ValueRow& o) {
+    if (node < R.n) {
+        const float4* p = R.rows + 8 * (size_t)node;
+        float4 q[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) q[j] = __ldg(p + j);
+#pragma unroll
+        for (int k = 0; k < 27; ++k) {
+            const float4& t = q[k >> 2];
+            o.x[k] = (k & 3) == 0 ? t.x : (k & 3) == 1 ? t.y : (k & 3) == 2 ? t.z : t.w;
+        }
+        o.enc = __float_as_int(q[6].w);
+        o.parent = __float_as_int(q[7].x);
+        o.first_child = __float_as_int(q[7].y);
+    } else {
+        int nb[27];
+#pragma unroll
+        for (int k = 0; k < 27; ++k) nb[k] = __ldg(R.neigh + (size_t)k * R.stride + node);
+        o.enc = __ldg(R.enc + node);
+        o.parent = __ldg(R.parent + node);
+        o.first_child = __ldg(R.first_child + node);
+#pragma unroll
+        for (int k = 0; k < 27; ++k) o.x[k] = __ldg(R.x + nb[k]);
+    }
+}
+
 // ---- Bernstein form of the implicit function on a cell --------------------------------
 // On a cell inside one cell of level l, every level-l translate b((x - c) 2^l) is a single
 // quadratic piece; with s in [-1, 1] across the cell (half width h) it is

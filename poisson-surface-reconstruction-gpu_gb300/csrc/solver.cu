@@ -1346,30 +1346,65 @@ __device__ __forceinline__ void decode3s(int e, int depth, int& ix, int& iy, int
 // (k_point_values_coarse; the partial sum is kept in `out`).  The depth-D terms are added
 // after the depth-D CG (k_point_values).  The iso-value is the FP64 mean of these float
 // values.
+// The value rows of the nodes above the finest depth (ValueRows), one thread per node; the rows go
+// out through shared memory, eight lanes a line.  Bound by its 54 reads a node.
+constexpr int kRowPitch = 36;   // floats: 16-byte aligned, rows on different banks
+__global__ void __launch_bounds__(kBlock) k_value_rows(const Counters* c, int depth, ValueRows R, float4* rows) {
+    PSR_CLOUD(c, R, rows);
+    __shared__ float s_row[kBlock / 32][32 * kRowPitch];
+    const int n = min(c->level_base[depth], R.n);
+    const int lane = lane_id();
+    float* buf = s_row[threadIdx.x >> 5];
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; b < n; b += gridDim.x * blockDim.x) {
+        const int node = b + lane;
+        if (node < n) {
+            int nb[27];
+#pragma unroll
+            for (int k = 0; k < 27; ++k) nb[k] = R.neigh[(size_t)k * R.stride + node];
+            float* o = buf + lane * kRowPitch;
+            o[27] = __int_as_float(R.enc[node]);
+            o[28] = __int_as_float(R.parent[node]);
+            o[29] = __int_as_float(R.first_child[node]);
+            o[30] = o[31] = 0.0f;
+            float xv[27];
+#pragma unroll
+            for (int k = 0; k < 27; ++k) xv[k] = R.x[nb[k]];
+#pragma unroll
+            for (int k = 0; k < 27; ++k) o[k] = xv[k];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int r = 4 * j + (lane >> 3);
+            if (b + r < n) rows[8 * (size_t)(b + r) + (lane & 7)] = *reinterpret_cast<const float4*>(buf + r * kRowPitch + 4 * (lane & 7));
+        }
+        __syncwarp();
+    }
+}
+
+template <bool kRows>
 __global__ void __launch_bounds__(kBlock) k_point_poly(const Counters* c, int depth, const float* ctr_x,
-                                                       const float* ctr_y, const float* ctr_z, const int* neigh,
-                                                       size_t stride, const int* parent, const int* enc,
-                                                       const float* x, float* coef, size_t cstride) {
-    PSR_CLOUD(c, ctr_x, ctr_y, ctr_z, neigh, parent, enc, x, coef);
+                                                       const float* ctr_y, const float* ctr_z, ValueRows R,
+                                                       float* coef, size_t cstride) {
+    PSR_CLOUD(c, ctr_x, ctr_y, ctr_z, R, coef);
+    R.n = kRows ? min(c->level_base[depth], R.n) : 0;
     const int d1 = depth - 1;
     const int n = c->level_count[d1];
     const int b = c->level_base[d1];
     PSR_GRID_STRIDE(a, n) {
         const int node = b + a;
         const float qx = ctr_x[node], qy = ctr_y[node], qz = ctr_z[node];
-        float C[27], y[27], mag = 0.0f;
+        float C[27], mag = 0.0f;
 #pragma unroll
         for (int k = 0; k < 27; ++k) C[k] = 0.0f;
-        for (int now = node; now >= 0; now = parent[now]) {
+        for (int now = node; now >= 0;) {
+            ValueRow r;
+            load_row(R, now, r);
             int ox, oy, oz;
-            decode3s(enc[now], depth, ox, oy, oz);
+            decode3s(r.enc, depth, ox, oy, oz);
             const int l = ilog2_dev(ox + 1);
-#pragma unroll
-            for (int k = 0; k < 27; ++k) {
-                const int v = neigh[(size_t)k * stride + now];
-                y[k] = (v >= 0) ? x[v] : 0.0f;
-            }
-            sign_level(y, ox, oy, oz, qx, qy, qz, __int_as_float((127 + l - depth) << 23), C, mag);   // h 2^l
+            now = r.parent;
+            sign_level(r.x, ox, oy, oz, qx, qy, qz, __int_as_float((127 + l - depth) << 23), C, mag);   // h 2^l
         }
 #pragma unroll
         for (int k = 0; k < 27; ++k) coef[(size_t)k * cstride + a] = C[k];
@@ -1603,10 +1638,16 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     const PointCoarse coarse{ws.parent, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.pv_coef, cstride};
     const int nb = ws.num_sms * 4;
     // sample values of all levels and the iso-value, once every depth is solved
+    const ValueRows rows = value_rows(ws);
     auto sample_values = [&]() {
-        k_point_poly<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, s>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.neigh,
-                                                                     (size_t)ws.cap.nodes, ws.parent, ws.enc, ws.xsol,
-                                                                     ws.pv_coef, cstride);
+        if (whole) {
+            k_value_rows<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, s>>>(ws.cnt, D, rows, ws.value_rows);
+            k_point_poly<true><<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, s>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z,
+                                                                               rows, ws.pv_coef, cstride);
+        } else {
+            k_point_poly<false><<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, s>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z,
+                                                                                rows, ws.pv_coef, cstride);
+        }
         k_point_values<true><<<PSR_GRID(ws, nb), kBlock, 0, s>>>(ws.cnt, ws.depth, ws.px, ws.py, ws.pz, ws.point2node,
                                                                  ws.neigh, (size_t)ws.cap.nodes, ws.enc, ws.xsol, coarse,
                                                                  ws.point_val, ws.iso_partial);
@@ -1660,9 +1701,8 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     // solved, beside the depth-D CG
     if (ncl > 1) e = cudaStreamWaitEvent(ws.aux, ws.ev_join3, 0);
     if (e == cudaSuccess) {
-        k_point_poly<<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, ws.aux>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.neigh,
-                                                            (size_t)ws.cap.nodes, ws.parent, ws.enc, ws.xsol,
-                                                            ws.pv_coef, cstride);
+        k_point_poly<false><<<PSR_GRID(ws, ws.num_sms * 4), kBlock, 0, ws.aux>>>(ws.cnt, D, ws.ctr_x, ws.ctr_y, ws.ctr_z,
+                                                                                 rows, ws.pv_coef, cstride);
         k_point_values_coarse<<<PSR_GRID(ws, nb), kBlock, 0, ws.aux>>>(ws.cnt, D, ws.px, ws.py, ws.pz, ws.point2node, coarse,
                                                                        ws.point_val);
         e = cudaEventRecord(ws.ev_join, ws.aux);

@@ -107,6 +107,8 @@ struct Workspace {
     float *cg_r, *cg_p, *cg_q, *cg_ap;   // residual, two direction buffers, A p (whole-GPU CG: x in cg_q)
     int* cg_nbg;            // [27][cap.nodes / 8 + 8]: neighbour groups of every sibling group (whole-GPU CG)
     float2* cg_rp;          // [8][cap.nodes / 8 + 8]: (r, p), sibling-major
+    float4* value_rows;     // after the CG of a tree of depth 8 or 9, in its vectors: [8] per node (ValueRows)
+    int cap_rows;
     ulonglong2* cg_part;    // [2][cg_part_cap]: sums of its virtual blocks
     int cg_part_cap;
     unsigned* cg_desc;      // [14][cap.nodes / 8 + 8]: packed neighbour groups (solver.cu)
@@ -218,6 +220,10 @@ inline int grid_for(const Workspace& ws, long long work) {
 // warp too long).  Trees of depth 7 keep D - 2 = 5 by the same measure.
 constexpr int kDivChunk = 512;
 inline int div_split(int D) { return D >= 8 ? 5 : (D >= 2 ? D - 2 : 0); }
+
+inline ValueRows value_rows(const Workspace& ws) {
+    return ValueRows{ws.value_rows, ws.cap_rows, ws.neigh, (size_t)ws.cap.nodes, ws.parent, ws.first_child, ws.enc, ws.xsol};
+}
 
 // stage entry points (each issues kernels on ws.stream; no host synchronisation)
 cudaError_t octree_build(Workspace& ws);
