@@ -992,26 +992,22 @@ __device__ __forceinline__ int sub_first_root(const Counters* c, int d) {
 // a root's number less this is its index among the roots of depth d
 __device__ __forceinline__ int sub_root_shift(const Counters* c, int d) { return c->sub_rstart[d] - sub_first_root(c, d); }
 
-// Neighbour rows of the live entries e0 .. e0 + n - 1 (n <= 32) of depth d, whose depth is complete
-// (computeRebuildNeighbor :669-696): lane p of every warp works on entry e0 + p, the block's 8 warps
-// share the 27 slots, and found(slot, p, record, neighbour) gets each.  A neighbour is a child of one
-// of the parent's neighbours: of an octree node its octree child (or, for a root, the root of the
+// Slots k0, k0 + kstep, .. of the neighbour row of live entry e of depth d, whose depth is complete
+// (computeRebuildNeighbor :669-696); found(slot, record, neighbour) gets each.  A neighbour is a child
+// of one of the parent's neighbours: of an octree node its octree child (or, for a root, the root of the
 // same group that replaces it), of a live entry its child entry if that is live.  The chain of a slot
 // is four dependent loads (record, parent's row, children, what `found` reads), and all rows of a
 // depth are in flight at once.
 template <class Found>
 __device__ __forceinline__ void sub_rows(const Counters* c, const SubTree& o, const SubArrays& A, int d, int depth,
-                                         int e0, int n, Found found) {
-    const int p = (int)lane_id();
-    if (p >= n) return;
-    const int e = e0 + p;
+                                         int e, int k0, int kstep, Found found) {
     const int4 me = A.rec[e];
     const int son = (me.z >> (3 * (depth - d))) & 7;
     const bool root = me.x < 0;
     const int pa = root ? -2 - me.x : me.x;
     const int* row = root ? o.neigh + (pa >= 0 ? pa : 0) : A.neigh + pa;
     const size_t rstride = root ? o.stride : (size_t)A.cap_live;
-    for (int k = threadIdx.x >> 5; k < 27; k += kBlock / 32) {
+    for (int k = k0; k < 27; k += kstep) {
         int lp, lc;
         nb_lut(son, k, lp, lc);
         int v = -1;
@@ -1033,7 +1029,7 @@ __device__ __forceinline__ void sub_rows(const Counters* c, const SubTree& o, co
             }
         }
         A.neigh[(size_t)k * A.cap_live + e] = v;
-        found(k, p, me, v);
+        found(k, me, v);
     }
 }
 
@@ -1057,27 +1053,26 @@ struct SubLevelLoad {
         __shared__ int s_fc[32 * 27];
         return s_fc;
     }
-    // rows of the tile's parents; called by every thread of the block before the tile's loads
+    static __device__ unsigned char* contributes() {   // per parent: an octree neighbour, or a root
+        __shared__ unsigned char s_con[32];
+        return s_con;
+    }
+    // rows of the tile's parents, a warp for the four of its candidates; called by every thread of the
+    // block before the tile's loads
     __device__ void begin(int base) const {
-        __shared__ unsigned s_con[32];
-        const int f0 = base >> 3;
-        const int nf = min(c->sub_nlive[d - 1] - f0, 32);   // parents of this tile
-        if (nf <= 0) return;
-        const int e0 = c->sub_lbase[d - 1] + f0;
-        int* s_fc = first_children();
-        if (threadIdx.x < 32) s_con[threadIdx.x] = 0u;
-        __syncthreads();
-        sub_rows(c, o, A, d - 1, depth, e0, nf, [&](int k, int p, const int4& me, int v) {
-            const bool oct = v >= 0 && v < o.na;
-            s_fc[p * 27 + k] = oct ? __ldg(o.first_child + v) : -1;
-            // a contributing level has an octree neighbour or is a root's
-            if (oct || me.x < 0) s_con[p] = 1u;
-        });
-        __syncthreads();
-        if ((int)threadIdx.x < nf) {
-            const int e = e0 + (int)threadIdx.x;
-            A.jump[e] = s_con[threadIdx.x] ? e : A.jump[A.rec[e].x];
+        const int p = threadIdx.x >> 3, f = (base >> 3) + p;
+        bool con = false;
+        if (f < c->sub_nlive[d - 1]) {
+            int* s_fc = first_children() + p * 27;
+            sub_rows(c, o, A, d - 1, depth, c->sub_lbase[d - 1] + f, threadIdx.x & 7, 8, [&](int k, const int4& me, int v) {
+                const bool oct = v >= 0 && v < o.na;
+                s_fc[k] = oct ? __ldg(o.first_child + v) : -1;
+                con |= oct || me.x < 0;
+            });
         }
+        con = (__ballot_sync(0xffffffffu, con) >> (threadIdx.x & 24) & 0xffu) != 0;
+        if ((threadIdx.x & 7) == 0) contributes()[p] = con;
+        __syncwarp();
     }
     __device__ unsigned operator()(int i) const {
         if (i >= 8 * c->sub_nlive[d - 1]) return 1u;   // a root
@@ -1087,22 +1082,22 @@ struct SubLevelLoad {
         sub_octant(A.poly + pl, (size_t)A.cap_live, ch, C);
         float mag = A.poly[(size_t)27 * A.cap_live + pl];
         const int* s_fc = first_children() + p * 27;
-        int fc[27];
-        bool contrib = false, deeper = false;   // deeper: an octree neighbour with children
+        // the eight of its parent's neighbours that a child's neighbours are children of
+        const int sx = (ch >> 2) & 1, sy = (ch >> 1) & 1, sz = ch & 1;
+        int most = -1;
 #pragma unroll
-        for (int k = 0; k < 27; ++k) {
-            int lp, lc;
-            nb_lut(ch, k, lp, lc);
-            fc[k] = s_fc[lp];
-            contrib |= fc[k] >= 0;
-            fc[k] = fc[k] >= 0 ? fc[k] + lc : -1;
-        }
+        for (int j = 0; j < 8; ++j)
+            most = max(most, s_fc[9 * (sx + (j >> 2)) + 3 * (sy + ((j >> 1) & 1)) + sz + (j & 1)]);
+        const bool contrib = most >= 0;
+        bool deeper = false;   // an octree neighbour with children
         if (contrib) {   // its own level
             float y[27];
+            int v[27];
+            child_neighbours(ch, [](int j) { return j; }, [&](int j) { return s_fc[j]; }, v);
 #pragma unroll
             for (int k = 0; k < 27; ++k) {
-                y[k] = fc[k] >= 0 ? __ldg(o.x + fc[k]) : 0.0f;
-                if (fc[k] >= 0 && d < depth) deeper |= __ldg(o.first_child + fc[k]) != -1;
+                y[k] = __ldg(o.x + v[k]);   // x[-1] = 0
+                if (v[k] >= 0 && d < depth) deeper |= __ldg(o.first_child + v[k]) != -1;
             }
             const float4 q = sub_child_pos(A.pos[pl], ch, d);
             const float sc = (float)(1 << d);
@@ -1142,7 +1137,10 @@ struct SubLevelStore {
         const int pl = c->sub_lbase[d - 1] + (i >> 3);
         if (child) {   // the family's eight lanes are all here
             const unsigned fam = __ballot_sync(0xffu << (threadIdx.x & 24), keep) >> (threadIdx.x & 24);
-            if ((i & 7) == 0) A.kids[pl] = make_int2(at, (int)(fam & 0xffu));
+            if ((i & 7) == 0) {
+                A.kids[pl] = make_int2(at, (int)(fam & 0xffu));
+                A.jump[pl] = SubLevelLoad::contributes()[threadIdx.x >> 3] ? pl : A.jump[A.rec[pl].x];
+            }
         }
         if (!keep) return;
         int4 me;
@@ -1224,7 +1222,6 @@ __global__ void __launch_bounds__(kBlock) k_sub_coarse(SubLevelLoad load, SubLev
         unsigned run = 0;
         for (int base = 0; base < n; base += kBlock) {
             load.begin(base);
-            __syncthreads();
             const int i = base + (int)threadIdx.x;
             const unsigned v = i < n ? load(i) : 0u;
             unsigned excl;
@@ -1260,7 +1257,8 @@ __global__ void __launch_bounds__(kBlock) k_sub_owners(const Counters* c, int de
         const int n = min(nl - L0, 32);
         if (threadIdx.x < 32) s_con[threadIdx.x] = s_smaller[threadIdx.x] = 0u;
         __syncthreads();
-        sub_rows(c, o, A, depth, depth, lb + L0, n, [&](int k, int pp, const int4& me, int v) {
+        const int pp = (int)lane_id();   // a lane a cell, the block's warps share its slots
+        if (pp < n) sub_rows(c, o, A, depth, depth, lb + L0 + pp, threadIdx.x >> 5, kBlock / 32, [&](int k, const int4& me, int v) {
             if (v >= o.na) {
                 if (k != 13 && A.rec[v - o.na].z < me.z) atomicOr(&s_smaller[pp], 1u << k);
             } else if (v >= 0) {

@@ -69,7 +69,6 @@ __device__ __forceinline__ void scan_done(const S&, unsigned, long) {}
 template <class L>
 __device__ __forceinline__ auto scan_begin(const L& l, int base, int) -> decltype(l.begin(base), void()) {
     l.begin(base);
-    __syncthreads();
 }
 template <class L>
 __device__ __forceinline__ void scan_begin(const L&, int, long) {}
