@@ -154,12 +154,12 @@ __global__ void __launch_bounds__(kBlock) k_mesh_owners(const Counters* c, int d
     PSR_GRID_STRIDE(i, M) {
         const int myk = key[i];
         unsigned smaller = 0;
+        int nb[27];
 #pragma unroll
-        for (int k = 0; k < 27; ++k) {
-            if (k == 13) continue;
-            const int nb = neigh[(size_t)k * stride + i];
-            if (nb != -1 && key[nb] < myk) smaller |= 1u << k;
-        }
+        for (int k = 0; k < 27; ++k) nb[k] = neigh[(size_t)k * stride + i];
+#pragma unroll
+        for (int k = 0; k < 27; ++k)   // an absent neighbour is never smaller
+            if (k != 13 && key[nb[k] != -1 ? nb[k] : i] < myk) smaller |= 1u << k;
         unsigned m = 0;
 #pragma unroll
         for (int q = 0; q < 8; ++q) if (!(smaller & vertex_cells(q))) m |= 1u << q;
@@ -205,12 +205,13 @@ struct VertexStore {
         const unsigned m = vmask[i];
         const int d = ndepth[i];
         const float hw = 1.0f / (float)(1 << (d + 1));
+        const float x = cx[i], y = cy[i], z = cz[i];
         int o = (int)pre;
         for (int q = 0; q < 8; ++q) {
             if (!((m >> q) & 1)) continue;
-            vx[o] = __fadd_rn(cx[i], (float)(2 * (q & 1) - 1) * hw);
-            vy[o] = __fadd_rn(cy[i], (float)(2 * ((q >> 1) & 1) - 1) * hw);
-            vz[o] = __fadd_rn(cz[i], (float)(2 * ((q >> 2) & 1) - 1) * hw);
+            vx[o] = __fadd_rn(x, (float)(2 * (q & 1) - 1) * hw);
+            vy[o] = __fadd_rn(y, (float)(2 * ((q >> 1) & 1) - 1) * hw);
+            vz[o] = __fadd_rn(z, (float)(2 * ((q >> 2) & 1) - 1) * hw);
             vowner[o] = i;
             vkind[o] = q;
             vdepth[o] = d;
@@ -259,14 +260,14 @@ struct FaceStore {
         if ((int)(pre + cnt) > cap) { atomicOr(err, kErrCapacity); return; }
         const unsigned m = fmask[i];
         const int d = ndepth[i];
-        const int son = (key[i] >> (3 * (depth - d))) & 7;
+        const int son = (key[i] >> (3 * (depth - d))) & 7, pa = parent[i];
         int q = (int)pre;
         for (int f = 0; f < 6; ++f) {
             if (!((m >> f) & 1)) continue;
             fowner[q] = i;
             fkind[q] = f;
             face_hit[q] = 0;
-            fhas[q] = (parent[i] == -1) ? -1 : ((__ldg(&g_tab.parent_face_kind[son][f]) != -1) ? 1 : -1);
+            fhas[q] = (pa == -1) ? -1 : ((__ldg(&g_tab.parent_face_kind[son][f]) != -1) ? 1 : -1);
             ++q;
         }
     }
@@ -318,25 +319,33 @@ __global__ void __launch_bounds__(kBlock) k_mesh_maintain(Counters* c, int depth
         const int V = c->n_vertices;
         PSR_GRID_STRIDE(v, V) {
             const int ow = vowner[v];
-            int mx, my, mz;
+            int mx, my, mz, nb[8];
             corner_sides(vkind[v], mx, my, mz);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)   // all reads before the first store
+                nb[j] = neigh[(size_t)nslot((j & 1) ? mx : 0, (j & 2) ? my : 0, (j & 4) ? mz : 0) * stride + ow];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int ax = (j & 1) ? mx : 0, ay = (j & 2) ? my : 0, az = (j & 4) ? mz : 0;
-                const int nb = neigh[(size_t)nslot(ax, ay, az) * stride + ow];
-                if (nb != -1) node_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * stride + nb] = v + 1;
+                if (nb[j] != -1) node_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * stride + nb[j]] = v + 1;
             }
         }
     } else if (blockIdx.z == 1) {
         const int E = c->n_edges;
         PSR_GRID_STRIDE(ei, E) {
             const int ow = eowner[ei], kind = ekind[ei];
+            int nb[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 int a[3];
                 edge_offset(kind, j, a);
-                const int nb = neigh[(size_t)nslot(a[0], a[1], a[2]) * stride + ow];
-                if (nb != -1) node_edge[(size_t)edge_slot_of(kind, a) * stride + nb] = ei + 1;
+                nb[j] = neigh[(size_t)nslot(a[0], a[1], a[2]) * stride + ow];
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                int a[3];
+                edge_offset(kind, j, a);
+                if (nb[j] != -1) node_edge[(size_t)edge_slot_of(kind, a) * stride + nb[j]] = ei + 1;
             }
         }
     } else if (blockIdx.z == 2) {
@@ -344,13 +353,10 @@ __global__ void __launch_bounds__(kBlock) k_mesh_maintain(Counters* c, int depth
         PSR_GRID_STRIDE(fi, F) {
             const int ow = fowner[fi], kind = fkind[fi];
             const int orient = kind >> 1, m = 2 * (kind & 1) - 1;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                int a[3] = {0, 0, 0};
-                a[orient] = j ? m : 0;
-                const int nb = neigh[(size_t)nslot(a[0], a[1], a[2]) * stride + ow];
-                if (nb != -1) node_face[(size_t)((orient << 1) + (2 * a[orient] - m < 0 ? 1 : 0)) * stride + nb] = fi + 1;
-            }
+            const int step = orient == 0 ? 9 : (orient == 1 ? 3 : 1);
+            const int nb0 = neigh[(size_t)13 * stride + ow], nb1 = neigh[(size_t)(13 + m * step) * stride + ow];
+            if (nb0 != -1) node_face[(size_t)((orient << 1) + (m > 0 ? 1 : 0)) * stride + nb0] = fi + 1;
+            if (nb1 != -1) node_face[(size_t)((orient << 1) + (m < 0 ? 1 : 0)) * stride + nb1] = fi + 1;
         }
     } else {
         // run length of every occupied cell of level g at the last sample of its run (the samples are
@@ -1392,25 +1398,33 @@ __global__ void __launch_bounds__(kBlock) k_sub_maintain(const Counters* c, int 
         const int V = c->n_sub_vertices;
         PSR_GRID_STRIDE(v, V) {
             const int ow = vowner[v];
-            int mx, my, mz;
+            int mx, my, mz, nb[8];
             corner_sides(vkind[v], mx, my, mz);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)   // all reads before the first store
+                nb[j] = A.neigh[(size_t)nslot((j & 1) ? mx : 0, (j & 2) ? my : 0, (j & 4) ? mz : 0) * A.cap_live + lb + ow] - na - lb;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int ax = (j & 1) ? mx : 0, ay = (j & 2) ? my : 0, az = (j & 4) ? mz : 0;
-                const int nb = A.neigh[(size_t)nslot(ax, ay, az) * A.cap_live + lb + ow] - na - lb;
-                if (nb >= 0) s_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * dstride + nb] = v + 1;
+                if (nb[j] >= 0) s_vtx[(size_t)vertex_slot_of(ax, ay, az, mx, my, mz) * dstride + nb[j]] = v + 1;
             }
         }
     } else {
         const int E = c->n_sub_edges;
         PSR_GRID_STRIDE(ei, E) {
             const int ow = eowner[ei], kind = ekind[ei];
+            int nb[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 int a[3];
                 edge_offset(kind, j, a);
-                const int nb = A.neigh[(size_t)nslot(a[0], a[1], a[2]) * A.cap_live + lb + ow] - na - lb;
-                if (nb >= 0) s_edge[(size_t)edge_slot_of(kind, a) * dstride + nb] = ei + 1;
+                nb[j] = A.neigh[(size_t)nslot(a[0], a[1], a[2]) * A.cap_live + lb + ow] - na - lb;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                int a[3];
+                edge_offset(kind, j, a);
+                if (nb[j] >= 0) s_edge[(size_t)edge_slot_of(kind, a) * dstride + nb[j]] = ei + 1;
             }
         }
     }

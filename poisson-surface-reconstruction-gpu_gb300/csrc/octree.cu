@@ -155,10 +155,16 @@ struct GatherLoad {
         const float c0 = c->center[0], c1 = c->center[1], c2 = c->center[2], e = c->max_edge;
         const float nscale = (float)(2 << depth);
         const size_t o = sidx[i];
-        px[i] = normalise_coord(xyz[3 * o], c0, e);
-        py[i] = normalise_coord(xyz[3 * o + 1], c1, e);
-        pz[i] = normalise_coord(xyz[3 * o + 2], c2, e);
+        // every read of the scattered sample before the first store, which the compiler could not
+        // move a read across (106 -> 85 us for 2,000,000 samples)
+        const float x = xyz[3 * o], y = xyz[3 * o + 1], z = xyz[3 * o + 2];
         float a = nrm[3 * o], b = nrm[3 * o + 1], d = nrm[3 * o + 2];
+        uint8_t r = 0, g = 0, bl = 0;
+        if (rgb) { r = rgb[3 * o]; g = rgb[3 * o + 1]; bl = rgb[3 * o + 2]; }
+        const unsigned code = scode[i], before = i ? scode[i - 1] : ~code;
+        px[i] = normalise_coord(x, c0, e);
+        py[i] = normalise_coord(y, c1, e);
+        pz[i] = normalise_coord(z, c2, e);
         float len = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b)), __fmul_rn(d, d)));
         // reference quirk: a normal no longer than 1e-6 is multiplied by its length
         if (len > 1e-6f) len = __fdiv_rn(1.0f, len);
@@ -167,13 +173,13 @@ struct GatherLoad {
         ny[i] = __fmul_rn(b, len);
         nz[i] = __fmul_rn(d, len);
         if (rgb) {
-            cr[i] = __fdiv_rn((float)rgb[3 * o], 255.0f);
-            cg[i] = __fdiv_rn((float)rgb[3 * o + 1], 255.0f);
-            cb[i] = __fdiv_rn((float)rgb[3 * o + 2], 255.0f);
+            cr[i] = __fdiv_rn((float)r, 255.0f);
+            cg[i] = __fdiv_rn((float)g, 255.0f);
+            cb[i] = __fdiv_rn((float)bl, 255.0f);
         } else {
             cr[i] = cg[i] = cb[i] = 0.0f;
         }
-        return (i == 0 || scode[i] != scode[i - 1]) ? 1u : 0u;
+        return code != before ? 1u : 0u;
     }
     __device__ void rebase() { PSR_CLOUD(in, scode, sidx, c, px, py, pz, nx, ny, nz, cr, cg, cb); }   // to cloud blockIdx.y
 };
@@ -533,12 +539,23 @@ __global__ void __launch_bounds__(kBlock) k_finalize_nodes(const Counters* c, in
             const int sh = 3 * (depth - d);
             const int g = li >> 3, j = li & 7;
             const int gs = off + 8 * g;
-            int v = 0;
-            while (v < 8 && tpnum[gs + v] == 0) ++v;
-            if (v == 8) v = 0;   // cannot happen: every group holds a non-empty node
+            int gp[8], gd[8];   // the group's counts (a group starts on a 32-byte boundary)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int4 p4 = *reinterpret_cast<const int4*>(tpnum + gs + 4 * q);
+                const int4 d4 = *reinterpret_cast<const int4*>(tdnum + gs + 4 * q);
+                gp[4 * q] = p4.x; gp[4 * q + 1] = p4.y; gp[4 * q + 2] = p4.z; gp[4 * q + 3] = p4.w;
+                gd[4 * q] = d4.x; gd[4 * q + 1] = d4.y; gd[4 * q + 2] = d4.z; gd[4 * q + 3] = d4.w;
+            }
+            int v = 0;   // the first non-empty node (0: cannot happen, every group holds one)
+#pragma unroll
+            for (int q = 7; q >= 0; --q)
+                if (gp[q] != 0) v = q;
             k = (tkey[gs + v] & ~(7 << sh)) | (j << sh);
             int nowP = tpidx[gs + v], nowD = tdidx[gs + v];
-            for (int q = 0; q < j; ++q) { nowP += tpnum[gs + q]; nowD += tdnum[gs + q]; }
+#pragma unroll
+            for (int q = 0; q < 7; ++q)
+                if (q < j) { nowP += gp[q]; nowD += gd[q]; }
             pi = nowP;
             di = (d == depth) ? tdidx[t] : nowD;
             // reference quirk: the first non-empty node of the group passes its parent to
