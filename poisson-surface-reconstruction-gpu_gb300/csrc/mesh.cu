@@ -1436,114 +1436,15 @@ __global__ void __launch_bounds__(kBlock) k_sub_maintain(const Counters* c, int 
 // own plus the slot offset.  A subdivision node's own index comes from its centre
 // ((off + 1/2) / 2^d exactly).  The value is the sum, level after level from the owner's
 // nearest contributing node up to the root and then 27 neighbour terms in slot order, of
-// ((x Fx) Fy) Fz.  Eight lanes per vertex (four vertices per warp, whose chains of
-// dependent loads overlap): the group's first lane finds the levels (subdivision nodes
-// through the jump links, then the octree ancestors), the lanes evaluate the 3 basis values
-// per axis of each level and form the terms in parallel, and the first lane adds them in
-// that order (absent neighbours as +0, which leaves such a sum unchanged): the chain's
-// dependent loads are paid once per level instead of once per term.
-constexpr int kSvLanes = 8;
-constexpr int kSvBlock = 128;
-constexpr int kSvGroups = kSvBlock / kSvLanes;
-constexpr int kSvMaxLevels = kMaxDepth + 1;
-__global__ void __launch_bounds__(kSvBlock) k_sub_vertex_values(const Counters* c, int depth, const float* vx,
-                                                                const float* vy, const float* vz, const int* vowner,
-                                                                const int* neigh, size_t stride, const int* parent,
-                                                                const int* root_self, SubArrays A,
-                                                                const int* enc, const float* x, float* vvalue, int na) {
-    PSR_CLOUD(c, vx, vy, vz, vowner, neigh, parent, root_self, A, enc, x, vvalue);
-    __shared__ int s_node[kSvGroups][kSvMaxLevels];   // live entry (subdivision) or octree node
-    __shared__ int s_root[kSvGroups];                 // a root neighbour's number to its root index
-    __shared__ int s_o[kSvGroups][kSvMaxLevels][3];   // function index of the level's node
-    __shared__ float s_t[kSvGroups][kSvMaxLevels * 27];
-    __shared__ float s_b[kSvGroups][kSvMaxLevels][9];  // a level's 3 basis values per axis
-    const int V = c->n_sub_vertices;
-    const float iso = c->iso;
-    const int lb = c->sub_lbase[depth];
-    const int gl = threadIdx.x & (kSvLanes - 1), w = threadIdx.x / kSvLanes;
-    const unsigned gmask = 0xffu << (threadIdx.x & 24);   // the group's lanes in its warp
-    for (int v = blockIdx.x * kSvGroups + w; v < V; v += gridDim.x * kSvGroups) {
-        const float qx = vx[v], qy = vy[v], qz = vz[v];
-        const int own = lb + vowner[v];
-        int nsub = 0, nlev = 0;
-        if (gl == 0) {
-            // levels whose 27 neighbours are all zero-valued subdivision nodes add nothing:
-            // the jump links skip them
-            int sn = A.jump[own], now = -1;
-            while (nsub < kSvMaxLevels) {
-                s_node[w][nsub++] = sn;
-                const int p = A.rec[sn].x;
-                if (p < 0) { now = -2 - p; break; }
-                sn = A.jump[p];
-            }
-            nlev = nsub;
-            for (; now != -1 && nlev < kSvMaxLevels; now = parent[now]) s_node[w][nlev++] = now;
-        }
-        nsub = __shfl_sync(gmask, nsub, 0, kSvLanes);
-        nlev = __shfl_sync(gmask, nlev, 0, kSvLanes);
-        __syncwarp(gmask);
-        for (int l = gl; l < nlev; l += kSvLanes) {
-            const int nd = s_node[w][l];
-            int ox, oy, oz;
-            if (l < nsub) {
-                const float4 q = A.pos[nd];
-                const int d = __float_as_int(q.w);
-                const float sc = (float)(1 << d);
-                const int base = (1 << d) - 1;
-                ox = base + (int)__fmul_rn(q.x, sc);
-                oy = base + (int)__fmul_rn(q.y, sc);
-                oz = base + (int)__fmul_rn(q.z, sc);
-                if (l == nsub - 1) s_root[w] = sub_root_shift(c, d) - na;
-            } else {
-                decode_fn_index(enc[nd], depth, ox, oy, oz);
-            }
-            s_o[w][l][0] = ox;
-            s_o[w][l][1] = oy;
-            s_o[w][l][2] = oz;
-        }
-        __syncwarp(gmask);
-        // the 27 translates of a level share 3 basis values per axis: 9 evaluations per level
-        for (int t = gl; t < nlev * 9; t += kSvLanes) {
-            const int l = t / 9, r = t - 9 * l, a = r / 3;
-            s_b[w][l][r] = basis32(s_o[w][l][a] - 1 + (r - 3 * a), a == 0 ? qx : (a == 1 ? qy : qz));
-        }
-        __syncwarp(gmask);
-        for (int t = gl; t < nlev * 27; t += kSvLanes) {
-            const int l = t / 27, k = t - 27 * l;
-            const int nd = s_node[w][l];
-            int nb = (l < nsub) ? A.neigh[(size_t)k * A.cap_live + nd] : neigh[(size_t)k * stride + nd];
-            if (nb >= na) nb = (l == nsub - 1) ? root_self[nb + s_root[w]] : -1;
-            float term = 0.0f;
-            if (nb >= 0) {
-                const float bxk = s_b[w][l][k / 9];
-                const float byk = s_b[w][l][3 + (k / 3) % 3];
-                const float bzk = s_b[w][l][6 + k % 3];
-                term = __fmul_rn(__fmul_rn(__fmul_rn(x[nb], bxk), byk), bzk);
-            }
-            s_t[w][t] = term;
-        }
-        __syncwarp(gmask);
-        if (gl == 0) {
-            float val = 0.0f;
-            for (int l = 0; l < nlev; ++l) {
-#pragma unroll
-                for (int k = 0; k < 27; ++k) val = __fadd_rn(val, s_t[w][l * 27 + k]);
-            }
-            vvalue[v] = __fsub_rn(val, iso);
-        }
-        __syncwarp(gmask);
-    }
-}
-
-// The same values, one thread per vertex: from depth 8 on there are hundreds of thousands of
-// vertices, whose own parallelism hides the chains' loads, and the eight-lane form leaves seven
-// lanes idle while the first adds the terms one by one (1.24 ms of 2M points, depth 9, against
-// 0.5 ms).  Software-pipelined like k_vertex_values: the next level's neighbour row is read while
-// the current one's values are in flight.
-__global__ void __launch_bounds__(kBlock) k_sub_vertex_values_wide(const Counters* c, int depth, const float* vx,
-                                                                   const float* vy, const float* vz, const int* vowner,
-                                                                   const int* root_self, SubArrays A, ValueRows R,
-                                                                   float* vvalue, int na) {
+// ((x Fx) Fy) Fz (levels whose 27 neighbours are all zero-valued subdivision nodes add nothing:
+// the jump links skip them).  One thread per vertex: its 27 loads of a level are in flight together
+// and the next octree row is read during the terms.  Eight lanes per vertex, which form the terms in
+// parallel and leave seven idle while one adds them, took 115 us where this takes 25 (60,000 samples
+// with clutter, depth 7), and 28 against 17 for the few thousand vertices of 200,000 samples.
+__global__ void __launch_bounds__(kBlock) k_sub_vertex_values(const Counters* c, int depth, const float* vx,
+                                                              const float* vy, const float* vz, const int* vowner,
+                                                              const int* root_self, SubArrays A, ValueRows R,
+                                                              float* vvalue, int na) {
     PSR_CLOUD(c, vx, vy, vz, vowner, root_self, A, R, vvalue);
     R.n = min(c->level_base[depth], R.n);
     const int V = c->n_sub_vertices;
@@ -2027,13 +1928,8 @@ cudaError_t mesh_build_sub(Workspace& ws, const MeshBufs& mb) {
     const dim3 g2 = PSR_GRID(ws, gl);
     k_sub_maintain<<<dim3(g2.x, g2.y, 2), kBlock, 0, s>>>(c, D, A, na, dstride, ws.sv_owner, ws.sv_kind, ws.s_vtx,
                                                           ws.se_owner, ws.se_kind, ws.s_edge);
-    if (D >= 8)
-        k_sub_vertex_values_wide<<<PSR_GRID(ws, 8 * ws.num_sms), kBlock, 0, s>>>(
-            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.root_self, A, value_rows(ws), ws.sv_value, na);
-    else
-        k_sub_vertex_values<<<PSR_GRID(ws, 16 * ws.num_sms), kSvBlock, 0, s>>>(
-            c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.neigh, stride, ws.parent, ws.root_self, A, ws.enc,
-            ws.xsol, ws.sv_value, na);
+    k_sub_vertex_values<<<PSR_GRID(ws, 8 * ws.num_sms), kBlock, 0, s>>>(
+        c, D, ws.sv_x, ws.sv_y, ws.sv_z, ws.sv_owner, ws.root_self, A, value_rows(ws), ws.sv_value, na);
     // crossings: staged after the main part's vertices
     e = launch_scan<4>(SubCrossLoad{ws.se_owner, ws.se_kind, ws.s_vtx, dstride, ws.sv_value, err},
                        SubCrossStore{ws.se_owner, ws.se_kind, ws.s_vtx, dstride, ws.sv_value, ws.sv_x, ws.sv_y,

@@ -221,8 +221,8 @@ inline int grid_for(const Workspace& ws, long long work) {
 constexpr int kDivChunk = 512;
 inline int div_split(int D) { return D >= 8 ? 5 : (D >= 2 ? D - 2 : 0); }
 
-inline ValueRows value_rows(const Workspace& ws) {
-    return ValueRows{ws.value_rows, ws.cap_rows, ws.neigh, (size_t)ws.cap.nodes, ws.parent, ws.first_child, ws.enc, ws.xsol};
+inline ValueRows value_rows(const Workspace& ws) {   // none below depth 8
+    return ValueRows{ws.value_rows, ws.depth >= 8 ? ws.cap_rows : 0, ws.neigh, (size_t)ws.cap.nodes, ws.parent, ws.first_child, ws.enc, ws.xsol};
 }
 
 // stage entry points (each issues kernels on ws.stream; no host synchronisation)
