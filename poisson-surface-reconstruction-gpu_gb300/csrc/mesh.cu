@@ -705,96 +705,28 @@ struct RootLoad {
     __device__ void rebase() { PSR_CLOUD(node_vtx, node_face, vvalue, face_hit, first_child, err); }   // to cloud blockIdx.y
 };
 struct RootStore {
+    Counters* c;
+    int depth;
     int* sub_root;
     int cap;
     unsigned* err;
     __device__ void operator()(int i, unsigned pre, unsigned f) const {
+        // the roots are in depth order: the count before a level's first node (1 + a multiple of 8) is
+        // where the roots of its depth start
+        if ((i & 7) == 1)
+            for (int d = 1; d < depth; ++d)
+                if (c->level_base[d] == i) c->sub_rstart[d] = min((int)pre, cap);
         if (!f) return;
         if ((int)pre >= cap) { atomicOr(err, kErrCapacity); return; }
         sub_root[pre] = i;
     }
-    __device__ void rebase() { PSR_CLOUD(sub_root, err); }   // to cloud blockIdx.y
+    __device__ void rebase() { PSR_CLOUD(c, sub_root, err); }   // to cloud blockIdx.y
 };
 
 // Group table.  Group record (ints): 0 root depth, 1 first root, 2 root count,
 // 3 virtual node offset, 4 virtual node count.  Coarse roots (depth < D - 4) are one group each; the finer roots
 // of one depth form one group (mesh/ComputeTriangleIndices.cu:1475-1799, :1801-2194).
 constexpr int kGroupRec = 8;
-
-struct GroupFlagLoad {
-    const int* sub_root;
-    const int* ndepth;
-    int finer;
-    __device__ unsigned operator()(int r) const {
-        const int rd = ndepth[sub_root[r]];
-        if (r == 0 || rd < finer) return 1u;
-        return (ndepth[sub_root[r - 1]] != rd) ? 1u : 0u;
-    }
-    __device__ void rebase() { PSR_CLOUD(sub_root, ndepth); }   // to cloud blockIdx.y
-};
-struct GroupFlagStore {
-    Counters* c;
-    int* root_group;
-    int* groups;
-    int max_groups;
-    unsigned* err;
-    __device__ void operator()(int r, unsigned pre, unsigned v) const {
-        const int g = (int)(pre + v) - 1;
-        root_group[r] = g;
-        if (v) {
-            if (g >= max_groups) { atomicOr(err, kErrCapacity); return; }
-            groups[(size_t)g * kGroupRec + 1] = r;
-        }
-    }
-    __device__ void done(unsigned total) const {
-        int ng = (int)total;
-        if (ng > max_groups) { atomicOr(err, kErrCapacity); ng = 0; }
-        c->n_group_flags = ng;
-    }
-    __device__ void rebase() { PSR_CLOUD(c, root_group, groups, err); }   // to cloud blockIdx.y
-};
-
-// per-group sizes; their prefixes number the groups' virtual nodes
-struct GroupSizeLoad {
-    Counters* c;
-    int depth;
-    const int* sub_root;
-    const int* ndepth;
-    int* groups;
-    __device__ unsigned operator()(int g) const {
-        const int ng = c->n_group_flags, R = c->n_subroots;
-        int* G = groups + (size_t)g * kGroupRec;
-        const int first = G[1];
-        const int next = (g + 1 < ng) ? groups[(size_t)(g + 1) * kGroupRec + 1] : R;
-        const int rd = ndepth[sub_root[first]];
-        const long long n = next - first;
-        long long per = 0, dper = 1;
-        for (int d = rd; d <= depth; ++d) { per += dper; if (d < depth) dper *= 8; }
-        const long long nodes = per * n;
-        G[0] = rd;
-        G[2] = (int)n;
-        if (nodes > 0x3fffffffLL) atomicOr(&c->error, kErrCapacity);
-        G[4] = nodes > 0x3fffffffLL ? 0x3fffffff : (int)nodes;
-        return (unsigned)G[4];
-    }
-    __device__ void rebase() { PSR_CLOUD(c, sub_root, ndepth, groups); }   // to cloud blockIdx.y
-};
-struct GroupSizeStore {
-    Counters* c;
-    int* groups;
-    int na;
-    __device__ void operator()(int g, unsigned pre, unsigned) const { groups[(size_t)g * kGroupRec + 3] = (int)pre; }
-    // the virtual numbering of all groups must fit beside the octree indices (na + index)
-    __device__ void done(unsigned total) const {
-        int ng = c->n_group_flags;
-        if (total > 0x7fffffffu - (unsigned)na) {
-            atomicOr(&c->error, kErrCapacity);
-            ng = 0;
-        }
-        c->n_groups = ng;
-    }
-    __device__ void rebase() { PSR_CLOUD(c, groups); }   // to cloud blockIdx.y
-};
 
 // ---- subdivision, breadth-first over live nodes ----------------------------------------
 // Virtual numbering (singleRebuildArray :599-635 / wholeRebuildArray :1110-1168): group g
@@ -813,37 +745,67 @@ __device__ __forceinline__ int sub_level_off(int rd, int n, int d) {
     return off;
 }
 
-// per-depth candidate bookkeeping (Counters::sub_*): [d] for depth d; one thread per depth
-__device__ __forceinline__ void sub_setup(Counters* c, int depth, const int* sub_root, const int* ndepth,
-                                          int cap_nodes) {
-    const int d = threadIdx.x;
-    const int R = c->n_subroots;
-    __shared__ int s_end[kMaxDepth + 2];
-    if (d <= depth + 1) {
-        int lo = 0, hi = R;   // first root deeper than d (roots are in depth order)
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (ndepth[sub_root[mid]] <= d) lo = mid + 1;
-            else hi = mid;
+// The groups of a depth's roots.  The roots are in depth order, so with the first root of every depth
+// known the groups follow without a scan: a coarse root is group number its own, a finer depth is the
+// group after those of the depths before it, and a root of depth d brings (8^(D-d+1) - 1) / 7 virtual
+// nodes (two scans of up to 12 us each before).  In shared memory of every block; block 0 also sets up the
+// per-depth bookkeeping (Counters::sub_*).
+struct DepthGroups {
+    int start[kMaxDepth + 2];     // first root of the depth
+    int count[kMaxDepth + 2];
+    int group[kMaxDepth + 2];     // first group
+    long long per[kMaxDepth + 2];    // virtual nodes of a root
+    long long first[kMaxDepth + 2];  // first virtual node
+    int n_groups;
+};
+__device__ __forceinline__ void sub_setup(Counters* c, int depth, int max_groups, int na, int cap_nodes, DepthGroups& t) {
+    if (threadIdx.x == 0) {
+        const int R = c->n_subroots;
+        int start[kMaxDepth + 2];
+#pragma unroll
+        for (int d = 0; d <= kMaxDepth + 1; ++d)   // a level without nodes has no roots
+            start[d] = d == 0 ? 0 : (d < depth && c->level_count[min(d, kMaxDepth)] > 0 ? c->sub_rstart[d] : -1);
+        int next = R, ng = 0;
+#pragma unroll
+        for (int d = kMaxDepth + 1; d >= 0; --d) {
+            if (start[d] < 0) start[d] = next;
+            t.start[d] = start[d];
+            t.count[d] = next - start[d];
+            next = start[d];
         }
-        s_end[d] = lo;
+        long long virt = 0;
+        unsigned bad = 0;
+        for (int d = 0; d <= depth; ++d) {
+            const bool coarse = d < depth - 4;
+            long long per = 0, n = 1;
+            for (int e = d; e <= depth; ++e) { per += n; n *= 8; }
+            t.per[d] = per;
+            t.group[d] = ng;
+            t.first[d] = virt;
+            ng += coarse ? t.count[d] : (t.count[d] > 0 ? 1 : 0);
+            if (t.count[d] > 0 && per * (coarse ? 1 : t.count[d]) > 0x3fffffffLL) bad = 1;
+            virt += per * t.count[d];
+        }
+        // the numbering of the groups must fit the table, and their virtual nodes beside the octree's
+        if (ng > max_groups || virt > 0x7fffffffLL - na) { bad = 1; ng = 0; }
+        t.n_groups = ng;
+        if (blockIdx.x == 0) {
+            if (bad) atomicOr(&c->error, kErrCapacity);
+            c->n_groups = ng;
+            c->n_sub_nodes = 0;
+            c->n_sub_dnodes = 0;
+        }
     }
     __syncthreads();
-    if (d <= depth + 1) {
-        const int start = (d > 0) ? s_end[d - 1] : 0;
-        const int n = (c->n_groups > 0) ? s_end[d] - start : 0;
-        c->sub_rstart[d] = start;
+    const int d = threadIdx.x;
+    if (blockIdx.x == 0 && d <= depth + 1) {
+        const int n = t.n_groups > 0 ? t.count[d] : 0;
         c->sub_nroots[d] = n;
         c->sub_cbase[d] = 0;
         c->sub_lbase[d] = 0;
         c->sub_nlive[d] = 0;
-        c->sub_cand[d] = 0;
-        if (d == 1) {
-            if (n > cap_nodes) atomicOr(&c->error, kErrCapacity);
-            else c->sub_cand[1] = n;
-            c->n_sub_nodes = 0;
-            c->n_sub_dnodes = 0;
-        }
+        if (d == 1 && n > cap_nodes) atomicOr(&c->error, kErrCapacity);
+        c->sub_cand[d] = d == 1 && n <= cap_nodes ? n : 0;
     }
 }
 
@@ -887,29 +849,44 @@ struct SubArrays {
 // them by Bernstein subdivision: with the cell at [a, b] of the root's unit interval, the
 // new coefficients are the blossom values P(a, a), P(a, b), P(b, b) -- convex weights, exact
 // for these dyadic a, b.
-// Per root: the octree node it stands for, the redirected child slot of its parent (overlay) and
+// Per root: its group's record, the octree node it stands for, the redirected child slot of its parent (overlay) and
 // its polynomial; block 0 also sets up the per-depth bookkeeping.
 __global__ void __launch_bounds__(kBlock) k_root_setup(Counters* c, int depth, const int* sub_root, const int* ndepth,
-                                                       const int* key, const int* root_group, const int* groups,
-                                                       int* root_self, int* ov_group, int* ov_sub, const float* ctr_x,
+                                                       const int* key, int* root_group, int* groups, int max_groups,
+                                                       int na, int* root_self, int* ov_group, int* ov_sub, const float* ctr_x,
                                                        const float* ctr_y, const float* ctr_z, const int* neigh,
                                                        size_t stride, const int* parent, const int* enc, const float* x,
                                                        float* root_poly, int cap_poly, int cap_nodes) {
     PSR_CLOUD(c, sub_root, ndepth, key, root_group, groups, root_self, ov_group, ov_sub, ctr_x, ctr_y, ctr_z, neigh, parent, enc, x, root_poly);
-    if (blockIdx.x == 0) sub_setup(c, depth, sub_root, ndepth, cap_nodes);
+    __shared__ DepthGroups T;
+    sub_setup(c, depth, max_groups, na, cap_nodes, T);
     const int R = c->n_subroots;
-    const int ng = c->n_groups;
+    const int ng = T.n_groups;
     PSR_GRID_STRIDE(r, R) {
         const int node = sub_root[r];
         const int rd = ndepth[node];
         const int self = neigh[(size_t)13 * stride + node];   // its neighs[13] in the reference
         root_self[r] = (self == -1) ? node : self;
-        const int g = root_group[r];
+        const int q = r - T.start[rd];
+        const bool coarse = rd < depth - 4;
+        const int g = T.group[rd] + (coarse ? q : 0), head = coarse ? r : T.start[rd];
         const int pa = parent[node];
-        if (g >= 0 && g < ng && pa >= 0) {
-            const int son = (key[node] >> (3 * (depth - rd))) & 7;
-            ov_group[(size_t)son * stride + pa] = g;
-            ov_sub[(size_t)son * stride + pa] = r - groups[(size_t)g * kGroupRec + 1];
+        root_group[r] = g;
+        if (g < ng) {
+            if (r == head) {
+                int* G = groups + (size_t)g * kGroupRec;
+                const int n = coarse ? 1 : T.count[rd];
+                G[0] = rd;
+                G[1] = r;
+                G[2] = n;
+                G[3] = (int)(T.first[rd] + (coarse ? q * T.per[rd] : 0));
+                G[4] = (int)min(n * T.per[rd], 0x3fffffffLL);
+            }
+            if (pa >= 0) {
+                const int son = (key[node] >> (3 * (depth - rd))) & 7;
+                ov_group[(size_t)son * stride + pa] = g;
+                ov_sub[(size_t)son * stride + pa] = r - head;
+            }
         }
         if (r >= cap_poly) continue;
         const float qx = ctr_x[node], qy = ctr_y[node], qz = ctr_z[node];
@@ -1865,18 +1842,10 @@ cudaError_t mesh_build_impl(Workspace& ws, const MeshBufs& mb) {
     if (e != cudaSuccess) return e;
     // subdivision roots among nodes of depth < D
     e = launch_scan<1>(RootLoad{ws.node_vtx, ws.node_face, stride, ws.vvalue, ws.face_hit, ws.first_child, err},
-                    RootStore{ws.sub_root, ws.cap.nodes, err}, &c->level_base[D], 0, ws.scan, total, err, s, ScanCount{&c->n_subroots, ws.cap.nodes});
-    if (e != cudaSuccess) return e;
-    // subdivision groups
-    e = launch_scan<1>(GroupFlagLoad{ws.sub_root, ws.ndepth, D - 4},
-                       GroupFlagStore{c, ws.root_group, mb.groups, mb.max_groups, err}, &c->n_subroots, 0, ws.scan, total,
-                       err, s, ScanCount{}, 1);
-    if (e != cudaSuccess) return e;
-    e = launch_scan<1>(GroupSizeLoad{c, D, ws.sub_root, ws.ndepth, mb.groups}, GroupSizeStore{c, mb.groups, ws.cap.nodes},
-                       &c->n_group_flags, 0, ws.scan, total, err, s, ScanCount{}, 1);
+                    RootStore{c, D, ws.sub_root, ws.cap.nodes, err}, &c->level_base[D], 0, ws.scan, total, err, s, ScanCount{&c->n_subroots, ws.cap.nodes});
     if (e != cudaSuccess) return e;
     k_root_setup<<<PSR_GRID(ws, 4 * ws.num_sms), kBlock, 0, s>>>(
-        c, D, ws.sub_root, ws.ndepth, ws.key, ws.root_group, mb.groups, ws.root_self, mb.ov_group, mb.ov_sub, ws.ctr_x,
+        c, D, ws.sub_root, ws.ndepth, ws.key, ws.root_group, mb.groups, mb.max_groups, ws.cap.nodes, ws.root_self, mb.ov_group, mb.ov_sub, ws.ctr_x,
         ws.ctr_y, ws.ctr_z, ws.neigh, stride, ws.parent, ws.enc, ws.xsol, ws.root_poly, ws.cap_poly, ws.cap.sub_nodes);
     return cudaGetLastError();
 }

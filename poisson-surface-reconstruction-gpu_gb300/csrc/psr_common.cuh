@@ -33,7 +33,6 @@ struct Counters {
     int n_vertices, n_edges, n_faces;
     int n_cross, n_tri;
     int n_subroots;
-    int n_group_flags;            // subdivision groups before the check of their numbering
     int n_div_items;              // chunks of the coarse divergence
     // subdivision, per depth d: candidates, their first compact slot, the first entry of
     // the depth's live list, live nodes, first root index and roots of depth d
