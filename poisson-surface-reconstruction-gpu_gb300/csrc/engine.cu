@@ -47,7 +47,7 @@ struct GraphEntry {
 struct psr_handle {
     psr_config cfg;
     Workspace ws;
-    InputRef* h_params = nullptr;   // pinned, one per slot: written by the host, copied to ws.d_params per call
+    InputRef* h_params = nullptr;   // pinned, one per slot: written by the host before each run
     std::map<long long, GraphEntry> graphs;
     int use_graphs = 1;
     int last_kernels = 0;
@@ -456,6 +456,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     e = cudaMallocHost(&h->cnt_host_all, sizeof(Counters) * (size_t)h->clouds);
     ws.cnt_host = h->cnt_host_all;
     if (e == cudaSuccess) e = cudaMallocHost(&h->h_params, sizeof(InputRef) * (size_t)h->clouds);
+    ws.h_params = h->h_params;
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking);
     for (int i = 0; i < 7 && e == cudaSuccess; ++i) e = cudaEventCreate(&h->ev[i]);
     h->ws.ev_cg = h->ev[6];
@@ -541,19 +542,37 @@ psr_status psr_destroy(psr_handle* h) {
 
 // copies the mesh of the last run into device-resident caller buffers (counts read on the
 // device, clamped to the caller's capacities), so a device-output call needs no host wait
+struct EmitTo {
+    float* v;   // null: not asked for, or copied by the host
+    int* t;
+    float *c, *n;
+    int vcap, tcap;
+};
+extern "C++" {   // templates
+template <int kClouds>
+struct EmitArgs {
+    EmitTo to[kClouds];
+};
+template <int kClouds>
 __global__ void __launch_bounds__(kBlock) k_emit_mesh(const Counters* c, const float* v, const int* t,
-                                                      const float* col, const float* nrm, float* ov, int* ot,
-                                                      float* oc, float* on, int vcap, int tcap) {
-    const int nv = 3 * min(max(c->n_mesh_vertices, 0), vcap);
-    const int nt = 3 * min(max(c->n_mesh_triangles, 0), tcap);
+                                                      const float* col, const float* nrm, EmitArgs<kClouds> a,
+                                                      Counters* host) {
+    PSR_CLOUD(c, v, t, col, nrm);
+    const EmitTo& to = a.to[kClouds > 1 ? blockIdx.y : 0];
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < (int)(sizeof(Counters) / 4); i += kBlock)
+            ((unsigned*)(host + blockIdx.y))[i] = ((const unsigned*)c)[i];
+    const int nv = 3 * min(max(c->n_mesh_vertices, 0), to.vcap);
+    const int nt = 3 * min(max(c->n_mesh_triangles, 0), to.tcap);
     PSR_GRID_STRIDE(i, max(nv, nt)) {
         if (i < nv) {
-            if (ov) ov[i] = v[i];
-            if (oc) oc[i] = col[i];
-            if (on) on[i] = nrm[i];
+            if (to.v) to.v[i] = v[i];
+            if (to.c) to.c[i] = col[i];
+            if (to.n) to.n[i] = nrm[i];
         }
-        if (i < nt && ot) ot[i] = t[i];
+        if (i < nt && to.t) to.t[i] = t[i];
     }
+}
 }
 
 // The whole pipeline for the clouds set by set_batch, issued on `qs` (captured into a graph
@@ -702,9 +721,7 @@ static cudaError_t stage_inputs(psr_handle* h, const psr_points* pts, int k, cud
         if (e == cudaSuccess) e = cudaMemcpyAsync((void*)hp->nrm, pts->normals, 3 * sizeof(float) * (size_t)n, kind, s);
         if (e == cudaSuccess && pts->rgb) e = cudaMemcpyAsync((void*)hp->rgb, pts->rgb, 3 * (size_t)n, kind, s);
     }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(slot_ptr(ws.d_params, k), hp, sizeof(InputRef), cudaMemcpyHostToDevice, s);
-    return e;
+    return e;   // the pipeline's first kernel reads *hp
 }
 
 // Device address of a host output buffer the GPU can write (pinned or registered host
@@ -723,30 +740,39 @@ static void* device_view(void* p, bool& ok) {
     return nullptr;
 }
 
-// Enqueues the count read-back of slot k and the copy of its mesh into the caller's
-// buffers by a kernel that reads the counts on the device (no host wait): for device
-// outputs, and for host outputs in pinned or registered memory, which the kernel writes
-// through their device addresses.  Other host outputs are copied when the work has
-// completed (*emitted = false).
-static cudaError_t stage_outputs(psr_handle* h, psr_mesh* mesh, int k, int want_colour, int want_normals,
-                                 cudaStream_t s, bool* emitted) {
+// Enqueues the read-back of the counts of slots 0 .. count - 1 and the copy of their meshes into
+// the caller's buffers: one kernel that reads the counts on the device (no host wait) and writes
+// counts and host outputs in pinned or registered memory through their device addresses (a copy per
+// cloud each way and a kernel per cloud took 150 us of a 16-cloud batch).  Other host outputs are
+// copied when the work has completed (emitted[k] = 0).
+static cudaError_t stage_outputs(psr_handle* h, psr_mesh* meshes, int count, int want_colour, int want_normals,
+                                 cudaStream_t s, std::vector<char>& emitted) {
     Workspace& ws = h->ws;
-    cudaError_t e =
-        cudaMemcpyAsync(h->cnt_host_all + k, slot_ptr(ws.cnt, k), sizeof(Counters), cudaMemcpyDeviceToHost, s);
-    bool ok = true;
-    void* dv = device_view(mesh->vertices, ok);
-    void* dt = device_view(mesh->triangles, ok);
-    void* dc = want_colour ? device_view(mesh->colors, ok) : nullptr;
-    void* dn = want_normals ? device_view(mesh->normals, ok) : nullptr;
-    *emitted = ok;
-    if (e == cudaSuccess && ok) {
-        k_emit_mesh<<<ws.num_sms * 4, kBlock, 0, s>>>(slot_ptr(ws.cnt, k), slot_ptr(ws.mesh_v, k),
-                                                      slot_ptr(ws.mesh_t, k), slot_ptr(ws.mesh_c, k),
-                                                      slot_ptr(ws.mesh_n, k), (float*)dv, (int*)dt, (float*)dc,
-                                                      (float*)dn, mesh->vertex_capacity, mesh->triangle_capacity);
-        e = cudaGetLastError();
+    EmitArgs<kMaxBatchClouds> a;
+    emitted.assign(count, 0);
+    for (int k = 0; k < count; ++k) {
+        psr_mesh* mesh = meshes + k;
+        bool ok = true;
+        EmitTo to;
+        to.v = (float*)device_view(mesh->vertices, ok);
+        to.t = (int*)device_view(mesh->triangles, ok);
+        to.c = (float*)(want_colour ? device_view(mesh->colors, ok) : nullptr);
+        to.n = (float*)(want_normals ? device_view(mesh->normals, ok) : nullptr);
+        to.vcap = mesh->vertex_capacity;
+        to.tcap = mesh->triangle_capacity;
+        a.to[k] = ok ? to : EmitTo{nullptr, nullptr, nullptr, nullptr, 0, 0};
+        emitted[k] = ok;
     }
-    return e;
+    const dim3 grid((unsigned)std::max(1, ws.num_sms * 4 / count), (unsigned)count);
+    if (count == 1) {
+        EmitArgs<1> one;
+        one.to[0] = a.to[0];
+        k_emit_mesh<1><<<grid, kBlock, 0, s>>>(ws.cnt, ws.mesh_v, ws.mesh_t, ws.mesh_c, ws.mesh_n, one, h->cnt_host_all);
+    } else {
+        k_emit_mesh<kMaxBatchClouds><<<grid, kBlock, 0, s>>>(ws.cnt, ws.mesh_v, ws.mesh_t, ws.mesh_c, ws.mesh_n, a,
+                                                             h->cnt_host_all);
+    }
+    return cudaGetLastError();
 }
 
 static psr_status check_points(psr_handle* h, const psr_points* pts, const psr_mesh* mesh) {
@@ -786,12 +812,7 @@ static psr_status submit_clouds(psr_handle* h, const psr_points* pts, int count,
     for (int k = 0; k < count && e == cudaSuccess; ++k) e = stage_inputs(h, pts + k, k, s);
     if (e != cudaSuccess) return cuda_fail(h, e, "input copy");
     e = launch_pipeline(h, depth, cg_iters, want_colour, want_normals, count, s);
-    h->pend_emitted.assign(count, 0);
-    for (int k = 0; k < count && e == cudaSuccess; ++k) {
-        bool em = false;
-        e = stage_outputs(h, meshes + k, k, want_colour, want_normals, s, &em);
-        h->pend_emitted[k] = em;
-    }
+    if (e == cudaSuccess) e = stage_outputs(h, meshes, count, want_colour, want_normals, s, h->pend_emitted);
     if (e == cudaSuccess) e = cudaEventRecord(h->done, s);
     if (e != cudaSuccess) return cuda_fail(h, e, "reconstruct");
     h->pending = true;

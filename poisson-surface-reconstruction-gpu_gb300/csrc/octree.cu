@@ -14,7 +14,8 @@ namespace psr {
 // bounding box (mesh/BuildOctree.cu:51-133) and normalisation parameters (:619-631)
 // ------------------------------------------------------------------------------------
 // the counters of a call, and the sort's
-__global__ void k_reset_counters(Counters* c, const InputRef* in, unsigned* sort_bins, float* x) {
+// The call's input reference is read from the host's pinned memory, a slot per cloud.
+__global__ void k_reset_counters(Counters* c, const InputRef* host_in, InputRef* in, unsigned* sort_bins, float* x) {
     PSR_CLOUD(c, in, sort_bins, x);
     static_assert(sizeof(Counters) % 4 == 0, "Counters is cleared word by word");
     unsigned* w = (unsigned*)c;
@@ -23,7 +24,9 @@ __global__ void k_reset_counters(Counters* c, const InputRef* in, unsigned* sort
     __syncthreads();
     if (threadIdx.x == 0) {
         x[-1] = 0.0f;   // the value of absent neighbours
-        c->n_points = in->n;
+        const InputRef ref = host_in[blockIdx.y];
+        *in = ref;
+        c->n_points = ref.n;
         for (int a = 0; a < 3; ++a) {
             // The reference seeds its reduction (padding threads, mesh/BuildOctree.cu:66-73)
             // and its host finish (mesh/BuildOctree.cpp:87-88) with -1e6 / 1e6, which gives a
@@ -640,7 +643,7 @@ cudaError_t octree_build(Workspace& ws) {
     Counters* c = ws.cnt;
     unsigned* err = &c->error;
     unsigned* total = (unsigned*)&c->scan_total;
-    k_reset_counters<<<PSR_GRID(ws, 1), 256, 0, s>>>(c, ws.d_params, ws.sort.bins, ws.xsol);
+    k_reset_counters<<<PSR_GRID(ws, 1), 256, 0, s>>>(c, ws.h_params, ws.d_params, ws.sort.bins, ws.xsol);
     const unsigned *scode = nullptr, *sidx = nullptr;
     cudaError_t e = encode_sort_points(ws, D, &scode, &sidx);
     if (e != cudaSuccess) return e;

@@ -176,7 +176,8 @@ struct Workspace {
     int* part_t;
     int part_cap_v, part_cap_t;
 
-    InputRef* d_params;     // the current call's input (written before each run)
+    InputRef* d_params;     // the current call's input (written by its first kernel)
+    const InputRef* h_params;   // and where that reads it: pinned host memory, one per cloud slot
 
     cudaStream_t stream;
     cudaStream_t aux = nullptr;         // second stream for work forked off `stream`
