@@ -361,14 +361,14 @@ def main():
         cg_bytes += st.level_count[d] * row_bytes * st.cg_iterations[d]
     cg_ms = float(np.mean(cg_samples)) if cg_samples else st.cg_kernel_ms
     roofline = {"bound": "hbm", "kernel": "CG of all depths: k_cg_cluster (depth D on 16 CTAs; D-1, D-2 on 8-CTA "
-                                          "clusters) and k_cg_cta (coarser depths), concurrent, timed together",
+                                          "clusters, a CTA for each coarser depth), concurrent, timed together",
                 "achieved": cg_bytes / (cg_ms * 1e-3) / 1e9 if cg_ms > 0 else None, "peak": peak_hbm,
                 "unit": "GB/s", "frac": None, "traffic": None,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6800 GB/s",
                 "algorithmic_bytes": cg_bytes, "launch_ms": cg_ms,
                 "note": "vectors resident in shared memory, descriptor table in L2 (DRAM traffic ~3 MB per "
                         "reconstruction): the HBM fraction does not bound it",
-                "limiter": "two cluster barriers and the distributed-shared-memory gathers of every iteration",
+                "limiter": "two cluster reductions and the shared-memory gathers of every iteration",
                 "us_per_iteration_depth_d": (1000.0 * st.cg_depth_ms[depth] / st.cg_iterations[depth]
                                              if st.cg_iterations[depth] else None),
                 "sm_ms_per_recon": None}

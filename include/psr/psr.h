@@ -55,7 +55,8 @@ typedef struct psr_config {
                                   corner entries and leaves an indefinite system) */
     int concurrent_stages;     /* 1: the octree-only mesh records and the colour grid run on a
                                   second stream beside the solve (lower latency of one call);
-                                  0: one chain (more throughput when many handles share the
+                                  0: one chain, up to depth 7 with one launch for the solves of
+                                  all depths (more throughput when many handles share the
                                   GPU, as in the served form) */
     int weld_vertices;         /* 1: vertices with bit-identical coordinates become one (the
                                   reference emits the vertices on the boundary of every
@@ -73,7 +74,7 @@ typedef struct psr_config {
                                   octree chain instead of from one cached polynomial per root
                                   (same mesh, slower) */
     int cg_residual_period;    /* CG iterative refinement: the true residual b - A x (exact
-                                  products, double-float sums, FP64 norm) is evaluated every
+                                  products, float-pair and fixed-point sums) is evaluated every
                                   this many iterations and when the recursive residual reaches
                                   the tolerance; the CG restarts from it when it is above the
                                   tolerance and the floor of an FP32 solution (2^-20 ||b||).
@@ -85,11 +86,13 @@ typedef struct psr_config {
                                   them (the clouds' data never mix; each result equals the
                                   one-cloud call's).  Device memory: K x psr_memory_bytes of a
                                   one-cloud handle */
-    int cg_cluster_ctas;       /* CTAs of the thread-block cluster that solves depth D (1..16;
-                                  0: the largest the device schedules, 16 on GB300).  Fewer
+    int cg_cluster_ctas;       /* CTAs of the thread-block cluster that solves depth D <= 7 (1..16;
+                                  0: the largest the device schedules, 16 on GB300, or 8 with
+                                  concurrent_stages = 0, where depth D-1 has as many).  Fewer
                                   CTAs take more rows each: longer per call, less SM time, which
-                                  is what many concurrent reconstructions share */
-    int cg_cluster_ctas_fine;  /* the same for depths D-1 and D-2 (0: 8) */
+                                  is what many concurrent reconstructions share.  Trees of depth 8
+                                  and 9 use the whole GPU */
+    int cg_cluster_ctas_fine;  /* the same for depths D-1 and D-2 with concurrent_stages = 1 (0: 8) */
 } psr_config;
 
 /* Oriented input cloud (the fields of DepthSurfel, base/CommonTypes.h:113-118, as SoA). */

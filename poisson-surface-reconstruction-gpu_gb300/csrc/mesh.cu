@@ -15,11 +15,6 @@ PSR_DEFINE_CONST_TABLES(upload_tables_mesh)
 
 namespace psr {
 
-__device__ __forceinline__ float sqdist3(float ax, float ay, float az, float bx, float by, float bz) {
-    float dx = __fsub_rn(ax, bx), dy = __fsub_rn(ay, by), dz = __fsub_rn(az, bz);
-    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-}
-
 // values behind N 1-based vertex pointers, every load issued before any check (a pointer
 // <= 0 is a broken record: it reads entry 0, yields 1.0f and flags the error)
 template <int N>
@@ -33,13 +28,6 @@ __device__ __forceinline__ void ptr_values(const float* vals, const int (&p)[N],
     if (bad) atomicOr(err, kErrInvalid);
 }
 
-__device__ __forceinline__ void decode3m(int e, int depth, int& ix, int& iy, int& iz) {
-    const int o1 = 1 << (depth + 1);
-    ix = e & (o1 - 1);
-    iy = (e >> (depth + 1)) & (o1 - 1);
-    iz = e >> (2 * (depth + 1));
-}
-
 // vertex slot of a neighbour centre relative to a vertex (mesh/BuildMeshGeometry.cu:133-144)
 __device__ __forceinline__ int vertex_slot(float ncx, float ncy, float ncz, float vx, float vy, float vz) {
     int idx = 0;
@@ -47,19 +35,6 @@ __device__ __forceinline__ int vertex_slot(float ncx, float ncy, float ncz, floa
     if (__fsub_rn(ncz, vz) < 0) idx |= 4;
     if (__fsub_rn(ncy, vy) < 0) idx += (idx & 1) ? 1 : 3;
     return idx;
-}
-
-__device__ __forceinline__ void edge_center(float cx, float cy, float cz, int e, float hw, float out[3]) {
-    const int orient = e >> 2;
-    const int off[2] = {e & 1, (e & 2) >> 1};
-    const float c[3] = {cx, cy, cz};
-    int dim = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        int m = 0;
-        if (orient != a) { m = 2 * off[dim] - 1; dim++; }
-        out[a] = __fadd_rn(c[a], (float)m * hw);
-    }
 }
 
 // Same-depth cells around a vertex, an edge or a face.  Neighbour slot k of a node is the

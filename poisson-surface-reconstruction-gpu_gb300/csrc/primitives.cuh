@@ -7,7 +7,6 @@
 namespace psr {
 
 constexpr int kScanItems = 8;                    // default items per thread
-constexpr int kScanTile = kBlock * kScanItems;   // 2048 elements per default tile
 constexpr int kScanMinTile = kBlock;             // smallest tile (1 item per thread)
 
 // Scratch of the scans: [0] tile counter, [1] blocks finished, [2] epoch, [3 + t] status
@@ -352,11 +351,6 @@ struct StoreExclusive {
         *reinterpret_cast<uint4*>(out + base + 4) = make_uint4(p[4], p[5], p[6], p[7]);
         return true;
     }
-    __device__ void rebase() { PSR_CLOUD(out); }   // to cloud blockIdx.y
-};
-struct StoreInclusive {
-    unsigned* out;
-    __device__ void operator()(int i, unsigned pre, unsigned v) const { out[i] = pre + v; }
     __device__ void rebase() { PSR_CLOUD(out); }   // to cloud blockIdx.y
 };
 

@@ -445,24 +445,6 @@ __device__ __forceinline__ float ff_to_float(FF a) { return __fadd_rn(a.hi, a.lo
 // the pair as one FP64 value (hi and lo are floats, so each converts exactly)
 __device__ __forceinline__ double ff_to_double(FF a) { return (double)a.hi + (double)a.lo; }
 
-// FP64 warp-wide sum (butterfly; IEEE addition is commutative, so every lane ends with the
-// same value, in a fixed order)
-__device__ __forceinline__ double dbl_warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// a / b rounded to float: float quotient of the leading parts, then one correction step
-// with the remainder a - q b evaluated with fused multiply-adds
-__device__ __forceinline__ float ff_div(FF a, FF b) {
-    const float q = __fdiv_rn(a.hi, b.hi);
-    float r = fmaf(-q, b.hi, a.hi);   // exact: a.hi - q * b.hi
-    r = __fadd_rn(r, a.lo);
-    r = fmaf(-q, b.lo, r);
-    return __fadd_rn(q, __fdiv_rn(r, b.hi));
-}
-
 #endif  // __CUDACC__
 
 // Iteration limit of every device-side wait; exceeding it sets kErrSpinTimeout.

@@ -8,12 +8,13 @@
 //
 // CG (mesh/solver/CGAlgorithm.cu:10-80): x0 = 0, r0 = b, stops when r.r <= tol^2 or after
 // max_iter iterations (or after a fixed count).  All depths are independent; they are
-// solved together in concurrent launches of thread-block clusters (see k_cg_cluster).
+// solved together, by thread-block clusters (k_cg_cluster) or, from depth 5 on of trees of
+// depth 8 and 9, by the whole GPU in one cooperative launch (k_cg_grid).
 // Precision: the operator, the vectors and the updates are FP32; the dot products and
-// residual norms are FP64 quantities (exact products, double-float sums within a warp, FP64
-// sums across warps and CTAs, in a fixed order).  Every res_period iterations and when the
+// residual norms are exact products summed as float pairs in a thread and as 57-bit fixed-point
+// integers across lanes, warps and CTAs (CgSum).  Every res_period iterations and when the
 // recursive residual reaches the tolerance, the true residual b - A x of the current x is
-// evaluated (exact products, double-float sums, FP64 norm); it drives iterative refinement:
+// evaluated the same way; it drives iterative refinement:
 // the CG restarts from it when it is above both the tolerance and the floor an FP32
 // solution can reach (2^-20 ||b||) and the recursive residual has converged or drifted.
 //
@@ -31,29 +32,25 @@ namespace cg = cooperative_groups;
 namespace psr {
 
 // ---- per-depth CG ---------------------------------------------------------------------
-// Every depth is an independent system.  The two finest depths (most rows, most
-// iterations) get one thread-block cluster each (k_cg_cluster: cluster barriers, sums
-// through distributed shared memory); the coarser depths get one CTA each (a cluster
-// of one, launched concurrently on a second stream).  Both run the same solver body: a cluster
-// of one CTA is a CTA.
+// Every depth is an independent system.  Up to depth 7 the two or three finest depths (most rows,
+// most iterations) get a thread-block cluster each; the coarser depths get one CTA each (a cluster
+// of one, on a second stream, or a CTA of a further cluster of the same launch).  All run the same
+// solver body: a cluster of one CTA is a CTA.
 //
-// Reductions: every product enters exactly (fma: TwoProduct) into a per-thread float pair,
-// warp butterflies sum the pairs (FF arithmetic on the FP32 pipes), one warp per CTA sums
-// the 32 warp partials in FP64 and writes the CTA's sum to its shared memory, and after
-// the barrier one warp of every CTA sums the CTAs' values in FP64 in a fixed order, so
-// every CTA holds the same result.  GB300 executes FP64 at a small fraction of its FP32
-// rate (an FP64 add per element cost 2.4 us per reduction against 0.3 us for the
-// cluster barrier), so FP64 arithmetic is kept to the 32 + 16 values of the cross-warp
-// and cross-CTA steps; the in-warp pairs carry about 44 bits, more than the reference's
-// float-rounded products summed in double (mesh/solver/CGAlgorithm.cu:106-133).  The
-// scalars of an iteration (alpha, beta, the continue flag) are computed once, by the
-// thread that finishes the sum, and read by every thread from shared memory.  The
-// partial buffers alternate between two slots, so a slot is only rewritten after a
-// barrier that follows its reads.
+// Reductions: every product enters exactly (fma: TwoProduct) into a per-thread float pair; a warp
+// adds its lanes' pairs as integers in three pieces aligned to the largest, a CTA its warps' and a
+// cluster its CTAs' sums as 57-bit integers (CgSum), which keeps more than the reference's
+// float-rounded products summed in double (mesh/solver/CGAlgorithm.cu:106-133) and stays off the
+// FP64 pipes (a dependent FP64 add takes 76 cycles here, an integer warp reduction about 50).  A CTA's
+// sum goes to every CTA of the cluster with st.async, whose arrival on an mbarrier is the barrier
+// (836 cycles; a cluster barrier and reads of the others' sums 1,442).  The scalars of an iteration
+// (alpha, beta, the continue flag) are computed once per CTA, by the thread that finishes the sum,
+// and read by every thread from shared memory.  The sums alternate between two slots, so a slot is
+// only rewritten after a reduction that follows its reads.
 //
 // True residual (iterative refinement): every res_period iterations, and when the
 // recursive r.r reaches tol^2, each row's b - sum_k st_k x[nb_k] is evaluated with exact
-// products and float-pair sums (staged in the A p buffer) and its FP64 norm is taken.  With
+// products and float-pair sums (staged in the A p buffer) and its norm is taken.  With
 // the reference's absolute tolerance (1e-5) and right-hand sides of norm ~1e7, the FP32
 // recursion ends with a true residual near 1e-7 ||b||, below what an FP32 x can resolve
 // (2^-20 ||b||, 16 ulps of b); refinement restarts the CG from the true residual only
@@ -64,7 +61,7 @@ namespace psr {
 // true residual at the FP32 floor with a recursive one far below it and the iteration
 // stalls (it ran to the 10,000-iteration cap on the depth-3 system of the superquadric).
 //
-// One iteration costs two barriers: the direction update p = r + beta p is fused into the
+// One iteration costs two reductions: the direction update p = r + beta p is fused into the
 // operator application (a row's neighbours rebuild their p values from r and the
 // previous p), so the FP32 operations per element are the textbook loop's:
 //   p_k = fma(beta, p_{k-1}, r_k)   Ap = sum_k st_k p_k[nb]   alpha = rr / (p.Ap)
@@ -172,7 +169,7 @@ struct CgcShared {
     int until_check;    // iterations until the next periodic true residual
     float st[27];
 };
-static_assert(kCgWarps == 32, "one FP64 lane per warp partial");
+static_assert(kCgWarps == 32, "one lane per warp sum");
 static_assert(kCgSmemBytes + sizeof(CgcShared) <= 227 * 1024, "shared memory of one CTA");
 static_assert(kCgGroups <= 2048, "11 bits of a packed neighbour group");
 

@@ -14,14 +14,6 @@ PSR_DEFINE_CONST_TABLES(upload_tables_transfer)
 namespace psr {
 
 
-__device__ __forceinline__ unsigned morton3(int x, int y, int z, int g) {
-    unsigned m = 0;
-    for (int l = 0; l < g; ++l)
-        m |= (((unsigned)(x >> l) & 1u) << (3 * l + 2)) | (((unsigned)(y >> l) & 1u) << (3 * l + 1)) |
-             (((unsigned)(z >> l) & 1u) << (3 * l));
-    return m;
-}
-
 // (d, i) lexicographic order: smaller squared distance first, then lower sample index
 __device__ __forceinline__ bool knn_less(float da, int ia, float db, int ib) {
     return da < db || (da == db && ia < ib);
