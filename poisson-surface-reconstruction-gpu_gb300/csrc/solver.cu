@@ -844,9 +844,11 @@ __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
 // 0.28M rows takes 10 us, of 1.2M 19 us and of 3.1M 41 us; with a whole-GPU barrier per step and the
 // sums read after it 11, 20 and 49 us, and as kernels in a CUDA-graph while node (7 launches per two
 // iterations) 27, 43 and 97 us.  What is left: 4k to 6k cycles per step for records to travel through
-// L2, and in A p the gather of 64 (r, p) pairs a group (8k cycles per 512 groups).  Keeping the
-// block's p in shared memory and reading only other blocks' groups from L2 was slower (5.0 ms a solve
-// against 3.4 of 3.1M rows): the scattered remote reads wait one by one.
+// L2, and in A p the gather of 64 (r, p) pairs a group (8k cycles per 512 groups).  Not kept:
+// the block's p in shared memory with other blocks' groups read from L2 (5.0 ms a solve against 3.4 of
+// 3.1M rows: the scattered reads wait one by one) or copied beside it every round (the gather falls to
+// 5.5k cycles, the copies and their block barrier take what it saves); the planes of the gather
+// pipelined by hand, 640 threads, virtual blocks of 128 (the same to 8% slower).
 constexpr int kGridBlock = 512;    // 128 registers a thread: a group's 27 neighbours and 32 loads in flight
 constexpr int kVbGroups = 256;                       // groups of a virtual block
 constexpr int kGridSubs = kGridBlock / kVbGroups;    // virtual blocks a block works on at once
