@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kBlock) k_na_encode(const float* xyz, NoAllocS
                 if (p[a] > cc[a]) { k |= 1u << (3 * l + 2 - a); cc[a] = __fadd_rn(cc[a], w); }
                 else cc[a] = __fsub_rn(cc[a], w);
             }
-            w = __fdiv_rn(w, 2.0f);
+            w = __fmul_rn(w, 0.5f);
         }
         code[i] = k;
         count.count(k);

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kBlock) k_encode(const InputRef* in, Counters*
                 if (p[a] > cc[a]) { k |= 1u << (3 * l + 2 - a); cc[a] = __fadd_rn(cc[a], w); }
                 else cc[a] = __fsub_rn(cc[a], w);
             }
-            w = __fdiv_rn(w, 2.0f);
+            w = __fmul_rn(w, 0.5f);
         }
         code[i] = k;
         count.count(k);
@@ -267,11 +267,16 @@ struct LeafPlaceStore {
 // (mesh/BuildOctree.cu:323-357), a scan over the groups that start a new father group gives the
 // father groups' addresses one level up (:359-375, :796-799), and every father goes to its slot
 // with the empty slots up to the next father's (:377-390).
+// the 8 entries of a group (a group starts on a 32-byte boundary of its array)
+__device__ __forceinline__ void load8(const int* p, int (&v)[8]) {
+    const int4 a = *reinterpret_cast<const int4*>(p), b = *reinterpret_cast<const int4*>(p + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
 // first non-empty slot of group g's 8 (the father's key is its key without the sibling bits)
 __device__ __forceinline__ int group_father_key(const LevelArrays& T, int base, int sh) {
     int pn[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) pn[j] = T.pnum[base + j];
+    load8(T.pnum + base, pn);
     int at = -1;
 #pragma unroll
     for (int j = 7; j >= 0; --j)
@@ -287,18 +292,24 @@ struct LevelLoad {
         const int off = c->level_tmp_off[d];
         const int sh = 3 * (depth - d), sh2 = 3 * (depth - d + 2);
         int fk = 0, pn = 0, pi = 0x7fffffff, dn = 0, di = 0x7fffffff;
+        const int t = off + 8 * g;
+        int pnum[8], dnum[8], didx[8], key[8], pidx[8];
+        load8(T.pnum + t, pnum);
+        load8(T.dnum + t, dnum);
+        load8(T.didx + t, didx);
+        load8(T.key + t, key);
+        load8(T.pidx + t, pidx);
+        const int before = g > 0 ? group_father_key(T, t - 8, sh) : 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const int t = off + 8 * g + j;
-            const int pnum = T.pnum[t], dnum = T.dnum[t], didx = T.didx[t], key = T.key[t], pidx = T.pidx[t];
-            if (pnum == 0) {
-                if (dnum != 0) { dn += dnum; di = min(di, didx); }
+            if (pnum[j] == 0) {
+                if (dnum[j] != 0) { dn += dnum[j]; di = min(di, didx[j]); }
             } else {
-                fk = key & ~(7 << sh);
-                pn += pnum;
-                pi = min(pi, pidx);
-                dn += dnum;
-                di = min(di, didx);
+                fk = key[j] & ~(7 << sh);
+                pn += pnum[j];
+                pi = min(pi, pidx[j]);
+                dn += dnum[j];
+                di = min(di, didx[j]);
             }
         }
         gkey[g] = fk;
@@ -307,7 +318,7 @@ struct LevelLoad {
         gdidx[g] = di;
         gdnum[g] = dn;
         if (g == 0) return 0u;
-        return ((group_father_key(T, off + 8 * (g - 1), sh) >> sh2) != (fk >> sh2)) ? 8u : 0u;
+        return ((before >> sh2) != (fk >> sh2)) ? 8u : 0u;
     }
     __device__ void rebase() { PSR_CLOUD(c, T, gkey, gpidx, gpnum, gdidx, gdnum); }   // to cloud blockIdx.y
 };
@@ -583,7 +594,7 @@ __global__ void __launch_bounds__(kBlock) k_finalize_nodes(const Counters* c, in
                 if ((k >> (3 * l + 2 - a)) & 1) cc[a] = __fadd_rn(cc[a], w);
                 else cc[a] = __fsub_rn(cc[a], w);
             }
-            w = __fdiv_rn(w, 2.0f);
+            w = __fmul_rn(w, 0.5f);
         }
         cx[i] = cc[0];
         cy[i] = cc[1];
