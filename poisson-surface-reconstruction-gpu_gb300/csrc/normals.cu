@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned
                         cnt = cell_start[(size_t)(m + 1) << (3 * up)] - base;
                     }
                 }
-                list_range8(gmask, cnt, base, s_off[gib], s_base[gib], used, running);
+                list_range<8>(gmask, cnt, base, s_off[gib], s_base[gib], used, running);
             }
             if (lane == 0) s_off[gib][used] = 0x7fffffff;
             __syncwarp(gmask);

@@ -22,29 +22,30 @@ struct ScanScratch {
 };
 constexpr int kScanHeader = 3;
 
-// Flattens ranges over the 8 lanes of a group (mask gmask): each lane hands in one range per call
+// Flattens ranges over the kLanes lanes of a group (mask gmask): each lane hands in one range per call
 // (cnt elements from `base`), ranges in lane order, call after call.  Only ranges with elements are
 // listed: list entry j starts at flat index off[j], and element t of it is t + from[j].  After the
 // last call one lane sets off[used] = 0x7fffffff, so that a walk over increasing t needs no other end.
 // Every lane walks the list, which is why it is short: of 27 cells around a surface point two thirds
 // are empty.
-__device__ __forceinline__ void list_range8(unsigned gmask, int cnt, int base, int* off, int* from, int& used,
-                                            int& running) {
-    const int lane = threadIdx.x & 7;
+template <int kLanes>
+__device__ __forceinline__ void list_range(unsigned gmask, int cnt, int base, int* off, int* from, int& used,
+                                           int& running) {
+    const int lane = threadIdx.x & (kLanes - 1);
     int incl = cnt;
 #pragma unroll
-    for (int q = 1; q < 8; q <<= 1) {
-        const int y = __shfl_up_sync(gmask, incl, q, 8);
+    for (int q = 1; q < kLanes; q <<= 1) {
+        const int y = __shfl_up_sync(gmask, incl, q, kLanes);
         if (lane >= q) incl += y;
     }
-    const unsigned some = __ballot_sync(gmask, cnt > 0) >> (threadIdx.x & 24);
+    const unsigned some = (__ballot_sync(gmask, cnt > 0) & gmask) >> (threadIdx.x & 31 & ~(kLanes - 1));
     if (cnt > 0) {
         const int at = used + __popc(some & ((1u << lane) - 1u));
         off[at] = running + incl - cnt;
         from[at] = base - (running + incl - cnt);
     }
-    used += __popc(some & 0xffu);
-    running += __shfl_sync(gmask, incl, 7, 8);
+    used += __popc(some);
+    running += __shfl_sync(gmask, incl, kLanes - 1, kLanes);
 }
 
 // optional count written by the last tile: min(total, cap) (overflow flags kErrCapacity)

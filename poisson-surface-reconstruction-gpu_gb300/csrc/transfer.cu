@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kBlock) k_colour_near(Counters* c, int gt, con
                                                    (float)(cz + k % 3 - 1) * w, w);
                     if (k == 13 || d2 > md[3]) cnt[r] = 0;
                 }
-                list_range8(gmask, cnt[r], base[r], s_off[gib], s_base[gib], used, running);
+                list_range<8>(gmask, cnt[r], base[r], s_off[gib], s_base[gib], used, running);
             }
             if (lane == 0) s_off[gib][used] = 0x7fffffff;
             __syncwarp(gmask);
