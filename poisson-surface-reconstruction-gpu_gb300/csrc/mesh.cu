@@ -155,8 +155,9 @@ __global__ void __launch_bounds__(kBlock) k_mesh_owners(const Counters* c, int d
         for (int k = 0; k < 12; ++k) node_edge[(size_t)k * stride + i] = 0;
 #pragma unroll
         for (int k = 0; k < 6; ++k) node_face[(size_t)k * stride + i] = 0;
+        if (i < bD)   // only nodes with children are looked up there
 #pragma unroll
-        for (int k = 0; k < 8; ++k) { ov_group[(size_t)k * stride + i] = -1; ov_sub[(size_t)k * stride + i] = -1; }
+            for (int k = 0; k < 8; ++k) { ov_group[(size_t)k * stride + i] = -1; ov_sub[(size_t)k * stride + i] = -1; }
     }
 }
 

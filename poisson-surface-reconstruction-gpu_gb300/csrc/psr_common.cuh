@@ -421,7 +421,13 @@ __device__ __forceinline__ FF ff_add(FF a, FF b) {
     return FF{h, __fsub_rn(e, __fsub_rn(h, s))};
 }
 
-__device__ __forceinline__ FF ff_add_float(FF a, float b) { return ff_add(a, FF{b, 0.0f}); }
+__device__ __forceinline__ FF ff_add_float(FF a, float b) {   // ff_add(a, FF{b, 0})
+    const float s = __fadd_rn(a.hi, b);
+    const float bv = __fsub_rn(s, a.hi);
+    const float e = __fadd_rn(__fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bv)), __fsub_rn(b, bv)), a.lo);
+    const float h = __fadd_rn(s, e);
+    return FF{h, __fsub_rn(e, __fsub_rn(h, s))};
+}
 
 // exact product of two floats as a float pair
 __device__ __forceinline__ FF ff_prod(float a, float b) {
