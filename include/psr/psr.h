@@ -88,11 +88,13 @@ typedef struct psr_config {
                                   one-cloud handle */
     int cg_cluster_ctas;       /* CTAs of the thread-block cluster that solves depth D <= 7 (1..16;
                                   0: the largest the device schedules, 16 on GB300, or 8 with
-                                  concurrent_stages = 0, where depth D-1 has as many).  Fewer
+                                  concurrent_stages = 0, where depth D-1 has as many, and for
+                                  batches of more clouds than the SMs hold).  Fewer
                                   CTAs take more rows each: longer per call, less SM time, which
                                   is what many concurrent reconstructions share.  Trees of depth 8
                                   and 9 use the whole GPU */
-    int cg_cluster_ctas_fine;  /* the same for depths D-1 and D-2 with concurrent_stages = 1 (0: 8) */
+    int cg_cluster_ctas_fine;  /* the same for depths D-1 and D-2 with concurrent_stages = 1 (0: 8, or 4
+                                  for such batches) */
 } psr_config;
 
 /* Oriented input cloud (the fields of DepthSurfel, base/CommonTypes.h:113-118, as SoA). */

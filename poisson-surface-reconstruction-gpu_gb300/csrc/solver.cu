@@ -1629,9 +1629,14 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     const bool whole = D >= 8;
     const int ncl = whole ? 0 : (D < 2 ? D : (D >= 5 ? 3 : 2));
     const int ncta = whole ? kGridDepth : D - ncl + 1;
-    int cl1 = ws.cg_ctas > 0 ? ws.cg_ctas : g_cg_cluster;
+    // Where the clouds of a launch need more SMs than there are, SM time counts, not the latency of a
+    // solve: half the CTAs, which hold 114,688 and 57,344 rows in shared memory (16 clouds of depth 7:
+    // 4.55 ms a batch with 16 and 8 CTAs, 4.27 with 16 and 4, 4.39 with 8 and 8, 4.15 with 8 and 4, 4.29
+    // with 8 and 2).
+    const bool crowded = ws.batch * (g_cg_cluster + 2 * 8 + ncta) > ws.num_sms;
+    int cl1 = ws.cg_ctas > 0 ? ws.cg_ctas : (crowded && g_cg_cluster > 8 ? 8 : g_cg_cluster);
     if (cl1 > g_cg_cluster) cl1 = g_cg_cluster;
-    int cl2 = ws.cg_ctas_fine > 0 ? ws.cg_ctas_fine : 8;
+    int cl2 = ws.cg_ctas_fine > 0 ? ws.cg_ctas_fine : (crowded ? 4 : 8);
     if (cl2 > g_cg_cluster) cl2 = g_cg_cluster;
     const size_t cstride = (size_t)ws.cap.dnodes / 8 + 64;
     const PointCoarse coarse{ws.parent, ws.ctr_x, ws.ctr_y, ws.ctr_z, ws.pv_coef, cstride};
