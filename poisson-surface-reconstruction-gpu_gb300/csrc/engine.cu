@@ -691,8 +691,8 @@ static cudaError_t launch_pipeline(psr_handle* h, int depth, int cg_iters, int w
     return e;
 }
 
-// Whether the kernels may read the caller's array in place: memory of the handle's device (or
-// managed).  Anything else is staged by a copy, which reports what it cannot read.
+// Whether the kernels may read the caller's array in place: device memory of the handle's device.
+// Anything else is staged by a copy, which reports what it cannot read.
 static bool readable_in_place(const psr_handle* h, const void* p) {
     if (!p) return true;
     cudaPointerAttributes at;
