@@ -129,6 +129,7 @@ typedef CUresult (*PfnRelease)(CUmemGenericAllocationHandle);
 typedef CUresult (*PfnMap)(CUdeviceptr, size_t, size_t, CUmemGenericAllocationHandle, unsigned long long);
 typedef CUresult (*PfnUnmap)(CUdeviceptr, size_t);
 typedef CUresult (*PfnSetAccess)(CUdeviceptr, size_t, const CUmemAccessDesc*, size_t);
+typedef CUresult (*PfnAttributes)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
 
 struct VmmApi {
     PfnGranularity granularity = nullptr;
@@ -140,6 +141,7 @@ struct VmmApi {
     PfnUnmap unmap = nullptr;
     PfnSetAccess set_access = nullptr;
     bool ok = false;
+    PfnAttributes attributes = nullptr;   // not one of the calls that `ok` speaks for
 };
 
 const VmmApi& vmm() {
@@ -155,6 +157,7 @@ const VmmApi& vmm() {
                get("cuMemCreate", (void**)&a.create) && get("cuMemRelease", (void**)&a.release) &&
                get("cuMemMap", (void**)&a.map) && get("cuMemUnmap", (void**)&a.unmap) &&
                get("cuMemSetAccess", (void**)&a.set_access);
+        if (!get("cuPointerGetAttributes", (void**)&a.attributes)) a.attributes = nullptr;
         return a;
     }();
     return api;
@@ -691,16 +694,24 @@ static cudaError_t launch_pipeline(psr_handle* h, int depth, int cg_iters, int w
     return e;
 }
 
-// Whether the kernels may read the caller's array in place: device memory of the handle's device.
-// Anything else is staged by a copy, which reports what it cannot read.
-static bool readable_in_place(const psr_handle* h, const void* p) {
+// Whether the kernels may read the caller's `bytes` at p in place: device memory of the handle's
+// device, on the boundary that loads of its elements need, and all of it inside one allocation.
+// Anything else is staged by a copy, which takes any address and reports what it cannot read.
+static bool readable_in_place(const psr_handle* h, const void* p, size_t bytes, size_t align) {
     if (!p) return true;
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return at.type == cudaMemoryTypeDevice && at.device == h->cfg.device;
+    const PfnAttributes attributes = vmm().attributes;
+    if ((size_t)p % align != 0 || !attributes) return false;
+    unsigned type = 0, managed = 0;
+    int device = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* data[] = {&type, &managed, &device, &start, &size};
+    if (attributes(5, which, data, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    const size_t at = (size_t)((CUdeviceptr)p - start);
+    return type == CU_MEMORYTYPE_DEVICE && !(managed & 0xffu) && device == h->cfg.device && at <= size && bytes <= size - at;
 }
 
 // Enqueues the input reference of slot k: the caller's device arrays themselves (the sort reads
@@ -711,14 +722,16 @@ static cudaError_t stage_inputs(psr_handle* h, const psr_points* pts, int k, cud
     const int n = pts->count;
     InputRef* hp = h->h_params + k;
     cudaError_t e = cudaSuccess;
-    if (pts->location == PSR_DEVICE && readable_in_place(h, pts->xyz) && readable_in_place(h, pts->normals) &&
-        readable_in_place(h, pts->rgb)) {
+    const size_t floats = 3 * sizeof(float) * (size_t)n;
+    if (pts->location == PSR_DEVICE && readable_in_place(h, pts->xyz, floats, alignof(float)) &&
+        readable_in_place(h, pts->normals, floats, alignof(float)) &&
+        readable_in_place(h, pts->rgb, 3 * (size_t)n, 1)) {
         *hp = InputRef{pts->xyz, pts->normals, pts->rgb, n};
     } else {
         const cudaMemcpyKind kind = (pts->location == PSR_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         *hp = InputRef{slot_ptr(ws.in_xyz, k), slot_ptr(ws.in_nrm, k), pts->rgb ? slot_ptr(ws.in_rgb, k) : nullptr, n};
-        e = cudaMemcpyAsync((void*)hp->xyz, pts->xyz, 3 * sizeof(float) * (size_t)n, kind, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync((void*)hp->nrm, pts->normals, 3 * sizeof(float) * (size_t)n, kind, s);
+        e = cudaMemcpyAsync((void*)hp->xyz, pts->xyz, floats, kind, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync((void*)hp->nrm, pts->normals, floats, kind, s);
         if (e == cudaSuccess && pts->rgb) e = cudaMemcpyAsync((void*)hp->rgb, pts->rgb, 3 * (size_t)n, kind, s);
     }
     return e;   // the pipeline's first kernel reads *hp
