@@ -75,6 +75,13 @@ __device__ __forceinline__ unsigned nrm_spread3(unsigned v) {
     v = (v | (v << 2)) & 0x09249249u;
     return v;
 }
+__device__ __forceinline__ int nrm_compact3(unsigned v) {   // the inverse, of every third bit
+    v &= 0x09249249u;
+    v = (v | (v >> 2)) & 0x030c30c3u;
+    v = (v | (v >> 4)) & 0x0300f00fu;
+    v = (v | (v >> 8)) & 0x030000ffu;
+    return (int)((v | (v >> 16)) & 0x3ffu);
+}
 __device__ __forceinline__ unsigned nrm_morton(int a, int b, int z) {
     return (nrm_spread3((unsigned)a) << 2) | (nrm_spread3((unsigned)b) << 1) | nrm_spread3((unsigned)z);
 }
@@ -136,13 +143,16 @@ __global__ void __launch_bounds__(kBlock) k_nrm_cells(Counters* c, const unsigne
 // at level 7 and, while that does not settle the point, at coarser levels (their cells are ranges
 // of the same table).  A level settles it when K points were found and the K-th is closer than one
 // cell width (every point outside the block is at least one width away).  A block with fewer than
-// K points is not scanned; one with more than kNrmNearCap, or a point that level kNrmNearCoarsest
-// leaves, goes to the far list.  Without the coarser levels a cloud whose spacing exceeds the level-7
-// cells went to the far pass point by point, a block each: 1.06 ms of 31k points, now part of the
-// 25 us of this pass.
+// K points is not scanned; a coarser one with more than kNrmNearCap, or a point that level
+// kNrmNearCoarsest leaves, goes to the far list.  Without the coarser levels a cloud whose spacing
+// exceeds the level-7 cells went to the far pass point by point, a block each: 1.06 ms of 31k points,
+// now part of the 25 us of this pass.  The cap is not for level 7, where eight lanes are the cheaper
+// form however crowded the block is: with it there, 4,000,000 points of a sphere took 122 ms instead of
+// 27.3, and 200,000 of a ground scan that thins out with the distance 11.7 ms instead of 4.9.  Four
+// blocks per SM (64 registers; at 75 and three 1,000,000 points took 2.90 ms instead of 2.67).
 constexpr int kNrmNearCap = 1024;
 constexpr int kNrmNearCoarsest = 3;
-__global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned* scode, const float* px,
+__global__ void __launch_bounds__(kBlock, 4) k_nrm_near(Counters* c, const unsigned* scode, const float* px,
                                                      const float* py, const float* pz, const int* cell_start,
                                                      int* nbr, int* far) {
     __shared__ int s_off[kNrmGroups][28];
@@ -155,25 +165,20 @@ __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned
     const int ngroups = (gridDim.x * blockDim.x) / kNrmLanes;
     for (int p = group; p < n; p += ngroups) {
         const float qx = px[p], qy = py[p], qz = pz[p];
-        // the point's cell from its code (x = bit 2 of every triple)
-        const unsigned code = scode[p];
-        int cxyz[3] = {0, 0, 0};
-#pragma unroll
-        for (int l = 0; l < kNrmGridLevel; ++l)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) cxyz[a] |= (int)((code >> (3 * l + 2 - a)) & 1u) << l;
         bool settled = false;
         for (int g = kNrmGridLevel; g >= kNrmNearCoarsest; --g) {   // uniform in the group
             const int G = 1 << g, up = kNrmGridLevel - g;
-            const float w = 1.0f / (float)G;
+            // the point's cell from its code (x = bit 2 of every triple), at every level anew: kept across
+            // the search it takes registers of a block
+            const unsigned code = scode[p] >> (3 * up);
+            const int cx = nrm_compact3(code >> 2), cy = nrm_compact3(code >> 1), cz = nrm_compact3(code);
             int running = 0, used = 0;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int k = lane + kNrmLanes * r;
                 int cnt = 0, base = 0;
                 if (k < 27) {
-                    const int a = (cxyz[0] >> up) + k / 9 - 1, b = (cxyz[1] >> up) + (k / 3) % 3 - 1,
-                              z = (cxyz[2] >> up) + k % 3 - 1;
+                    const int a = cx + k / 9 - 1, b = cy + (k / 3) % 3 - 1, z = cz + k % 3 - 1;
                     if (a >= 0 && a < G && b >= 0 && b < G && z >= 0 && z < G) {
                         const unsigned m = nrm_morton(a, b, z);
                         base = cell_start[(size_t)m << (3 * up)];
@@ -184,7 +189,7 @@ __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned
             }
             if (lane == 0) s_off[gib][used] = 0x7fffffff;
             __syncwarp(gmask);
-            if (running > kNrmNearCap) break;
+            if (g < kNrmGridLevel && running > kNrmNearCap) break;
             if (running < kNrmK && running < n) continue;   // the K-th is farther out
             float bd[kNrmK];
             int bi[kNrmK];
@@ -199,6 +204,7 @@ __global__ void __launch_bounds__(kBlock) k_nrm_near(Counters* c, const unsigned
             float md[kNrmK];
             int mi[kNrmK];
             nrm_group_merge<kNrmK>(bd, bi, md, mi, gmask, kNrmLanes);
+            const float w = __int_as_float((127 - g) << 23);   // 1 / G
             // fewer than K points in the whole cloud: all of them are the neighbours
             if (md[kNrmK - 1] < w * w || running == n) {
                 if (lane == 0) {
