@@ -28,13 +28,14 @@ __device__ __forceinline__ float bspline32(float t) {
     return a < 0.5f ? inner : (a < 1.5f ? outer : 0.0f);
 }
 
-// 4 lanes per D-level node (8 nodes per warp): the 27 neighbours' sample ranges are
+// 8 lanes per D-level node (4 nodes per warp): the 27 neighbours' sample ranges are
 // flattened over the group's lanes (a group scan gives the range offsets), every lane
-// accumulates its samples' weighted normals in two of eight interleaved sums, and the eight are
-// added in a fixed order.  Bound by instruction issue: a node has about ten samples, so eight lanes
-// left a third of the second round idle and listed the ranges for four nodes at a time (field stage
-// 2.15 -> 2.12 ms for 2,000,000 samples, depth 9; the sums are the same).
-constexpr int kVfLanes = 4;
+// accumulates its samples' weighted normals and a butterfly over the group combines the lanes (fixed
+// order).  Bound by instruction issue.  Four lanes with two of the eight sums each are 1.7% faster in
+// the field stage of 2,000,000 samples at depth 9 (1.67 against 1.70 ms), where a node has about ten
+// samples around it, and slower wherever it has more: 200,000 samples at depth 6 84 against 70 us,
+// 2,000,000 745 against 367.
+constexpr int kVfLanes = 8;
 constexpr int kVfGroups = kBlock / kVfLanes;
 __global__ void __launch_bounds__(kBlock) k_vector_field(const Counters* c, int depth, const float* px, const float* py,
                                                          const float* pz, const float* nx, const float* ny,
@@ -50,7 +51,7 @@ __global__ void __launch_bounds__(kBlock) k_vector_field(const Counters* c, int 
     const float s = (float)(1 << depth);
     const int lane = threadIdx.x & (kVfLanes - 1);
     const int gib = threadIdx.x / kVfLanes;
-    const unsigned gmask = 0xfu << (threadIdx.x & 28);   // the group's lanes in its warp
+    const unsigned gmask = 0xffu << (threadIdx.x & 24);   // the group's lanes in its warp
     const int group = (blockIdx.x * blockDim.x + threadIdx.x) / kVfLanes;
     const int ngroups = (gridDim.x * blockDim.x) / kVfLanes;
     for (int o = group; o < md; o += ngroups) {
@@ -58,7 +59,7 @@ __global__ void __launch_bounds__(kBlock) k_vector_field(const Counters* c, int 
         const float ox = cx[i], oy = cy[i], oz = cz[i];
         int running = 0, used = 0;
 #pragma unroll
-        for (int r = 0; r < 7; ++r) {
+        for (int r = 0; r < 4; ++r) {
             const int k = lane + kVfLanes * r;
             int cnt = 0, base = 0;
             if (k < 27) {
@@ -69,24 +70,16 @@ __global__ void __launch_bounds__(kBlock) k_vector_field(const Counters* c, int 
         }
         if (lane == 0) s_off[gib][used] = 0x7fffffff;
         __syncwarp(gmask);
-        float ax = 0.f, ay = 0.f, az = 0.f, bx = 0.f, by = 0.f, bz = 0.f;
+        float ax = 0.f, ay = 0.f, az = 0.f;
         int k = 0;
-        auto add = [&](int t, float& sx, float& sy, float& sz) {
+        for (int t = lane; t < running; t += kVfLanes) {
             while (s_off[gib][k + 1] <= t) ++k;
             const int p = t + s_base[gib][k];
             const float w = bspline32((px[p] - ox) * s) * bspline32((py[p] - oy) * s) * bspline32((pz[p] - oz) * s);
-            sx = fmaf(w, nx[p], sx);
-            sy = fmaf(w, ny[p], sy);
-            sz = fmaf(w, nz[p], sz);
-        };
-        // a lane keeps two of eight interleaved sums
-        for (int t = lane; t < running; t += 2 * kVfLanes) {
-            add(t, ax, ay, az);
-            if (t + kVfLanes < running) add(t + kVfLanes, bx, by, bz);
+            ax = fmaf(w, nx[p], ax);
+            ay = fmaf(w, ny[p], ay);
+            az = fmaf(w, nz[p], az);
         }
-        ax += bx;
-        ay += by;
-        az += bz;
 #pragma unroll
         for (int q = kVfLanes / 2; q > 0; q >>= 1) {
             ax += __shfl_xor_sync(gmask, ax, q);
