@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
     const int sub = tid / kVbGroups, subt = tid % kVbGroups;
     const int per = a.first - a.last + 1, nu = per * a.clouds;
     const unsigned long long t0 = global_ns();
-    unsigned* err = &a.v.cw->error;
+    auto fail = [&](int k, unsigned bits) { atomicOr(&at_cloud(a.v.cw, k)->error, bits); };
     // the units: cloud after cloud, depth after depth
     for (int u = tid; u < nu; u += kGridBlock) {
         CgGridUnit& q = U[u];
@@ -995,7 +995,8 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
     __syncthreads();
     const int total = s_total;
     if (total > a.part_cap) {   // uniform over the launch
-        if (blockIdx.x == 0 && tid == 0) atomicOr(err, kErrCapacity);
+        if (blockIdx.x == 0)
+            for (int k = tid; k < a.clouds; k += kGridBlock) fail(k, kErrCapacity);
         return;
     }
     // this block's virtual blocks, and the units they belong to
@@ -1303,7 +1304,10 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             q.resid = 0;
         });
     }
-    if (tid == 0 && (!ok || round >= most)) atomicOr(err, kErrSpinTimeout);
+    // a wait ran out: the block's units are unfinished, and with them those of every other block that
+    // waits for its records, so the clouds of all its units fail
+    if (!ok || round >= most)
+        for (int u = u0 + tid; u < u1; u += kGridBlock) fail(U[u].k, kErrSpinTimeout);
     // x in row order; the reports by the block that holds a unit's first virtual block
     for (int p = 0; p < npass; ++p) {
         const int vb = v0 + p * kGridSubs + sub;
