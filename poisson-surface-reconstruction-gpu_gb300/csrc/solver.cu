@@ -892,7 +892,6 @@ struct CgGridUnit {
     int G0, ng;           // first group (global number), groups
     int vb0, nvb;         // first virtual block of the launch, virtual blocks
     float w[4];           // centre, face, edge, corner
-    float own[8];         // p of the first group's rows where its table does not name itself
 };
 
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
@@ -1229,7 +1228,7 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
                 for (int q = 0; q < 16; ++q) {
                     const int p = 16 * bx + q;
                     const float v = fmaf(beta, e[q].y, e[q].x);
-                    if (cg_pos_group(p) == 13) pi[cg_pos_sib(p)] = v;   // the group itself, as its table says
+                    if (cg_pos_group(p) == 13) pi[cg_pos_sib(p)] = v;   // the group itself
 #pragma unroll
                     for (int s = 0; s < 8; ++s) {
                         const int ox = (p >> 4) - (s >> 2), oy = ((p >> 2) & 3) - ((s >> 1) & 1), oz = (p & 3) - (s & 1);
@@ -1243,11 +1242,16 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
                 ap[s * aps] = y[s];
                 acc = ff_add(acc, ff_prod(pi[s], y[s]));
             }
-            // Only a unit's first group can have a table that does not name the group itself (its
-            // parent is recorded as the first node of the level above): its p is what the table says
+            // Only a unit's first group can have a table that does not name the group itself (its parent is
+            // recorded as the first node of the level above): the operator takes what the table says,
+            // the rows' own p their own pairs
             if (g == 0 && nb[13] != (unsigned)G) {
-#pragma unroll
-                for (int s = 0; s < 8; ++s) q.own[s] = pi[s];
+                acc = ff_zero();
+#pragma unroll 1
+                for (int s = 0; s < 8; ++s) {
+                    const float2 o = rp[(unsigned)s * a.pitch + (unsigned)G];
+                    acc = ff_add(acc, ff_prod(fmaf(beta, o.y, o.x), ap[s * aps]));
+                }
             }
             return acc;
         });
@@ -1277,7 +1281,6 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             }
             float* xs = at_cloud(a.xs, q.k) + G;
             const float alpha = q.alpha, beta = q.beta;
-            const bool self = g != 0 || at_cloud(a.nbg, q.k)[13 * a.pitch + G] == G;
             float2 own[8];
             float xo[8], y[8];
 #pragma unroll
@@ -1288,7 +1291,7 @@ __global__ void __launch_bounds__(kGridBlock) k_cg_grid(CgGridArgs a) {
             }
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
-                const float pi = self ? fmaf(beta, own[s].y, own[s].x) : q.own[s];
+                const float pi = fmaf(beta, own[s].y, own[s].x);
                 xs[s * a.pitch] = fmaf(alpha, pi, xo[s]);
                 const float ri = fmaf(-alpha, y[s], own[s].x);
                 rp[s * a.pitch] = make_float2(ri, pi);
