@@ -37,11 +37,15 @@ namespace psr {
 // of one, on a second stream, or a CTA of a further cluster of the same launch).  All run the same
 // solver body: a cluster of one CTA is a CTA.
 //
-// Reductions: every product enters exactly (fma: TwoProduct) into a per-thread float pair; a warp
-// adds its lanes' pairs as integers in three pieces aligned to the largest, a CTA its warps' and a
-// cluster its CTAs' sums as 57-bit integers (CgSum), which keeps more than the reference's
-// float-rounded products summed in double (mesh/solver/CGAlgorithm.cu:106-133) and stays off the
-// FP64 pipes (a dependent FP64 add takes 76 cycles here, an integer warp reduction about 50).  A CTA's
+// Reductions: every product enters exactly (fma: TwoProduct); the 8 products of a sibling group are
+// added as float pairs in one order (cg_group_sum), and the groups' sums as integers: four digits of
+// 19 bits on a fixed grid of exponents (CgDig), of which the lowest are dropped below the largest
+// group's.  What a group contributes depends on the group alone and integers add in any order, so a
+// sum is the same however many CTAs, threads or turns its groups are dealt to: a cloud gets the same
+// bits from every cluster size, alone, served and in a batch.  It keeps 58 to 76 bits below the largest
+// group, more than the reference's float-rounded products summed in double
+// (mesh/solver/CGAlgorithm.cu:106-133), and stays off the FP64 pipes (a dependent FP64 add takes 76
+// cycles here, an integer warp reduction about 50).  A CTA's
 // sum goes to every CTA of the cluster with st.async, whose arrival on an mbarrier is the barrier
 // (836 cycles; a cluster barrier and reads of the others' sums 1,442).  The scalars of an iteration
 // (alpha, beta, the continue flag) are computed once per CTA, by the thread that finishes the sum,
@@ -151,9 +155,19 @@ struct alignas(16) CgSum {
     long long e;      // >= 512: not a number
 };
 
+// A sum in digits: (d[0] 2^57 + d[1] 2^38 + d[2] 2^19 + d[3]) 2^(19 (b - 3) - 127).  The digits of the
+// bins below the highest, b, are kept apart, so that a sum of a higher bin can drop the lowest ones and
+// nothing else.  A digit of a group is below 2^19 and a half: those of up to 4095 groups fit 32 bits.
+struct CgDig {
+    int4 d;
+    int b;            // -1: nothing added yet; above 13: not a number
+};
+
 struct CgcShared {
-    int4 warp[kCgWarps];           // the warps' sums: three pieces and their exponent
-    CgSum slot[2][16];             // the cluster's CTA sums, written by the CTAs
+    int4 warp[kCgWarps];           // the warps' sums
+    int warp_b[kCgWarps];
+    int4 slot[2][16];              // the cluster's CTA sums, written by the CTAs
+    int slot_b[2][16];
     unsigned long long bar[2];     // their arrivals
     CgSum rr;           // r.r of the recursive residual
     CgSum pap;
@@ -248,6 +262,113 @@ __device__ __forceinline__ double cgs_double(const CgSum& s) {
     return (double)s.m * __hiloint2double((1023 + max((int)s.e - 183, -1000)) << 20, 0);   // a power of two: exact
 }
 
+// The digits of the sum of kLanes lanes' float pairs, kTerms a lane, in every lane: each pair is rounded
+// to the lowest unit of the four bins, which start at the largest pair's.  What a pair leaves in the bins
+// from any unit upwards is the pair rounded to that unit (to even), whatever bin its digits start at.
+template <int kTerms, class Sum, class Max>
+__device__ __forceinline__ CgDig cgd_of(FF (&v)[kTerms], int lanes, Sum sum, Max max_of) {
+    int E = 0;
+#pragma unroll
+    for (int q = 0; q < kTerms; ++q) E = max(E, __float_as_int(v[q].hi) & 0x7f800000);
+    E = max_of(E) >> 23;   // the largest is below 2^(E - 126)
+    if (E == 255) return CgDig{make_int4(1, 0, 0, 0), 31};   // infinite or not a number
+    const int b = E / 19;
+    int at = b;
+    if (b < 2 || b > 12) {   // keep the units of the digits normal numbers
+        const int up = b < 2 ? 2 : -1;
+#pragma unroll
+        for (int q = 0; q < kTerms; ++q) {
+            v[q].hi *= pow2f_exact(19 * up);
+            v[q].lo *= pow2f_exact(19 * up);
+        }
+        at += up;
+    }
+    // a digit against 1.5 * 2^23 of its units: the addition rounds to the unit and leaves the integer in
+    // the low bits (less those of the constant, taken off the sum); what is left over is exact.  lo is at
+    // most 2^-24 hi and has none in the first bin.
+    const int c0 = ((19 * at + 23) << 23) | 0x400000, c1 = c0 - (19 << 23), c2 = c1 - (19 << 23), c3 = c2 - (19 << 23);
+    auto take = [](float& r, int c) -> int {
+        const float f = __int_as_float(c);
+        const float t = __fadd_rn(r, f);
+        r = __fsub_rn(r, __fsub_rn(t, f));
+        return __float_as_int(t);
+    };
+    unsigned d0 = 0, d1 = 0, d2 = 0, d3 = 0;   // modulo 2^32
+#pragma unroll
+    for (int q = 0; q < kTerms; ++q) {
+        d0 += take(v[q].hi, c0);
+        d1 += take(v[q].hi, c1);
+        d2 += take(v[q].hi, c2);
+        d3 += take(v[q].hi, c3);
+        d1 += take(v[q].lo, c1);
+        d2 += take(v[q].lo, c2);
+        d3 += take(v[q].lo, c3);
+    }
+    const unsigned n = (unsigned)(lanes * kTerms);
+    return CgDig{make_int4((int)(sum(d0) - n * c0), (int)(sum(d1) - 2 * n * c1), (int)(sum(d2) - 2 * n * c2),
+                           (int)(sum(d3) - 2 * n * c3)), b};
+}
+// of a warp's pairs
+template <int kTerms>
+__device__ __forceinline__ CgDig cgd_warp_sum(FF (&v)[kTerms]) {
+    return cgd_of(v, 32, [](unsigned d) { return __reduce_add_sync(0xffffffffu, d); },
+                  [](int e) { return __reduce_max_sync(0xffffffffu, e); });
+}
+// of one lane's pair
+__device__ __forceinline__ CgDig cgd_of(FF v) {
+    FF t[1] = {v};
+    return cgd_of(t, 1, [](unsigned d) { return d; }, [](int e) { return e; });
+}
+// the digits of a sum whose highest bin is s bins higher (the lowest s are dropped)
+template <class D>
+__device__ __forceinline__ void cgd_drop(D& d, int s) {
+    if (s & 1) { d.w = d.z; d.z = d.y; d.y = d.x; d.x = 0; }
+    if (s & 2) { d.w = d.y; d.z = d.x; d.y = d.x = 0; }
+    if (s > 3) d.x = d.y = d.z = d.w = 0;
+}
+__device__ __forceinline__ void cgd_add(CgDig& a, FF v) {
+    CgDig t = cgd_of(v);
+    const int b = max(a.b, t.b);
+    cgd_drop(a.d, b - a.b);
+    cgd_drop(t.d, b - t.b);
+    a = CgDig{make_int4(a.d.x + t.d.x, a.d.y + t.d.y, a.d.z + t.d.z, a.d.w + t.d.w), b};
+}
+// the lanes' sum, in every lane
+__device__ __forceinline__ CgDig cgd_warp_sum(CgDig v) {
+    const int b = __reduce_max_sync(0xffffffffu, v.b);
+    cgd_drop(v.d, b - v.b);
+    return CgDig{make_int4(__reduce_add_sync(0xffffffffu, v.d.x), __reduce_add_sync(0xffffffffu, v.d.y),
+                           __reduce_add_sync(0xffffffffu, v.d.z), __reduce_add_sync(0xffffffffu, v.d.w)), b};
+}
+// the sum of up to 16 lanes' digits as one number, in every lane (digits of all groups: below 2^38)
+template <class D>
+__device__ __forceinline__ CgSum cgd_total(D d, int lane_b) {
+    const int b = __reduce_max_sync(0xffffffffu, lane_b);
+    cgd_drop(d, b - lane_b);
+    auto add = [](long long m) -> long long {   // |sum| < 2^57
+        const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)m & 0x3ffffffu);
+        return ((long long)__reduce_add_sync(0xffffffffu, (int)(m >> 26)) << 26) + (long long)lo;
+    };
+    const long long hi = add(((long long)d.x << 19) + (long long)d.y), lo = add(((long long)d.z << 19) + (long long)d.w);
+    if (b > 13) return CgSum{1ll << 56, 1024};
+    const int k = min(38, 61 - (64 - __clzll(hi < 0 ? -hi : hi)));
+    return CgSum{(hi << k) + (lo >> (38 - k)), 19 * (b - 3) - 127 + 38 - k + 183};
+}
+
+// the sum of a sibling group's 8 terms, in one order: ((0 + 1) + (2 + 3)) + ((4 + 5) + (6 + 7))
+template <class Term>
+__device__ __forceinline__ FF cg_group_sum(Term term) {
+    FF h[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const FF t0 = term(4 * q), t1 = term(4 * q + 1);
+        const FF a = ff_add(t0, t1);
+        const FF t2 = term(4 * q + 2), t3 = term(4 * q + 3);
+        h[q] = ff_add(a, ff_add(t2, t3));
+    }
+    return ff_add(h[0], h[1]);
+}
+
 // a shared-memory address of this CTA in the window of cluster CTA `rank`
 __device__ __forceinline__ unsigned cg_map(unsigned sa, unsigned rank) {
     unsigned ra;
@@ -274,16 +395,22 @@ __device__ __forceinline__ void cgc_barriers_init(CgcShared& sh) {
 // mbarrier arrivals with release.  `n` counts the reductions: they alternate between two
 // slots and barriers, and a CTA reuses a slot only after every peer has sent to the other one.
 // The wait is bounded; `error` is then flagged and the solve stops.
-template <bool kPublish, class Post>
-__device__ __forceinline__ void cgc_allreduce(unsigned nb, unsigned me, CgcShared& sh, unsigned& n, FF v,
+template <bool kPublish, int kTerms, class Post>
+__device__ __forceinline__ void cgc_allreduce(unsigned nb, unsigned me, CgcShared& sh, unsigned& n, FF (&terms)[kTerms],
                                               unsigned* error, Post post) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int4 ws = make_int4(0, 0, 0, 0);
-    if (__any_sync(0xffffffffu, v.hi != 0.0f)) ws = cgs_warp_sum(v);   // not a number differs from 0 too
-    if (lane == 0) sh.warp[warp] = ws;
+    CgDig v{make_int4(0, 0, 0, 0), -1};
+    bool some = false;
+#pragma unroll
+    for (int q = 0; q < kTerms; ++q) some |= terms[q].hi != 0.0f;   // not a number differs from 0 too
+    if (__any_sync(0xffffffffu, some)) v = cgd_warp_sum(terms);
+    if (lane == 0) {
+        sh.warp[warp] = v.d;
+        sh.warp_b[warp] = v.b;
+    }
     __syncthreads();
     if (warp == 0) {
-        CgSum t = cgs_warp_sum(cgs_join(sh.warp[lane]));
+        v = cgd_warp_sum(CgDig{sh.warp[lane], sh.warp_b[lane]});
         bool late = false;
         if (nb > 1) {
             const int buf = (int)(n & 1u);
@@ -291,14 +418,21 @@ __device__ __forceinline__ void cgc_allreduce(unsigned nb, unsigned me, CgcShare
             const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh.bar[buf]);
             if (kPublish) asm volatile("fence.acq_rel.cluster;" ::: "memory");
             if (lane == 0)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(nb * 16u) : "memory");
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(nb * 20u) : "memory");
             __syncwarp();
             if ((unsigned)lane < nb) {
-                const unsigned slot = cg_map((unsigned)__cvta_generic_to_shared(&sh.slot[buf][me]), (unsigned)lane);
+                const unsigned peer_bar = cg_map(bar, (unsigned)lane);
+                const long long d01 = (long long)(unsigned)v.d.x | (long long)v.d.y << 32;
+                const long long d23 = (long long)(unsigned)v.d.z | (long long)v.d.w << 32;
                 asm volatile(
-                    "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(slot),
-                    "l"(t.m), "l"(t.e), "r"(cg_map(bar, (unsigned)lane))
+                    "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
+                        cg_map((unsigned)__cvta_generic_to_shared(&sh.slot[buf][me]), (unsigned)lane)),
+                    "l"(d01), "l"(d23), "r"(peer_bar)
                     : "memory");
+                asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(
+                                 cg_map((unsigned)__cvta_generic_to_shared(&sh.slot_b[buf][me]), (unsigned)lane)),
+                             "r"(v.b), "r"(peer_bar)
+                             : "memory");
             }
             unsigned done = 0;
             for (int spin = 0; spin < kSpinLimit && !done; ++spin)
@@ -310,10 +444,12 @@ __device__ __forceinline__ void cgc_allreduce(unsigned nb, unsigned me, CgcShare
                     : "r"(bar), "r"(parity)
                     : "memory");
             late = !done;
-            t = CgSum{0, 0};
-            if ((unsigned)lane < nb) t = sh.slot[buf][lane];
-            t = cgs_warp_sum(t);
+            v = CgDig{make_int4(0, 0, 0, 0), -1};
+            if ((unsigned)lane < nb) v = CgDig{sh.slot[buf][lane], sh.slot_b[buf][lane]};
+        } else if (lane > 0) {
+            v = CgDig{make_int4(0, 0, 0, 0), -1};
         }
+        const CgSum t = cgd_total(v.d, v.b);
         if (lane == 0) {
             post(t);
             if (late) {
@@ -477,6 +613,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     float* sap = sx + 8 * GP;
     constexpr int kDescPitch = kMode == kCgOne ? kCgcBlock : kCgRowGroups;
     unsigned* sdesc = reinterpret_cast<unsigned*>(sap + 8 * GP);   // [kCgDescWords][kDescPitch]
+    FF* sterm = reinterpret_cast<FF*>(sdesc + kCgDescWords * kDescPitch);   // kCgRows: [8][kCgRowGroups]
     const unsigned me = u.me, nb = u.nb;
     unsigned* err = &v.cw->error;
     const int tid = threadIdx.x;
@@ -552,26 +689,39 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
         rp[tid * GP + GP - 1] = make_float2(0.0f, 0.0f);
         sx[tid * GP + GP - 1] = 0.0f;
     }
-    // every row of this thread: body(element, row of the unit's arrays)
-    auto for_rows = [&](auto body) {
-        if (kMode == kCgRows) {
-            if (row_on) body(rs * GP + rg);
-        } else {
-            for (int g = tid; g < ng; g += kCgcBlock)
+    // A thread's groups' sums of this step's terms.
+    constexpr int kTerms = kMode == kCgMany ? 2 : 1;
+    FF acc[kTerms];
+    // body(group) for the thread's groups, its sum to acc
+    auto for_groups = [&](auto body) {
 #pragma unroll
-                for (int s = 0; s < 8; ++s) body(s * GP + g);
+        for (int q = 0; q < kTerms; ++q) {
+            const int g = tid + q * kCgcBlock;
+            acc[q] = ff_zero();
+            if (g < ng) acc[q] = body(g);
         }
     };
-    // r0 = b, p_{-1} = 0, x0 = 0 (rows in order: coalesced; A p starts as scratch)
-    FF acc = ff_zero();
+    // The sums of term(element) over the groups.  Where a row has a thread of its own, the terms of a
+    // group meet in shared memory and one thread adds them.
+    auto sum_rows = [&](auto term) {
+        if (kMode == kCgRows) {
+            sterm[tid] = row_on ? term(rs * GP + rg) : ff_zero();
+            __syncthreads();
+            acc[0] = ff_zero();
+            if (tid < kCgRowGroups) acc[0] = cg_group_sum([&](int s) { return sterm[s * kCgRowGroups + tid]; });
+        } else {
+            for_groups([&](int g) { return cg_group_sum([&](int s) { return term(s * GP + g); }); });
+        }
+    };
+    // r0 = b, p_{-1} = 0, x0 = 0 (rows in order: coalesced)
     const int mlo = 1 + 8 * gbase;
     for (int l = tid; l < 8 * ng; l += kCgcBlock) {
-        const float bi = v.b[mlo + l];
         const int e = (l & 7) * GP + (l >> 3);
-        rp[e] = make_float2(bi, 0.0f);
+        rp[e] = make_float2(v.b[mlo + l], 0.0f);
         sx[e] = 0.0f;
-        acc = ff_add(acc, ff_prod(bi, bi));
     }
+    __syncthreads();
+    sum_rows([&](int e) { return ff_prod(rp[e].x, rp[e].x); });
     unsigned nred = 0;
     cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_start(sh, a, t); });
     bool ran = false;
@@ -579,10 +729,8 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     while (sh.go) {
         const float beta = sh.beta;
         // (A) A p_k from the neighbours' (r_k, p_{k-1}), p.Ap
-        acc = ff_zero();
         if (kMode == kCgRows) {
-            if (row_on) {
-                const int e = rs * GP + rg;
+            sum_rows([&](int e) {
                 float y = 0.0f;
 #pragma unroll
                 for (int k = 0; k < 27; ++k) {
@@ -591,10 +739,10 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
                 }
                 const float2 own = rp[e];
                 sap[e] = y;
-                acc = ff_add(acc, ff_prod(fmaf(beta, own.y, own.x), y));
-            }
+                return ff_prod(fmaf(beta, own.y, own.x), y);
+            });
         } else {
-            for (int g = tid; g < ng; g += kCgcBlock) {
+            for_groups([&](int g) {
                 float y[8];
 #pragma unroll
                 for (int s = 0; s < 8; ++s) y[s] = 0.0f;
@@ -604,25 +752,23 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
                         return fmaf(beta, q.y, q.x);
                     },
                     [&](int s, int c, float p) { y[s] = fmaf(w[c], p, y[s]); });
-#pragma unroll
-                for (int s = 0; s < 8; ++s) {
+                return cg_group_sum([&](int s) {
                     const float2 own = rp[s * GP + g];
                     sap[s * GP + g] = y[s];
-                    acc = ff_add(acc, ff_prod(fmaf(beta, own.y, own.x), y[s]));
-                }
-            }
+                    return ff_prod(fmaf(beta, own.y, own.x), y[s]);
+                });
+            });
         }
         cgc_allreduce<false>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_alpha(sh, t); });
         const float alpha = sh.alpha;
         // (B) x and r, r.r; every CTA has read the pairs (the barrier of the last reduction)
-        acc = ff_zero();
-        for_rows([&](int e) {
+        sum_rows([&](int e) {
             const float2 own = rp[e];
             const float pi = fmaf(beta, own.y, own.x);
             sx[e] = fmaf(alpha, pi, sx[e]);
             const float ri = fmaf(-alpha, sap[e], own.x);
             rp[e] = make_float2(ri, pi);
-            acc = ff_add(acc, ff_prod(ri, ri));
+            return ff_prod(ri, ri);
         });
         cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_rr(sh, a, t, it); });
         ran = true;
@@ -631,20 +777,19 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
             // (C) true residual b - A x of the current x from the neighbours' x (the barrier
             // of the last reduction published every CTA's x), with exact products and
             // float-pair sums; staged in the A p array, which holds nothing live here
-            acc = ff_zero();
             // the entry of an offset that moves on `axes` of x and y, and by kz - 1 on z
             auto w_of = [&](int axes, int kz) {
                 return kz == 1 ? (axes == 0 ? w[0] : axes == 1 ? w[1] : w[2]) : (axes == 0 ? w[1] : axes == 1 ? w[2] : w[3]);
             };
-            auto residual = [&](int g, int s, FF y) {
+            auto residual = [&](int g, int s, FF y) -> FF {
                 const float ri = ff_to_float(ff_add(FF{v.b[mlo + 8 * g + s], 0.0f}, FF{-y.hi, -y.lo}));
                 sap[s * GP + g] = ri;
-                acc = ff_add(acc, ff_prod(ri, ri));
+                return ff_prod(ri, ri);
             };
             // rolled over the z-lines of the block: straight-line code that runs twice per solve
             // would come from L2
             if (kMode == kCgRows) {
-                if (row_on) {
+                sum_rows([&](int) {
                     FF y = ff_zero();
 #pragma unroll 1
                     for (int q = 0; q < 9; ++q) {
@@ -656,10 +801,10 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
                             y = ff_add(y, ff_prod(wk, cg_ld1(base_of(desc_of(rg, n), x_sa, 4u) + (unsigned)(sib * GP * 4))));
                         }
                     }
-                    residual(rg, rs, y);
-                }
+                    return residual(rg, rs, y);
+                });
             } else {
-                for (int g = tid; g < ng; g += kCgcBlock) {
+                for_groups([&](int g) {
                     FF y[8];
 #pragma unroll
                     for (int s = 0; s < 8; ++s) y[s] = ff_zero();
@@ -687,13 +832,18 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
                                 }
                         }
                     }
-#pragma unroll
-                    for (int s = 0; s < 8; ++s) residual(g, s, y[s]);
-                }
+                    return cg_group_sum([&](int s) { return residual(g, s, y[s]); });
+                });
             }
             cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_true(sh, a, t, it); });
             if (sh.replace) {   // refinement restart: CG continues from the true residual
-                for_rows([&](int e) { rp[e].x = sap[e]; });
+                if (kMode == kCgRows) {
+                    if (row_on) rp[rs * GP + rg].x = sap[rs * GP + rg];
+                } else {
+                    for (int g = tid; g < ng; g += kCgcBlock)
+#pragma unroll
+                        for (int s = 0; s < 8; ++s) rp[s * GP + g].x = sap[s * GP + g];
+                }
                 // before any CTA reads a neighbour's new r
                 if (nb > 1) cl.sync();
                 else __syncthreads();
@@ -709,33 +859,105 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     if (ran && me == 0 && tid == 0) cgc_report(v, u.d, sh, it - 1);
 }
 
-// Global-memory path (any size, any depth).  The peers' vectors are read through L1, so every
-// published step also passes the cluster barrier.
+// The same sum for any number of groups a thread (digits of 64 bits), by cluster barriers, which also
+// publish the CTAs' vectors in global memory.
+struct CgWide {
+    long long x, y, z, w;
+};
+struct CgWideShared {
+    CgWide warp[kCgWarps], cta[2];
+    int warp_b[kCgWarps], cta_b[2];
+    FF term[kCgWarps][32 * 9];   // the terms of 32 groups a warp
+};
+static_assert(sizeof(CgWideShared) <= kCgSmemBytes, "in the resident path's shared memory");
+// the lanes' sum of d, |d| < 2^44
+__device__ __forceinline__ long long cgd_add_lanes(long long d) {
+    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)d & 0xfffffu);
+    return ((long long)__reduce_add_sync(0xffffffffu, (int)(d >> 20)) << 20) + (long long)lo;
+}
+template <class Post>
+__device__ __forceinline__ void cgc_allreduce_wide(cg::cluster_group& cl, unsigned nb, CgWideShared& sw, unsigned& n,
+                                                   CgDig v, Post post) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, buf = (int)(n & 1u);
+    auto lanes_sum = [](CgWide d, int& lane_b) -> CgWide {
+        const int b = __reduce_max_sync(0xffffffffu, lane_b);
+        cgd_drop(d, b - lane_b);
+        lane_b = b;
+        return CgWide{cgd_add_lanes(d.x), cgd_add_lanes(d.y), cgd_add_lanes(d.z), cgd_add_lanes(d.w)};
+    };
+    const CgWide w = lanes_sum(CgWide{v.d.x, v.d.y, v.d.z, v.d.w}, v.b);
+    if (lane == 0) {
+        sw.warp[warp] = w;
+        sw.warp_b[warp] = v.b;
+    }
+    __syncthreads();
+    CgWide t{0, 0, 0, 0};
+    int tb = -1;
+    if (warp == 0) {
+        tb = sw.warp_b[lane];
+        t = lanes_sum(sw.warp[lane], tb);
+        if (lane == 0) {
+            sw.cta[buf] = t;
+            sw.cta_b[buf] = tb;
+        }
+    }
+    if (nb > 1) cl.sync();
+    if (warp == 0) {
+        if (nb > 1 && (unsigned)lane < nb) {
+            t = *cl.map_shared_rank(&sw.cta[buf], lane);
+            tb = *cl.map_shared_rank(&sw.cta_b[buf], lane);
+        } else if (nb > 1 || lane > 0) {
+            t = CgWide{0, 0, 0, 0};
+            tb = -1;
+        }
+        const CgSum sum = cgd_total(t, tb);
+        if (lane == 0) post(sum);
+    }
+    ++n;
+    __syncthreads();
+}
+
+// Global-memory path (any size, any depth).  A row has a lane, so that a warp reads consecutive rows, and
+// every eight turns a lane adds the terms of one group; the peers' vectors are read through L1, and every reduction passes the cluster
+// barrier.
 __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh, const CgcArgs& a,
-                                           const CgcVec& v, const CgUnit& u) {
+                                           const CgcVec& v, const CgUnit& u, float4* dyn) {
     const unsigned me = u.me, nb = u.nb;
-    unsigned* err = &v.cw->error;
-    const int tid = me * blockDim.x + threadIdx.x;
-    const int nthr = nb * blockDim.x;
-    FF acc = ff_zero();
-    for (int i = u.row0 + tid; i < u.row1; i += nthr) {
+    CgWideShared& sw = *reinterpret_cast<CgWideShared*>(dyn);
+    const int lane = threadIdx.x & 31;
+    const int first = u.row0 + (int)(me * blockDim.x + threadIdx.x), nthr = nb * blockDim.x;
+    // the digits of term(row) over the rows of this thread, added group by group in cg_group_sum's order
+    auto sum_rows = [&](auto term) -> CgDig {
+        CgDig acc{make_int4(0, 0, 0, 0), -1};
+        FF* buf = sw.term[threadIdx.x >> 5];
+        for (int i0 = first - lane; i0 < u.row1; i0 += 8 * nthr) {
+#pragma unroll 1
+            for (int q = 0; q < 8; ++q) {
+                const int i = i0 + q * nthr + lane;
+                buf[9 * (4 * q + (lane >> 3)) + (lane & 7)] = i < u.row1 ? term(i) : ff_zero();
+            }
+            __syncwarp();
+            cgd_add(acc, cg_group_sum([&](int s) { return buf[9 * lane + s]; }));
+            __syncwarp();
+        }
+        return acc;
+    };
+    unsigned nred = 0;
+    CgDig acc = sum_rows([&](int i) {
         const float bi = v.b[i];
         v.r[i] = bi;
         v.pa[i] = 0.0f;
         v.x[i] = 0.0f;
-        acc = ff_add(acc, ff_prod(bi, bi));
-    }
-    unsigned nred = 0;
-    cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_start(sh, a, t); });
-    if (nb > 1) cl.sync();
+        return ff_prod(bi, bi);
+    });
+    cgc_allreduce_wide(cl, nb, sw, nred, acc, [&](const CgSum& t) { cgc_start(sh, a, t); });
     bool ran = false;
     const float* pprev = v.pa;
     float* pcur = v.pb;
     int it = 1;
     while (sh.go) {
         const float beta = sh.beta;
-        acc = ff_zero();
-        for (int i = u.row0 + tid; i < u.row1; i += nthr) {
+        acc = sum_rows([&](int i) {
             const float pi = fmaf(beta, pprev[i], v.r[i]);
             float y = 0.0f;
 #pragma unroll 9
@@ -745,19 +967,17 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
             }
             pcur[i] = pi;
             v.ap[i] = y;
-            acc = ff_add(acc, ff_prod(pi, y));
-        }
-        cgc_allreduce<false>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_alpha(sh, t); });
+            return ff_prod(pi, y);
+        });
+        cgc_allreduce_wide(cl, nb, sw, nred, acc, [&](const CgSum& t) { cgc_alpha(sh, t); });
         const float alpha = sh.alpha;
-        acc = ff_zero();
-        for (int i = u.row0 + tid; i < u.row1; i += nthr) {
+        acc = sum_rows([&](int i) {
             v.x[i] = fmaf(alpha, pcur[i], v.x[i]);
             const float ri = fmaf(-alpha, v.ap[i], v.r[i]);
             v.r[i] = ri;
-            acc = ff_add(acc, ff_prod(ri, ri));
-        }
-        cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_rr(sh, a, t, it); });
-        if (nb > 1) cl.sync();
+            return ff_prod(ri, ri);
+        });
+        cgc_allreduce_wide(cl, nb, sw, nred, acc, [&](const CgSum& t) { cgc_after_rr(sh, a, t, it); });
         ran = true;
         float* t = const_cast<float*>(pprev);
         pprev = pcur;
@@ -765,8 +985,7 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
         ++it;
         if (sh.check) {
             // true residual r = b - A x (the barrier of the last reduction published x)
-            acc = ff_zero();
-            for (int i = u.row0 + tid; i < u.row1; i += nthr) {
+            acc = sum_rows([&](int i) {
                 FF y = ff_zero();
                 for (int k = 0; k < 27; ++k) {
                     const int nb = __ldg(&v.neigh[(size_t)k * a.stride + i]);
@@ -774,12 +993,11 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
                 }
                 const float ri = ff_to_float(ff_add(FF{v.b[i], 0.0f}, FF{-y.hi, -y.lo}));
                 v.ap[i] = ri;   // staged; A p holds nothing live here
-                acc = ff_add(acc, ff_prod(ri, ri));
-            }
-            cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_true(sh, a, t, it); });
-            if (nb > 1) cl.sync();
+                return ff_prod(ri, ri);
+            });
+            cgc_allreduce_wide(cl, nb, sw, nred, acc, [&](const CgSum& t) { cgc_after_true(sh, a, t, it); });
             if (sh.replace) {   // refinement restart: CG continues from the true residual
-                for (int i = u.row0 + tid; i < u.row1; i += nthr) v.r[i] = v.ap[i];
+                for (int i = first; i < u.row1; i += nthr) v.r[i] = v.ap[i];
                 if (nb > 1) cl.sync();
                 else __syncthreads();
             }
@@ -816,7 +1034,7 @@ __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
         const int m = u.row1 - u.row0;
         const int chunk = cg_chunk_groups(m, (int)u.nb);
         const bool fits = cg_fits_resident(u.d, m, (int)u.nb);   // the same in all CTAs of the unit
-        if (!fits) cgc_global(cl, sh, a, v, u);
+        if (!fits) cgc_global(cl, sh, a, v, u, cg_dyn);
         else if (chunk <= kCgRowGroups) cgc_resident<kCgRows>(cl, sh, a, v, u, chunk, cg_dyn);
         else if (chunk <= kCgcBlock) cgc_resident<kCgOne>(cl, sh, a, v, u, chunk, cg_dyn);
         else cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);

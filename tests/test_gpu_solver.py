@@ -43,3 +43,45 @@ def test_rows_outside_their_own_table_against_oracle(oracle_mod, seed, depth, gr
     ref = o.get("x")
     assert parity.rel_l2(x, ref) <= parity.REL_L2
     assert parity.rel_l2(x[b:b + 8], ref[b:b + 8]) <= parity.REL_L2
+
+
+def solution(r):
+    st = r.stats()
+    return (r.debug("x", np.float32), st.iso_value, list(st.cg_iterations), list(st.cg_residual),
+            list(st.cg_true_residual), list(st.cg_restarts))
+
+
+def equal(a, b):
+    np.testing.assert_array_equal(a[0], b[0])
+    assert a[1:] == b[1:]
+
+
+# systems that give a row, a group and several groups to a thread, and systems that outgrow the shared
+# memory of the smaller clusters
+@pytest.mark.parametrize("name,cloud,n,depth", [("sphere20k", 0, 4000, 5), ("mix", 1, 40000, 6), ("mix", 2, 60000, 7),
+                                               ("torus_ellipsoid200k", 0, 150000, 7), ("serve", 3, 300000, 7)])
+def test_solution_does_not_depend_on_the_cluster_size(name, cloud, n, depth):
+    """Every sum of the CG is the same however its rows are dealt to CTAs and threads: iterations,
+    residuals (as doubles) and solutions are equal bit for bit for every cluster size, from the global-memory
+    path, in one chain, and in a batch."""
+    import psr
+    p, nr, _, _ = syn.workload(name, cloud=cloud, n=n, colour=False)
+    caps = dict(max_depth=7, max_points=300000)
+    with psr.PoissonReconstruction(**caps) as r:
+        r.SolvePoissionReconstructionMesh(p, nr, depth=depth)
+        want = solution(r)
+    for options in (dict(cg_cluster_ctas=1, cg_cluster_ctas_fine=1), dict(cg_cluster_ctas=2, cg_cluster_ctas_fine=4),
+                    dict(cg_cluster_ctas=5, cg_cluster_ctas_fine=3), dict(cg_cluster_ctas=8, cg_cluster_ctas_fine=16),
+                    dict(concurrent_stages=False), dict(concurrent_stages=False, cg_cluster_ctas=3),
+                    dict(disable_graphs=True)):
+        with psr.PoissonReconstruction(**caps, **options) as r:
+            r.SolvePoissionReconstructionMesh(p, nr, depth=depth)
+            equal(want, solution(r))
+    count = 5   # enough that the launch takes its smaller clusters
+    with psr.PoissonReconstruction(batch_clouds=count, max_mesh_vertices=200000, max_triangles=400000, **caps) as r:
+        r.reconstruct_batch([(p, nr, None)] * count, depth=depth)
+        for k in (0, count - 1):
+            status, st = r.batch_result(k)
+            assert status == psr.PSR_OK
+            assert want[1:] == (st.iso_value, list(st.cg_iterations), list(st.cg_residual), list(st.cg_true_residual),
+                                list(st.cg_restarts))
