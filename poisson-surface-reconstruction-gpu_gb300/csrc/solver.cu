@@ -11,8 +11,8 @@
 // solved together, by thread-block clusters (k_cg_cluster) or, from depth 5 on of trees of
 // depth 8 and 9, by the whole GPU in one cooperative launch (k_cg_grid).
 // Precision: the operator, the vectors and the updates are FP32; the dot products and
-// residual norms are exact products summed as float pairs in a thread and as 57-bit fixed-point
-// integers across lanes, warps and CTAs (CgSum).  Every res_period iterations and when the
+// residual norms are exact products summed as float pairs in a sibling group (k_cg_grid: in a thread)
+// and as integers across lanes, warps and CTAs (CgDig, CgSum).  Every res_period iterations and when the
 // recursive residual reaches the tolerance, the true residual b - A x of the current x is
 // evaluated the same way; it drives iterative refinement:
 // the CG restarts from it when it is above both the tolerance and the floor an FP32
@@ -86,7 +86,8 @@ namespace psr {
 // groups (CTA rank, local group: 15 bits) are found once per solve and stay packed in 14
 // words a group, in shared memory where they fit (up to 1024 groups).
 // A chunk of at most kCgRowGroups groups (the coarser depths) gives every row a thread of
-// its own instead, 27 loads each, for a shorter chain.  The first version fetched a group's
+// its own instead, 27 loads each, for a shorter chain (the terms of a group then meet in shared memory,
+// one block barrier more a reduction).  The first version fetched a group's
 // block with 8 lanes through a staging block in shared memory (8 stores and 27 reads a row
 // besides the 8 loads) and was bound by the shared-memory queue.  Since p is rebuilt from
 // (r, p) after the first barrier, phase B overwrites the one copy of the pair that phase A
@@ -113,11 +114,9 @@ struct CgcVec {
     const float* stencil;
     const float* b;
     float* x;
-    float* r;
-    float* pa;
-    float* pb;
+    float2* rp;         // global-memory path: (r_k, p_{k-1}) per row
     float* ap;
-    __device__ void rebase() { PSR_CLOUD(c, cw, neigh, parent, first_child, desc, stencil, b, x, r, pa, pb, ap); }
+    __device__ void rebase() { PSR_CLOUD(c, cw, neigh, parent, first_child, desc, stencil, b, x, rp, ap); }
 };
 
 // a workspace pointer of cloud 0 moved to cloud k (null stays null)
@@ -854,7 +853,6 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     for (int l = tid; l < 8 * ng; l += kCgcBlock) {
         const int e = (l & 7) * GP + (l >> 3);
         v.x[mlo + l] = sx[e];
-        v.r[mlo + l] = rp[e].x;
     }
     if (ran && me == 0 && tid == 0) cgc_report(v, u.d, sh, it - 1);
 }
@@ -918,7 +916,8 @@ __device__ __forceinline__ void cgc_allreduce_wide(cg::cluster_group& cl, unsign
 }
 
 // Global-memory path (any size, any depth).  A row has a lane, so that a warp reads consecutive rows, and
-// every eight turns a lane adds the terms of one group; the peers' vectors are read through L1, and every reduction passes the cluster
+// every eight turns a lane adds the terms of one group.  r and p are one pair, so a neighbour is one
+// load (278,000 rows on 16 CTAs: 109 -> 95 us an iteration); the peers' vectors are read through L1, and every reduction passes the cluster
 // barrier.
 __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh, const CgcArgs& a,
                                            const CgcVec& v, const CgUnit& u, float4* dyn) {
@@ -945,43 +944,41 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
     unsigned nred = 0;
     CgDig acc = sum_rows([&](int i) {
         const float bi = v.b[i];
-        v.r[i] = bi;
-        v.pa[i] = 0.0f;
+        v.rp[i] = make_float2(bi, 0.0f);
         v.x[i] = 0.0f;
         return ff_prod(bi, bi);
     });
     cgc_allreduce_wide(cl, nb, sw, nred, acc, [&](const CgSum& t) { cgc_start(sh, a, t); });
     bool ran = false;
-    const float* pprev = v.pa;
-    float* pcur = v.pb;
     int it = 1;
     while (sh.go) {
         const float beta = sh.beta;
         acc = sum_rows([&](int i) {
-            const float pi = fmaf(beta, pprev[i], v.r[i]);
+            const float2 own = v.rp[i];
             float y = 0.0f;
 #pragma unroll 9
             for (int k = 0; k < 27; ++k) {
                 const int nb = __ldg(&v.neigh[(size_t)k * a.stride + i]);
-                if (nb >= 0) y = fmaf(sh.st[k], fmaf(beta, pprev[nb], v.r[nb]), y);
+                if (nb >= 0) {
+                    const float2 q = v.rp[nb];
+                    y = fmaf(sh.st[k], fmaf(beta, q.y, q.x), y);
+                }
             }
-            pcur[i] = pi;
             v.ap[i] = y;
-            return ff_prod(pi, y);
+            return ff_prod(fmaf(beta, own.y, own.x), y);
         });
         cgc_allreduce_wide(cl, nb, sw, nred, acc, [&](const CgSum& t) { cgc_alpha(sh, t); });
         const float alpha = sh.alpha;
         acc = sum_rows([&](int i) {
-            v.x[i] = fmaf(alpha, pcur[i], v.x[i]);
-            const float ri = fmaf(-alpha, v.ap[i], v.r[i]);
-            v.r[i] = ri;
+            const float2 own = v.rp[i];
+            const float pi = fmaf(beta, own.y, own.x);
+            v.x[i] = fmaf(alpha, pi, v.x[i]);
+            const float ri = fmaf(-alpha, v.ap[i], own.x);
+            v.rp[i] = make_float2(ri, pi);
             return ff_prod(ri, ri);
         });
         cgc_allreduce_wide(cl, nb, sw, nred, acc, [&](const CgSum& t) { cgc_after_rr(sh, a, t, it); });
         ran = true;
-        float* t = const_cast<float*>(pprev);
-        pprev = pcur;
-        pcur = t;
         ++it;
         if (sh.check) {
             // true residual r = b - A x (the barrier of the last reduction published x)
@@ -997,7 +994,7 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
             });
             cgc_allreduce_wide(cl, nb, sw, nred, acc, [&](const CgSum& t) { cgc_after_true(sh, a, t, it); });
             if (sh.replace) {   // refinement restart: CG continues from the true residual
-                for (int i = first; i < u.row1; i += nthr) v.r[i] = v.ap[i];
+                for (int i = first; i < u.row1; i += nthr) v.rp[i].x = v.ap[i];
                 if (nb > 1) cl.sync();
                 else __syncthreads();
             }
@@ -1835,9 +1832,7 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     a.v.stencil = ws.stencil;
     a.v.b = ws.divg;
     a.v.x = ws.xsol;
-    a.v.r = ws.cg_r;
-    a.v.pa = ws.cg_p;
-    a.v.pb = ws.cg_q;
+    a.v.rp = ws.cg_p;
     a.v.ap = ws.cg_ap;
     a.tol2 = cg_tol * cg_tol;
     // a fixed iteration count replaces the reference's max_iter (10000); the tolerance
