@@ -21,6 +21,7 @@
 // Iso-value (:269-305): mean of the implicit function at the sample points, evaluated in
 // FP32 per point and averaged in FP64.
 #include <cooperative_groups.h>
+#include <type_traits>
 #include <vector>
 #include "workspace.h"
 #include "tables.cuh"
@@ -83,7 +84,7 @@ namespace psr {
 // (r, p) once (own shared memory, or a peer's through distributed shared memory) and adds
 // it to every row it belongs to, which keeps each row's sum in neighbour order.  Nothing is
 // staged and nothing is reread: a group costs 64 loads and 216 FMAs, and the neighbour
-// groups (CTA rank, local group: 15 bits) are found once per solve and stay packed in 14
+// groups (CTA rank, local group: 16 bits) are found once per solve and stay packed in 14
 // words a group, in shared memory where they fit (up to 1024 groups).
 // A chunk of at most kCgRowGroups groups (the coarser depths) gives every row a thread of
 // its own instead, 27 loads each, for a shorter chain (the terms of a group then meet in shared memory,
@@ -91,12 +92,17 @@ namespace psr {
 // block with 8 lanes through a staging block in shared memory (8 stores and 27 reads a row
 // besides the 8 loads) and was bound by the shared-memory queue.  Since p is rebuilt from
 // (r, p) after the first barrier, phase B overwrites the one copy of the pair that phase A
-// read.  Otherwise (the root, or more rows than fit) the vectors live in global memory and
-// the neighbour table is read row by row.
+// read.
+// A chunk of 1792 to 3583 groups keeps the pairs alone in shared memory; x and A p, which an iteration
+// reads once and writes once by the thread that owns them, go through L2 (32 us an iteration for 278,000
+// rows on 16 CTAs, where the path below takes 95).  It is what lets small clusters and single CTAs
+// take systems larger than those they are sized for.  Otherwise (the root, or more rows than fit)
+// the vectors live in global memory and the neighbour table is read row by row.
 constexpr int kCgcBlock = 1024;
 constexpr int kCgWarps = kCgcBlock / 32;
 constexpr int kCgGroups = 1792;                   // local groups of a CTA's arrays; the last one is the zero group
                                                   //   (absent neighbours: (0, 0), x = 0)
+constexpr int kCgPairGroups = 2 * kCgGroups;      // the same of the pairs alone
 constexpr int kCgRowGroups = kCgcBlock / 8;       // at most this many groups: a thread per row
 constexpr int kCgDescWords = 14;                  // 27 neighbour groups, two per word
 constexpr size_t kCgSmemBytes = (size_t)kCgGroups * 8 * (sizeof(float2) + 2 * sizeof(float));   // (r, p), x, A p
@@ -115,8 +121,9 @@ struct CgcVec {
     const float* b;
     float* x;
     float2* rp;         // global-memory path: (r_k, p_{k-1}) per row
-    float* ap;
-    __device__ void rebase() { PSR_CLOUD(c, cw, neigh, parent, first_child, desc, stencil, b, x, rp, ap); }
+    float* ap;          //   and A p
+    float *xs, *aps;    // x and A p of chunks whose pairs alone fit shared memory: [8][dstride], sibling-major
+    __device__ void rebase() { PSR_CLOUD(c, cw, neigh, parent, first_child, desc, stencil, b, x, rp, ap, xs, aps); }
 };
 
 // a workspace pointer of cloud 0 moved to cloud k (null stays null)
@@ -139,11 +146,11 @@ struct CgcArgs {
                         // solve a coarser depth each
 };
 
-// The resident path holds a depth when its cluster's chunk of groups fits a CTA's shared
-// memory (the last group is the zero group); the root never does.
+// The resident path holds a depth when the (r, p) pairs of its cluster's chunk of groups fit a CTA's
+// shared memory (the last group is the zero group); the root never does.
 __device__ __forceinline__ int cg_chunk_groups(int m, int nblk) { return ((m >> 3) + nblk - 1) / nblk; }
 __device__ __forceinline__ bool cg_fits_resident(int d, int m, int nblk) {
-    return d >= 1 && cg_chunk_groups(m, nblk) < kCgGroups;
+    return d >= 1 && cg_chunk_groups(m, nblk) < kCgPairGroups;
 }
 
 // A sum in fixed point: m * 2^(e - 183), |m| < 2^62.  The lanes of a warp are added as 57-bit
@@ -184,7 +191,7 @@ struct CgcShared {
 };
 static_assert(kCgWarps == 32, "one lane per warp sum");
 static_assert(kCgSmemBytes + sizeof(CgcShared) <= 227 * 1024, "shared memory of one CTA");
-static_assert(kCgGroups <= 2048, "11 bits of a packed neighbour group");
+static_assert(kCgPairGroups <= 4096, "12 bits of a packed neighbour group, 4 of its CTA");
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -264,8 +271,8 @@ __device__ __forceinline__ double cgs_double(const CgSum& s) {
 // The digits of the sum of kLanes lanes' float pairs, kTerms a lane, in every lane: each pair is rounded
 // to the lowest unit of the four bins, which start at the largest pair's.  What a pair leaves in the bins
 // from any unit upwards is the pair rounded to that unit (to even), whatever bin its digits start at.
-template <int kTerms, class Sum, class Max>
-__device__ __forceinline__ CgDig cgd_of(FF (&v)[kTerms], int lanes, Sum sum, Max max_of) {
+template <int kTerms, class Sum, class Max, class Any>
+__device__ __forceinline__ CgDig cgd_of(FF (&v)[kTerms], int lanes, Sum sum, Max max_of, Any any) {
     int E = 0;
 #pragma unroll
     for (int q = 0; q < kTerms; ++q) E = max(E, __float_as_int(v[q].hi) & 0x7f800000);
@@ -293,8 +300,11 @@ __device__ __forceinline__ CgDig cgd_of(FF (&v)[kTerms], int lanes, Sum sum, Max
         return __float_as_int(t);
     };
     unsigned d0 = 0, d1 = 0, d2 = 0, d3 = 0;   // modulo 2^32
+    unsigned n = 0;
 #pragma unroll
     for (int q = 0; q < kTerms; ++q) {
+        if (kTerms > 1 && !any(v[q].hi != 0.0f)) continue;
+        n += (unsigned)lanes;
         d0 += take(v[q].hi, c0);
         d1 += take(v[q].hi, c1);
         d2 += take(v[q].hi, c2);
@@ -303,20 +313,24 @@ __device__ __forceinline__ CgDig cgd_of(FF (&v)[kTerms], int lanes, Sum sum, Max
         d2 += take(v[q].lo, c2);
         d3 += take(v[q].lo, c3);
     }
-    const unsigned n = (unsigned)(lanes * kTerms);
     return CgDig{make_int4((int)(sum(d0) - n * c0), (int)(sum(d1) - 2 * n * c1), (int)(sum(d2) - 2 * n * c2),
                            (int)(sum(d3) - 2 * n * c3)), b};
 }
 // of a warp's pairs
 template <int kTerms>
 __device__ __forceinline__ CgDig cgd_warp_sum(FF (&v)[kTerms]) {
+    bool some = false;
+#pragma unroll
+    for (int q = 0; q < kTerms; ++q) some |= v[q].hi != 0.0f;   // not a number differs from 0 too
+    if (!__any_sync(0xffffffffu, some)) return CgDig{make_int4(0, 0, 0, 0), -1};
     return cgd_of(v, 32, [](unsigned d) { return __reduce_add_sync(0xffffffffu, d); },
-                  [](int e) { return __reduce_max_sync(0xffffffffu, e); });
+                  [](int e) { return __reduce_max_sync(0xffffffffu, e); },
+                  [](bool some) { return __any_sync(0xffffffffu, some) != 0; });
 }
 // of one lane's pair
 __device__ __forceinline__ CgDig cgd_of(FF v) {
     FF t[1] = {v};
-    return cgd_of(t, 1, [](unsigned d) { return d; }, [](int e) { return e; });
+    return cgd_of(t, 1, [](unsigned d) { return d; }, [](int e) { return e; }, [](bool some) { return some; });
 }
 // the digits of a sum whose highest bin is s bins higher (the lowest s are dropped)
 template <class D>
@@ -394,15 +408,11 @@ __device__ __forceinline__ void cgc_barriers_init(CgcShared& sh) {
 // mbarrier arrivals with release.  `n` counts the reductions: they alternate between two
 // slots and barriers, and a CTA reuses a slot only after every peer has sent to the other one.
 // The wait is bounded; `error` is then flagged and the solve stops.
-template <bool kPublish, int kTerms, class Post>
-__device__ __forceinline__ void cgc_allreduce(unsigned nb, unsigned me, CgcShared& sh, unsigned& n, FF (&terms)[kTerms],
+template <bool kPublish, class Terms, class Post>
+__device__ __forceinline__ void cgc_allreduce(unsigned nb, unsigned me, CgcShared& sh, unsigned& n, Terms& terms,
                                               unsigned* error, Post post) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    CgDig v{make_int4(0, 0, 0, 0), -1};
-    bool some = false;
-#pragma unroll
-    for (int q = 0; q < kTerms; ++q) some |= terms[q].hi != 0.0f;   // not a number differs from 0 too
-    if (__any_sync(0xffffffffu, some)) v = cgd_warp_sum(terms);
+    CgDig v = cgd_warp_sum(terms);
     if (lane == 0) {
         sh.warp[warp] = v.d;
         sh.warp_b[warp] = v.b;
@@ -577,12 +587,17 @@ __device__ __forceinline__ int cg_neighbour_group(const CgcVec& v, size_t stride
 enum CgMode {
     kCgRows,     // a thread per row (thread t: sibling t / kCgRowGroups of group t % kCgRowGroups)
     kCgOne,      // a thread per group, the packed neighbour groups in shared memory
-    kCgMany      // groups in turn, their neighbour groups packed in global memory
+    kCgMany,     // groups in turn, their neighbour groups packed in global memory
+    kCgPairs     // the same with x and A p in global memory too
 };
 // groups of the sibling-major arrays of a mode (the last one is the zero group)
 __host__ __device__ constexpr int cg_pitch(int mode) {
-    return mode == kCgMany ? kCgGroups : mode == kCgOne ? kCgcBlock + 8 : kCgRowGroups + 8;
+    return mode == kCgPairs  ? kCgPairGroups
+           : mode == kCgMany ? kCgGroups
+           : mode == kCgOne  ? kCgcBlock + 8
+                             : kCgRowGroups + 8;
 }
+static_assert((size_t)cg_pitch(kCgPairs) * 8 * sizeof(float2) <= kCgSmemBytes, "kCgPairs");
 static_assert((size_t)cg_pitch(kCgOne) * 8 * 16 + (size_t)kCgDescWords * kCgcBlock * 4 <= kCgSmemBytes, "kCgOne");
 
 // The operator of one group: adds st * val(position) to every row the position neighbours, in
@@ -623,16 +638,16 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     const unsigned rp_sa = (unsigned)__cvta_generic_to_shared(rp);
     const unsigned x_sa = (unsigned)__cvta_generic_to_shared(sx);
     const float w[4] = {sh.st[13], sh.st[14], sh.st[17], sh.st[26]};   // centre, face, edge, corner
-    // q / chunk = umulhi(q, ceil(2^32 / chunk)): exact for q < 16 * chunk, chunk <= 2^11
+    // q / chunk = umulhi(q, ceil(2^32 / chunk)): exact for q < 16 * chunk, chunk <= 2^12
     const unsigned magic = (unsigned)((0x100000000ull + (unsigned)chunk - 1) / (unsigned)chunk);
-    // rank << 11 | local group of global group G (absent or outside the unit: the zero group)
+    // rank << 12 | local group of global group G (absent or outside the unit: the zero group)
     auto locate = [&](int G) -> unsigned {
         const unsigned q = (unsigned)(G - ((u.row0 - 1) >> 3));
-        if (G < 0 || q >= (unsigned)ngroups) return ((u.rank0 + me) << 11) | (unsigned)(GP - 1);
+        if (G < 0 || q >= (unsigned)ngroups) return ((u.rank0 + me) << 12) | (unsigned)(GP - 1);
         const unsigned own = chunk > 1 ? __umulhi(q, magic) : q;   // q / chunk
-        return ((u.rank0 + own) << 11) | (q - own * (unsigned)chunk);
+        return ((u.rank0 + own) << 12) | (q - own * (unsigned)chunk);
     };
-    auto base_of = [&](unsigned d, unsigned sa, unsigned elem) { return cg_map(sa + (d & 2047u) * elem, d >> 11); };
+    auto base_of = [&](unsigned d, unsigned sa, unsigned elem) { return cg_map(sa + (d & 4095u) * elem, d >> 12); };
 
     // kCgRows: this thread's row and the mapped addresses of its 27 neighbours' pairs
     const int rs = tid / kCgRowGroups, rg = tid % kCgRowGroups;
@@ -649,7 +664,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
         const unsigned lo = locate(cg_neighbour_group(v, a.stride, pa, 2 * j));
         const unsigned hi = (2 * j + 1 < 27) ? locate(cg_neighbour_group(v, a.stride, pa, 2 * j + 1)) : 0u;
         const unsigned q = lo | (hi << 16);
-        if (kMode == kCgMany) v.desc[(size_t)j * a.dstride + gbase + g] = q;
+        if (kMode >= kCgMany) v.desc[(size_t)j * a.dstride + gbase + g] = q;
         else sdesc[j * kDescPitch + g] = q;
     };
     if (kMode == kCgRows) {   // a word per thread and turn
@@ -667,7 +682,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     }
     // neighbour group slot n of group g (packed)
     auto desc_of = [&](int g, int n) -> unsigned {
-        const unsigned q = kMode == kCgMany ? v.desc[(size_t)(n >> 1) * a.dstride + gbase + g]
+        const unsigned q = kMode >= kCgMany ? v.desc[(size_t)(n >> 1) * a.dstride + gbase + g]
                                             : sdesc[(n >> 1) * kDescPitch + g];
         return (n & 1) ? q >> 16 : q & 0xffffu;
     };
@@ -684,43 +699,66 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
             }
         }
     }
+    // x and A p of sibling s of local group g
+    const unsigned dpitch = (unsigned)a.dstride;
+    auto x_at = [&](int s, int g) -> float& {
+        return kMode == kCgPairs ? v.xs[(unsigned)s * dpitch + (unsigned)(gbase + g)] : sx[s * GP + g];
+    };
+    auto ap_at = [&](int s, int g) -> float& {
+        return kMode == kCgPairs ? v.aps[(unsigned)s * dpitch + (unsigned)(gbase + g)] : sap[s * GP + g];
+    };
     if (tid < 8) {
         rp[tid * GP + GP - 1] = make_float2(0.0f, 0.0f);
-        sx[tid * GP + GP - 1] = 0.0f;
+        if (kMode == kCgPairs) v.xs[(unsigned)tid * dpitch + dpitch - 1u] = 0.0f;   // the same in every CTA
+        else sx[tid * GP + GP - 1] = 0.0f;
     }
     // A thread's groups' sums of this step's terms.
     constexpr int kTerms = kMode == kCgMany ? 2 : 1;
-    FF acc[kTerms];
+    std::conditional_t<kMode == kCgPairs, CgDig, FF[kTerms]> acc;
     // body(group) for the thread's groups, its sum to acc
     auto for_groups = [&](auto body) {
-#pragma unroll
-        for (int q = 0; q < kTerms; ++q) {
-            const int g = tid + q * kCgcBlock;
-            acc[q] = ff_zero();
-            if (g < ng) acc[q] = body(g);
+        if constexpr (kMode == kCgPairs) {
+            acc = CgDig{make_int4(0, 0, 0, 0), -1};
+#pragma unroll 1
+            for (int g = tid; g < ng; g += kCgcBlock) cgd_add(acc, body(g));
+        } else {
+            acc[0] = acc[kTerms - 1] = ff_zero();
+            if constexpr (kTerms == 1) {
+                if (tid < ng) acc[0] = body(tid);
+            } else {
+#pragma unroll 1
+                for (int g = tid; g < ng; g += kCgcBlock) {   // twice at most; one copy of the body
+                    const FF t = body(g);
+                    if (g == tid) acc[0] = t;
+                    else acc[kTerms - 1] = t;
+                }
+            }
         }
     };
-    // The sums of term(element) over the groups.  Where a row has a thread of its own, the terms of a
+    // The sums of term(sibling, group) over the groups.  Where a row has a thread of its own, the terms of a
     // group meet in shared memory and one thread adds them.
     auto sum_rows = [&](auto term) {
-        if (kMode == kCgRows) {
-            sterm[tid] = row_on ? term(rs * GP + rg) : ff_zero();
+        if constexpr (kMode == kCgRows) {
+            sterm[tid] = row_on ? term(rs, rg) : ff_zero();
             __syncthreads();
             acc[0] = ff_zero();
             if (tid < kCgRowGroups) acc[0] = cg_group_sum([&](int s) { return sterm[s * kCgRowGroups + tid]; });
         } else {
-            for_groups([&](int g) { return cg_group_sum([&](int s) { return term(s * GP + g); }); });
+            for_groups([&](int g) { return cg_group_sum([&](int s) { return term(s, g); }); });
         }
     };
     // r0 = b, p_{-1} = 0, x0 = 0 (rows in order: coalesced)
     const int mlo = 1 + 8 * gbase;
     for (int l = tid; l < 8 * ng; l += kCgcBlock) {
-        const int e = (l & 7) * GP + (l >> 3);
-        rp[e] = make_float2(v.b[mlo + l], 0.0f);
-        sx[e] = 0.0f;
+        rp[(l & 7) * GP + (l >> 3)] = make_float2(v.b[mlo + l], 0.0f);
+        if (kMode != kCgPairs) sx[(l & 7) * GP + (l >> 3)] = 0.0f;
     }
     __syncthreads();
-    sum_rows([&](int e) { return ff_prod(rp[e].x, rp[e].x); });
+    sum_rows([&](int s, int g) {
+        if (kMode == kCgPairs) x_at(s, g) = 0.0f;
+        const float r = rp[s * GP + g].x;
+        return ff_prod(r, r);
+    });
     unsigned nred = 0;
     cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_start(sh, a, t); });
     bool ran = false;
@@ -729,15 +767,15 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
         const float beta = sh.beta;
         // (A) A p_k from the neighbours' (r_k, p_{k-1}), p.Ap
         if (kMode == kCgRows) {
-            sum_rows([&](int e) {
+            sum_rows([&](int s, int g) {
                 float y = 0.0f;
 #pragma unroll
                 for (int k = 0; k < 27; ++k) {
                     const float2 q = cg_ld2(adr[kMode == kCgRows ? k : 0]);
                     y = fmaf(w[cg_class(k)], fmaf(beta, q.y, q.x), y);
                 }
-                const float2 own = rp[e];
-                sap[e] = y;
+                const float2 own = rp[s * GP + g];
+                sap[s * GP + g] = y;
                 return ff_prod(fmaf(beta, own.y, own.x), y);
             });
         } else {
@@ -753,7 +791,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
                     [&](int s, int c, float p) { y[s] = fmaf(w[c], p, y[s]); });
                 return cg_group_sum([&](int s) {
                     const float2 own = rp[s * GP + g];
-                    sap[s * GP + g] = y[s];
+                    ap_at(s, g) = y[s];
                     return ff_prod(fmaf(beta, own.y, own.x), y[s]);
                 });
             });
@@ -761,14 +799,27 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
         cgc_allreduce<false>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_alpha(sh, t); });
         const float alpha = sh.alpha;
         // (B) x and r, r.r; every CTA has read the pairs (the barrier of the last reduction)
-        sum_rows([&](int e) {
-            const float2 own = rp[e];
+        auto update = [&](int s, int g, float xo, float y) -> FF {
+            const float2 own = rp[s * GP + g];
             const float pi = fmaf(beta, own.y, own.x);
-            sx[e] = fmaf(alpha, pi, sx[e]);
-            const float ri = fmaf(-alpha, sap[e], own.x);
-            rp[e] = make_float2(ri, pi);
+            x_at(s, g) = fmaf(alpha, pi, xo);
+            const float ri = fmaf(-alpha, y, own.x);
+            rp[s * GP + g] = make_float2(ri, pi);
             return ff_prod(ri, ri);
-        });
+        };
+        if (kMode == kCgPairs) {
+            for_groups([&](int g) {
+                float xo[8], y[8];   // in flight together
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    xo[s] = x_at(s, g);
+                    y[s] = ap_at(s, g);
+                }
+                return cg_group_sum([&](int s) { return update(s, g, xo[s], y[s]); });
+            });
+        } else {
+            sum_rows([&](int s, int g) { return update(s, g, sx[s * GP + g], sap[s * GP + g]); });
+        }
         cgc_allreduce<true>(nb, me, sh, nred, acc, err, [&](const CgSum& t) { cgc_after_rr(sh, a, t, it); });
         ran = true;
         ++it;
@@ -776,19 +827,25 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
             // (C) true residual b - A x of the current x from the neighbours' x (the barrier
             // of the last reduction published every CTA's x), with exact products and
             // float-pair sums; staged in the A p array, which holds nothing live here
+            if (kMode == kCgPairs && nb > 1) cl.sync();   // x is in global memory
+            auto x_of = [&](unsigned d, int sib) -> float {   // x of sibling sib of a packed group
+                if (kMode != kCgPairs) return cg_ld1(base_of(d, x_sa, 4u) + (unsigned)(sib * GP * 4));
+                const unsigned local = d & 4095u, G = (unsigned)(gbase - g0) + ((d >> 12) - u.rank0) * (unsigned)chunk + local;
+                return __ldcg(v.xs + (unsigned)sib * dpitch + (local == (unsigned)(GP - 1) ? dpitch - 1u : G));
+            };
             // the entry of an offset that moves on `axes` of x and y, and by kz - 1 on z
             auto w_of = [&](int axes, int kz) {
                 return kz == 1 ? (axes == 0 ? w[0] : axes == 1 ? w[1] : w[2]) : (axes == 0 ? w[1] : axes == 1 ? w[2] : w[3]);
             };
             auto residual = [&](int g, int s, FF y) -> FF {
                 const float ri = ff_to_float(ff_add(FF{v.b[mlo + 8 * g + s], 0.0f}, FF{-y.hi, -y.lo}));
-                sap[s * GP + g] = ri;
+                ap_at(s, g) = ri;
                 return ff_prod(ri, ri);
             };
             // rolled over the z-lines of the block: straight-line code that runs twice per solve
             // would come from L2
             if (kMode == kCgRows) {
-                sum_rows([&](int) {
+                sum_rows([&](int, int) {
                     FF y = ff_zero();
 #pragma unroll 1
                     for (int q = 0; q < 9; ++q) {
@@ -797,7 +854,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
                             int n, sib;
                             slot_of(rs, q / 3, q % 3, kz, n, sib);
                             const float wk = w_of((q / 3 != 1) + (q % 3 != 1), kz);
-                            y = ff_add(y, ff_prod(wk, cg_ld1(base_of(desc_of(rg, n), x_sa, 4u) + (unsigned)(sib * GP * 4))));
+                            y = ff_add(y, ff_prod(wk, x_of(desc_of(rg, n), sib)));
                         }
                     }
                     return residual(rg, rs, y);
@@ -814,9 +871,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
                         const int sxy = 4 * ((bx + 1) & 1) + 2 * ((by + 1) & 1);
                         float xv[4];
 #pragma unroll
-                        for (int bz = 0; bz < 4; ++bz)
-                            xv[bz] = cg_ld1(base_of(desc_of(g, nxy + cg_pos_axis(bz)), x_sa, 4u) +
-                                            (unsigned)((sxy + ((bz + 1) & 1)) * GP * 4));
+                        for (int bz = 0; bz < 4; ++bz) xv[bz] = x_of(desc_of(g, nxy + cg_pos_axis(bz)), sxy + ((bz + 1) & 1));
 #pragma unroll
                         for (int sxy2 = 0; sxy2 < 4; ++sxy2) {   // the rows (sx, sy) this line neighbours
                             const int ox = bx - (sxy2 >> 1), oy = by - (sxy2 & 1);
@@ -841,7 +896,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
                 } else {
                     for (int g = tid; g < ng; g += kCgcBlock)
 #pragma unroll
-                        for (int s = 0; s < 8; ++s) rp[s * GP + g].x = sap[s * GP + g];
+                        for (int s = 0; s < 8; ++s) rp[s * GP + g].x = ap_at(s, g);
                 }
                 // before any CTA reads a neighbour's new r
                 if (nb > 1) cl.sync();
@@ -851,8 +906,7 @@ __device__ __forceinline__ void cgc_resident(cg::cluster_group& cl, CgcShared& s
     }
     __syncthreads();
     for (int l = tid; l < 8 * ng; l += kCgcBlock) {
-        const int e = (l & 7) * GP + (l >> 3);
-        v.x[mlo + l] = sx[e];
+        v.x[mlo + l] = x_at(l & 7, l >> 3);
     }
     if (ran && me == 0 && tid == 0) cgc_report(v, u.d, sh, it - 1);
 }
@@ -1003,13 +1057,29 @@ __device__ __forceinline__ void cgc_global(cg::cluster_group& cl, CgcShared& sh,
     if (ran && me == 0 && threadIdx.x == 0) cgc_report(v, u.d, sh, it - 1);
 }
 
+// the CTA's shared state, for the kernel and what it calls out of line
+__device__ __forceinline__ CgcShared& cgc_shared() {
+    __shared__ CgcShared sh;
+    return sh;
+}
+
+// Out of line: in the kernel its registers would cost the other modes 200 bytes of spills (4% of an
+// iteration).
+__device__ __noinline__ void cgc_pairs(const CgcArgs a, const CgUnit u, int chunk) {
+    extern __shared__ float4 cg_dyn[];
+    cg::cluster_group cl = cg::this_cluster();
+    CgcVec v = a.v;
+    v.rebase();
+    cgc_resident<kCgPairs>(cl, cgc_shared(), a, v, u, chunk, cg_dyn);
+}
+
 // One depth per cluster; behind the first a.clusters clusters, one depth per CTA.  Cluster
 // barriers are passed by every CTA the same number of times only where a whole cluster solves.
 __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
     cg::cluster_group cl = cg::this_cluster();
     CgcVec v = a.v;
     v.rebase();
-    __shared__ CgcShared sh;
+    CgcShared& sh = cgc_shared();
     extern __shared__ float4 cg_dyn[];
     const unsigned long long t_start = global_ns();
     const unsigned size = cl.num_blocks(), rank = cl.block_rank();
@@ -1034,7 +1104,8 @@ __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
         if (!fits) cgc_global(cl, sh, a, v, u, cg_dyn);
         else if (chunk <= kCgRowGroups) cgc_resident<kCgRows>(cl, sh, a, v, u, chunk, cg_dyn);
         else if (chunk <= kCgcBlock) cgc_resident<kCgOne>(cl, sh, a, v, u, chunk, cg_dyn);
-        else cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);
+        else if (chunk < kCgGroups) cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);
+        else cgc_pairs(a, u, chunk);
         if (u.me == 0 && threadIdx.x == 0) v.cw->cg_depth_ns[u.d] = global_ns() - t_start;
     }
     cl.sync();   // no CTA exits while others may still read its shared memory
@@ -1833,6 +1904,8 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     a.v.b = ws.divg;
     a.v.x = ws.xsol;
     a.v.rp = ws.cg_p;
+    a.v.xs = ws.cg_q;
+    a.v.aps = (float*)ws.cg_partial;   // free once the divergence is summed
     a.v.ap = ws.cg_ap;
     a.tol2 = cg_tol * cg_tol;
     // a fixed iteration count replaces the reference's max_iter (10000); the tolerance
@@ -1850,9 +1923,9 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
     const int ncl = whole ? 0 : (D < 2 ? D : (D >= 5 ? 3 : 2));
     const int ncta = whole ? kGridDepth : D - ncl + 1;
     // Where the clouds of a launch need more SMs than there are, SM time counts, not the latency of a
-    // solve: half the CTAs, which hold 114,688 and 57,344 rows in shared memory (16 clouds of depth 7:
+    // solve: half the CTAs, which hold 114,624 and 57,312 rows in shared memory (16 clouds of depth 7:
     // 4.55 ms a batch with 16 and 8 CTAs, 4.27 with 16 and 4, 4.39 with 8 and 8, 4.15 with 8 and 4, 4.29
-    // with 8 and 2).
+    // with 8 and 2) and the pairs of twice as many.
     const bool crowded = ws.batch * (g_cg_cluster + 2 * 8 + ncta) > ws.num_sms;
     int cl1 = ws.cg_ctas > 0 ? ws.cg_ctas : (crowded && g_cg_cluster > 8 ? 8 : g_cg_cluster);
     if (cl1 > g_cg_cluster) cl1 = g_cg_cluster;
@@ -1881,7 +1954,10 @@ cudaError_t solve_build(Workspace& ws, int cg_mode, int cg_iters, float cg_tol, 
         // One launch for every depth: clusters of at most 8 CTAs for the two finest, a CTA each for
         // the rest in the clusters behind them.  A chain without forks takes one hardware queue,
         // so that the resident slots of a server run side by side (the driver has 8 by default:
-        // with three branches a graph, eight depth-5 clouds took 245 us each, 158 with 32 queues).
+        // with three branches a graph, eight depth-5 clouds took 245 us each, 158 with 32 queues).  The
+        // one CTA of depth 5 holds the pairs of 28,656 rows; samples throughout the box, which is enlarged 1.25
+        // times, make 21,952 (16 served clouds of 200,000 samples, 2% of them scattered in the box: 24.1 ms
+        // with all of depth 5 in global memory, 9.4 now).
         const int cs = ws.cg_ctas > 0 ? cl1 : (g_cg_cluster < 8 ? g_cg_cluster : 8);
         CgcArgs b = a;
         b.first = D;

@@ -85,3 +85,32 @@ def test_solution_does_not_depend_on_the_cluster_size(name, cloud, n, depth):
             assert status == psr.PSR_OK
             assert want[1:] == (st.iso_value, list(st.cg_iterations), list(st.cg_residual), list(st.cg_true_residual),
                                 list(st.cg_restarts))
+
+
+def test_systems_that_fill_their_box_against_oracle(oracle_mod):
+    """Samples throughout a box: depths 5 to 7 hold 20,000 to several 100,000 rows, which leave the pairs
+    alone in shared memory (depth 5 on the one CTA of the chain, 6 on small clusters) or nothing (7)."""
+    import psr
+    rng = np.random.default_rng(7)
+    p = rng.uniform(-1, 1, (120000, 3)).astype(np.float32)
+    nr = (p / np.linalg.norm(p, axis=1, keepdims=True)).astype(np.float32)
+    o = oracle_mod.Oracle()
+    assert o.run(p, nr, None, depth=7, stop_after=3) == 0
+    ref, base = o.get("x"), o.get("base")
+    want = None
+    for options in (dict(), dict(concurrent_stages=False), dict(cg_cluster_ctas=8, cg_cluster_ctas_fine=6),
+                    dict(cg_cluster_ctas=16, cg_cluster_ctas_fine=1)):
+        with psr.PoissonReconstruction(max_depth=7, max_points=120000, max_nodes=2000000, **options) as r:
+            try:
+                r.SolvePoissionReconstructionMesh(p, nr, depth=7)
+            except psr.PsrError as e:   # whether the reference's algorithm can mesh it is not the question
+                assert e.status == psr.PSR_INVALID_INPUT
+            got = solution(r)
+            counts = list(r.stats().level_count)
+        assert counts[5] // 8 > 1791 and counts[6] // 8 > 6 * 1791 and counts[7] > 200000
+        if want is None:
+            want = got
+            for d in (5, 6, 7):
+                s = slice(int(base[d]), int(base[d]) + counts[d])
+                assert parity.rel_l2(got[0][s], ref[s]) <= parity.REL_L2
+        equal(want, got)
