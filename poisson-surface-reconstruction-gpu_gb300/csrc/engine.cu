@@ -856,7 +856,7 @@ static const char* status_message(psr_status st) {
 
 static void fill_stats(const psr_handle* h, const Counters& c, int depth, psr_stats& st) {
     memset(&st, 0, sizeof(st));
-    st.points = c.n_points; st.unique_leaves = c.n_unique; st.nodes = c.n_nodes; st.depth = depth;
+    st.points = c.n_input; st.unique_leaves = c.n_unique; st.nodes = c.n_nodes; st.depth = depth;
     for (int d = 0; d <= kMaxDepth; ++d) {
         st.level_count[d] = c.level_count[d];
         st.cg_iterations[d] = c.cg_iters[d];

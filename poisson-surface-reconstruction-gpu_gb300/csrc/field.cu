@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kBlock) k_div_coarse_reduce(DivArgs a) {
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n_nodes; i += nwarps) {
         const int t0 = (int)a.item_start[i];
-        const int t1 = (i + 1 < n_nodes) ? (int)a.item_start[i + 1] : n_items;
+        const int t1 = (i + 1 < n_nodes) ? min((int)a.item_start[i + 1], n_items) : n_items;
         FF s = ff_zero();
         for (int t = t0 + lane; t < t1; t += 32) s = ff_add(s, a.partial[t]);
         s = ff_warp_sum(s);

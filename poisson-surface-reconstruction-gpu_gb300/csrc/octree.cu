@@ -26,7 +26,7 @@ __global__ void k_reset_counters(Counters* c, const InputRef* host_in, InputRef*
         x[-1] = 0.0f;   // the value of absent neighbours
         const InputRef ref = host_in[blockIdx.y];
         *in = ref;
-        c->n_points = ref.n;
+        c->n_points = c->n_input = ref.n;
         for (int a = 0; a < 3; ++a) {
             // The reference seeds its reduction (padding threads, mesh/BuildOctree.cu:66-73)
             // and its host finish (mesh/BuildOctree.cpp:87-88) with -1e6 / 1e6, which gives a
@@ -393,9 +393,15 @@ __device__ __forceinline__ unsigned block_inclusive_scan_1024(unsigned v, unsign
     return r;
 }
 
-// every level is counted: their places in the node arrays
+// Every level is counted: their places in the node arrays.  A tree that outgrew its arrays is left
+// without nodes and points, because its records stop at the capacity and the later stages would follow
+// indices into records that were never written.
 __device__ __forceinline__ void levels_done(Counters* c, int depth) {
     int b = 0;
+    if (atomicOr(&c->error, 0u) & kErrCapacity) {
+        c->n_points = 0;
+        for (int d = 0; d <= depth; ++d) c->level_count[d] = 0;
+    }
     for (int d = 0; d <= depth; ++d) {
         c->level_base[d] = b;
         b += c->level_count[d];

@@ -29,6 +29,7 @@ struct Counters {
     int level_groups[kMaxDepth + 1];    // sibling groups of each level (level_count / 8)
     unsigned long long grid_bar;  // arrivals of the whole-GPU solver's blocks
     unsigned ticket[3];           // blocks done of the bounding box, the encoder, the sample values
+    int n_input;          // points of the call (n_points: of its octree, none when that overflowed)
     int n_nodes;
     int n_vertices, n_edges, n_faces;
     int n_cross, n_tri;

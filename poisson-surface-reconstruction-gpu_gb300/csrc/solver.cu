@@ -148,7 +148,7 @@ struct CgcArgs {
 
 // The resident path holds a depth when the (r, p) pairs of its cluster's chunk of groups fit a CTA's
 // shared memory (the last group is the zero group); the root never does.
-__device__ __forceinline__ int cg_chunk_groups(int m, int nblk) { return ((m >> 3) + nblk - 1) / nblk; }
+__device__ __forceinline__ int cg_chunk_groups(int m, int nblk) { return max(1, ((m >> 3) + nblk - 1) / nblk); }
 __device__ __forceinline__ bool cg_fits_resident(int d, int m, int nblk) {
     return d >= 1 && cg_chunk_groups(m, nblk) < kCgPairGroups;
 }
