@@ -105,6 +105,7 @@ psr_status fail(psr_handle* h, psr_status s, const char* msg) {
 
 psr_status cuda_fail(psr_handle* h, cudaError_t e, const char* where) {
     if (h) h->last_error = std::string(where) + ": " + cudaGetErrorString(e);
+    (void)cudaGetLastError();   // reported by the status: not left for the caller's next CUDA call
     return PSR_CUDA_ERROR;
 }
 
@@ -714,27 +715,41 @@ static bool readable_in_place(const psr_handle* h, const void* p, size_t bytes, 
     return type == CU_MEMORYTYPE_DEVICE && !(managed & 0xffu) && device == h->cfg.device && at <= size && bytes <= size - at;
 }
 
+// An input reference written by the work itself: what a caller captures has to read the arrays of its
+// own call on every replay, whatever the host submitted in between.
+__global__ void k_set_input(InputRef* to, InputRef ref) { *to = ref; }
+
 // Enqueues the input reference of slot k: the caller's device arrays themselves (the sort reads
 // them once and gathers from them once, so a copy would only add traffic and three launches), or
-// copies of host arrays in the slot's staging buffers.
+// copies of other arrays in the slot's staging buffers.
 static cudaError_t stage_inputs(psr_handle* h, const psr_points* pts, int k, cudaStream_t s) {
     Workspace& ws = h->ws;
     const int n = pts->count;
-    InputRef* hp = h->h_params + k;
+    InputRef ref;
     cudaError_t e = cudaSuccess;
     const size_t floats = 3 * sizeof(float) * (size_t)n;
     if (pts->location == PSR_DEVICE && readable_in_place(h, pts->xyz, floats, alignof(float)) &&
         readable_in_place(h, pts->normals, floats, alignof(float)) &&
         readable_in_place(h, pts->rgb, 3 * (size_t)n, 1)) {
-        *hp = InputRef{pts->xyz, pts->normals, pts->rgb, n};
+        ref = InputRef{pts->xyz, pts->normals, pts->rgb, n};
     } else {
         const cudaMemcpyKind kind = (pts->location == PSR_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-        *hp = InputRef{slot_ptr(ws.in_xyz, k), slot_ptr(ws.in_nrm, k), pts->rgb ? slot_ptr(ws.in_rgb, k) : nullptr, n};
-        e = cudaMemcpyAsync((void*)hp->xyz, pts->xyz, floats, kind, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync((void*)hp->nrm, pts->normals, floats, kind, s);
-        if (e == cudaSuccess && pts->rgb) e = cudaMemcpyAsync((void*)hp->rgb, pts->rgb, 3 * (size_t)n, kind, s);
+        ref = InputRef{slot_ptr(ws.in_xyz, k), slot_ptr(ws.in_nrm, k), pts->rgb ? slot_ptr(ws.in_rgb, k) : nullptr, n};
+        e = cudaMemcpyAsync((void*)ref.xyz, pts->xyz, floats, kind, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync((void*)ref.nrm, pts->normals, floats, kind, s);
+        if (e == cudaSuccess && pts->rgb) e = cudaMemcpyAsync((void*)ref.rgb, pts->rgb, 3 * (size_t)n, kind, s);
     }
-    return e;   // the pipeline's first kernel reads *hp
+    if (e != cudaSuccess) return e;
+    // the pipeline's first kernel reads it
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    e = cudaStreamIsCapturing(s, &cap);
+    if (e == cudaSuccess && cap == cudaStreamCaptureStatusActive) {
+        k_set_input<<<1, 1, 0, s>>>(h->h_params + k, ref);
+        e = cudaGetLastError();
+    } else {
+        h->h_params[k] = ref;
+    }
+    return e;
 }
 
 // Device address of a host output buffer the GPU can write (pinned or registered host

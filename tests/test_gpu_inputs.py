@@ -41,3 +41,34 @@ def test_byte_shifted_device_inputs_equal_staged(ox, on):
         np.testing.assert_array_equal(v[:m.vertex_count].cpu().numpy(), a.vertices)
         np.testing.assert_array_equal(t[:m.triangle_count].cpu().numpy(), a.triangles)
 
+
+
+def test_captured_submission_replays_its_own_inputs():
+    """A caller's own capture of psr_submit (kernels issued one by one): a replay reconstructs the cloud
+    that was captured, also after other clouds went through the handle."""
+    import torch
+    import psr
+    clouds = []
+    for n, seed in ((3001, 0), (2500, 1)):
+        p, nr, _, _ = syn.workload("torus_ellipsoid200k", cloud=seed, n=n)
+        clouds.append((torch.from_numpy(p).cuda(), torch.from_numpy(nr).cuda(), n))
+    with psr.PoissonReconstruction(max_depth=6, max_points=4000, disable_graphs=True) as r:
+        want = [r.SolvePoissionReconstructionMesh(x.cpu().numpy(), q.cpu().numpy(), depth=6) for x, q, _ in clouds]
+        x, q, n = clouds[0]
+        v, t, m = outputs()
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            r.submit_device(x.data_ptr(), q.data_ptr(), None, n, m, depth=6, stream=stream.cuda_stream)
+        with pytest.raises(psr.PsrError):   # its completion is the caller's to wait for
+            r.wait()
+        x, q, n = clouds[1]
+        v1, t1, m1 = outputs()
+        r.reconstruct_device(x.data_ptr(), q.data_ptr(), None, n, depth=6, out=m1)
+        np.testing.assert_array_equal(v1[:m1.vertex_count].cpu().numpy(), want[1].vertices)
+        graph.replay()
+        torch.cuda.synchronize()
+    nv, nt = len(want[0].vertices), len(want[0].triangles)
+    np.testing.assert_array_equal(v[:nv].cpu().numpy(), want[0].vertices)
+    np.testing.assert_array_equal(t[:nt].cpu().numpy(), want[0].triangles)
+    assert not v[nv:].any() and not t[nt:].any()
