@@ -423,7 +423,7 @@ def main():
                          "plain": "cg_cluster_ctas 16 (the device's widest cluster), fine 8"}}
     line.update(side_legs(psr, r, caps, d_xyz, d_nrm, d_rgb, n, depth, dev_mesh, stream, torch, st))
     try:
-        line["batch"] = batch_leg(psr, {**caps, **tuned_kw}, dclouds, args.steps, torch, dev, args.batch)
+        line["batch"] = batch_leg(psr, caps, dclouds, args.steps, torch, dev, args.batch)
         line["batch"]["vs_plain"] = line["batch"]["value"] / plain_value
     except Exception as e:   # reported, not fatal: the headline legs are above
         line["batch"] = {"error": str(e)}

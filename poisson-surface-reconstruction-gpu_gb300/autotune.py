@@ -1,18 +1,20 @@
-"""Launch-shape autotuner for the served forms.
+"""Launch-shape autotuner for the served form.
 
 A single call is latency-bound: its depth-D CG runs on the widest thread-block cluster the
-device schedules (16 CTAs) and depths D-1, D-2 on 8-CTA clusters, which leaves most SMs to
-the other stages.  When many reconstructions share the GPU (the resident slots of
-serve.Server, or a multi-cloud pass), the SM time of each one is what bounds throughput,
-and a CG cluster with fewer CTAs (more rows each) spends less SM time for a somewhat
-longer solve.  The tuner measures the served throughput of a workload for each candidate
-pair (psr_config.cg_cluster_ctas, cg_cluster_ctas_fine) and returns the best, with the
-table of measurements.  Candidates whose rows do not fit the CG's shared-memory budget run
-on its global-memory path and lose on their own.
+device schedules (16 CTAs), which leaves most SMs to the other stages.  When many
+reconstructions share the GPU (the resident slots of serve.Server), the SM time of each one
+is what bounds throughput, and a CG cluster with fewer CTAs (more rows each) spends less SM
+time for a somewhat longer solve.  A slot's pipeline is one chain, whose solves are one
+launch: psr_config.cg_cluster_ctas sizes the clusters of depths D and D-1 alike, and the
+coarser depths share one more of that size (cg_cluster_ctas_fine has no effect there).  The
+tuner measures the served throughput of a workload for each candidate (cg_cluster_ctas,
+cg_cluster_ctas_fine = 0) and returns the best, with the table of measurements.
+Candidates whose rows do not fit the CG's shared memory run on its global-memory path and
+lose on their own.
 """
 import time
 
-CANDIDATES = ((16, 8), (16, 4), (12, 8), (12, 4), (10, 4))
+CANDIDATES = ((16, 0), (12, 0), (10, 0), (8, 0), (6, 0), (5, 0), (4, 0))   # 8: the default of a chain
 
 
 def measure_served(server, requests_fn, torch, dev, rounds=3):
