@@ -94,8 +94,8 @@ namespace psr {
 // (r, p) after the first barrier, phase B overwrites the one copy of the pair that phase A
 // read.
 // A chunk of 1792 to 3583 groups keeps the pairs alone in shared memory; x and A p, which an iteration
-// reads once and writes once by the thread that owns them, go through L2 (32 us an iteration for 278,000
-// rows on 16 CTAs, where the path below takes 95).  It is what lets small clusters and single CTAs
+// reads once and writes once by the thread that owns them, go through L2 (28 us an iteration for 389,000
+// rows on 16 CTAs; the path below takes 95 for 278,000).  It is what lets small clusters and single CTAs
 // take systems larger than those they are sized for.  Otherwise (the root, or more rows than fit)
 // the vectors live in global memory and the neighbour table is read row by row.
 constexpr int kCgcBlock = 1024;
@@ -1063,8 +1063,15 @@ __device__ __forceinline__ CgcShared& cgc_shared() {
     return sh;
 }
 
-// Out of line: in the kernel its registers would cost the other modes 200 bytes of spills (4% of an
+// Out of line: in the kernel their registers would cost the other modes 200 bytes of spills (4% of an
 // iteration).
+__device__ __noinline__ void cgc_far(const CgcArgs a, const CgUnit u) {
+    extern __shared__ float4 cg_dyn[];
+    cg::cluster_group cl = cg::this_cluster();
+    CgcVec v = a.v;
+    v.rebase();
+    cgc_global(cl, cgc_shared(), a, v, u, cg_dyn);
+}
 __device__ __noinline__ void cgc_pairs(const CgcArgs a, const CgUnit u, int chunk) {
     extern __shared__ float4 cg_dyn[];
     cg::cluster_group cl = cg::this_cluster();
@@ -1101,7 +1108,7 @@ __global__ void __launch_bounds__(kCgcBlock) k_cg_cluster(CgcArgs a) {
         const int m = u.row1 - u.row0;
         const int chunk = cg_chunk_groups(m, (int)u.nb);
         const bool fits = cg_fits_resident(u.d, m, (int)u.nb);   // the same in all CTAs of the unit
-        if (!fits) cgc_global(cl, sh, a, v, u, cg_dyn);
+        if (!fits) cgc_far(a, u);
         else if (chunk <= kCgRowGroups) cgc_resident<kCgRows>(cl, sh, a, v, u, chunk, cg_dyn);
         else if (chunk <= kCgcBlock) cgc_resident<kCgOne>(cl, sh, a, v, u, chunk, cg_dyn);
         else if (chunk < kCgGroups) cgc_resident<kCgMany>(cl, sh, a, v, u, chunk, cg_dyn);
