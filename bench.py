@@ -392,7 +392,7 @@ def main():
     roofline["sm_ms_per_recon"] = round(sm_ms, 3)
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": tot_sdev / args.steps, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f32 (CG dots and norms in 57-bit fixed point, iso-value sums in f64)", "data": "synthetic",
+            "scaling": "weak", "vs_baseline": None, "dtype": "f32 (CG dots and norms in exact products and integer sums of 57 bits or more, iso-value sums in f64)", "data": "synthetic",
             "impl": "gpu",
             "config": {"workload": f"{args.workload} (N={n}, depth {depth}, colour, normals)",
                        "path": f"served: Server with {K} slots (handle + stream + CUDA graphs each), one host "

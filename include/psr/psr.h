@@ -97,7 +97,9 @@ typedef struct psr_config {
                                   for such batches) */
 } psr_config;
 
-/* Oriented input cloud (the fields of DepthSurfel, base/CommonTypes.h:113-118, as SoA). */
+/* Oriented input cloud (the fields of DepthSurfel, base/CommonTypes.h:113-118, as SoA).  Device
+ * arrays are read where they are when the floats lie on 4-byte boundaries and inside one
+ * allocation of the handle's device; otherwise, and for host arrays, from copies. */
 typedef struct psr_points {
     const float* xyz;      /* 3 * count, x y z interleaved */
     const float* normals;  /* 3 * count */

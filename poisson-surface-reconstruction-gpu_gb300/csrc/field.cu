@@ -282,7 +282,7 @@ __device__ __forceinline__ void div_chunks(const DivArgs& a) {
 
 // The three parts only read the vector field: one launch, blockIdx.z a part (the longest first).
 // Bound by instruction issue (two thirds of the slots) once enough warps hide the table look-ups:
-// five blocks per SM, 48 registers (four: 2% slower at 500,000 samples, depth 9).
+// five blocks per SM, 48 registers with 24 bytes spilled (four: 2% slower at 500,000 samples, depth 9).
 __global__ void __launch_bounds__(kBlock, 5) k_divergence(DivArgs a) {
     __shared__ int s_off[kBlock / 32][33];
     __shared__ int s_base[kBlock / 32][32];

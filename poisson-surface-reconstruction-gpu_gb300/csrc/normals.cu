@@ -8,10 +8,12 @@
 // Here: the points are Morton-sorted on a 128^3 grid of the reference's normalised
 // coordinates (the octree encoder and radix sort), a cell -> first point table is built
 // by a scan, and the exact k nearest of every point are found like the colour search's:
-// an 8-lane near pass over the 3x3x3 cell block (exact when the k-th is within one cell
-// width), then one block per remaining point over coarser levels and shells.  Neighbour
-// distances are compared in normalised coordinates (a uniform scale of the input), ties
-// towards the lower sorted index.  The 3x3 eigenproblem is solved in FP64.
+// an 8-lane near pass over the 3x3x3 cell block, at the grid's level and then at coarser ones
+// (exact when the k-th is within one cell width), then one block per remaining point over
+// coarser levels and shells.  Neighbour distances are compared in normalised coordinates (a
+// uniform scale of the input), ties towards the lower sorted index.  The covariance is summed
+// as float pairs from the neighbours' exact offsets, its smallest eigenvalue found by Newton
+// steps in FP64 from an FP32 start.
 #include "workspace.h"
 
 namespace psr {

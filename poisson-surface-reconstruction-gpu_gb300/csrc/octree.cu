@@ -263,10 +263,6 @@ struct LeafPlaceStore {
     __device__ void rebase() { PSR_CLOUD(ucode, ufirst, c, uslot, T, err); }   // to cloud blockIdx.y
 };
 
-// One level of the build: the sibling groups of level d aggregate into their fathers
-// (mesh/BuildOctree.cu:323-357), a scan over the groups that start a new father group gives the
-// father groups' addresses one level up (:359-375, :796-799), and every father goes to its slot
-// with the empty slots up to the next father's (:377-390).
 // the 8 entries of a group (a group starts on a 32-byte boundary of its array)
 __device__ __forceinline__ void load8(const int* p, int (&v)[8]) {
     const int4 a = *reinterpret_cast<const int4*>(p), b = *reinterpret_cast<const int4*>(p + 4);
@@ -283,6 +279,10 @@ __device__ __forceinline__ int group_father_key(const LevelArrays& T, int base, 
         if (pn[j] != 0) at = j;
     return at < 0 ? 0 : T.key[base + at] & ~(7 << sh);
 }
+// One level of the build: the sibling groups of level d aggregate into their fathers
+// (mesh/BuildOctree.cu:323-357), a scan over the groups that start a new father group gives the
+// father groups' addresses one level up (:359-375, :796-799), and every father goes to its slot
+// with the empty slots up to the next father's (:377-390).
 struct LevelLoad {
     const Counters* c;
     int d, depth;
@@ -361,8 +361,8 @@ struct LevelStore {
 // ---- coarse levels in one CTA --------------------------------------------------------
 // The levels near the root hold few nodes, so their per-level passes (group aggregate,
 // father-group scan, level set-up, father placement) run inside one 1024-thread CTA with
-// block barriers between steps instead of five launches per level.  Same arithmetic as
-// the per-level kernels above.
+// block barriers between steps instead of a scan of their own per level.  Same arithmetic as
+// the per-level scans above.
 constexpr int kLevelBlock = 1024;
 constexpr int kCoarseLevels = 4;   // levels up to this one: at most 4096 nodes, 4 rounds of the CTA
 
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kLevelBlock) k_levels_block(Counters* c, int d
 }
 
 // 27-neighbour tables of levels 1..dmax in one CTA (levels in order: a level reads its
-// parents' table)
+// parents' table).  1024 threads leave 64 registers each: 56 bytes of the row spill.
 __global__ void __launch_bounds__(kLevelBlock) k_neighbours_block(const Counters* c, int dmax, int depth,
                                                                   const int* key, const int* parent,
                                                                   const int* first_child, int* neigh, size_t stride) {

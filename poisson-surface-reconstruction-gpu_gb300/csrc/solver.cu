@@ -1637,14 +1637,6 @@ __device__ __forceinline__ void decode3s(int e, int depth, int& ix, int& iy, int
     iz = e >> (2 * (depth + 1));
 }
 
-// Implicit value at a sample point: the 27 neighbour terms ((x * Fx) * Fy) * Fz of every
-// level of its chain (its depth-D node and that node's ancestors).  The levels up to D-1
-// are summed first, as soon as their systems are solved, beside the depth-D CG: on the cell
-// of a depth-(D-1) node they form one tensor-product quadratic (k_point_poly: its 27
-// Bernstein coefficients, one thread per node), evaluated at each sample of the cell
-// (k_point_values_coarse; the partial sum is kept in `out`).  The depth-D terms are added
-// after the depth-D CG (k_point_values).  The iso-value is the FP64 mean of these float
-// values.
 // The value rows of the nodes above the finest depth (ValueRows), one thread per node; the rows go
 // out through shared memory, eight lanes a line.  Bound by its 54 reads a node.
 constexpr int kRowPitch = 36;   // floats: 16-byte aligned, rows on different banks
@@ -1681,6 +1673,14 @@ __global__ void __launch_bounds__(kBlock) k_value_rows(const Counters* c, int de
     }
 }
 
+// Implicit value at a sample point: the 27 neighbour terms ((x * Fx) * Fy) * Fz of every
+// level of its chain (its depth-D node and that node's ancestors).  The levels up to D-1
+// are summed first, as soon as their systems are solved, beside the depth-D CG: on the cell
+// of a depth-(D-1) node they form one tensor-product quadratic (k_point_poly: its 27
+// Bernstein coefficients, one thread per node), evaluated at each sample of the cell
+// (k_point_values_coarse; the partial sum is kept in `out`).  The depth-D terms are added
+// after the depth-D CG (k_point_values).  The iso-value is the FP64 mean of these float
+// values.
 template <bool kRows>
 __global__ void __launch_bounds__(kBlock) k_point_poly(const Counters* c, int depth, const float* ctr_x,
                                                        const float* ctr_y, const float* ctr_z, ValueRows R,
