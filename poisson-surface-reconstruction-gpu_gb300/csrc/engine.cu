@@ -742,8 +742,8 @@ static cudaError_t stage_inputs(psr_handle* h, const psr_points* pts, int k, cud
     if (e != cudaSuccess) return e;
     // the pipeline's first kernel reads it
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    e = cudaStreamIsCapturing(s, &cap);
-    if (e == cudaSuccess && cap == cudaStreamCaptureStatusActive) {
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) (void)cudaGetLastError();   // then not `s` itself
+    if (cap == cudaStreamCaptureStatusActive) {
         k_set_input<<<1, 1, 0, s>>>(h->h_params + k, ref);
         e = cudaGetLastError();
     } else {

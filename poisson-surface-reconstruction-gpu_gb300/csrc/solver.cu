@@ -153,7 +153,7 @@ __device__ __forceinline__ bool cg_fits_resident(int d, int m, int nblk) {
     return d >= 1 && cg_chunk_groups(m, nblk) < kCgPairGroups;
 }
 
-// A sum in fixed point: m * 2^(e - 183), |m| < 2^62.  The lanes of a warp are added as 57-bit
+// A sum in fixed point: m * 2^(e - 183), |m| < 2^62.  k_cg_grid adds the lanes of a warp as 57-bit
 // integers aligned to the largest of them, in three integer warp reductions (what falls off a
 // smaller term is below 2^-57 of the largest); warps and CTAs the same way.
 struct alignas(16) CgSum {
