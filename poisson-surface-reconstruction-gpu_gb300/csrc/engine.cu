@@ -346,7 +346,7 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     A.add(ws.divg, (size_t)nodes);
     A.add(ws.xsol, (size_t)nodes + 64);   // from entry 64 on: x[-1] = 0 stands for absent neighbours
     const size_t pitch = (size_t)nodes / 8 + 8;   // sibling groups, and a zero group at the end
-    A.add(ws.cg_r, (size_t)nodes); A.add(ws.cg_p, (size_t)nodes); A.add(ws.cg_q, 8 * pitch);
+    A.add(ws.cg_p, (size_t)nodes); A.add(ws.cg_q, 8 * pitch);
     A.add(ws.cg_ap, 8 * pitch);
     if (cfg.max_depth >= 8) {   // the whole-GPU CG
         A.add(ws.cg_nbg, 27 * pitch);
@@ -437,9 +437,9 @@ psr_status psr_create(const psr_config* cfg_in, psr_handle** out) {
     }
     h->arena_bytes = A.bytes;
     A.assign((char*)h->arena);
-    if (cfg.max_depth >= 8) {   // from cg_r to cg_rp: free once the CG is done
-        ws.value_rows = (float4*)ws.cg_r;
-        ws.cap_rows = (int)(((char*)ws.cg_part - (char*)ws.cg_r) / (8 * sizeof(float4)));
+    if (cfg.max_depth >= 8) {   // from cg_p to cg_rp: free once the CG is done
+        ws.value_rows = (float4*)ws.cg_p;
+        ws.cap_rows = (int)(((char*)ws.cg_part - (char*)ws.cg_p) / (8 * sizeof(float4)));
     }
     ws.xsol += 64;
     set_batch(ws, 1);

@@ -325,7 +325,7 @@ cudaError_t field_build(Workspace& ws) {
     // numbered beside the mesh records
     const int dsplit = div_split(D);
     const DivArgs a{c, D, dsplit, ws.res, ws.enc, ws.didx, ws.dnum, ws.neigh, stride, ws.leaf, ws.dff,
-                    (const unsigned*)ws.cg_r, reinterpret_cast<FF*>(ws.cg_partial), ws.divg};
+                    (const unsigned*)ws.cg_p, reinterpret_cast<FF*>(ws.cg_partial), ws.divg};
     if (!ws.chain) {
         const cudaError_t e = cudaStreamWaitEvent(s, ws.ev_geo, 0);
         if (e != cudaSuccess) return e;

@@ -1776,7 +1776,7 @@ cudaError_t mesh_geometry_impl(Workspace& ws, const MeshBufs& mb, unsigned* tota
     cudaError_t e;
     if (dsplit > 0)
         e = launch_scans(scan_job<1>(DivChunkLoad{ws.neigh, stride, ws.dnum},
-                                     DivChunkStore{(unsigned*)ws.cg_r, c, ws.cap.nodes},   // as many float pairs
+                                     DivChunkStore{(unsigned*)ws.cg_p, c, ws.cap.nodes},   // as many float pairs
                                      &c->level_base[dsplit], ws.scan_side[2], side + 2),
                          vertices, faces, edges, err, s);
     else

@@ -104,8 +104,8 @@ struct Workspace {
     float* xsol;            // M, with xsol[-1] = 0
     cudaEvent_t ev_cg = nullptr;   // recorded right after the CG kernel (stage timing)
     unsigned ev_flags = 0;         // flags of the stage-timing event records (external in a capture)
-    float* cg_r;            // M: where the coarse divergence's chunks start
-    float2* cg_p;           // M: (r, p) of the cluster CG's global-memory path
+    float2* cg_p;           // M: (r, p) of the cluster CG's global-memory path; before the solve, where the
+                            //   coarse divergence's chunks start
     float *cg_q, *cg_ap;    // x (sibling-major) and A p of the whole-GPU CG; A p of the global-memory path
     int* cg_nbg;            // [27][cap.nodes / 8 + 8]: neighbour groups of every sibling group (whole-GPU CG)
     float2* cg_rp;          // [8][cap.nodes / 8 + 8]: (r, p), sibling-major
